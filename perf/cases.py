@@ -20,8 +20,7 @@ import torch
 import matfree_gb300 as mf
 from matfree_gb300.autodiff import rbf_logdet
 
-S2, ELL, TAU = 1.0, 0.2, 1e-2  # the repository's kernel: variance, length scale, nugget
-WELL = 0.5  # the nugget of its solves
+S2, ELL, TAU = 1.0, 0.2, 2.0  # the kernel: variance, length scale, nugget (noisy observations)
 HEAT = -0.1  # exp(HEAT x), the serving stream's other function
 SHIFT = 0.1  # of the Laplacian
 
@@ -53,8 +52,8 @@ def listed():
         {"name": "laplace 1m", "kind": "sparse", "m": 1024, "k": 100, "p": 64},
         # the plain float64 log-determinant of a dense matrix
         {"name": "dense f64", "kind": "dense64", "n": 1000, "k": 30, "p": 100},
-        # a function of a kernel matrix times vectors (its square root: samples of a process)
-        {"name": "sqrt samples", "kind": "funm", "n": 5000, "k": 40, "p": 48},
+        # a function of a kernel matrix times vectors, here its heat kernel
+        {"name": "heat vectors", "kind": "funm", "n": 5000, "k": 40, "p": 48},
         # a linear solve with a kernel matrix by conjugate gradients
         {"name": "solve", "kind": "solve", "n": 8192, "p": 1},
     ]
@@ -123,7 +122,6 @@ def _inputs(case, seed):
     n, p = case.get("n"), case["p"]
     if kind == "product":
         A = torch.randn((n, n), generator=g, device="cuda") * (0.5 / math.sqrt(n))
-        A.diagonal().add_(2.0)
         return {"A": A, "probes": _signs(g, p, n, torch.float32)}
     if kind == "sparse":
         weight = float(torch.rand(1, generator=g, device="cuda") * 0.2 + 0.9)
@@ -135,7 +133,7 @@ def _inputs(case, seed):
         return {"A": A, "probes": _signs(g, p, n, torch.float64)}
     s = {"x": torch.rand((n, 3), generator=g, device="cuda")}
     if kind == "train":
-        start = torch.tensor([0.0, math.log(ELL), math.log(10 * TAU)])
+        start = torch.tensor([0.0, math.log(ELL), math.log(TAU)])
         s["theta"] = start + 0.1 * torch.rand(3, generator=g, device="cuda").cpu()
         s["probes"] = _signs(g, p, n, torch.float32)
     elif kind in ("funm", "solve"):
@@ -154,16 +152,16 @@ def prepare(case, seed):
         if kind == "sparse":
             s["op"] = mf.CSROperator(*_grid_csr(case["m"], s["weight"]), n, shift=SHIFT)
     elif kind == "product":
-        s["op"] = mf.DenseOperator(s.pop("A"), precision="bf16x3")
+        s["op"] = mf.DenseOperator(s.pop("A"), precision="bf16x3", shift=2.0)
         s["op"].transpose()  # kept by the operator
         s["integrand"] = mf.funm.monte_carlo_funm_product_logdet(mf.decomp.bidiag(case["k"]))
     elif kind == "dense64":
         s["op"] = mf.DenseOperator(s.pop("A"), precision="fp64")
         s["integrand"] = mf.funm.monte_carlo_funm_sym_logdet(mf.decomp.tridiag_sym(case["k"]))
     elif kind in ("funm", "solve"):
-        s["op"] = mf.RBFKernelOperator(s["x"], s2=S2, ell=ELL, tau=WELL)
+        s["op"] = mf.RBFKernelOperator(s["x"], s2=S2, ell=ELL, tau=TAU)
         if kind == "funm":
-            s["apply"] = mf.funm.funm_lanczos_sym(mf.funm.funm_pow(0.5), mf.decomp.tridiag_sym(case["k"]))
+            s["apply"] = mf.funm.funm_lanczos_sym(mf.funm.funm_exp(HEAT), mf.decomp.tridiag_sym(case["k"]))
     return s
 
 
@@ -213,7 +211,7 @@ def work(case):
     if kind == "funm":
         return {"bytes": 4.0 * n * n + 8.0 * n * p, "flops": 2.0 * n * n * p * k + basis + 2.0 * n * p * k}
     # the number of iterations is the problem's: about sqrt(condition) of them
-    its = 0.5 * math.sqrt(0.02 * n / WELL) * math.log(2e5)
+    its = 0.5 * math.sqrt(0.02 * n / TAU) * math.log(2e5)
     return {"bytes": 4.0 * n * n + 8.0 * n * p, "flops": 2.0 * n * n * p * its}
 
 
@@ -380,12 +378,13 @@ def exact(case, seed):
     if kind == "product":
         # Lanczos on A^T A gives the bidiagonalisation's B^T B
         A = s["A"].double()
+        A.diagonal().add_(2.0)
         return _quadrature64(lambda q: (q @ A.T) @ A, s["probes"], k, torch.log)
-    K, _ = _kernel64(s["x"], S2, ELL, WELL)
+    K, _ = _kernel64(s["x"], S2, ELL, TAU)
     V = s["rhs"].double()
     if kind == "solve":
         return torch.linalg.solve(K, V.T).T
     Q, d, e, length = _lanczos64(lambda q: q @ K, V, k)
     w, S = _eigh64(d, e)
-    coef = length[:, None] * torch.einsum("pij,pj->pi", S, w.sqrt() * S[:, 0])
+    coef = length[:, None] * torch.einsum("pij,pj->pi", S, torch.exp(HEAT * w) * S[:, 0])
     return torch.einsum("pk,pkn->pn", coef, Q)
