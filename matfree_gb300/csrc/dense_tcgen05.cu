@@ -6,21 +6,22 @@
 // (p rows of bf16, hi and optionally lo) are both K-major, so one tile of the
 // product is the UMMA D[M = 128 rows of A][N = probes] += A_tile[M][K] B[N][K]^T.
 //
-// CTA organisation (192 threads, one output tile of 128 rows x BN probes):
-//   warp 0      TMA producer: one elected lane streams 32-wide K slices of A
+// CTA organisation (192 threads; the split-K form's numbers, the CTA-pair forms
+// differ as their comments say):
+//   warp 0      TMA producer: one elected lane streams 64-wide K slices of A
 //               (and A_lo) and of the panel (and its lo part) into a ring of
-//               shared-memory stages (64-byte swizzled rows, 1024-byte aligned
-//               tiles; 4 stages in split mode, 8 in plain bf16) and arms the
-//               stage's "full" mbarrier with the transaction bytes.
-//   warp 1      allocates the TMEM accumulator (BN fp32 columns x 128 lanes);
-//               one lane issues tcgen05.mma (kind::f16, bf16 inputs, fp32
-//               accumulate), 2 per K slice (K = 16 each), 6 for the split
-//               product hi*hi + hi*lo + lo*hi, then tcgen05.commit to the
-//               stage's "empty" mbarrier; a final commit signals the epilogue.
+//               shared-memory stages (128-byte swizzled rows, 1024-byte aligned
+//               tiles) and arms the stage's "full" mbarrier with the
+//               transaction bytes.  Rows of 64 bytes (32-wide slices) bound an
+//               SM's intake at 58 GB/s; 128-byte rows take 79 (n = 8192, 32
+//               probes, 64 CTAs: 90 -> 73 us).
+//   warp 1      allocates the TMEM accumulators (fp32, 128 lanes); one lane
+//               issues tcgen05.mma (kind::f16, bf16 inputs, fp32 accumulate),
+//               three per 16-wide step of the split product hi*hi + hi*lo +
+//               lo*hi, then tcgen05.commit to the stage's "empty" mbarrier; a
+//               final commit signals the epilogue.
 //   warps 2-5   epilogue: tcgen05.ld 32 lanes x 16 columns at a time (each
-//               warp owns the TMEM lane quarter its warp index allows), add
-//               shift * Vf and store; 32 lanes write 32 consecutive rows of
-//               one probe (128-byte coalesced stores).
+//               warp owns the TMEM lane quarter its warp index allows).
 //
 // Every mbarrier wait is bounded.  A role that gives up records
 // MFG_ERR_TIMEOUT in *status and raises a shared abort flag; the others leave
@@ -44,9 +45,11 @@ constexpr int kUmmaK = 16;          // K per tcgen05.mma of kind::f16
 constexpr int kGemmThreads = 192;
 constexpr int64_t kPairMinRows = 1024;  // CTA pairs from this operator size on
 
+constexpr int kGemmMaxStages = 12;
+
 struct GemmShared {
-  uint64_t full[8];
-  uint64_t empty[8];
+  uint64_t full[kGemmMaxStages];
+  uint64_t empty[kGemmMaxStages];
   uint64_t tmem_full;
   uint64_t drain;
   uint32_t tmem_base;
@@ -99,13 +102,14 @@ __device__ __forceinline__ void tc_fence_after() {
 // 8 * kRowBytes, descriptor version 1, layout type 4 (SWIZZLE_64B) or 2
 // (SWIZZLE_128B).  The leading-byte offset is not used by swizzled K-major
 // layouts and is set to 1.
+template <int kRow = kRowBytes>
 __device__ __forceinline__ uint64_t sw_desc(uint32_t saddr) {
   uint64_t d = 0;
   d |= (uint64_t)((saddr >> 4) & 0x3FFFu);
   d |= (uint64_t)1u << 16;
-  d |= (uint64_t)((8u * kRowBytes) >> 4) << 32;
+  d |= (uint64_t)((8u * kRow) >> 4) << 32;
   d |= (uint64_t)1u << 46;
-  d |= (uint64_t)(kRowBytes == 128 ? 2u : 4u) << 61;
+  d |= (uint64_t)(kRow == 128 ? 2u : 4u) << 61;
   return d;
 }
 
@@ -142,156 +146,6 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
   for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
-}
-
-template <bool kSplit>
-__global__ void __launch_bounds__(kGemmThreads, 1)
-dense_tcgen05_kernel(const __grid_constant__ CUtensorMap map_ahi,
-                     const __grid_constant__ CUtensorMap map_alo,
-                     const __grid_constant__ CUtensorMap map_bhi,
-                     const __grid_constant__ CUtensorMap map_blo, const float *__restrict__ Vf,
-                     int64_t ldvf, float *__restrict__ W, int64_t ldw, int n, int p, int BN,
-                     int stages, uint32_t tmem_cols, float shift, int *status) {
-  extern __shared__ __align__(1024) uint8_t smem_raw[];
-  // 1024-byte aligned stage ring, then the barrier block
-  uint8_t *tiles = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  const uint32_t a_bytes = kBM * kBK * 2;
-  const uint32_t b_bytes = (uint32_t)BN * kBK * 2;
-  const uint32_t stage_bytes = (kSplit ? 2u : 1u) * (a_bytes + b_bytes);
-  GemmShared *sh = reinterpret_cast<GemmShared *>(tiles + (size_t)stages * stage_bytes);
-
-  const int warp = threadIdx.x >> 5;
-  const int lane = threadIdx.x & 31;
-  const int m0 = blockIdx.x * kBM;
-  const int b0 = blockIdx.y * BN;
-  const int num_k = (n + kBK - 1) / kBK;
-  volatile int *abort_flag = &sh->abort;
-
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < stages; ++s) {
-      mbar_init(&sh->full[s], 1);
-      mbar_init(&sh->empty[s], 1);
-    }
-    mbar_init(&sh->tmem_full, 1);
-    mbar_init(&sh->drain, 1);
-    sh->abort = 0;
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                     smem_u32(&sh->tmem_base)),
-                 "r"(tmem_cols)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = sh->tmem_base;
-
-  if (warp == 0) {
-    if (lane == 0) {
-      int issued = 0;
-      for (int kt = 0; kt < num_k; ++kt) {
-        const int s = kt % stages;
-        const uint32_t ph = (uint32_t)(kt / stages) & 1u;
-        if (!mbar_wait(&sh->empty[s], ph ^ 1u, abort_flag, status)) break;
-        uint8_t *st = tiles + (size_t)s * stage_bytes;
-        mbar_arrive_expect_tx(&sh->full[s], stage_bytes);
-        const int kx = kt * kBK;
-        tma_load_2d(st, &map_ahi, &sh->full[s], kx, m0);
-        tma_load_2d(st + a_bytes, &map_bhi, &sh->full[s], kx, b0);
-        if (kSplit) {
-          tma_load_2d(st + a_bytes + b_bytes, &map_alo, &sh->full[s], kx, m0);
-          tma_load_2d(st + 2 * a_bytes + b_bytes, &map_blo, &sh->full[s], kx, b0);
-        }
-        ++issued;
-      }
-      // drain: copies still in flight complete their stage's "full" phase
-      if (*abort_flag) {
-        for (int kt = (issued > stages ? issued - stages : 0); kt < issued; ++kt) {
-          const int s = kt % stages;
-          const uint32_t ph = (uint32_t)(kt / stages) & 1u;
-          mbar_wait_bounded(smem_u32(&sh->full[s]), ph, nullptr, kMbarWaitNs / 8);
-        }
-      }
-    }
-  } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc = instr_desc_bf16(kBM, BN);
-      int done = 0;
-      for (int kt = 0; kt < num_k; ++kt) {
-        const int s = kt % stages;
-        const uint32_t ph = (uint32_t)(kt / stages) & 1u;
-        if (!mbar_wait(&sh->full[s], ph, abort_flag, status)) break;
-        tc_fence_after();
-        const uint32_t st = smem_u32(tiles + (size_t)s * stage_bytes);
-        const uint32_t ahi = st, bhi = st + a_bytes;
-        const uint32_t alo = st + a_bytes + b_bytes, blo = st + 2 * a_bytes + b_bytes;
-#pragma unroll
-        for (int kk = 0; kk < kBK / kUmmaK; ++kk) {
-          const uint32_t off = (uint32_t)kk * kUmmaK * 2;  // 32 bytes along K inside the atom
-          const uint32_t acc = (kt > 0 || kk > 0) ? 1u : 0u;
-          umma_bf16(tmem, sw_desc(ahi + off), sw_desc(bhi + off), idesc, acc);
-          if (kSplit) {
-            umma_bf16(tmem, sw_desc(ahi + off), sw_desc(blo + off), idesc, 1u);
-            umma_bf16(tmem, sw_desc(alo + off), sw_desc(bhi + off), idesc, 1u);
-          }
-        }
-        umma_commit(&sh->empty[s]);
-        ++done;
-      }
-      // every MMA issued so far completes before this arrives
-      umma_commit(done == num_k ? &sh->tmem_full : &sh->drain);
-      if (done != num_k) {
-        mbar_wait_bounded(smem_u32(&sh->drain), 0, nullptr, kMbarWaitNs / 8);
-      }
-    }
-  } else {
-    // epilogue: warps 2..5 -> TMEM lane quarters 2, 3, 0, 1
-    const int quarter = warp & 3;
-    const int row = quarter * 32 + lane;
-    const int m = m0 + row;
-    // The shift term's probe values (shift * V[b][m]) are loaded one group of
-    // 16 probes ahead of the accumulator reads, the first group while the
-    // main loop runs, so their latency stays off the epilogue's path.
-    float sv[16], svn[16];
-    auto load_shift = [&](int c, float(&dst)[16]) {
-#pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        const int b = b0 + c + j;
-        dst[j] = (shift != 0.f && m < n && b < p) ? __ldg(Vf + (int64_t)b * ldvf + m) : 0.f;
-      }
-    };
-    load_shift(0, sv);
-    // warp-uniform decision: tcgen05.ld is executed by all 32 lanes or none
-    // the epilogue sleeps through the main loop
-    const bool ok = __all_sync(0xffffffffu, mbar_wait<true>(&sh->tmem_full, 0, abort_flag, status));
-    tc_fence_after();
-    if (ok) {
-      for (int c = 0; c < BN; c += 16) {
-        if (c + 16 < BN) load_shift(c + 16, svn);
-        float v[16];
-        tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)c, v);
-        if (m < n) {
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            const int b = b0 + c + j;
-            if (b < p) W[(int64_t)b * ldw + m] = fmaf(shift, sv[j], v[j]);
-          }
-        }
-#pragma unroll
-        for (int j = 0; j < 16; ++j) sv[j] = svn[j];
-      }
-    }
-  }
-  tc_fence_before();
-  __syncthreads();
-  if (warp == 1) {
-    tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tmem_cols)
-                 : "memory");
-  }
 }
 
 // ---------------------------------------------------------------------------
@@ -531,6 +385,214 @@ dense_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_ahi,
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tmem_cols)
                  : "memory");
   }
+}
+
+// ---------------------------------------------------------------------------
+// Split-K cluster form: a cluster of S CTAs computes one tile of 128 operator
+// rows x BN <= 128 probes, CTA r the r-th of S equal ranges of K.  Each
+// accumulates its partial product in its own TMEM, writes it to its own
+// shared memory (the ring, free by then), and after a cluster barrier CTA r
+// adds the S partial tiles of its share of the probe columns over distributed
+// shared memory, in rank order, adds the shift term and stores.  No zeroed
+// W, no atomics, one launch, and every output row has the same S accumulation
+// chains of n / S terms (the tensor pipe's fp32 accumulation truncates, so
+// shorter chains are also closer to the exact product).
+//
+// What bounds it: the operator stream (4 n^2 bytes in split mode).  The ring
+// takes under half of an SM's shared memory, so two CTAs share an SM and one
+// streams while the other fills its pipeline or reduces.
+// ---------------------------------------------------------------------------
+
+__device__ __forceinline__ float4 ld_dsmem_f4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "r"(addr)
+               : "memory");
+  return v;
+}
+
+constexpr int kSplitKBK = 64;  // K per stage: 128-byte rows
+constexpr int kSplitKMaxBN = 128;
+constexpr int kSplitKMaxS = 8;  // portable cluster size
+constexpr size_t kSplitKRing = 220 * 1024;
+
+template <bool kSplit, int MT>
+__global__ void __launch_bounds__(kGemmThreads, 1)
+dense_tcgen05_splitk_kernel(const __grid_constant__ CUtensorMap map_ahi,
+                            const __grid_constant__ CUtensorMap map_alo,
+                            const __grid_constant__ CUtensorMap map_bhi,
+                            const __grid_constant__ CUtensorMap map_blo,
+                            const float *__restrict__ Vf, int64_t ldvf, float *__restrict__ W,
+                            int64_t ldw, int n, int p, int BN, int stages, uint32_t tmem_cols,
+                            float shift, int vec_ok, int *status) {
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t *tiles = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  const uint32_t a_bytes = MT * kBM * kSplitKBK * 2;
+  const uint32_t b_bytes = (uint32_t)BN * kSplitKBK * 2;
+  const uint32_t stage_bytes = (kSplit ? 2u : 1u) * (a_bytes + b_bytes);
+  const uint32_t part_bytes = (uint32_t)BN * (MT * kBM) * 4u;  // the partial tile [BN][rows] in the ring
+  const uint32_t ring_bytes = (uint32_t)stages * stage_bytes;
+  GemmShared *sh = reinterpret_cast<GemmShared *>(tiles + (ring_bytes > part_bytes ? ring_bytes : part_bytes));
+
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  const int S = (int)gridDim.x, part = (int)blockIdx.x;  // the cluster spans grid.x
+  const int m0 = blockIdx.y * (MT * kBM);
+  const int b0 = blockIdx.z * BN;
+  const int num_k_all = (n + kSplitKBK - 1) / kSplitKBK;
+  const int kb0 = (int)((int64_t)num_k_all * part / S);
+  const int num_k = (int)((int64_t)num_k_all * (part + 1) / S) - kb0;  // >= 1: S <= num_k_all
+  volatile int *abort_flag = &sh->abort;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < stages; ++s) {
+      mbar_init(&sh->full[s], 1);
+      mbar_init(&sh->empty[s], 1);
+    }
+    mbar_init(&sh->tmem_full, 1);
+    mbar_init(&sh->drain, 1);
+    sh->abort = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     smem_u32(&sh->tmem_base)),
+                 "r"(tmem_cols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = sh->tmem_base;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      int issued = 0, s = 0;
+      uint32_t ph = 0;
+      for (int kt = 0; kt < num_k; ++kt) {
+        if (!mbar_wait(&sh->empty[s], ph ^ 1u, abort_flag, status)) break;
+        uint8_t *st = tiles + (size_t)s * stage_bytes;
+        mbar_arrive_expect_tx(&sh->full[s], stage_bytes);
+        const int kx = (kb0 + kt) * kSplitKBK;
+        tma_load_2d(st, &map_ahi, &sh->full[s], kx, m0);
+        if (kSplit) tma_load_2d(st + a_bytes + b_bytes, &map_alo, &sh->full[s], kx, m0);
+        tma_load_2d(st + a_bytes, &map_bhi, &sh->full[s], kx, b0);
+        if (kSplit) tma_load_2d(st + 2 * a_bytes + b_bytes, &map_blo, &sh->full[s], kx, b0);
+        ++issued;
+        if (++s == stages) {
+          s = 0;
+          ph ^= 1u;
+        }
+      }
+      if (*abort_flag) {
+        for (int kt = (issued > stages ? issued - stages : 0); kt < issued; ++kt)
+          mbar_wait_bounded(smem_u32(&sh->full[kt % stages]), (uint32_t)(kt / stages) & 1u, nullptr,
+                            kMbarWaitNs / 8);
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      const uint32_t idesc = instr_desc_bf16(kBM, BN);
+      int done = 0, s = 0;
+      uint32_t ph = 0;
+      for (int kt = 0; kt < num_k; ++kt) {
+        if (!mbar_wait(&sh->full[s], ph, abort_flag, status)) break;
+        tc_fence_after();
+        const uint32_t st = smem_u32(tiles + (size_t)s * stage_bytes);
+        const uint32_t ahi = st, bhi = st + a_bytes;
+        const uint32_t alo = st + a_bytes + b_bytes, blo = st + 2 * a_bytes + b_bytes;
+#pragma unroll
+        for (int kk = 0; kk < kSplitKBK / kUmmaK; ++kk) {
+          const uint32_t off = (uint32_t)kk * kUmmaK * 2;
+#pragma unroll
+          for (int t = 0; t < MT; ++t) {  // row tiles share the panel slice
+            const uint32_t acc = tmem + (uint32_t)(t * BN), ta = off + (uint32_t)t * (kBM * kSplitKBK * 2);
+            umma_bf16(acc, sw_desc<2 * kSplitKBK>(ahi + ta), sw_desc<2 * kSplitKBK>(bhi + off), idesc, (kt > 0 || kk > 0) ? 1u : 0u);
+            if (kSplit) {
+              umma_bf16(acc, sw_desc<2 * kSplitKBK>(ahi + ta), sw_desc<2 * kSplitKBK>(blo + off), idesc, 1u);
+              umma_bf16(acc, sw_desc<2 * kSplitKBK>(alo + ta), sw_desc<2 * kSplitKBK>(bhi + off), idesc, 1u);
+            }
+          }
+        }
+        umma_commit(&sh->empty[s]);
+        ++done;
+        if (++s == stages) {
+          s = 0;
+          ph ^= 1u;
+        }
+      }
+      umma_commit(done == num_k ? &sh->tmem_full : &sh->drain);
+      if (done != num_k) mbar_wait_bounded(smem_u32(&sh->drain), 0, nullptr, kMbarWaitNs / 8);
+    }
+  } else {
+    // warps 2..5 -> TMEM lane quarters 2, 3, 0, 1: the partial tile into this
+    // CTA's shared memory, probe-major (32 lanes write 32 consecutive rows).
+    // Every copy has landed and every MMA has read its stage once tmem_full
+    // completes, so the ring may be overwritten.
+    const int quarter = warp & 3;
+    float *dst = reinterpret_cast<float *>(tiles) + quarter * 32 + lane;
+    const bool ok = __all_sync(0xffffffffu, mbar_wait<true>(&sh->tmem_full, 0, abort_flag, status));
+    tc_fence_after();
+    if (ok) {
+#pragma unroll
+      for (int t = 0; t < MT; ++t)
+        for (int c = 0; c < BN; c += 16) {
+          float v[16];
+          tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(t * BN + c), v);
+#pragma unroll
+          for (int j = 0; j < 16; ++j) dst[(c + j) * (MT * kBM) + t * kBM] = v[j];
+        }
+    }
+  }
+  __syncwarp();
+  tc_fence_before();
+  cluster_sync_all();  // the S partial tiles are complete
+  if (warp == 1) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tmem_cols)
+                 : "memory");
+  }
+  // this CTA's columns [c0, c1) of the tile; a warp takes whole columns, a
+  // lane four consecutive rows
+  const int c0 = BN * part / S, c1 = BN * (part + 1) / S;
+  const uint32_t base = smem_u32(tiles) + (uint32_t)lane * 16u;
+  for (int i = warp; i < MT * (c1 - c0); i += kGemmThreads / 32) {
+    const int c = c0 + i / MT, t = i % MT;
+    const int b = b0 + c, m = m0 + t * kBM + lane * 4;
+    if (b >= p || m >= n) continue;
+    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 x[kSplitKMaxS];
+#pragma unroll
+    for (int r = 0; r < kSplitKMaxS; ++r)
+      if (r < S) x[r] = ld_dsmem_f4(map_to_rank(base + (uint32_t)(c * MT + t) * (kBM * 4u), (uint32_t)r));
+#pragma unroll
+    for (int r = 0; r < kSplitKMaxS; ++r)
+      if (r < S) {
+        sum.x += x[r].x;
+        sum.y += x[r].y;
+        sum.z += x[r].z;
+        sum.w += x[r].w;
+      }
+    float *w = W + (int64_t)b * ldw + m;
+    const float *vf = Vf + (int64_t)b * ldvf + m;
+    if (vec_ok && m + 4 <= n) {
+      if (shift != 0.f) {
+        const float4 sv = __ldg(reinterpret_cast<const float4 *>(vf));
+        sum = make_float4(fmaf(shift, sv.x, sum.x), fmaf(shift, sv.y, sum.y), fmaf(shift, sv.z, sum.z),
+                          fmaf(shift, sv.w, sum.w));
+      }
+      *reinterpret_cast<float4 *>(w) = sum;
+    } else {
+      const float o[4] = {sum.x, sum.y, sum.z, sum.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (m + j < n) w[j] = shift != 0.f ? fmaf(shift, __ldg(vf + j), o[j]) : o[j];
+    }
+  }
+  __syncwarp();
+  cluster_sync_all();  // no CTA leaves while the others may read its partial tile
 }
 
 // ---------------------------------------------------------------------------
@@ -828,17 +890,17 @@ static PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
 // 2-D bf16 map: inner extent `cols` (K), `rows` rows `ld` elements apart,
 // box 64 x box_rows, 128-byte swizzle, zero fill out of bounds.
 static bool make_map(CUtensorMap *map, const void *base, int64_t cols, int64_t rows, int64_t ld,
-                     uint32_t box_rows) {
+                     uint32_t box_rows, int bk = kBK) {
   auto fn = encode_fn();
   if (!fn) return false;
   cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
   cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
-  cuuint32_t box[2] = {(cuuint32_t)kBK, box_rows};
+  cuuint32_t box[2] = {(cuuint32_t)bk, box_rows};
   cuuint32_t estr[2] = {1, 1};
   const CUresult r =
       fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(base), dims, strides, box,
          estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-         kRowBytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+         bk == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) record_error(__FILE__, __LINE__, "cuTensorMapEncodeTiled (bf16 tile) failed");
   return r == CUDA_SUCCESS;
@@ -1162,6 +1224,130 @@ int64_t schedule_cost(const PairSchedule &sc, int K) {
   return cost;
 }
 
+// CTAs of clusters of S = 1 .. 8 that the GPU holds at a time (kernels with
+// TMEM run one CTA per SM; larger clusters leave SMs of a GPC over: 152, 152,
+// 138, 144, 140, 138, 105, 120 on a GB300).
+struct SplitKSlots {
+  int cta[kSplitKMaxS + 1];
+  SplitKSlots() {
+    int dev = 0, sms = 152;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+      sms = 152;
+    auto kern = dense_tcgen05_splitk_kernel<true, 1>;
+    const int smem = 1024 + (int)kSplitKRing + (int)sizeof(GemmShared);
+    const bool set = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess;
+    for (int S = 1; S <= kSplitKMaxS; ++S) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3((unsigned)S, 1024, 1);
+      cfg.blockDim = dim3(kGemmThreads);
+      cfg.dynamicSmemBytes = (size_t)smem;
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = (unsigned)S;
+      attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      int clusters = 0;
+      if (!set || cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) != cudaSuccess || clusters < 1)
+        clusters = sms / S > 0 ? sms / S : 1;
+      cta[S] = clusters * S;
+    }
+    cta[0] = sms;
+    (void)cudaGetLastError();
+  }
+};
+
+struct SplitKPlan {
+  int bn, S, mt;  // probe tile, K ranges, 128-row tiles per CTA
+};
+
+// The cheapest (S, mt) by the time of the rounds of CTAs: a 64-wide K slice
+// takes as long as the slowest of the SM's own intake (measured 75 GB/s with
+// three or more stages in the ring, 62 with two), the operator's share of HBM
+// (6.4 TB/s over the CTAs running) and the L2 share of everything read
+// (11 TB/s); a round adds 6 us of pipeline fill and cluster reduction, and
+// 20 ns per accumulator column.  The model ranks the measured (n, p) grid
+// right to within a few percent: e.g. n = 23170, 32 probes S = 3 of two row
+// tiles (334 us; S = 1: 452 with one, 352 with two), n = 5000, 48 probes S = 3
+// (27 us; S = 1: 56, S = 4: 39, a second round), n = 512 S = 8 (11 us; S = 1: 17).
+static SplitKPlan splitk_plan(int64_t n, int64_t p, bool split) {
+  static const SplitKSlots slots;
+  const int64_t tiles_p = ceil_div(p, kSplitKMaxBN);
+  SplitKPlan best{(int)(ceil_div(ceil_div(p, tiles_p), 16) * 16), 1, 1};
+  const int64_t slices = ceil_div(n, kSplitKBK);
+  const double copies = split ? 2.0 : 1.0, v = copies * best.bn * kSplitKBK * 2.0;
+  double best_us = 1e300;
+  for (int mt = 1; mt <= 2; ++mt) {
+    const double a = copies * mt * kBM * kSplitKBK * 2.0;
+    const int64_t tiles = ceil_div(n, mt * kBM) * tiles_p;
+    const double intake = kSplitKRing >= 3.0 * (a + v) ? 75e3 : 62e3;  // bytes per us
+    for (int S = 1; S <= kSplitKMaxS && S <= slices; ++S) {
+      const double ks = (double)ceil_div(slices, S), fixed = 6.0 + 0.02 * best.bn * mt;
+      auto round_us = [&](double ctas) {
+        double t = (a + v) / intake;
+        if (ctas * a / 6.4e6 > t) t = ctas * a / 6.4e6;
+        if (ctas * (a + v) / 11e6 > t) t = ctas * (a + v) / 11e6;
+        return ks * t + fixed;
+      };
+      const int64_t full = tiles * S / slots.cta[S], rest = tiles * S % slots.cta[S];
+      const double us = full * round_us((double)slots.cta[S]) + (rest ? round_us((double)rest) : 0.0);
+      if (us < best_us) {
+        best_us = us;
+        best.S = S;
+        best.mt = mt;
+      }
+    }
+  }
+  return best;
+}
+
+// Split-K cluster form (see dense_tcgen05_splitk_kernel).
+static int launch_splitk(const __nv_bfloat16 *A_hi, const __nv_bfloat16 *A_lo, int64_t lda,
+                         const __nv_bfloat16 *V_hi, const __nv_bfloat16 *V_lo, int64_t ldvb,
+                         const float *Vf, int64_t ldvf, float *W, int64_t ldw, int64_t n, int64_t p,
+                         const SplitKPlan &plan, double shift, int *status, cudaStream_t s) {
+  const int bn = plan.bn, S = plan.S, mt = plan.mt;
+  const bool split = A_lo != nullptr;
+  const uint32_t rows = (uint32_t)(mt * kBM);
+  const uint32_t stage_bytes = (split ? 2u : 1u) * (rows + (uint32_t)bn) * kSplitKBK * 2;
+  int stages = (int)(kSplitKRing / stage_bytes);
+  if (stages > kGemmMaxStages) stages = kGemmMaxStages;
+  const size_t ring = (size_t)stages * stage_bytes, part = (size_t)bn * rows * 4;
+  const size_t smem = 1024 + (ring > part ? ring : part) + sizeof(GemmShared);
+  CUtensorMap mahi, malo, mbhi, mblo;
+  if (!make_map(&mahi, A_hi, n, n, lda, rows, kSplitKBK)) return MFG_ERR_CUDA;
+  if (!make_map(&mbhi, V_hi, n, p, ldvb, (uint32_t)bn, kSplitKBK)) return MFG_ERR_CUDA;
+  if (split) {
+    if (!make_map(&malo, A_lo, n, n, lda, rows, kSplitKBK)) return MFG_ERR_CUDA;
+    if (!make_map(&mblo, V_lo, n, p, ldvb, (uint32_t)bn, kSplitKBK)) return MFG_ERR_CUDA;
+  } else {
+    malo = mahi;
+    mblo = mbhi;
+  }
+  uint32_t cols = 32;
+  while ((int)cols < mt * bn) cols <<= 1;
+  const int vec_ok = ldw % 4 == 0 && ldvf % 4 == 0 && ((uintptr_t)W & 15) == 0 && ((uintptr_t)Vf & 15) == 0;
+  auto kern = mt == 2 ? (split ? dense_tcgen05_splitk_kernel<true, 2> : dense_tcgen05_splitk_kernel<false, 2>)
+                      : (split ? dense_tcgen05_splitk_kernel<true, 1> : dense_tcgen05_splitk_kernel<false, 1>);
+  MFG_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)S, (unsigned)ceil_div(n, rows), (unsigned)ceil_div(p, bn));
+  cfg.blockDim = dim3(kGemmThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)S;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  MFG_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, mahi, malo, mbhi, mblo, Vf, ldvf, W, ldw, (int)n, (int)p,
+                                  bn, stages, cols, (float)shift, vec_ok, status));
+  return MFG_LAUNCH_STATUS();
+}
+
 int launch_dense_tcgen05(const __nv_bfloat16 *A_hi, const __nv_bfloat16 *A_lo, int64_t lda,
                          const __nv_bfloat16 *V_hi, const __nv_bfloat16 *V_lo, int64_t ldvb,
                          const float *Vf, int64_t ldvf, float *W, int64_t ldw, int64_t n, int64_t p,
@@ -1174,17 +1360,34 @@ int launch_dense_tcgen05(const __nv_bfloat16 *A_hi, const __nv_bfloat16 *A_lo, i
     return MFG_ERR_BAD_ARG;
   if (p <= kGemvMaxP)
     return launch_dense_gemv(A_hi, A_lo, lda, V_hi, V_lo, ldvb, Vf, ldvf, W, ldw, n, p, shift, s);
-  // probes per tile: a multiple of 16 in [16, 256]
   const GemmRule rule = n >= kPairMinRows ? gemm_rule_for(n, p) : GemmRule{0, 0, 0, 0, 0, 0};
+  // Few probes are bound by the operator stream, and few tiles leave SMs
+  // idle: the split-K cluster form.  More than 128 probes re-read the operator
+  // per probe tile there, which pays while the tiles (of one K range) cover
+  // up to 5/9 of the SMs (256 probes: n = 5000 52 against 71 us for CTA pairs;
+  // n = 6144 73 against 66).  Rules of the autotuner name CTA-pair forms.
+  static int sms = 0;
+  if (sms == 0) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+      sms = 152;
+  }
+  const bool pair_rule = (rule.split != 0 || rule.bn != 0) && p >= 64;
+  const int64_t row_tiles = ceil_div(n, kBM);
+  if (!pair_rule && (n < kPairMinRows || p <= kSplitKMaxBN ||
+                     row_tiles * ceil_div(p, kSplitKMaxBN) * 9 <= (int64_t)sms * 5)) {
+    const SplitKPlan plan = splitk_plan(n, p, split);
+    return launch_splitk(A_hi, A_lo, lda, V_hi, V_lo, ldvb, Vf, ldvf, W, ldw, n, p, plan, shift, status, s);
+  }
+  // CTA pairs (2-SM MMAs, M = 256); probes per tile: a multiple of 32 in [64, 256]
   const int64_t pt = p < 256 ? p : 256;
-  int BN = (int)((pt + 15) / 16 * 16);
+  int BN = (int)((pt + 31) / 32 * 32);
   if (rule.bn > 0 && rule.bn < BN) BN = rule.bn;  // a narrower probe tile: more tiles per operator
   uint32_t cols = 32;
   while ((int)cols < BN) cols <<= 1;
-  // CTA pairs (2-SM MMAs, M = 256) once the operator spans several pair tiles
-  const bool pair = n >= kPairMinRows && BN >= 64 && BN % 32 == 0;
   const uint32_t a_bytes = kBM * kBK * 2;
-  const uint32_t b_bytes = (uint32_t)(pair ? BN / 2 : BN) * kBK * 2;
+  const uint32_t b_bytes = (uint32_t)(BN / 2) * kBK * 2;
   const uint32_t stage_bytes = (split ? 2u : 1u) * (a_bytes + b_bytes);
   const size_t budget = 200 * 1024;
   int stages = (int)(budget / stage_bytes);
@@ -1193,7 +1396,7 @@ int launch_dense_tcgen05(const __nv_bfloat16 *A_hi, const __nv_bfloat16 *A_lo, i
   const size_t smem = 1024 + (size_t)stages * stage_bytes + sizeof(GemmShared);
 
   CUtensorMap mahi, malo, mbhi, mblo;
-  const uint32_t b_rows = (uint32_t)(pair ? BN / 2 : BN);
+  const uint32_t b_rows = (uint32_t)(BN / 2);
   if (!make_map(&mahi, A_hi, n, n, lda, kBM)) return MFG_ERR_CUDA;
   if (!make_map(&mbhi, V_hi, n, p, ldvb, b_rows)) return MFG_ERR_CUDA;
   if (split) {
@@ -1203,20 +1406,13 @@ int launch_dense_tcgen05(const __nv_bfloat16 *A_hi, const __nv_bfloat16 *A_lo, i
     malo = mahi;
     mblo = mbhi;
   }
-  if (pair) {
+  {
     // grid.x: two CTAs per 256-row tile (the cluster dimension).  When the
     // tiles cover fewer than 60 % of the SMs (e.g. n = 8192: 64 CTAs), each
     // CTA streams its rows at a fixed rate and the SMs idle, so K is split in
     // two halves (grid.z) whose partial products add into a zeroed W.
     dim3 grid((unsigned)(2 * ((n + 2 * kBM - 1) / (2 * kBM))), (unsigned)((p + BN - 1) / BN));
     if (grid.y > 65535) return MFG_ERR_UNSUPPORTED;
-    static int sms = 0;
-    if (sms == 0) {
-      int dev = 0;
-      if (cudaGetDevice(&dev) != cudaSuccess ||
-          cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-        sms = 152;
-    }
     const int num_k_all = (int)((n + kBK - 1) / kBK);
     const bool split_default = (int64_t)grid.x * grid.y * 5 < (int64_t)sms * 3;
     const bool split_k = rule.split == 0 ? split_default : rule.split == 2;
@@ -1285,22 +1481,6 @@ int launch_dense_tcgen05(const __nv_bfloat16 *A_hi, const __nv_bfloat16 *A_lo, i
     }
     return MFG_LAUNCH_STATUS();
   }
-  dim3 grid((unsigned)((n + kBM - 1) / kBM), (unsigned)((p + BN - 1) / BN));
-  if (grid.y > 65535) return MFG_ERR_UNSUPPORTED;
-  if (split) {
-    MFG_CUDA_TRY(cudaFuncSetAttribute(dense_tcgen05_kernel<true>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    dense_tcgen05_kernel<true><<<grid, kGemmThreads, smem, s>>>(
-        mahi, malo, mbhi, mblo, Vf, ldvf, W, ldw, (int)n, (int)p, BN, stages, cols, (float)shift,
-        status);
-  } else {
-    MFG_CUDA_TRY(cudaFuncSetAttribute(dense_tcgen05_kernel<false>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    dense_tcgen05_kernel<false><<<grid, kGemmThreads, smem, s>>>(
-        mahi, malo, mbhi, mblo, Vf, ldvf, W, ldw, (int)n, (int)p, BN, stages, cols, (float)shift,
-        status);
-  }
-  return MFG_LAUNCH_STATUS();
 }
 
 }  // namespace mfg
