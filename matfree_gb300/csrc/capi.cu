@@ -88,8 +88,8 @@ static void prof_end(size_t e0, int cls, double bytes, double flops, cudaStream_
 
 struct WsLayout {
   size_t w, panel, norm, len0, h2, partials, counters, status, hi, lo, q, h, values, eig, fsq;
-  // two-sweep Arnoldi: qt (float panel), X2 (p (2k + 1)), dots (p 3), nu (p),
-  // finish coefficients (p 4), full coefficients Hh (p (k + 1) k)
+  // two-sweep Arnoldi: qt (float panel), X2 (p (2k + 1)), dots (p 3), nu
+  // (p (k + 1)), finish coefficients (p 4), full coefficients Hh (p (k + 1) k)
   size_t vt, x2, dots, nu, cf, hh;
   size_t total;
 };
@@ -143,7 +143,7 @@ static WsLayout layout(const mfg_operator *op, int64_t k, int64_t p, int64_t ld,
     L.vt = take((size_t)p * ld * es);
     L.x2 = take((size_t)p * (2 * kk + 1) * 8);
     L.dots = take((size_t)p * 3 * 8);
-    L.nu = take((size_t)p * 8);
+    L.nu = take((size_t)p * (kk + 1) * 8);
     L.cf = take((size_t)p * 4 * 8);
     L.hh = take((size_t)p * (kk + 1) * kk * 8);
   }
@@ -253,7 +253,7 @@ static void apply_cost(const mfg_operator *op, int64_t p, double *bytes, double 
 // raises MFG_ERR_RETRY in the device status word.
 template <typename T>
 static int run_two_sweep(const mfg_operator *op, int64_t k, int64_t p, int64_t ld, T *Q,
-                         double *H, T *R, const WsLayout &L, char *ws, cudaStream_t s) {
+                         double *H, bool full_h, T *R, const WsLayout &L, char *ws, cudaStream_t s) {
   if constexpr (sizeof(T) != 4) {
     return MFG_ERR_UNSUPPORTED;
   } else {
@@ -279,46 +279,63 @@ static int run_two_sweep(const mfg_operator *op, int64_t k, int64_t p, int64_t l
     const double bfb = hi ? (double)n * (double)p * 2.0 * (lo ? 2.0 : 1.0) : 0.0;
     const int64_t qb = k * ld;
     const int64_t koff = k, xs = 2 * k + 1;
-    // step 0 as the reference: w = A q_0, h_0 = q_0 . w, u_1 = w - q_0 h_0
-    MFG_LAUNCH(MFG_PROF_APPLY, ab, af, apply_op<T>(op, Q, qb, Wb, ld, p, hi, lo, ld, panel, status, s));
-    MFG_LAUNCH(MFG_PROF_PROJ, 2.0 * vecb, 2.0 * vecb / sizeof(T),
-               launch_proj<T>(Q, qb, ld, 1, Wb, ld, n, p, partials, counters, H, k * k, k, s, status));
-    MFG_LAUNCH(MFG_PROF_SUB, 3.0 * vecb, 4.0 * vecb / sizeof(T),
-               launch_sub<T>(Q, qb, ld, 1, H, k * k, k, Wb, Wb, ld, n, p, true, true, partials,
-                             counters, nu, nullptr, 0, s, status));
-    // qt_1 = u_1 / ||u_1|| (and its bf16 copies when another product follows)
-    MFG_LAUNCH(MFG_PROF_SCALE, 2.0 * vecb + (k > 1 ? bfb : 0.0), vecb / sizeof(T),
-               launch_scale<T>(Wb, ld, n, p, nu, Vt, ld, k > 1 ? hi : nullptr, lo, ld, s));
-    for (int64_t j = 1; j < k; ++j) {
-      const int nc = (int)j;
-      MFG_LAUNCH(MFG_PROF_APPLY, ab, af, apply_op<T>(op, Vt, ld, Wb, ld, p, hi, lo, ld, panel, status, s));
-      // [Q^T qt | Q^T w | qt . w] from one read of the basis, in column blocks
-      // of at most kTwoSweepPassCols vectors (the later blocks' qt . w goes to
-      // a scratch slot: it is the first block's value again)
-      for (int c0 = 0; c0 < nc; c0 += kTwoSweepPassCols) {
-        const int cn = nc - c0 < kTwoSweepPassCols ? nc - c0 : kTwoSweepPassCols;
-        MFG_LAUNCH(MFG_PROF_PROJ, (cn + 2.0) * vecb, 4.0 * cn * vecb / sizeof(T),
-                   launch_proj2<T>(Q, qb, ld, c0, cn, Wb, Vt, ld, n, p, partials, counters,
-                                   X2 + c0, xs, koff, c0 > 0 ? dots : nullptr, 3, status, s));
+    const bool fused = arnoldi_cluster_applies(n);
+    if (fused) {
+      // a step is the product and one launch: while a probe's vector fits the
+      // registers of a cluster (n <= 32768)
+      for (int64_t j = 0; j < k; ++j) {
+        MFG_LAUNCH(MFG_PROF_APPLY, ab, af,
+                   apply_op<T>(op, j == 0 ? Q : Vt, j == 0 ? qb : ld, Wb, ld, p, hi, lo, ld, panel, status, s));
+        const bool more = j + 1 < k;
+        MFG_LAUNCH(MFG_PROF_SUBPROJ, (j + (more || R ? 4.0 : 3.0)) * vecb + (more ? bfb : 0.0),
+                   (8.0 * j + 10.0) * vecb / sizeof(T),
+                   launch_arnoldi_step((int)j, k, n, p, Q, qb, ld, Wb, j == 0 ? Q : Vt, j == 0 ? qb : ld,
+                                       (more || R) ? Vt : nullptr, more ? hi : nullptr, lo, H, Hh, nu, status, s));
       }
-      // q_j (unnormalised) = qt - Q Q^T qt into row j, w <- w - Q Q^T w; a
-      // later column block continues from the first block's results
-      for (int c0 = 0; c0 < nc; c0 += kTwoSweepPassCols) {
-        const int cn = nc - c0 < kTwoSweepPassCols ? nc - c0 : kTwoSweepPassCols;
-        const T *bin = c0 == 0 ? Vt : Q + j * ld;
-        const int64_t bstr = c0 == 0 ? ld : qb;
-        MFG_LAUNCH(MFG_PROF_SUBPROJ, (cn + 4.0) * vecb, 4.0 * cn * vecb / sizeof(T),
-                   launch_sub2<T>(Q, qb, ld, c0, cn, X2 + c0, xs, koff, Wb, ld, bin, bstr,
-                                  Q + j * ld, qb, n, p, partials, counters, dots, status, s));
+      MFG_LAUNCH(MFG_PROF_OTHER, 24.0 * p * k * k, full_h ? 2.0 / 3.0 * p * k * k * k : 0.0,
+                 launch_arnoldi_h(k, p, H, Hh, nu, !full_h, R ? cf : nullptr, s));
+    } else {
+      // step 0 as the reference: w = A q_0, h_0 = q_0 . w, u_1 = w - q_0 h_0
+      MFG_LAUNCH(MFG_PROF_APPLY, ab, af, apply_op<T>(op, Q, qb, Wb, ld, p, hi, lo, ld, panel, status, s));
+      MFG_LAUNCH(MFG_PROF_PROJ, 2.0 * vecb, 2.0 * vecb / sizeof(T),
+                 launch_proj<T>(Q, qb, ld, 1, Wb, ld, n, p, partials, counters, H, k * k, k, s, status));
+      MFG_LAUNCH(MFG_PROF_SUB, 3.0 * vecb, 4.0 * vecb / sizeof(T),
+                 launch_sub<T>(Q, qb, ld, 1, H, k * k, k, Wb, Wb, ld, n, p, true, true, partials,
+                               counters, nu, nullptr, 0, s, status));
+      // qt_1 = u_1 / ||u_1|| (and its bf16 copies when another product follows)
+      MFG_LAUNCH(MFG_PROF_SCALE, 2.0 * vecb + (k > 1 ? bfb : 0.0), vecb / sizeof(T),
+                 launch_scale<T>(Wb, ld, n, p, nu, Vt, ld, k > 1 ? hi : nullptr, lo, ld, s));
+      for (int64_t j = 1; j < k; ++j) {
+        const int nc = (int)j;
+        MFG_LAUNCH(MFG_PROF_APPLY, ab, af, apply_op<T>(op, Vt, ld, Wb, ld, p, hi, lo, ld, panel, status, s));
+        // [Q^T qt | Q^T w | qt . w] from one read of the basis, in column blocks
+        // of at most kTwoSweepPassCols vectors (the later blocks' qt . w goes to
+        // a scratch slot: it is the first block's value again)
+        for (int c0 = 0; c0 < nc; c0 += kTwoSweepPassCols) {
+          const int cn = nc - c0 < kTwoSweepPassCols ? nc - c0 : kTwoSweepPassCols;
+          MFG_LAUNCH(MFG_PROF_PROJ, (cn + 2.0) * vecb, 4.0 * cn * vecb / sizeof(T),
+                     launch_proj2<T>(Q, qb, ld, c0, cn, Wb, Vt, ld, n, p, partials, counters,
+                                     X2 + c0, xs, koff, c0 > 0 ? dots : nullptr, 3, status, s));
+        }
+        // q_j (unnormalised) = qt - Q Q^T qt into row j, w <- w - Q Q^T w; a
+        // later column block continues from the first block's results
+        for (int c0 = 0; c0 < nc; c0 += kTwoSweepPassCols) {
+          const int cn = nc - c0 < kTwoSweepPassCols ? nc - c0 : kTwoSweepPassCols;
+          const T *bin = c0 == 0 ? Vt : Q + j * ld;
+          const int64_t bstr = c0 == 0 ? ld : qb;
+          MFG_LAUNCH(MFG_PROF_SUBPROJ, (cn + 4.0) * vecb, 4.0 * cn * vecb / sizeof(T),
+                     launch_sub2<T>(Q, qb, ld, c0, cn, X2 + c0, xs, koff, Wb, ld, bin, bstr,
+                                    Q + j * ld, qb, n, p, partials, counters, dots, status, s));
+        }
+        MFG_LAUNCH(MFG_PROF_OTHER, 8.0 * p * (3.0 * k + 2.0 * j), 2.0 * p * j * j,
+                   launch_twosweep_coef((int)j, (int)k, p, X2, koff, dots, H, Hh, nu, cf, status, s));
+        const bool more = j + 1 < k;
+        MFG_LAUNCH(MFG_PROF_SCALE, (more || R ? 4.0 : 2.0) * vecb + (more ? bfb : 0.0),
+                   3.0 * vecb / sizeof(T),
+                   launch_twosweep_finish<T>(Q + j * ld, qb, Wb, ld, n, p, cf,
+                                             (more || R) ? Vt : nullptr, more ? hi : nullptr, lo,
+                                             ld, s));
       }
-      MFG_LAUNCH(MFG_PROF_OTHER, 8.0 * p * (3.0 * k + 2.0 * j), 2.0 * p * j * j,
-                 launch_twosweep_coef((int)j, (int)k, p, X2, koff, dots, H, Hh, nu, cf, status, s));
-      const bool more = j + 1 < k;
-      MFG_LAUNCH(MFG_PROF_SCALE, (more || R ? 4.0 : 2.0) * vecb + (more ? bfb : 0.0),
-                 3.0 * vecb / sizeof(T),
-                 launch_twosweep_finish<T>(Q + j * ld, qb, Wb, ld, n, p, cf,
-                                           (more || R) ? Vt : nullptr, more ? hi : nullptr, lo,
-                                           ld, s));
     }
     if (R) {
       // the reference's last reorthogonalisation: R = nu_k (qt_k - Q Q^T qt_k)
@@ -328,7 +345,7 @@ static int run_two_sweep(const mfg_operator *op, int64_t k, int64_t p, int64_t l
       MFG_LAUNCH(MFG_PROF_SUB, (nc + 2.0) * vecb, 2.0 * nc * vecb / sizeof(T),
                  launch_sub<T>(Q, qb, ld, nc, X2, xs, 1, Vt, R, ld, n, p, false, true, partials,
                                counters, nullptr, nullptr, 0, s, status));
-      MFG_LAUNCH(MFG_PROF_OTHER, 16.0 * p, (double)p, launch_inv(nu, cf, p, s));
+      if (!fused) MFG_LAUNCH(MFG_PROF_OTHER, 16.0 * p, (double)p, launch_inv(nu, cf, p, s));
       MFG_LAUNCH(MFG_PROF_SCALE, 2.0 * vecb, vecb / sizeof(T),
                  launch_scale<T>(R, ld, n, p, cf, R, ld, nullptr, nullptr, ld, s));
     }
@@ -338,7 +355,7 @@ static int run_two_sweep(const mfg_operator *op, int64_t k, int64_t p, int64_t l
 
 template <typename T>
 static int run_hessenberg(const mfg_operator *op, int64_t k, int64_t p, const T *V, int64_t ld,
-                          int reortho, T *Q, double *H, T *R, double *init_len_inv,
+                          int reortho, T *Q, double *H, bool full_h, T *R, double *init_len_inv,
                           const WsLayout &L, char *ws, cudaStream_t s) {
   const int64_t n = op->n;
   const double vecb = (double)n * (double)p * (double)sizeof(T);  // one panel
@@ -377,7 +394,7 @@ static int run_hessenberg(const mfg_operator *op, int64_t k, int64_t p, const T 
   }
   MFG_LAUNCH(MFG_PROF_SCALE, 2.0 * vecb + bfb, vecb / sizeof(T),
              launch_scale<T>(V, ld, n, p, len0, Q, qb, hi, lo, ld, s));
-  if (reortho == 3) return run_two_sweep<T>(op, k, p, ld, Q, H, R, L, ws, s);
+  if (reortho == 3) return run_two_sweep<T>(op, k, p, ld, Q, H, full_h, R, L, ws, s);
 
   for (int64_t j = 0; j < k; ++j) {
     const T *qj = Q + j * ld;
@@ -1125,8 +1142,8 @@ int mfg_hessenberg(const mfg_operator *op, int64_t k, int64_t p, const void *V, 
   cudaStream_t s = as_stream(stream);
   if (op->precision == MFG_PREC_FP64)
     return run_hessenberg<double>(op, k, p, (const double *)V, ld, reortho, (double *)Q, H,
-                                  (double *)residual, init_len_inv, L, ws, s);
-  return run_hessenberg<float>(op, k, p, (const float *)V, ld, reortho, (float *)Q, H,
+                                  true, (double *)residual, init_len_inv, L, ws, s);
+  return run_hessenberg<float>(op, k, p, (const float *)V, ld, reortho, (float *)Q, H, true,
                                (float *)residual, init_len_inv, L, ws, s);
 }
 
@@ -1235,10 +1252,10 @@ static int slq_impl(const mfg_operator *op, int64_t k, int64_t p, const void *pr
   if (Q && !aligned16(Q)) return MFG_ERR_BAD_ARG;
   if (op->precision == MFG_PREC_FP64)
     MFG_TRY(run_hessenberg<double>(op, k, p, (const double *)probes, ld, 1, (double *)Qb, Hb,
-                                   nullptr, nullptr, L, ws, s));
+                                   true, nullptr, nullptr, L, ws, s));
   else
     MFG_TRY(run_hessenberg<float>(op, k, p, (const float *)probes, ld, two ? 3 : 1, (float *)Qb, Hb,
-                                  nullptr, nullptr, L, ws, s));
+                                  H != nullptr, nullptr, nullptr, L, ws, s));
   // funm.py:240-241: length^2 * e1^T f(T) e1 with length = ||v||
   MFG_LAUNCH(MFG_PROF_OTHER, 16.0 * p, (double)p, launch_square(len0, scale, p, s));
   MFG_LAUNCH(MFG_PROF_QUAD, 8.0 * p * k * k + 16.0 * p * k, 0.0,

@@ -55,6 +55,13 @@ template <typename T>
 int launch_twosweep_finish(T *Qj, int64_t q_bstride, const T *Z, int64_t w_bstride, int64_t n,
                            int64_t p, const double *cf, T *qt, __nv_bfloat16 *hi,
                            __nv_bfloat16 *lo, int64_t bf_bstride, cudaStream_t s);
+// arnoldi_cluster.cu: the same step as one launch (float bases of n up to 32768)
+bool arnoldi_cluster_applies(int64_t n);
+int launch_arnoldi_step(int j, int64_t k, int64_t n, int64_t p, float *Q, int64_t qb, int64_t ld, const float *W,
+                        const float *Vin, int64_t vb, float *Vout, __nv_bfloat16 *hi, __nv_bfloat16 *lo, double *H,
+                        double *Hh, double *nu, int *status, cudaStream_t s);
+int launch_arnoldi_h(int64_t k, int64_t p, double *H, const double *Hh, const double *nu, bool band,
+                     double *nu_last_inv, cudaStream_t s);
 // conjugate gradients on probe-major panels (lanczos_kernels.cu)
 template <typename T>
 int launch_cg_init(const T *B, T *X, T *R, T *P, int64_t ld, int64_t n, int64_t p,
