@@ -331,13 +331,10 @@ static int launch_tridiag_eigh_ql(int64_t k, int64_t p, const double *H, double 
 //    [f; 0]^T u_j and [0; l]^T u_j.
 //
 // One CTA owns one problem.  The serial parts of a merge (the sorted merge
-// of the two halves and the deflation scan) run on one thread per merge; the
-// roots, the Loewner products and the vector rows run on one group of lanes
-// per root, over all merges of a level at once: one lane for merges of up to
-// 16 poles, four lanes (each taking every fourth term of the sums) above.  The float64 work of a problem spreads over up
-// to 4k threads in place of the single serial chain of the QL chase; GB300
-// issues float64 at two lanes per clock per SM, and the many independent
-// chains keep that pipe fed.
+// of the two halves with deflated poles, the deflation scan) run on one thread per
+// merge; the merge where nothing deflates runs on a thread per element, and the roots,
+// the Loewner products and the vector rows on a group of lanes per root, over all
+// merges of a level at once.
 
 constexpr int kDcMinK = 16;          // below this the QL chase is as fast
 constexpr int kDcMaxK = 2048;        // shared-memory bound (about 200 KB)
@@ -357,163 +354,181 @@ __host__ __device__ inline DcLayout dc_layout(int k) {
   return L;
 }
 
-// root in (P1, P2) of c + s1/(P1 - x) + s2/(P2 - x) = 0, one of P1, P2 zero
-__device__ __forceinline__ double dc_quad_root(double c, double P1, double P2, double s1,
-                                               double s2) {
-  const double a1 = c * (P1 + P2) + s1 + s2;
-  const double a0 = c * P1 * P2 + s1 * P2 + s2 * P1;
-  // g(x) = c x^2 - a1 x + a0 is positive at P1 and negative at P2, so the
-  // root inside is (a1 - sqrt(a1^2 - 4 c a0)) / (2c) for either sign of c
-  const double sq = sqrt(fmax(a1 * a1 - 4.0 * c * a0, 0.0));
-  return a1 > 0.0 ? 2.0 * a0 / (a1 + sq) : (a1 - sq) / (2.0 * c);
-}
-
-// step eta with c + s1/(A - eta) + s2/(B - eta) = 0, A < 0 < B, where the
-// model equals f at eta = 0 (so its constant term is A B f)
-__device__ __forceinline__ double dc_quad_step(double c, double A, double B, double s1,
-                                               double s2, double f) {
-  const double a1 = c * (A + B) + s1 + s2;
-  const double a0 = A * B * f;
-  const double sq = sqrt(fmax(a1 * a1 - 4.0 * c * a0, 0.0));
-  return a1 > 0.0 ? 2.0 * a0 / (a1 + sq) : (a1 - sq) / (2.0 * c);
-}
-
-// step eta > A with c + s0/(A0 - eta) + s1/(A - eta) = 0, A0 < A < 0 (the
-// largest root: both poles below it, so the root is the larger one)
-__device__ __forceinline__ double dc_quad_step_right(double c, double A0, double A, double s0,
-                                                     double s1, double f) {
-  const double a1 = c * (A0 + A) + s0 + s1;
-  const double a0 = A0 * A * f;
-  const double sq = sqrt(fmax(a1 * a1 - 4.0 * c * a0, 0.0));
-  return a1 >= 0.0 ? (a1 + sq) / (2.0 * c) : 2.0 * a0 / (a1 - sq);
-}
-
-// 1/x from the hardware's approximate float64 reciprocal (rcp.approx.ftz.f64)
-// refined by two Newton-Raphson steps y <- y + y (1 - x y), each of which
-// squares the relative error: a few ulp from 1/x for x in the normal range,
-// in four FMAs in place of a correctly rounded division.  The secular sums,
-// Loewner products and vector entries below carry rounding errors of that
+// 1/x from the hardware's approximate float64 reciprocal (relative error e of
+// about 2^-20) and one third-order step y (1 + e + e^2), which leaves e^3: a few
+// ulp from 1/x for x in the normal range, in three dependent FMAs.  The secular
+// sums, Loewner products and vector entries below carry rounding errors of that
 // size anyway.
 __device__ __forceinline__ double rcp_nr(double x) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  double e = fma(-x, y, 1.0);
-  y = fma(y, e, y);
-  e = fma(-x, y, 1.0);
-  return fma(y, e, y);
+  const double e = fma(-x, y, 1.0);
+  return fma(y, fma(e, e, e), y);
 }
 
-// Sum (product) over the G lanes of a group (lanes G m .. G m + G - 1 of a
-// warp, G = 1 or 4).  Every lane gets the same bits ((v0+v1)+(v2+v3) in some
-// operand order; IEEE addition and multiplication commute), so the lanes of a
-// group take the same branches afterwards.
+// 1 / rho of a coupling, which may be as small as the whole problem's scale
+__device__ __forceinline__ double rcp_any(double x) { return x > 1e-290 ? rcp_nr(x) : 1.0 / x; }
+
+// Square root and quotient of an iteration's step: one Newton step (relative
+// error about 1e-12).  The iterate they lead to is judged by f itself.
+__device__ __forceinline__ double sqrt_step(double v) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(v));
+  const double h = v * y;
+  const double r = fma(0.5 * h, fma(-h, y, 1.0), h);
+  return v > 1e-290 ? r : 0.0;
+}
+__device__ __forceinline__ double div_step(double num, double den) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(den));
+  y = fma(y, fma(-den, y, 1.0), y);
+  return num * y;
+}
+
+// A double's bits as an integer of the same order (-0 sorts below +0, NaN beyond
+// the infinities).
+__device__ __forceinline__ long long order_key(double x) {
+  const long long v = __double_as_longlong(x);
+  return v ^ ((v >> 63) & 0x7fffffffffffffffll);
+}
+__device__ __forceinline__ bool less_than(double x, double y) { return order_key(x) < order_key(y); }
+__device__ __forceinline__ bool positive(double x) { return order_key(x) > 0; }
+
+// Root of c x^2 - 2 h x + a0 with c + s0/(U - x) + s1/(V - x) = 0, U < V its poles:
+// the one between them, or (right) the one above both, for c > 0.  The
+// cancelling form of the quadratic formula is avoided for either sign of h;
+// one square root and one quotient on every path.
+__device__ __forceinline__ double dc_quadratic(double c, double h, double a0, bool right) {
+  double disc = fma(h, h, -c * a0);
+  disc = positive(disc) ? disc : 0.0;
+  const double sq = sqrt_step(disc);
+  const bool up = positive(h);
+  const double t = up ? h + sq : h - sq;
+  const bool small = up != right;  // the root of smaller modulus: a0 / t
+  return div_step(small ? a0 : t, small ? t : c);
+}
+
+// Sum (product) over the G lanes of a group (lanes G m .. G m + G - 1 of a warp).
+// Every lane gets the same bits (each level adds the same two values in either
+// order), so the lanes of a group take the same branches afterwards.
 template <int G>
 __device__ __forceinline__ double group_sum(double v, unsigned mask) {
-  if (G >= 2) v += __shfl_xor_sync(mask, v, 1);
-  if (G >= 4) v += __shfl_xor_sync(mask, v, 2);
+#pragma unroll
+  for (int o = 1; o < G; o <<= 1) v += __shfl_xor_sync(mask, v, o);
   return v;
 }
 template <int G>
 __device__ __forceinline__ double group_prod(double v, unsigned mask) {
-  if (G >= 2) v *= __shfl_xor_sync(mask, v, 1);
-  if (G >= 4) v *= __shfl_xor_sync(mask, v, 2);
+#pragma unroll
+  for (int o = 1; o < G; o <<= 1) v *= __shfl_xor_sync(mask, v, o);
   return v;
 }
 
 // Root j of the secular equation of the kept poles P[0..mk) (ascending) with
 // weights ZZ[i] = z_i^2 and coupling rho > 0; upper bounds the largest root.
-// The G lanes of a group (sub = 0..G-1, lane mask gm) each sum every G-th
-// term and take identical steps.  Every term runs through one loop whose trip
-// count is the same for all roots of a merge (the two poles of the model are
-// masked out rather than skipped), so the groups of a warp stay converged.
+// The G lanes of a group (sub = 0..G-1, lane mask gm) each sum every G-th term
+// and take identical steps.  A warp has one float64 instruction under way at a
+// time, 64 clocks each whatever its active lanes, and an SM about four warps'
+// (measured), so what counts is the number of a warp's float64 instructions:
+// comparisons run on integers, and a step is one chain for all its cases.
 // Returns false when the iteration limit is reached.
 template <int G>
 __device__ bool dc_secular_root(const double *P, const double *ZZ, int mk, int j, double rho,
                                 double upper, int sub, unsigned gm, double &x_out, int &o_out) {
-  const double ir = 1.0 / rho;
+  o_out = j;
+  if (mk == 1) {
+    x_out = rho * ZZ[0];
+    return true;
+  }
+  const double ir = rcp_any(rho);
   const bool last = j + 1 >= mk;
-  const double lo_pole = P[j];
-  const double hi_pole = last ? upper : P[j + 1];
+  // the poles of the model: (j, j + 1) inside, (j - 1, j) for the largest root
+  const int m0 = last ? j - 1 : j, m1 = m0 + 1;
+  const int lane0 = (int)(threadIdx.x & 31 & ~(G - 1));
+  const double PU = P[m0], PV = P[m1], w0 = ZZ[m0], w1 = ZZ[m1], wh = 0.5 * (w0 + w1);
+  const double lo_pole = P[j], hi_pole = last ? upper : PV;
+  // one pass over the poles at base + x: the sums of all but the model's terms below
+  // (negative) and above (positive) the root, their derivative, and the model's two
+  double below, above, slope, t0, t1;
+  auto pass = [&](double base, double x) {
+    below = above = slope = t0 = t1 = 0.0;
+    for (int i = sub; i < mk; i += G) {
+      const double inv = rcp_nr((P[i] - base) - x);
+      const double t = ZZ[i] * inv;
+      if (i == m0) {
+        t0 = t;
+      } else if (i == m1) {
+        t1 = t;
+      } else {
+        slope = fma(t, inv, slope);
+        const double acc = (i < m0 ? below : above) + t;
+        if (i < m0)
+          below = acc;
+        else
+          above = acc;
+      }
+    }
+    below = group_sum<G>(below, gm);
+    above = group_sum<G>(above, gm);
+    slope = group_sum<G>(slope, gm);
+    if (G > 1) {
+      t0 = __shfl_sync(gm, t0, lane0 + (m0 & (G - 1)));
+      t1 = __shfl_sync(gm, t1, lane0 + (m1 & (G - 1)));
+    }
+  };
+  // the sign at the midpoint names the nearer pole, the origin of the offsets
   const double xma = 0.5 * (lo_pole + hi_pole);
-  double fpart = 0.0;
-  for (int i = sub; i < mk; i += G) fpart = fma(ZZ[i], rcp_nr(P[i] - xma), fpart);
-  const double fmid = ir + group_sum<G>(fpart, gm);
-  const double zzj = ZZ[j];
-  const double zzj1 = last ? 0.0 : ZZ[j + 1];
-  const bool two_below = last && mk > 1;
-  const double zzjm = two_below ? ZZ[j - 1] : 0.0;
-  const int o = (!last && fmid < 0.0) ? j + 1 : j;
+  pass(0.0, xma);
+  const double cmid = ir + (below + above), fmid = cmid + (t0 + t1);
+  const int o = (!last && !positive(fmid)) ? j + 1 : j;
   const double base = P[o];
   double lo = lo_pole - base, hi = hi_pole - base;
-  const double P1 = P[j] - base;
-  const double P2 = last ? hi : P[j + 1] - base;
-  const double P0 = two_below ? P[j - 1] - base : 0.0;
+  const double U = PU - base, V = PV - base, M = 0.5 * (U + V);
   const double xm = 0.5 * (lo + hi);
   // first guess: the two poles of the model exact, the other terms frozen at
   // the midpoint of the interval
   double x;
-  if (mk == 1) {
-    x = rho * zzj;
-  } else if (last) {
-    const double c = fmid - zzj * rcp_nr(P[j] - xma) - zzjm * rcp_nr(P[j - 1] - xma);
-    x = c > 0.0 ? xm + dc_quad_step_right(c, P0 - xm, P1 - xm, zzjm, zzj, fmid) : xm;
+  if (last) {
+    const double u = U - xm, v = V - xm;
+    x = xm + dc_quadratic(cmid, fma(cmid, M - xm, wh), u * v * fmid, true);
+    if (!positive(cmid)) x = xm;
   } else {
-    const double c = fmid - zzj * rcp_nr(P[j] - xma) - zzj1 * rcp_nr(P[j + 1] - xma);
-    x = dc_quad_root(c, P1, P2, zzj, zzj1);
+    x = dc_quadratic(cmid, fma(cmid, M, wh), fma(cmid, U * V, fma(w0, V, w1 * U)), false);
   }
-  if (!(lo < x && x < hi)) x = xm;
-  // the poles of the model: (j, j+1) inside, (j-1, j) for the largest root
-  const int m0 = two_below ? j - 1 : j;
-  const int m1 = last ? j : j + 1;
+  if (!(less_than(lo, x) && less_than(x, hi))) x = xm;
   bool conv = false;
+  const double eps_mk = DBL_EPSILON * mk;
   for (int it = 0; it < kSecularMaxIt; ++it) {
-    // the rest of the sum (poles below contribute t < 0, above t > 0), its
-    // derivative and its absolute sum
-    double rs = 0.0, drs = 0.0, ab = 0.0;
-    for (int i = sub; i < mk; i += G) {
-      const double inv = rcp_nr((P[i] - base) - x);
-      double t = ZZ[i] * inv;
-      t = (i >= m0 && i <= m1) ? 0.0 : t;
-      rs += t;
-      drs = fma(t, inv, drs);
-      ab += fabs(t);
-    }
-    rs = group_sum<G>(rs, gm);
-    drs = group_sum<G>(drs, gm);
-    ab = group_sum<G>(ab, gm);
-    const double A = P1 - x;
-    const double B = P2 - x;
-    const double A0 = P0 - x;
-    const double tj = zzj * rcp_nr(A);
-    const double tj1 = last ? 0.0 : zzj1 * rcp_nr(B);
-    const double tjm = two_below ? zzjm * rcp_nr(A0) : 0.0;
-    const double f = ir + rs + tj + tj1 + tjm;
-    const double sab = ab + fabs(tj) + fabs(tj1) + fabs(tjm);
-    if (f > 0.0)
+    pass(base, x);
+    const double c0 = ir + (below + above);
+    const double f = c0 + (t0 + t1);
+    if (positive(f))
       hi = x;
     else
       lo = x;
-    if (fabs(f) <= DBL_EPSILON * mk * (ir + sab) ||
-        hi - lo <= 2.0 * DBL_EPSILON * fmax(fabs(lo), fabs(hi))) {
+    // |f| within the rounding of its terms
+    const double mag = (ir + (above - below)) + (fabs(t0) + fabs(t1));
+    if (!less_than(eps_mk * mag, fabs(f))) {
       conv = true;
       break;
     }
-    double eta;
-    if (last && mk == 1) {
-      eta = A + zzj * rho;
-    } else if (last) {
-      const double c = ir + rs - drs * A0;
-      eta = c > 0.0 ? dc_quad_step_right(c, A0, A, zzjm + drs * A0 * A0, zzj, f) : nan("");
-    } else {
-      eta = (o == j) ? dc_quad_step(ir + rs - drs * B, A, B, zzj, zzj1 + drs * B * B, f)
-                     : dc_quad_step(ir + rs - drs * A, A, B, zzj + drs * A * A, zzj1, f);
-    }
-    if (fabs(eta) <= 2.0 * DBL_EPSILON * fabs(x)) {
+    // the rest's derivative goes to the pole E that is not the origin
+    const double u = U - x, v = V - x;
+    const double E = (last || o != j) ? u : v, se = slope * E;
+    const double c = c0 - se;
+    const double eta = dc_quadratic(c, fma(c, M - x, fma(se, 0.5 * E, wh)), u * v * f, last);
+    if (!less_than(2.0 * DBL_EPSILON * fabs(x), fabs(eta))) {
       conv = true;
       break;
     }
     double xn = x + eta;
-    if (!(lo < xn && xn < hi)) xn = 0.5 * (lo + hi);  // also catches a NaN step
+    if (!(less_than(lo, xn) && less_than(xn, hi)) || (last && !positive(c))) {  // also a NaN step
+      xn = 0.5 * (lo + hi);
+      if (hi - lo <= 2.0 * DBL_EPSILON * fmax(fabs(lo), fabs(hi))) {
+        conv = true;
+        break;
+      }
+    }
     x = xn;
   }
   x_out = x;
@@ -526,25 +541,86 @@ struct DcArrays {
   int *O, *MS;
 };
 constexpr int kFlipBit = 1 << 30;   // in MS: the merge was negated
-constexpr int kDcNarrow = 16;       // merges up to this size: one lane per root
+
+// Phase A of one level where nothing deflates, on all threads: the merged
+// position of each element of the two halves by binary search in the other half,
+// its value, weight and rows written there.  A merge with a negligible weight or
+// two close poles gets MS[q] = -1 and is left to the serial scan.  kVec: the
+// weights come from the eigenvector columns S, and CI keeps each pole's column.
+template <bool kVec>
+__device__ void dc_sorted_merge(const DcArrays &Ar, const double *LAM, const double *FR, const double *LR,
+                                const double *EO, const double *S, int *CI, int k, int s, int nm, double *RH,
+                                double *UB) {
+  const int w = 1 << s;
+  int *MS = Ar.MS;
+  for (int q = threadIdx.x; q < nm; q += blockDim.x) MS[q] = 0;
+  for (int r = threadIdx.x; r < k; r += blockDim.x) {
+    const int q = r >> (s + 1);
+    if (q >= nm) continue;
+    const int a = q * 2 * w, mid = a + w, hi = min(a + 2 * w, k);
+    const bool flip = EO[mid - 1] < 0.0, first = r < mid;
+    // order within the half, and in the other half the count of values below
+    // (first half: strictly; equal values of the first half come first)
+    const int own = flip ? (first ? mid - 1 - r : hi - 1 - r) : (first ? r - a : r - mid);
+    const double v = flip ? -LAM[r] : LAM[r];
+    const long long key = order_key(v);
+    int lo = 0, up = first ? hi - mid : w;
+    while (lo < up) {
+      const int c = (lo + up) >> 1;
+      const int i = first ? (flip ? hi - 1 - c : mid + c) : (flip ? mid - 1 - c : a + c);
+      const long long other = order_key(flip ? -LAM[i] : LAM[i]);
+      if (first ? other < key : other <= key)
+        lo = c + 1;
+      else
+        up = c;
+    }
+    const int pos = a + own + lo;
+    const double z = kVec ? S[(size_t)r * k + (first ? mid - 1 : mid)] : (first ? LR[r] : FR[r]);
+    Ar.D[pos] = v;
+    Ar.Z[pos] = z;
+    Ar.NF[pos] = z * z;
+    if (kVec) {
+      CI[pos] = r;
+    } else {
+      Ar.F[pos] = first ? FR[r] : 0.0;
+      Ar.L[pos] = first ? 0.0 : LR[r];
+    }
+  }
+  __syncthreads();
+  for (int r = threadIdx.x; r < k; r += blockDim.x) {
+    const int q = r >> (s + 1);
+    if (q >= nm) continue;
+    const int a = q * 2 * w, mid = a + w, hi = min(a + 2 * w, k);
+    const double rho = fabs(EO[mid - 1]);
+    const double maxabs = fmax(fabs(Ar.D[a]), fabs(Ar.D[hi - 1]));  // of the sorted values
+    const double tol = 8.0 * DBL_EPSILON * fmax(maxabs, 2.0 * rho);
+    const double d = Ar.D[r];
+    if (!(rho * fabs(Ar.Z[r]) > tol) || (r > a && !(d - Ar.D[r - 1] > tol))) MS[q] = -1;
+    if (r == hi - 1) {
+      RH[q] = rho;
+      // the weights are two unit rows: the largest root lies below d + 2 rho
+      UB[q] = d + 2.0 * rho * (1.0 + 1e-12) + 16.0 * DBL_EPSILON * fabs(d);
+    }
+  }
+  __syncthreads();
+}
 
 // Phases B-D of one level (merges of width 2^(s+1)): the secular roots, the
-// Loewner zhat and the new first/last rows, one group of G lanes per root.
+// Loewner zhat and the new first/last rows, G lanes per root.
 // kVec: instead of new first/last rows, the normalised coefficients u of
 // each root's vector in the kept poles' columns, U[r * k + i] (r the root's
 // index in the problem, i < mk).
-template <int G, bool kVec = false>
-__device__ bool dc_merge_roots(const DcArrays &Ar, int k, int s, int nm, double *U = nullptr) {
+template <int G, bool kVec>
+__device__ bool dc_merge_roots(const DcArrays &Ar, int k, int s, int nm, double *U) {
   double *D = Ar.D, *Z = Ar.Z, *F = Ar.F, *L = Ar.L, *X = Ar.X, *NF = Ar.NF, *NL = Ar.NL;
   const double *RH = Ar.RH, *UB = Ar.UB;
   int *O = Ar.O;
   const int *MS = Ar.MS;
-  const int tid = threadIdx.x;
-  const int sub = tid & (G - 1);
-  const int grp = tid / G, ngrp = (int)blockDim.x / G;
-  const unsigned gm = (G == 1 ? 1u : (1u << G) - 1u) << (tid & 31 & ~(G - 1));
+  const int sub = threadIdx.x & (G - 1);
+  const int grp = threadIdx.x / G, ngrp = (int)blockDim.x / G;
+  const unsigned gm = (G == 1 ? 1u : (1u << G) - 1u) << (threadIdx.x & 31 & ~(G - 1));
   bool ok = true;
-  // B: secular roots, one group per root over all merges of the level
+  // B: secular roots over all merges of the level
   for (int r = grp; r < k; r += ngrp) {
     const int q = r >> (s + 1);
     if (q >= nm) continue;
@@ -572,9 +648,12 @@ __device__ bool dc_merge_roots(const DcArrays &Ar, int k, int s, int nm, double 
     if (i >= mk) continue;
     const double *P = D + a;
     const double di = P[i];
-    double prod = sub == 0 ? ((P[O[a + mk - 1]] - di) + X[a + mk - 1]) / RH[q] : 1.0;
-    for (int j = sub; j < mk - 1; j += G)
-      prod *= ((P[O[a + j]] - di) + X[a + j]) * rcp_nr(P[j < i ? j : j + 1] - di);
+    double prod = 1.0;
+    for (int j = sub; j < mk; j += G) {
+      // factor j, the last one with rho in place of a pole's distance
+      const double den = j + 1 < mk ? P[j < i ? j : j + 1] - di : RH[q];
+      prod *= ((P[O[a + j]] - di) + X[a + j]) * (j + 1 < mk ? rcp_nr(den) : rcp_any(den));
+    }
     prod = group_prod<G>(prod, gm);
     if (sub == 0) Z[r] = copysign(sqrt(fmax(prod, 0.0)), Z[r]);
   }
@@ -598,11 +677,10 @@ __device__ bool dc_merge_roots(const DcArrays &Ar, int k, int s, int nm, double 
         sl = fma(L[a + i], u, sl);
       }
     }
-    s2 = group_sum<G>(s2, gm);  // in every lane of the group
+    s2 = group_sum<G>(s2, gm);
     const double rn = rsqrt(s2);
     if (kVec) {
-      for (int i = sub; i < mk; i += G)
-        U[(size_t)r * k + i] = Z[a + i] * rcp_nr((P[i] - ox) - x) * rn;
+      for (int i = sub; i < mk; i += G) U[(size_t)r * k + i] = Z[a + i] * rcp_nr((P[i] - ox) - x) * rn;
     } else {
       sf = group_sum<G>(sf, gm);
       sl = group_sum<G>(sl, gm);
@@ -619,8 +697,50 @@ __device__ bool dc_merge_roots(const DcArrays &Ar, int k, int s, int nm, double 
   return ok;
 }
 
+// Lanes per root for p problems of size k: a pass over the poles costs a warp
+// about 8 k / G + 3 log2 G + 29 float64 instructions of 64 clocks, and the SM's
+// warps share one such instruction per 19 clocks; a warp of more roots waits for
+// the slowest of more of them, which other warps hide where an SM has several
+// problems.  Measured: k = 16, 32 problems 252 us with one lane per root -> 98 us
+// (8); k = 32, 64: 320 -> 146 (4); k = 40, 48: 281 with 2, 219 with 4; k = 64, 256:
+// 866 -> 552 (2; with 1 654); k = 96, 32: 919 with 1, 639 with 4; k = 64, 1000: 2806 ->
+// 1593 (1).
+static int dc_group(int64_t k, int64_t p) {
+  static int sms = 0;
+  if (sms == 0) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+      sms = 152;
+  }
+  int best = 1;
+  double best_clk = 1e300;
+  for (int G = 1, lg = 0; G <= 8; G *= 2, ++lg) {
+    if (k * G > kDcMaxThreads && G > 1) break;
+    const double per_sm = p > sms ? (double)p / sms : 1.0;
+    const double share = 19.2 * (double)ceil_div(k * G, 32) * per_sm;
+    const double wait = 9.0 - (per_sm > 2.0 ? 0.0 : (per_sm > 1.0 ? 0.6 : 1.0)) * lg;
+    const double clk = (8.0 * k / G + 3.0 * lg + 29.0) * (share > 64.0 ? share : 64.0) * wait;
+    if (clk < best_clk) {
+      best_clk = clk;
+      best = G;
+    }
+  }
+  return best;
+}
+
+template <bool kVec>
+__device__ bool dc_merge_level(int G, const DcArrays &Ar, int k, int s, int nm, double *U = nullptr) {
+  switch (G) {
+    case 8: return dc_merge_roots<8, kVec>(Ar, k, s, nm, U);
+    case 4: return dc_merge_roots<4, kVec>(Ar, k, s, nm, U);
+    case 2: return dc_merge_roots<2, kVec>(Ar, k, s, nm, U);
+    default: return dc_merge_roots<1, kVec>(Ar, k, s, nm, U);
+  }
+}
+
 __global__ void __launch_bounds__(kDcMaxThreads, 1)
-    tridiag_dc_kernel(int k, int64_t p, const double *__restrict__ H, int fun, double param,
+    tridiag_dc_kernel(int k, int64_t p, int G, const double *__restrict__ H, int fun, double param,
                       const double *__restrict__ scale, double *__restrict__ values,
                       double *__restrict__ eigvals, double *__restrict__ first_sq,
                       int *__restrict__ status) {
@@ -660,11 +780,17 @@ __global__ void __launch_bounds__(kDcMaxThreads, 1)
   for (int s = 0; (1 << s) < k; ++s) {
     const int w = 1 << s;
     const int nm = (k - w - 1) / (2 * w) + 1;
-    // A: sorted merge of the two halves and deflation, one thread per merge
+    // A: sorted merge of the two halves, and deflation by one thread per merge that
+    // has any (a merge of 32 took that thread 31000 clocks, all threads 2000)
+    dc_sorted_merge<false>(Ar, LAM, FR, LR, EO, nullptr, nullptr, k, s, nm, RH, UB);
     for (int q = tid; q < nm; q += nt) {
       const int a = q * 2 * w, mid = a + w, hi = min(a + 2 * w, k);
       double rho = EO[mid - 1];
       const bool flip = rho < 0.0;
+      if (MS[q] == 0) {
+        MS[q] = (hi - a) | (flip ? kFlipBit : 0);
+        continue;
+      }
       const double sg = flip ? -1.0 : 1.0;
       rho = fabs(rho);
       const double maxabs = fmax(fmax(fabs(LAM[a]), fabs(LAM[mid - 1])),
@@ -760,12 +886,24 @@ __global__ void __launch_bounds__(kDcMaxThreads, 1)
                      : 0.0;
     }
     __syncthreads();
-    ok &= (2 << s) > kDcNarrow ? dc_merge_roots<4>(Ar, k, s, nm) : dc_merge_roots<1>(Ar, k, s, nm);
+    ok &= dc_merge_level<false>(G, Ar, k, s, nm);
     // E: merge the roots [a, a+mk) with the dropped poles [a+mk, hi), both
     // ascending; a negated merge is negated back and reversed
+    for (int r = tid; r < k; r += nt) {  // merges without dropped poles
+      const int q = r >> (s + 1);
+      if (q >= nm) continue;
+      const int a = q * 2 * w, hi = min(a + 2 * w, k);
+      if ((MS[q] & (kFlipBit - 1)) != hi - a) continue;
+      const bool flip = (MS[q] & kFlipBit) != 0;
+      const int pos = flip ? hi - 1 - (r - a) : r;
+      LAM[pos] = flip ? -X[r] : X[r];
+      FR[pos] = NF[r];
+      LR[pos] = NL[r];
+    }
     for (int q = tid; q < nm; q += nt) {
       const int a = q * 2 * w, hi = min(a + 2 * w, k);
       const int mk = MS[q] & (kFlipBit - 1);
+      if (mk == hi - a) continue;
       const bool flip = (MS[q] & kFlipBit) != 0;
       const double sg = flip ? -1.0 : 1.0;
       int c1 = a, c2 = a + mk;
@@ -849,7 +987,7 @@ __host__ inline size_t dcv_smem_bytes(int k) {
 }
 
 __global__ void __launch_bounds__(kDcMaxThreads, 1)
-    tridiag_dcv_kernel(int k, int64_t p, const double *__restrict__ H, double *__restrict__ w_out,
+    tridiag_dcv_kernel(int k, int64_t p, int G, const double *__restrict__ H, double *__restrict__ w_out,
                        double *__restrict__ S_out, int *__restrict__ status) {
   extern __shared__ double sm[];
   const int tid = threadIdx.x;
@@ -890,10 +1028,15 @@ __global__ void __launch_bounds__(kDcMaxThreads, 1)
     const int span = 2 * w;
     const int nm = (k - w - 1) / span + 1;
     // A
+    dc_sorted_merge<true>(Ar, LAM, nullptr, nullptr, EO, S, CI, k, s, nm, RH, UB);
     for (int q = tid; q < nm; q += nt) {
       const int a = q * span, mid = a + w, hi = min(a + span, k);
       double rho = EO[mid - 1];
       const bool flip = rho < 0.0;
+      if (MS[q] == 0) {
+        MS[q] = (hi - a) | (flip ? kFlipBit : 0);
+        continue;
+      }
       const double sg = flip ? -1.0 : 1.0;
       rho = fabs(rho);
       const double maxabs = fmax(fmax(fabs(LAM[a]), fabs(LAM[mid - 1])),
@@ -984,8 +1127,7 @@ __global__ void __launch_bounds__(kDcMaxThreads, 1)
                      : 0.0;
     }
     __syncthreads();
-    ok &= span > kDcNarrow ? dc_merge_roots<4, true>(Ar, k, s, nm, U)
-                           : dc_merge_roots<1, true>(Ar, k, s, nm, U);
+    ok &= dc_merge_level<true>(G, Ar, k, s, nm, U);
     // D': the merged columns into S2 (rows a..hi-1)
     for (int idx = tid; idx < nm * span * span; idx += nt) {
       const int q = idx / (span * span);
@@ -1006,9 +1148,20 @@ __global__ void __launch_bounds__(kDcMaxThreads, 1)
     }
     // E: ascending merge of the roots [a, a+mk) and the dropped poles
     // [a+mk, hi); a negated merge is negated back and reversed
+    for (int r = tid; r < k; r += nt) {  // merges without dropped poles
+      const int q = r >> (s + 1);
+      if (q >= nm) continue;
+      const int a = q * span, hi = min(a + span, k);
+      if ((MS[q] & (kFlipBit - 1)) != hi - a) continue;
+      const bool flip = (MS[q] & kFlipBit) != 0;
+      const int pos = flip ? hi - 1 - (r - a) : r;
+      LAM[pos] = flip ? -X[r] : X[r];
+      O[pos] = r;
+    }
     for (int q = tid; q < nm; q += nt) {
       const int a = q * span, hi = min(a + span, k);
       const int mk = MS[q] & (kFlipBit - 1);
+      if (mk == hi - a) continue;
       const bool flip = (MS[q] & kFlipBit) != 0;
       const double sg = flip ? -1.0 : 1.0;
       int c1 = a, c2 = a + mk;
@@ -1054,13 +1207,15 @@ int launch_tridiag_quadrature(int64_t k, int64_t p, const double *H, int32_t fun
                               double *first_sq, int *status, cudaStream_t s) {
   if (p <= 0 || k <= 0) return MFG_OK;
   if (k >= kDcMinK && k <= kDcMaxK) {
-    // one problem per CTA, a quad of lanes per root: 4k threads up to 512
+    // one problem per CTA, G lanes per root, up to 512 threads
     const size_t smem = dc_layout((int)k).words * sizeof(double);
     if (smem > 48 * 1024)
       MFG_CUDA_TRY(cudaFuncSetAttribute(tridiag_dc_kernel,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const int threads = (int)(k >= kDcMaxThreads / 4 ? kDcMaxThreads : (4 * k + 31) / 32 * 32);
-    tridiag_dc_kernel<<<(unsigned)p, threads, smem, s>>>((int)k, p, H, fun, param, scale, values,
+    const int G = dc_group(k, p);
+    const int64_t want = (k * G + 31) / 32 * 32;
+    const int threads = (int)(want < kDcMaxThreads ? want : kDcMaxThreads);
+    tridiag_dc_kernel<<<(unsigned)p, threads, smem, s>>>((int)k, p, G, H, fun, param, scale, values,
                                                         eigvals, first_sq, status);
     return MFG_LAUNCH_STATUS();
   }
@@ -1131,8 +1286,10 @@ int launch_tridiag_eigh_full(int64_t k, int64_t p, const double *H, double *w, d
     const size_t smem = dcv_smem_bytes((int)k);
     MFG_CUDA_TRY(cudaFuncSetAttribute(tridiag_dcv_kernel,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const int threads = (int)((4 * k + 31) / 32 * 32);
-    tridiag_dcv_kernel<<<(unsigned)p, threads, smem, s>>>((int)k, p, H, w, S, status);
+    const int G = dc_group(k, p);
+    const int64_t want = k * G;  // at least 4 k threads for the merged columns
+    const int threads = (int)(((want > 4 * k ? want : 4 * k) + 31) / 32 * 32);
+    tridiag_dcv_kernel<<<(unsigned)p, threads, smem, s>>>((int)k, p, G, H, w, S, status);
     return MFG_LAUNCH_STATUS();
   }
   return launch_tridiag_eigh_ql(k, p, H, w, S, Z, status, s);
