@@ -1,4 +1,4 @@
-// Operator kernels on CUDA cores: dense W = A V (float32 / float64), CSR
+// Operator kernels: dense W = A V in float32 / float64, CSR
 // SpMM, and builders of the dense RBF kernel matrix and its bf16 split.
 #include "common.cuh"
 #include "kernels.cuh"
@@ -6,146 +6,226 @@
 namespace mfg {
 
 // ---------------------------------------------------------------------------
-// Dense W[b][m] = sum_k A[m][k] V[b][k] + shift V[b][m]  (CUDA cores)
+// Dense W[b][m] = sum_k A[m][k] V[b][k] + shift V[b][m] in float32 (FMA pipes)
+// and float64 (m8n8k4 MMAs).
 //
-// CTA tile: BM rows of A x BP probes, K in steps of BK staged through shared
-// memory (A tile stored k-major so each thread reads its TM contiguous rows
-// with 16-byte loads).  Global loads of the next K step are issued before
-// the FMAs of the current one (register double buffering).
+// A CTA forms a tile of BM rows x BP probes over one of S equal ranges of K, a
+// cluster of S CTAs covers K and adds its partial tiles over distributed shared
+// memory in rank order (small operators have too few tiles for the GPU; n = 2000,
+// 64 probes: 32 tiles).  Both operands are K-major; slices of BK columns go to
+// shared memory as they are (cp.async, three stages, rows padded by 16 bytes so
+// that 16-byte reads of neighbouring rows fall into different banks).
 // ---------------------------------------------------------------------------
 
-template <typename T> struct SimtCfg;
-template <> struct SimtCfg<float> {
-  static constexpr int BM = 128, BP = 64, BK = 16, TM = 8, TP = 4;
-};
-template <> struct SimtCfg<double> {
-  static constexpr int BM = 128, BP = 64, BK = 8, TM = 8, TP = 4;
-};
-// Small tiles for operators whose large-tile grid would not fill the GPU
-// (e.g. n = 1000, p = 100: 16 CTAs of 128 x 64 against 128 of 32 x 32).
-template <typename T> struct SimtCfgSmall;
-template <> struct SimtCfgSmall<float> {
-  static constexpr int BM = 32, BP = 32, BK = 32, TM = 2, TP = 2;
-};
-template <> struct SimtCfgSmall<double> {
-  static constexpr int BM = 32, BP = 32, BK = 16, TM = 2, TP = 2;
-};
+constexpr int kDStages = 3;
+constexpr int kDMaxS = 8;
 
-template <typename T, typename C>
+__device__ __forceinline__ uint32_t d_smem(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+// 16 bytes to shared memory, the first `bytes` of them from global memory, the rest zero
+__device__ __forceinline__ void cp_async16(void *dst, const void *src, int bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d_smem(dst)), "l"(src), "r"(bytes) : "memory");
+}
+
+__device__ __forceinline__ void d_cluster_sync() {
+  __syncthreads();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+template <typename T>
+__device__ __forceinline__ T d_load_rank(const T *local, int rank) {
+  uint32_t at;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(d_smem(local)), "r"(rank));
+  T v;
+  if constexpr (sizeof(T) == 4)
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(at) : "memory");
+  else
+    asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(at) : "memory");
+  return v;
+}
+
+// Slices [kb, ke) of BK columns of A's rows m0.. and V's probes b0.. through the
+// stages; body(As, Vs) consumes one.  Columns past n, rows past n and probes past
+// p read as zero.
+template <typename T, int BM, int BP, int BK, int THREADS, typename F>
+__device__ __forceinline__ void d_pipeline(T *stages, const T *__restrict__ A, int64_t lda, const T *__restrict__ V,
+                                           int64_t ldv, int64_t n, int64_t p, int64_t m0, int64_t b0, int64_t kb,
+                                           int64_t ke, F body) {
+  constexpr int VW = Vec<T>::width, LD = BK + VW, PER = BK / VW;
+  constexpr int64_t kStage = (int64_t)(BM + BP) * LD;
+  auto load = [&](int64_t slice) {
+    if (slice < ke) {
+      T *st = stages + (slice - kb) % kDStages * kStage;
+      for (int i = threadIdx.x; i < (BM + BP) * PER; i += THREADS) {
+        const int r = i / PER, c = i % PER * VW;
+        const int64_t k = slice * BK + c;
+        const bool isA = r < BM;
+        const int64_t row = isA ? m0 + r : b0 + (r - BM);
+        const int64_t left = row < (isA ? n : p) ? n - k : 0;
+        const int bytes = left >= VW ? 16 : (left > 0 ? (int)(left * sizeof(T)) : 0);
+        const T *src = bytes ? (isA ? A + row * lda : V + row * ldv) + k : A;
+        cp_async16(st + (int64_t)r * LD + c, src, bytes);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll
+  for (int s = 0; s < kDStages - 1; ++s) load(kb + s);
+  for (int64_t slice = kb; slice < ke; ++slice) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kDStages - 2) : "memory");
+    __syncthreads();  // this slice has landed, and the stage loaded next is no longer read
+    load(slice + kDStages - 1);
+    const T *st = stages + (slice - kb) % kDStages * kStage;
+    body(st, st + (int64_t)BM * LD);
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+}
+
+// The cluster's partial tiles part[BP][BM] into W, this CTA's share of the probes.
+template <typename T, int BM, int BP, int THREADS>
+__device__ __forceinline__ void d_reduce_store(const T *part, const T *__restrict__ V, int64_t ldv, T *__restrict__ W,
+                                               int64_t ldw, int64_t n, int64_t p, int64_t m0, int64_t b0, int rank,
+                                               int S, T shift) {
+  d_cluster_sync();
+  const int c0 = BP * rank / S, c1 = BP * (rank + 1) / S;
+  for (int i = threadIdx.x; i < (c1 - c0) * BM; i += THREADS) {
+    const int c = c0 + i / BM, r = i % BM;
+    const int64_t m = m0 + r, b = b0 + c;
+    if (m >= n || b >= p) continue;
+    T x[kDMaxS];
+#pragma unroll
+    for (int q = 0; q < kDMaxS; ++q) x[q] = q < S ? d_load_rank(part + c * BM + r, q) : (T)0;
+    T sum = x[0];
+#pragma unroll
+    for (int q = 1; q < kDMaxS; ++q)
+      if (q < S) sum += x[q];
+    W[b * ldw + m] = fma(shift, __ldg(V + b * ldv + m), sum);
+  }
+  d_cluster_sync();
+}
+
+// float32: 256 threads, TM x TP outputs each, rows tx + i BM / TM and probes ty + j
+// BP / TP; four columns at a time from 16-byte reads, 8 of them for 64 FMAs.  Bound by
+// the FMA pipes and, for small operators, by too few tiles.  Against 32 x 32 and
+// 128 x 64 tiles staged through registers: n = 2000, 64 probes 54 -> 27 us; n = 512, 32
+// 17 -> 7; n = 4096, 256 598 -> 279 (31 TFLOP/s); n = 16384, 256 5.84 -> 4.18 ms.
+template <int BM, int BP, int TM, int TP>
 __global__ void __launch_bounds__(256)
-dense_simt_kernel(const T *__restrict__ A, int64_t lda, const T *__restrict__ V, int64_t ldv,
-                  T *__restrict__ W, int64_t ldw, int64_t n, int64_t p, T shift) {
-  constexpr int BM = C::BM, BP = C::BP, BK = C::BK, TM = C::TM, TP = C::TP;
-  constexpr int VW = Vec<T>::width;
-  using VT = typename Vec<T>::type;
-  constexpr int A_VECS = BM * BK / VW / 256;  // 16-byte loads per thread for the A tile
-  constexpr int V_VECS = BP * BK / VW / 256;
-  static_assert(A_VECS >= 1 && V_VECS >= 1, "tile too small for 256 threads");
-  static_assert((BM / TM) * (BP / TP) == 256, "thread layout");
-  __shared__ __align__(16) T As[BK][BM];
-  __shared__ __align__(16) T Vs[BK][BP];
-
-  const int t = threadIdx.x;
-  const int tx = t % (BM / TM);  // row group
-  const int ty = t / (BM / TM);  // probe group
-  const int64_t m0 = (int64_t)blockIdx.x * BM;
-  const int64_t b0 = (int64_t)blockIdx.y * BP;
-
-  T acc[TM][TP];
+dense_f32_kernel(const float *__restrict__ A, int64_t lda, const float *__restrict__ V, int64_t ldv,
+                 float *__restrict__ W, int64_t ldw, int64_t n, int64_t p, float shift) {
+  constexpr int BK = 32, LD = BK + 4, RX = BM / TM, RY = BP / TP;
+  static_assert(RX * RY == 256, "thread layout");
+  extern __shared__ __align__(16) uint8_t d_raw[];
+  float *stages = reinterpret_cast<float *>(d_raw);
+  const int S = (int)gridDim.x, rank = (int)blockIdx.x;
+  const int64_t m0 = (int64_t)blockIdx.y * BM, b0 = (int64_t)blockIdx.z * BP;
+  const int64_t slices = (n + BK - 1) / BK;
+  const int tx = threadIdx.x % RX, ty = threadIdx.x / RX;
+  float acc[TM][TP];
 #pragma unroll
   for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int j = 0; j < TP; ++j) acc[i][j] = (T)0;
+    for (int j = 0; j < TP; ++j) acc[i][j] = 0.f;
+  d_pipeline<float, BM, BP, BK, 256>(
+      stages, A, lda, V, ldv, n, p, m0, b0, slices * rank / S, slices * (rank + 1) / S,
+      [&](const float *As, const float *Vs) {
+#pragma unroll
+        for (int k = 0; k < BK; k += 4) {
+          float a[TM][4], v[TP][4];
+#pragma unroll
+          for (int i = 0; i < TM; ++i) vec_to_array<float>(*reinterpret_cast<const float4 *>(As + (tx + i * RX) * LD + k), a[i]);
+#pragma unroll
+          for (int j = 0; j < TP; ++j) vec_to_array<float>(*reinterpret_cast<const float4 *>(Vs + (ty + j * RY) * LD + k), v[j]);
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int i = 0; i < TM; ++i)
+#pragma unroll
+              for (int j = 0; j < TP; ++j) acc[i][j] = fmaf(a[i][u], v[j][u], acc[i][j]);
+        }
+      });
+#pragma unroll
+  for (int j = 0; j < TP; ++j)
+#pragma unroll
+    for (int i = 0; i < TM; ++i) stages[(ty + j * RY) * BM + tx + i * RX] = acc[i][j];
+  d_reduce_store<float, BM, BP, 256>(stages, V, ldv, W, ldw, n, p, m0, b0, rank, S, shift);
+}
 
-  T ra[A_VECS][VW], rv[V_VECS][VW];
-  auto gload = [&](int64_t k0) {
-#pragma unroll
-    for (int e = 0; e < A_VECS; ++e) {
-      const int f = t + e * 256;
-      const int row = f / (BK / VW), kq = (f % (BK / VW)) * VW;
-      const int64_t m = m0 + row, kk = k0 + kq;
-      if (m < n && kk + VW <= n) {
-        vec_to_array<T>(__ldg(reinterpret_cast<const VT *>(A + m * lda + kk)), ra[e]);
-      } else {
-#pragma unroll
-        for (int u = 0; u < VW; ++u) ra[e][u] = (m < n && kk + u < n) ? A[m * lda + kk + u] : (T)0;
-      }
-    }
-#pragma unroll
-    for (int e = 0; e < V_VECS; ++e) {
-      const int f = t + e * 256;
-      const int pb = f / (BK / VW), kq = (f % (BK / VW)) * VW;
-      const int64_t b = b0 + pb, kk = k0 + kq;
-      if (b < p && kk + VW <= n) {
-        vec_to_array<T>(__ldg(reinterpret_cast<const VT *>(V + b * ldv + kk)), rv[e]);
-      } else {
-#pragma unroll
-        for (int u = 0; u < VW; ++u) rv[e][u] = (b < p && kk + u < n) ? V[b * ldv + kk + u] : (T)0;
-      }
-    }
-  };
-  auto sstore = [&]() {
-#pragma unroll
-    for (int e = 0; e < A_VECS; ++e) {
-      const int f = t + e * 256;
-      const int row = f / (BK / VW), kq = (f % (BK / VW)) * VW;
-#pragma unroll
-      for (int u = 0; u < VW; ++u) As[kq + u][row] = ra[e][u];
-    }
-#pragma unroll
-    for (int e = 0; e < V_VECS; ++e) {
-      const int f = t + e * 256;
-      const int pb = f / (BK / VW), kq = (f % (BK / VW)) * VW;
-#pragma unroll
-      for (int u = 0; u < VW; ++u) Vs[kq + u][pb] = rv[e][u];
-    }
-  };
+// float64: four warps, warp w the probes 8 w .. 8 w + 7 of the tile, its rows as M / 8
+// m8n8k4 MMAs.  An SM runs 1.76 float64 FMAs a clock as MMAs and 1.68 as FMA
+// instructions (measured), whatever a warp's independent chains, so tiles are small
+// and many: up to five CTAs share an SM's pipe, MMAs past the last row or probe are
+// left out, and no operand is reused in registers.  Against 32 x 32 tiles of FMA
+// instructions on one CTA each: n = 1000, 100 probes 272 -> 242 us (0.83 TFLOP/s, 0.80 of
+// that rate); n = 1500, 100 785 -> 480; n = 700, 37 193 -> 57; n = 200, 16 60 -> 11.
+constexpr int kF64M = 16, kF64P = 32, kF64K = 32;
 
-  gload(0);
-  for (int64_t k0 = 0; k0 < n; k0 += BK) {
-    __syncthreads();
-    sstore();
-    __syncthreads();
-    if (k0 + BK < n) gload(k0 + BK);
+__global__ void __launch_bounds__(128)
+dense_f64_kernel(const double *__restrict__ A, int64_t lda, const double *__restrict__ V, int64_t ldv,
+                 double *__restrict__ W, int64_t ldw, int64_t n, int64_t p, double shift) {
+  constexpr int M = kF64M, LD = kF64K + 2, kRows = M / 8;
+  extern __shared__ __align__(16) uint8_t d_raw[];
+  double *stages = reinterpret_cast<double *>(d_raw);
+  const int S = (int)gridDim.x, rank = (int)blockIdx.x;
+  const int64_t m0 = (int64_t)blockIdx.y * M, b0 = (int64_t)blockIdx.z * kF64P;
+  const int64_t slices = (n + kF64K - 1) / kF64K;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int fr = lane >> 2, fk = lane & 3;  // fragment row (A) or probe (V), and column
+  // warp-uniform: MMAs of 8 rows with any row and probe in range
+  const int live = b0 + warp * 8 < p ? (int)(n - m0 < M ? (n - m0 + 7) / 8 : kRows) : 0;
+  double c[kRows][2];
 #pragma unroll
-    for (int kk = 0; kk < BK; ++kk) {
-      T a[TM], v[TP];
-      if constexpr (TM % VW == 0 && TP % VW == 0) {
+  for (int i = 0; i < kRows; ++i) c[i][0] = c[i][1] = 0.0;
+  d_pipeline<double, M, kF64P, kF64K, 128>(
+      stages, A, lda, V, ldv, n, p, m0, b0, slices * rank / S, slices * (rank + 1) / S,
+      [&](const double *As, const double *Vs) {
+        if (live == 0) return;
+        const double *a = As + fr * LD + fk, *v = Vs + (warp * 8 + fr) * LD + fk;
 #pragma unroll
-        for (int i = 0; i < TM; i += VW) vec_to_array<T>(*reinterpret_cast<const VT *>(&As[kk][tx * TM + i]), a + i);
+        for (int k = 0; k < kF64K; k += 4) {
+          const double vb = v[k];
 #pragma unroll
-        for (int j = 0; j < TP; j += VW) vec_to_array<T>(*reinterpret_cast<const VT *>(&Vs[kk][ty * TP + j]), v + j);
-      } else {  // thread tiles narrower than a 16-byte vector
+          for (int i = 0; i < kRows; ++i)
+            if (i < live)
+              asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                           : "+d"(c[i][0]), "+d"(c[i][1])
+                           : "d"(a[i * 8 * LD + k]), "d"(vb));
+        }
+      });
 #pragma unroll
-        for (int i = 0; i < TM; ++i) a[i] = As[kk][tx * TM + i];
+  for (int i = 0; i < kRows; ++i)
 #pragma unroll
-        for (int j = 0; j < TP; ++j) v[j] = Vs[kk][ty * TP + j];
-      }
-#pragma unroll
-      for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TP; ++j) acc[i][j] = fma(a[i], v[j], acc[i][j]);
-    }
-  }
+    for (int e = 0; e < 2; ++e) stages[(warp * 8 + 2 * fk + e) * M + i * 8 + fr] = c[i][e];
+  d_reduce_store<double, M, kF64P, 128>(stages, V, ldv, W, ldw, n, p, m0, b0, rank, S, shift);
+}
 
-#pragma unroll
-  for (int j = 0; j < TP; ++j) {
-    const int64_t b = b0 + ty * TP + j;
-    if (b >= p) continue;
-    const int64_t mb = m0 + tx * TM;
-#pragma unroll
-    for (int i = 0; i < TM; ++i) {
-      const int64_t m = mb + i;
-      if (m < n) W[b * ldw + m] = fma(shift, V[b * ldv + m], acc[i][j]);
-    }
-  }
+template <typename K, typename T>
+static int launch_dense_cluster(K kern, int bm, int bp, int threads, size_t smem, int S, const T *A, int64_t lda,
+                                const T *V, int64_t ldv, T *W, int64_t ldw, int64_t n, int64_t p, T shift,
+                                cudaStream_t s) {
+  const int64_t gy = ceil_div(n, bm), gz = ceil_div(p, bp);
+  if (gy > 65535 || gz > 65535) return MFG_ERR_UNSUPPORTED;
+  MFG_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)S, (unsigned)gy, (unsigned)gz);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)S;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  MFG_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, A, lda, V, ldv, W, ldw, n, p, shift));
+  return MFG_LAUNCH_STATUS();
 }
 
 template <typename T>
 int launch_dense_simt(const T *A, int64_t lda, const T *V, int64_t ldv, T *W, int64_t ldw,
                       int64_t n, int64_t p, double shift, cudaStream_t s) {
-  using C = SimtCfg<T>;
-  using CS = SimtCfgSmall<T>;
   if (n <= 0 || p <= 0) return MFG_OK;
   static int sms = 0;
   if (sms == 0) {
@@ -154,18 +234,38 @@ int launch_dense_simt(const T *A, int64_t lda, const T *V, int64_t ldv, T *W, in
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
       sms = 152;
   }
-  const int64_t gx = ceil_div(n, C::BM), gy = ceil_div(p, C::BP);
-  if (gx * gy < sms) {
-    const int64_t sy = ceil_div(p, CS::BP);
-    if (sy > 65535) return MFG_ERR_UNSUPPORTED;
-    dim3 grid((unsigned)ceil_div(n, CS::BM), (unsigned)sy);
-    dense_simt_kernel<T, CS><<<grid, 256, 0, s>>>(A, lda, V, ldv, W, ldw, n, p, (T)shift);
-    return MFG_LAUNCH_STATUS();
+  if constexpr (sizeof(T) == 8) {
+    // the K ranges of least time: an SM's CTAs one after the other on its pipe (five
+    // at a time; past that a tail of two), slower with few of them to hide each
+    // other's waits; clusters of three leave SMs of a GPC over
+    const int64_t slices = ceil_div(n, kF64K), tiles = ceil_div(n, kF64M) * ceil_div(p, kF64P);
+    int S = 1;
+    double best = 1e300;
+    for (int c : {1, 2, 3, 4, 8}) {
+      if (c > slices) break;
+      const double ctas = (double)(tiles * c) / sms;
+      const double rounds = ctas <= 5.0 ? (double)ceil_div(tiles * c, sms) : ctas + 2.0;
+      const double cost = rounds * (double)(ceil_div(slices, c) + 1) * (1.0 + 0.25 / ctas) * (c == 3 ? 1.1 : 1.0);
+      if (cost < best) {
+        best = cost;
+        S = c;
+      }
+    }
+    const size_t smem = (size_t)kDStages * (kF64M + kF64P) * (kF64K + 2) * sizeof(double);
+    return launch_dense_cluster(dense_f64_kernel, kF64M, kF64P, 128, smem, S, A, lda, V, ldv, W, ldw, n, p, shift, s);
+  } else {
+    // four to eight K ranges of at least two slices (n = 2000, 64 probes: one range 104
+    // us, two 56, four 31, eight 27; n = 4096, 256: 330, 322, 279, 299)
+    const int bp = p <= 32 ? 32 : 64;
+    const int64_t tiles = ceil_div(n, 64) * ceil_div(p, bp), slices = ceil_div(n, 32);
+    int64_t S = ceil_div(4 * (int64_t)sms, tiles);
+    S = S < 4 ? 4 : (S > kDMaxS ? kDMaxS : S);
+    if (S > slices / 2) S = slices / 2;
+    if (S < 1) S = 1;
+    const size_t smem = (size_t)kDStages * (64 + bp) * 36 * sizeof(float);
+    return launch_dense_cluster(bp == 32 ? dense_f32_kernel<64, 32, 4, 2> : dense_f32_kernel<64, 64, 4, 4>, 64, bp, 256,
+                                smem, (int)S, A, lda, V, ldv, W, ldw, n, p, (float)shift, s);
   }
-  if (gy > 65535) return MFG_ERR_UNSUPPORTED;
-  dim3 grid((unsigned)gx, (unsigned)gy);
-  dense_simt_kernel<T, C><<<grid, 256, 0, s>>>(A, lda, V, ldv, W, ldw, n, p, (T)shift);
-  return MFG_LAUNCH_STATUS();
 }
 template int launch_dense_simt<float>(const float *, int64_t, const float *, int64_t, float *,
                                       int64_t, int64_t, int64_t, double, cudaStream_t);
