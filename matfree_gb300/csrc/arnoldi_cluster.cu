@@ -37,19 +37,12 @@
 // Waits are bounded; after a failure a CTA's warps run on without waiting or
 // computing, still meeting every barrier, and the copies in flight are drained.
 
-#include "common.cuh"
+#include "cluster.cuh"
 #include "kernels.cuh"
 
 namespace mfg {
 
-constexpr int kCWarps = 8;             // compute warps
-constexpr int kCThreads = 32 * kCWarps;
-constexpr int kCRows = 256;            // rows of a warp: 8 per lane
-constexpr int kCMaxSlots = 32;
 constexpr int kCMaxCols = kTwoSweepMaxK - 1;  // basis vectors of a step
-constexpr int kCMaxS = 16;
-constexpr size_t kCSmem = 112 * 1024;  // dynamic shared memory of a CTA: two per SM
-
 static_assert(kCMaxCols == 128, "shared arrays");
 
 struct CStepArgs {
@@ -67,117 +60,6 @@ struct CStepArgs {
   int *status;
 };
 
-__device__ __forceinline__ uint32_t c_smem(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ uint32_t c_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-
-__device__ __forceinline__ uint32_t c_map(uint32_t saddr, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
-  return r;
-}
-
-__device__ __forceinline__ double c_ld_f64(uint32_t addr) {
-  double v;
-  asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(addr) : "memory");
-  return v;
-}
-
-__device__ __forceinline__ void c_bulk(uint32_t dst, const float *src, uint32_t bytes, uint64_t *bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-               "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes), "r"(c_smem(bar))
-               : "memory");
-}
-
-__device__ __forceinline__ void c_expect(uint64_t *bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(c_smem(bar)), "r"(bytes) : "memory");
-}
-
-__device__ __forceinline__ void c_arrive(uint64_t *bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(c_smem(bar)) : "memory");
-}
-
-// the compute warps' barrier; the warp is converged on both sides
-__device__ __forceinline__ void c_sync() {
-  __syncwarp();
-  asm volatile("barrier.sync 1, %0;" ::"n"(kCThreads) : "memory");
-  __syncwarp();
-}
-
-__device__ __forceinline__ void c_cluster_arrive() {
-  __syncwarp();
-  asm volatile("barrier.cluster.arrive.release;" ::: "memory");
-}
-__device__ __forceinline__ void c_cluster_wait() {
-  asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
-  __syncwarp();
-}
-
-// s + e += x, exactly up to the rounding of e
-__device__ __forceinline__ void two_add(float &s, float &e, float x) {
-  const float t = s + x, z = t - s;
-  e += (s - (t - z)) + (x - z);
-  s = t;
-}
-
-// Sum of the lanes' two-float values in float64 (all lanes).
-__device__ __forceinline__ double warp_sum2(float s, float e) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float s2 = __shfl_xor_sync(0xffffffffu, s, o), e2 = __shfl_xor_sync(0xffffffffu, e, o);
-    two_add(s, e, s2);
-    e += e2;
-  }
-  return (double)s + (double)e;
-}
-
-// The same for three values.
-__device__ __forceinline__ void warp_sum2x3(float (&s)[3], float (&e)[3], double (&out)[3]) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    float s2[3], e2[3];
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      s2[i] = __shfl_xor_sync(0xffffffffu, s[i], o);
-      e2[i] = __shfl_xor_sync(0xffffffffu, e[i], o);
-    }
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      two_add(s[i], e[i], s2[i]);
-      e[i] += e2[i];
-    }
-  }
-#pragma unroll
-  for (int i = 0; i < 3; ++i) out[i] = (double)s[i] + (double)e[i];
-}
-
-// Halving butterfly: N per-lane values to their warp sums; lane l ends with the
-// sum of value idx(l), kept by the lanes of equal idx (32 / N of them).
-template <int N>
-__device__ __forceinline__ float c_xsum(float (&v)[N], int lane, int &idx) {
-  idx = 0;
-#pragma unroll
-  for (int s = 0; s < 5; ++s) {
-    const int o = 16 >> s, half = N >> (s + 1);
-    if (half >= 1) {
-      const bool up = (lane & o) != 0;
-#pragma unroll
-      for (int i = 0; i < half; ++i) {
-        const float send = up ? v[i] : v[i + half], keep = up ? v[i + half] : v[i];
-        v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-      }
-      if (up) idx += half;
-    } else {
-      v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
-    }
-  }
-  return v[0];
-}
-
 struct CShared {
   uint64_t full[kCMaxSlots], empty[kCMaxSlots];
   uint64_t wq_full, wq_empty;
@@ -192,49 +74,6 @@ struct CShared {
   float fin[3];
   int fail;
 };
-
-// Bounded wait of a whole warp (warp-uniform result) for the phase of `bar` with
-// the given parity: false, with the flag and the status raised, after the limit
-// or another warp's failure.  kCluster: acquires what other CTAs wrote.
-template <bool kCluster = false>
-__device__ __forceinline__ bool c_wait(uint64_t *bar, uint32_t parity, volatile int *fail, int *status) {
-  const uint32_t at = c_smem(bar);
-  uint64_t t0 = 0;
-  for (uint32_t it = 0;; ++it) {
-    uint32_t ok;
-    if constexpr (kCluster)
-      asm volatile(
-          "{\n\t.reg .pred p;\n\t"
-          "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-          "selp.u32 %0, 1, 0, p;\n\t}\n"
-          : "=r"(ok)
-          : "r"(at), "r"(parity)
-          : "memory");
-    else
-      ok = mbar_try_wait_parity<false>(at, parity);
-    if (__all_sync(0xffffffffu, ok)) return true;
-    if ((it & 63u) == 0) {
-      const uint64_t now = global_ns();
-      if (it == 0) t0 = now;
-      if (__any_sync(0xffffffffu, *fail != 0 || now - t0 > kMbarWaitNs)) break;
-    }
-  }
-  if ((threadIdx.x & 31) == 0 && !*fail) {
-    *fail = 1;
-    if (status) atomicExch(status, (int)MFG_ERR_TIMEOUT);
-  }
-  __syncwarp();
-  return false;
-}
-
-// This CTA has reached a meeting point of the cluster: its shared-memory writes
-// before it (all warps', after a c_sync()) are released to every CTA.
-__device__ __forceinline__ void c_meet_arrive(uint64_t *bar, int S) {
-  if (S > 1 && (int)threadIdx.x < S)
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(c_map(c_smem(bar), threadIdx.x))
-                 : "memory");
-  __syncwarp();
-}
 
 // kWR warps cover the CTA's R <= 256 kWR rows; the 8 / kWR groups of warps take
 // the basis slots s in turn (group s % kWC), each group from a ring of its own
@@ -771,11 +610,8 @@ __global__ void arnoldi_h_band_kernel(double *__restrict__ H, const double *__re
 // Host side
 // ---------------------------------------------------------------------------
 
-constexpr int kCMaxR = kCRows * kCWarps;
-
 bool arnoldi_cluster_applies(int64_t n) { return n <= (int64_t)kCMaxS * kCMaxR; }
 
-static int c_wr(int R) { return R <= kCRows ? 1 : (R <= 2 * kCRows ? 2 : (R <= 4 * kCRows ? 4 : 8)); }
 static int c_gc(int wr) { return wr >= 4 ? 2 : 4; }
 
 using CKernel = void (*)(const CStepArgs);
@@ -794,39 +630,14 @@ static size_t c_fixed(int R, int wr) {
   return (sizeof(CShared) + 127) / 128 * 128 + (size_t)(2 * R + (kCWarps / wr - 1) * 2 * R) * 4;
 }
 
-// Clusters of S = 1, 2, 4, 8, 16 CTAs that the GPU holds at a time, per number
-// of row warps.
+// clusters held at a time, per log2 of the row warps
 struct CSlots {
   int clusters[4][5];
   CSlots() {
-    int dev = 0, sms = 152;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-      sms = 152;
     for (int w = 0; w < 4; ++w) {
-      auto kern = c_kernel<false>(1 << w);
-      bool set = true;
-      for (auto kk : {kern, c_kernel<true>(1 << w)}) {
-        set = set && cudaFuncSetAttribute(kk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCSmem) == cudaSuccess;
-        set = set && cudaFuncSetAttribute(kk, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
-      }
-      for (int i = 0; i < 5; ++i) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(1024);
-        cfg.blockDim = dim3(kCThreads + 32);
-        cfg.dynamicSmemBytes = kCSmem;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = 1u << i;
-        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        int c = 0;
-        if (!set || cudaOccupancyMaxActiveClusters(&c, kern, &cfg) != cudaSuccess) c = 0;
-        clusters[w][i] = c;
-      }
+      c_prepare(c_kernel<true>(1 << w));
+      c_count_clusters(c_kernel<false>(1 << w), clusters[w]);
     }
-    (void)cudaGetLastError();
   }
 };
 
@@ -849,7 +660,7 @@ static CPlan c_plan(int64_t n, int64_t p, int j) {
     const int S = 1 << i;
     const int64_t R = ceil_div(ceil_div(n, S), 4) * 4;
     if (R > kCMaxR) continue;
-    const int wr = c_wr((int)R);
+    const int wr = c_row_warps(R);
     int w = 0;
     while ((1 << w) < wr) ++w;
     const int c = slots.clusters[w][i];
@@ -902,19 +713,8 @@ int launch_arnoldi_step(int j, int64_t k, int64_t n, int64_t p, float *Q, int64_
   a.nu = nu;
   a.status = status;
   auto kern = j == 0 ? c_kernel<true>(plan.wr) : c_kernel<false>(plan.wr);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(plan.S * (p < plan.clusters ? p : plan.clusters)));
-  cfg.blockDim = dim3(kCThreads + 32);
-  cfg.dynamicSmemBytes = c_fixed(plan.R, plan.wr) + (size_t)plan.slots * (kCWarps / plan.wr) * c_gc(plan.wr) * plan.R * 4;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)plan.S;
-  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  MFG_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, a));
-  return MFG_LAUNCH_STATUS();
+  const size_t smem = c_fixed(plan.R, plan.wr) + (size_t)plan.slots * (kCWarps / plan.wr) * c_gc(plan.wr) * plan.R * 4;
+  return c_launch(kern, plan.S, plan.S * (p < plan.clusters ? p : plan.clusters), smem, a, s);
 }
 
 // H of every probe from what the steps left (`band`: its tridiagonal part only);

@@ -423,11 +423,19 @@ static int run_hessenberg(const mfg_operator *op, int64_t k, int64_t p, const T 
                    launch_scale<T>(Wb, ld, n, p, norm, Q + (j + 1) * ld, qb, hi, lo, ld, s));
       continue;
     }
+    const bool last = (j + 1 == k);
+    double *hsub = last ? nullptr : H + (j + 1) * k + j;
+    if (gs_cluster_applies(n, ncols, 0)) {
+      // the step after the product as one launch
+      MFG_LAUNCH(MFG_PROF_SUBPROJ, (ncols + 2.0) * vecb + (last ? 0.0 : bfb), (reortho ? 4.0 : 2.0) * pf,
+                 launch_gs_cluster<T>(Q, qb, ld, ncols, Wb, n, p, reortho ? 4 : 2, nullptr, 0, nullptr, 0, H + j,
+                                      k * k, k, norm, hsub, k * k, last ? Wb : nullptr,
+                                      last ? nullptr : Q + (j + 1) * ld, qb, last ? nullptr : hi, lo, status, s));
+      continue;
+    }
     // first pass: h = Q^T w into column j of H
     MFG_LAUNCH(MFG_PROF_PROJ, pb, pf,
                launch_proj<T>(Q, qb, ld, ncols, Wb, ld, n, p, partials, counters, H + j, k * k, k, s, status));
-    const bool last = (j + 1 == k);
-    double *hsub = last ? nullptr : H + (j + 1) * k + j;
     if (reortho && sub_proj_rows_per_thread<T>(ncols) > 0) {
       // w' = w - Q h1 and h2 = Q^T w' from one read of the basis
       MFG_LAUNCH(MFG_PROF_SUBPROJ, (ncols + 2.0) * vecb, 2.0 * pf,
@@ -565,6 +573,28 @@ static int run_adjoint(const mfg_operator *op, int64_t k, int64_t p, int64_t ld,
              launch_sub<T>(Q, qb, ld, (int)k, coef, k, 1, lam, lam, ld, n, p, false, true, partials,
                            counters, nullptr, nullptr, 0, s, status));
 
+  if (gs_cluster_applies(n, k, 2 * k)) {
+    // lambda of step k - 1 reprojected (decomp.py:576-584), then a step is the product
+    // and one launch
+    MFG_LAUNCH(MFG_PROF_PROJ, (k + 1.0) * vecb, 2.0 * k * vecb / sizeof(T),
+               launch_proj<T>(Q, qb, ld, (int)k, lam, ld, n, p, partials, counters, h, k, 1, s, status));
+    MFG_LAUNCH(MFG_PROF_OTHER, 16.0 * p * k, (double)p * k,
+               launch_adj_reortho_coef(h, dH, (int)k, p, (int)(k - 1), (int)k, coef, s));
+    MFG_LAUNCH(MFG_PROF_SUB, (k + 2.0) * vecb, 2.0 * k * vecb / sizeof(T),
+               launch_sub<T>(Q, qb, ld, (int)k, coef, k, 1, lam, lam, ld, n, p, false, true, partials,
+                             counters, nullptr, nullptr, 0, s, status));
+    MFG_CUDA_TRY(cudaMemcpy2DAsync(Lam + (k - 1) * ld, qb * sizeof(T), lam, ld * sizeof(T), ld * sizeof(T), p,
+                                   cudaMemcpyDeviceToDevice, s));
+    if (hi) MFG_TRY(launch_split_bf16((const float *)lam, p, n, ld, hi, lo, ld, s));
+    for (int64_t idx = k - 1; idx >= 0; --idx) {
+      MFG_LAUNCH(MFG_PROF_APPLY, ab, af,
+                 apply_op<T>(op, Lam + idx * ld, qb, U, ld, p, hi, lo, ld, panel, status, s));
+      MFG_LAUNCH(MFG_PROF_SUBPROJ, (2.0 * k - idx + 4.0) * vecb, (4.0 * k + 4.0 * idx + 8.0) * vecb / sizeof(T),
+                 launch_adj_cluster<T>(Q, qb, ld, (int)k, (int)idx, U, Lam, R, dQ ? dQ + idx * ld : nullptr, H, Pi, dH,
+                                       gamma, Gamma, c, dv, n, p, hi, lo, status, s));
+    }
+    return MFG_OK;
+  }
   for (int64_t idx = k - 1; idx >= 0; --idx) {
     const int ncr = (int)(idx + 2 < k ? idx + 2 : k);
     // masked re-projection: lambda -= Q_m (Q_m^T lambda - dH[:, idx]_m)   (decomp.py:576-584)
@@ -755,9 +785,23 @@ static int run_bidiag(const mfg_operator *A, const mfg_operator *At, int64_t k, 
   };
 
   for (int64_t i = 0; i < k; ++i) {
+    const bool last = i + 1 == k;
     // left vector: u_i = (A v_i - beta_i u_{i-1}) reorthogonalised, / alpha_i
     MFG_LAUNCH(MFG_PROF_APPLY, ab, af,
                apply_op<T>(A, Vb + i * ld, qb, Wb, ld, p, hiA, loA, ld, panel, status, s));
+    if (gs_cluster_applies(n, i + 1, 0)) {
+      // everything of a side after its product as one launch
+      MFG_LAUNCH(MFG_PROF_SUBPROJ, (i + 3.0) * vecb, (8.0 * i + 6.0) * vecb / sizeof(T),
+                 launch_gs_cluster<T>(U, qb, ld, (int)i, Wb, n, p, 4, i > 0 ? U + (i - 1) * ld : nullptr, qb, betas + i,
+                                      k, h1, k, 1, norm, alphas + i, k, nullptr, U + i * ld, qb, hi, lo, status, s));
+      MFG_LAUNCH(MFG_PROF_APPLY, tb, tf,
+                 apply_op<T>(At, U + i * ld, qb, Wb, ld, p, hiT, loT, ld, panel, status, s));
+      MFG_LAUNCH(MFG_PROF_SUBPROJ, (i + 4.0) * vecb, (8.0 * i + 14.0) * vecb / sizeof(T),
+                 launch_gs_cluster<T>(Vb, qb, ld, (int)(i + 1), Wb, n, p, 4, Vb + i * ld, qb, alphas + i, k, h1, k, 1,
+                                      norm, last ? nullptr : betas + i + 1, k, last ? Wb : nullptr,
+                                      last ? nullptr : Vb + (i + 1) * ld, qb, last ? nullptr : hi, lo, status, s));
+      continue;
+    }
     if (i > 0)
       MFG_LAUNCH(MFG_PROF_SUB, 3.0 * vecb, 2.0 * vecb / sizeof(T),
                  launch_sub<T>(U + (i - 1) * ld, qb, ld, 1, betas + i, k, 1, Wb, Wb, ld, n, p, false,
@@ -771,7 +815,6 @@ static int run_bidiag(const mfg_operator *A, const mfg_operator *At, int64_t k, 
     MFG_LAUNCH(MFG_PROF_SUB, 3.0 * vecb, 2.0 * vecb / sizeof(T),
                launch_sub<T>(Vb + i * ld, qb, ld, 1, alphas + i, k, 1, Wb, Wb, ld, n, p, false, true,
                              partials, counters, norm, nullptr, 0, s, status));
-    const bool last = i + 1 == k;
     MFG_TRY(cgs2(Vb, (int)(i + 1), last ? nullptr : betas + i + 1, k));
     if (!last)
       MFG_LAUNCH(MFG_PROF_SCALE, 2.0 * vecb, vecb / sizeof(T),

@@ -1,0 +1,220 @@
+// Building blocks of the kernels that give a probe to a cluster of CTAs: eight
+// compute warps, a copy warp, shared-memory rings filled by bulk copies, and sums
+// met over distributed shared memory (arnoldi_cluster.cu, gs_cluster.cu).
+#pragma once
+
+#include "common.cuh"
+
+namespace mfg {
+
+constexpr int kCWarps = 8;             // compute warps
+constexpr int kCThreads = 32 * kCWarps;
+constexpr int kCRows = 256;            // rows of a warp: 8 per lane
+constexpr int kCMaxSlots = 32;
+constexpr int kCMaxS = 16;
+constexpr size_t kCSmem = 112 * 1024;  // dynamic shared memory of a CTA: two per SM
+constexpr int kCMaxR = kCRows * kCWarps;
+
+__device__ __forceinline__ uint32_t c_smem(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+__device__ __forceinline__ uint32_t c_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+
+__device__ __forceinline__ uint32_t c_map(uint32_t saddr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
+  return r;
+}
+
+__device__ __forceinline__ double c_ld_f64(uint32_t addr) {
+  double v;
+  asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(addr) : "memory");
+  return v;
+}
+
+__device__ __forceinline__ void c_bulk(uint32_t dst, const void *src, uint32_t bytes, uint64_t *bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+               "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes), "r"(c_smem(bar))
+               : "memory");
+}
+
+__device__ __forceinline__ void c_expect(uint64_t *bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(c_smem(bar)), "r"(bytes) : "memory");
+}
+
+__device__ __forceinline__ void c_arrive(uint64_t *bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(c_smem(bar)) : "memory");
+}
+
+// the compute warps' barrier; the warp is converged on both sides
+__device__ __forceinline__ void c_sync() {
+  __syncwarp();
+  asm volatile("barrier.sync 1, %0;" ::"n"(kCThreads) : "memory");
+  __syncwarp();
+}
+
+__device__ __forceinline__ void c_cluster_arrive() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+}
+__device__ __forceinline__ void c_cluster_wait() {
+  asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+  __syncwarp();
+}
+
+// s + e += x, exactly up to the rounding of e
+__device__ __forceinline__ void two_add(float &s, float &e, float x) {
+  const float t = s + x, z = t - s;
+  e += (s - (t - z)) + (x - z);
+  s = t;
+}
+
+// Sum of the lanes' two-float values in float64 (all lanes).
+__device__ __forceinline__ double warp_sum2(float s, float e) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const float s2 = __shfl_xor_sync(0xffffffffu, s, o), e2 = __shfl_xor_sync(0xffffffffu, e, o);
+    two_add(s, e, s2);
+    e += e2;
+  }
+  return (double)s + (double)e;
+}
+
+// The same for three values.
+__device__ __forceinline__ void warp_sum2x3(float (&s)[3], float (&e)[3], double (&out)[3]) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    float s2[3], e2[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      s2[i] = __shfl_xor_sync(0xffffffffu, s[i], o);
+      e2[i] = __shfl_xor_sync(0xffffffffu, e[i], o);
+    }
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      two_add(s[i], e[i], s2[i]);
+      e[i] += e2[i];
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 3; ++i) out[i] = (double)s[i] + (double)e[i];
+}
+
+// Halving butterfly: N per-lane values to their warp sums; lane l ends with the
+// sum of value idx(l), kept by the lanes of equal idx (32 / N of them).
+template <int N, typename T>
+__device__ __forceinline__ T c_xsum(T (&v)[N], int lane, int &idx) {
+  idx = 0;
+#pragma unroll
+  for (int s = 0; s < 5; ++s) {
+    const int o = 16 >> s, half = N >> (s + 1);
+    if (half >= 1) {
+      const bool up = (lane & o) != 0;
+#pragma unroll
+      for (int i = 0; i < half; ++i) {
+        const T send = up ? v[i] : v[i + half], keep = up ? v[i + half] : v[i];
+        v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+      }
+      if (up) idx += half;
+    } else {
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+    }
+  }
+  return v[0];
+}
+
+// Bounded wait of a whole warp (warp-uniform result) for the phase of `bar` with
+// the given parity: false, with the flag and the status raised, after the limit
+// or another warp's failure.  kCluster: acquires what other CTAs wrote.
+template <bool kCluster = false>
+__device__ __forceinline__ bool c_wait(uint64_t *bar, uint32_t parity, volatile int *fail, int *status) {
+  const uint32_t at = c_smem(bar);
+  uint64_t t0 = 0;
+  for (uint32_t it = 0;; ++it) {
+    uint32_t ok;
+    if constexpr (kCluster)
+      asm volatile(
+          "{\n\t.reg .pred p;\n\t"
+          "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+          "selp.u32 %0, 1, 0, p;\n\t}\n"
+          : "=r"(ok)
+          : "r"(at), "r"(parity)
+          : "memory");
+    else
+      ok = mbar_try_wait_parity<false>(at, parity);
+    if (__all_sync(0xffffffffu, ok)) return true;
+    if ((it & 63u) == 0) {
+      const uint64_t now = global_ns();
+      if (it == 0) t0 = now;
+      if (__any_sync(0xffffffffu, *fail != 0 || now - t0 > kMbarWaitNs)) break;
+    }
+  }
+  if ((threadIdx.x & 31) == 0 && !*fail) {
+    *fail = 1;
+    if (status) atomicExch(status, (int)MFG_ERR_TIMEOUT);
+  }
+  __syncwarp();
+  return false;
+}
+
+// This CTA has reached a meeting point of the cluster: its shared-memory writes
+// before it (all warps', after a c_sync()) are released to every CTA.
+__device__ __forceinline__ void c_meet_arrive(uint64_t *bar, int S) {
+  if (S > 1 && (int)threadIdx.x < S)
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(c_map(c_smem(bar), threadIdx.x))
+                 : "memory");
+  __syncwarp();
+}
+
+// Row warps for R rows of a CTA, and the clusters of S = 1, 2, 4, 8, 16 CTAs that
+// the GPU holds at a time for a kernel of kCThreads + 32 threads and kCSmem bytes.
+inline int c_row_warps(int64_t R) { return R <= kCRows ? 1 : (R <= 2 * kCRows ? 2 : (R <= 4 * kCRows ? 4 : 8)); }
+
+template <typename K>
+inline bool c_prepare(K kern) {
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCSmem) == cudaSuccess &&
+         cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+}
+
+template <typename K>
+inline void c_count_clusters(K kern, int (&clusters)[5]) {
+  const bool set = c_prepare(kern);
+  for (int i = 0; i < 5; ++i) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(1024);
+    cfg.blockDim = dim3(kCThreads + 32);
+    cfg.dynamicSmemBytes = kCSmem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1u << i;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int c = 0;
+    if (!set || cudaOccupancyMaxActiveClusters(&c, kern, &cfg) != cudaSuccess) c = 0;
+    clusters[i] = c;
+  }
+  (void)cudaGetLastError();
+}
+
+template <typename K, typename A>
+inline int c_launch(K kern, int S, int64_t ctas, size_t smem, const A &args, cudaStream_t s) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)ctas);
+  cfg.blockDim = dim3(kCThreads + 32);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)S;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  MFG_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, args));
+  return MFG_LAUNCH_STATUS();
+}
+
+}  // namespace mfg

@@ -62,6 +62,19 @@ int launch_arnoldi_step(int j, int64_t k, int64_t n, int64_t p, float *Q, int64_
                         double *Hh, double *nu, int *status, cudaStream_t s);
 int launch_arnoldi_h(int64_t k, int64_t p, double *H, const double *Hh, const double *nu, bool band,
                      double *nu_last_inv, cudaStream_t s);
+// gs_cluster.cu: Gram-Schmidt twice with the norm and the normalisation, and a step
+// of the adjoint, as one launch each (n up to 32768)
+bool gs_cluster_applies(int64_t n, int64_t ncols, int64_t nextra);
+template <typename T>
+int launch_gs_cluster(const T *Q, int64_t qb, int64_t ld, int ncols, const T *W, int64_t n, int64_t p, int passes,
+                      const T *prev, int64_t prev_b, const double *prev_c, int64_t prev_cs, double *h, int64_t h_bs,
+                      int64_t h_is, double *norm, double *norm2, int64_t norm2_bs, T *w_out, T *next, int64_t next_b,
+                      __nv_bfloat16 *hi, __nv_bfloat16 *lo, int *status, cudaStream_t s);
+template <typename T>
+int launch_adj_cluster(const T *Q, int64_t qb, int64_t ld, int k, int idx, const T *U, T *Lam, const T *res,
+                       const T *dq, const double *H, const double *Pi, const double *dH, const double *gamma,
+                       double *Gamma, const double *c, T *dv, int64_t n, int64_t p, __nv_bfloat16 *hi,
+                       __nv_bfloat16 *lo, int *status, cudaStream_t s);
 // conjugate gradients on probe-major panels (lanczos_kernels.cu)
 template <typename T>
 int launch_cg_init(const T *B, T *X, T *R, T *P, int64_t ld, int64_t n, int64_t p,

@@ -193,3 +193,138 @@ def test_every_interleaving_ends_with_the_right_data(wr, slots, S, ns):
 def test_the_model_sees_a_slot_released_too_early():
     with pytest.raises(AssertionError):
         simulate(8, 3, 1, 9, probes=3, seed=0, keep_bug=True)
+
+
+def simulate_passes(wr, slots, S, ns, nsx, passes, norm, probes, seed):
+    """The Gram-Schmidt / adjoint kernel (csrc/gs_cluster.cu): nsx slots read once, then `passes` passes over
+    ns slots in rotated orders, a meeting of the cluster after every other pass (and after the norm)."""
+    rng = random.Random(seed)
+    ctas = [Cta(wr, slots, S) for _ in range(S)]
+    for c in ctas:
+        c.meet = [Barrier(S) for _ in range(3)]
+        c.part = {}
+    wc = WARPS // wr
+    flying = []
+
+    def of(g, n=ns):
+        return (n - g + wc - 1) // wc if g < n else 0
+
+    def copier(c):
+        fills, pos, par = [0] * wc, [0] * wc, [0] * wc
+
+        def fill(g, what):
+            if fills[g] >= slots:
+                while not c.empty[g][pos[g]].done(par[g] ^ 1):
+                    yield
+            c.full[g][pos[g]].arrive(1)
+
+            def land(at=pos[g]):
+                c.data[g][at] = what
+                c.full[g][at].complete(1)
+
+            flying.append(land)
+            fills[g] += 1
+            pos[g] += 1
+            if pos[g] == slots:
+                pos[g], par[g] = 0, par[g] ^ 1
+            yield
+
+        for b in range(probes):
+            for s in range(nsx):
+                yield from fill(s % wc, (b, "x", s))
+            for t in range(1, passes + 1):
+                for i in range(of(0)):
+                    for g in range(wc):
+                        gs = of(g)
+                        gk = min(gs, slots)
+                        if i >= gs or (t > 1 and i < gk):
+                            continue
+                        yield from fill(g, (b, "q", (i + (t - 1) * (gs - gk)) % gs * wc + g))
+
+    def cta_sync(c):
+        gen = c.sync_gen
+        c.sync_n += 1
+        if c.sync_n == WARPS:
+            c.sync_n, c.sync_gen = 0, gen + 1
+        while c.sync_gen == gen:
+            yield
+
+    def meet(c, warp, which, b):
+        yield from cta_sync(c)
+        if warp == 0:
+            c.part[which, b & 1] = b
+        yield from cta_sync(c)
+        if S > 1:
+            if warp == 0:
+                for other in ctas:
+                    other.meet[which].arrive()
+                    yield
+            while not c.meet[which].done(b & 1):
+                yield
+            for other in ctas:
+                assert other.part[which, b & 1] == b
+                yield
+            yield from cta_sync(c)
+
+    def compute(c, warp):
+        group = warp // wr
+        full, empty, data = c.full[group], c.empty[group], c.data[group]
+        gs = of(group)
+        gk = min(gs, slots)
+        pos = sp = 0
+
+        def advance():
+            nonlocal pos, sp
+            pos, sp = (0, sp ^ 1) if pos + 1 == slots else (pos + 1, sp)
+
+        def use(what, release):
+            while not full[pos].done(sp):
+                yield
+            assert data[pos] == what
+            yield
+            assert data[pos] == what
+            if release:
+                empty[pos].arrive()
+            advance()
+
+        for b in range(probes):
+            for u in range(of(group, nsx)):
+                yield from use((b, "x", u * wc + group), True)
+            for t in range(1, passes + 1):
+                u = (t - 1) * (gs - gk) % gs if gs else 0
+                kept = (pos, sp)
+                for i in range(gs):
+                    if i == gs - gk:
+                        kept = (pos, sp)
+                    yield from use((b, "q", u * wc + group), t == passes or i < gs - gk)
+                    u = 0 if u + 1 == gs else u + 1
+                if t < passes:
+                    pos, sp = kept
+                if t % 2:
+                    yield from meet(c, warp, t // 2, b)
+                elif wc > 1:
+                    yield from cta_sync(c)
+            if norm:
+                yield from meet(c, warp, 2, b)
+
+    agents = [copier(c) for c in ctas] + [compute(c, w) for c in ctas for w in range(WARPS)]
+    steps = 0
+    while agents:
+        if flying and rng.random() < 0.3:
+            flying.pop(rng.randrange(len(flying)))()
+        a = rng.choice(agents)
+        try:
+            next(a)
+        except StopIteration:
+            agents.remove(a)
+        steps += 1
+        assert steps < 4_000_000, "a wait that does not end"
+    assert not flying
+
+
+@pytest.mark.parametrize("wr,slots,S", [(8, 5, 2), (8, 2, 1), (4, 3, 2), (2, 2, 4), (1, 2, 1)])
+@pytest.mark.parametrize("ns,nsx,passes,norm", [(0, 0, 4, True), (1, 0, 4, True), (7, 0, 2, True), (13, 0, 4, True),
+                                                (1, 9, 2, False), (6, 4, 4, False), (17, 2, 4, False)])
+def test_rotated_passes_end_with_the_right_data(wr, slots, S, ns, nsx, passes, norm):
+    for seed in range(2):
+        simulate_passes(wr, slots, S, ns, nsx, passes, norm, probes=3, seed=seed)
