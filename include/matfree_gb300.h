@@ -281,6 +281,16 @@ MFG_API int mfg_rbf_build(const float *x, int64_t n, int32_t dim, double s2, dou
 MFG_API int mfg_rbf_build_dlogell(const float *x, int64_t n, int32_t dim, double s2, double ell,
                                   int32_t precision, void *a, void *a_lo, int64_t lda, void *stream);
 
+/* The parameter part of the reverse pass over all stacked adjoint states
+ * (matfree/decomp.py:587-589): with rows vectors q_r of Q and lam_r of Lam (ld
+ * elements apart), out (device, 3 float64) = (sum lam_r^T A q_r, sum lam_r^T dA q_r,
+ * shift sum lam_r^T q_r) for the dense A (taken without its shift) and dA of one
+ * size and precision, summed in float64 accuracy. */
+MFG_API size_t mfg_theta_contractions_workspace_bytes(const mfg_operator *op, int64_t rows, int64_t ld);
+MFG_API int mfg_theta_contractions(const mfg_operator *op, const mfg_operator *dop, int64_t rows,
+                                   int64_t ld, const void *Q, const void *Lam, double *out,
+                                   void *workspace, size_t workspace_bytes, void *stream);
+
 /* Split a float32 matrix into bf16 hi = bf16(a) and lo = bf16(a - hi). */
 /* ---- Golub-Kahan bidiagonalisation and product quadrature --------------- */
 

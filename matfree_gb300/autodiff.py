@@ -209,16 +209,37 @@ def rbf_theta_contractions(op: RBFKernelOperator, x, Q, Lam, dl=None) -> torch.T
     """
     p, k, ld = Q.shape
     n = op.n
+    if dl is None:
+        dl = _rbf_dlogell_operator(op, x)
+    live = torch.is_grad_enabled() and (Q.requires_grad or Lam.requires_grad)
+    if (not live and Q.dtype == Lam.dtype == op.basis_dtype and Q.shape == Lam.shape and p * k > 0
+            and dl.precision == op.precision and dl.n == n and ld >= n and ld % 8 == 0):
+        Q, Lam = Q.contiguous(), Lam.contiguous()
+        if Q.data_ptr() % 16 == 0 and Lam.data_ptr() % 16 == 0:
+            return _device_contractions(op, dl, Q, Lam)
+    # panels the kernel does not read in place, mixed types
     rows = Q.reshape(p * k, ld)[:, :n]
     lam = Lam.reshape(p * k, ld)[:, :n].double()
     # the stored exponential part (without the nugget) is dK/dlog s2
     base = DenseOperator._from_storage(n, op.precision, op.a, op.a_lo, 0.0)
     g0 = (lam * base.matmat(rows).double()).sum()
-    if dl is None:
-        dl = _rbf_dlogell_operator(op, x)
     g1 = (lam * dl.matmat(rows).double()).sum()
     g2 = op.tau * (lam * rows.double()).sum()
     return torch.stack([g0, g1, g2])
+
+
+def _device_contractions(op: RBFKernelOperator, dl: DenseOperator, Q, Lam) -> torch.Tensor:
+    p, k, ld = Q.shape
+    out = torch.empty(3, dtype=torch.float64, device=Q.device)
+    lib = _lib.lib()
+    s, d = op.c_struct(), dl.c_struct()
+    nbytes = lib.mfg_theta_contractions_workspace_bytes(ctypes.byref(s), p * k, ld)
+    ws = torch.empty(nbytes, dtype=torch.uint8, device=Q.device)
+    st = lib.mfg_theta_contractions(ctypes.byref(s), ctypes.byref(d), p * k, ld, ctypes.c_void_p(Q.data_ptr()),
+                                    ctypes.c_void_p(Lam.data_ptr()), ctypes.c_void_p(out.data_ptr()),
+                                    ctypes.c_void_p(ws.data_ptr()), nbytes, stream_ptr())
+    _lib.check(st, "mfg_theta_contractions")
+    return out
 
 
 def _rbf_dlogell_operator(op: RBFKernelOperator, x) -> DenseOperator:

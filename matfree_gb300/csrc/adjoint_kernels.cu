@@ -6,7 +6,7 @@
 // updates, operator application) that the driver issues with the forward
 // kernels.  Index conventions follow the float64 restatement of
 // matfree/decomp.py:480-600: step idx runs from k-1 down to 0.
-#include "common.cuh"
+#include "cluster.cuh"
 #include "kernels.cuh"
 
 namespace mfg {
@@ -198,6 +198,150 @@ template int launch_basis_combine<double>(const double *, int64_t, int64_t, int6
 int launch_axpy_f64(double a, const double *x, double *y, int64_t m, cudaStream_t s) {
   if (m <= 0) return MFG_OK;
   axpy_f64_kernel<<<blocks(m, 256), 256, 0, s>>>(a, x, y, m);
+  return MFG_LAUNCH_STATUS();
+}
+
+// <Lam, Y> (and <Lam, Q> from the same read of Lam) over the n valid columns of
+// `rows` panel rows, in float64: the parameter contractions of the reverse pass.
+//
+// Bound by the read of the two or three panels.  A float64 multiply-add or
+// conversion costs an SM about 19 cycles a warp, several times what the load of its
+// operands takes, so products of floats are kept as exact two-float pairs (product
+// and fma remainder) and summed with error-free additions: ten float instructions
+// an element, some 2^-45 of the sum of |lam y| against float64.  Four products
+// outside [2^-90, 2^100], where a remainder could underflow or the sum overflow,
+// are added in float64.  6144 rows of 8192, all of the contractions with their two
+// products and the split: 4.87 ms with float64 copies of the panels and one pass per
+// conversion, product and sum, 3.24 ms so (of which the products 2.6 at the GEMM's rate).
+// 1024 columns a CTA step, 8 CTAs an SM; partials are summed in a fixed order.
+constexpr int kDotCols = kThreads * 4;
+constexpr int kDotBlocks = 152 * 8;
+
+struct Dot2 {
+  float s = 0.0f, e = 0.0f;
+  double d = 0.0;
+  __device__ __forceinline__ void add(const float4 &l, const float4 &y) {
+    const float a[4] = {l.x, l.y, l.z, l.w}, b[4] = {y.x, y.y, y.z, y.w};
+    float p[4], m = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      p[i] = a[i] * b[i];
+      m = fmaxf(m, fabsf(p[i]));
+    }
+    if (m < 0x1p-90f || m > 0x1p100f) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) d += (double)a[i] * (double)b[i];
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        e += fmaf(a[i], b[i], -p[i]);
+        two_add(s, e, p[i]);
+      }
+    }
+  }
+  __device__ __forceinline__ double value() const { return d + ((double)s + (double)e); }
+};
+
+// the valid ones of four panel elements from column c on; padding counts as zero
+__device__ __forceinline__ float4 dot_load(const float *row, int64_t c, int64_t n) {
+  float4 v = __ldg(reinterpret_cast<const float4 *>(row + c));
+  if (c + 4 > n) {
+    if (c + 1 >= n) v.y = 0.0f;
+    if (c + 2 >= n) v.z = 0.0f;
+    if (c + 3 >= n) v.w = 0.0f;
+  }
+  return v;
+}
+
+template <typename T, bool kQ>
+__global__ void __launch_bounds__(kThreads) panel_dot_kernel(const T *__restrict__ Y,
+                                                             const T *__restrict__ Lam,
+                                                             const T *__restrict__ Q, int64_t rows,
+                                                             int64_t n, int64_t ld, int slot,
+                                                             double *__restrict__ part) {
+  __shared__ double sh[2][kWarps];
+  const int64_t nch = (n + kDotCols - 1) / kDotCols;
+  double dy = 0.0, dq = 0.0;
+  Dot2 ay, aq;
+  for (int64_t it = blockIdx.x; it < rows * nch; it += gridDim.x) {
+    const int64_t r = it / nch, c = (it - r * nch) * kDotCols + threadIdx.x * 4;
+    if (c >= n) continue;
+    const int64_t o = r * ld;
+    if constexpr (sizeof(T) == 4) {
+      const float4 l = dot_load(Lam + o, c, n), y = dot_load(Y + o, c, n);
+      if constexpr (kQ) {
+        const float4 q = dot_load(Q + o, c, n);
+        aq.add(l, q);
+      }
+      ay.add(l, y);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (c + i < n) {
+          const double l = Lam[o + c + i];
+          dy = fma(l, Y[o + c + i], dy);
+          if constexpr (kQ) dq = fma(l, Q[o + c + i], dq);
+        }
+    }
+  }
+  if constexpr (sizeof(T) == 4) {
+    dy = ay.value();
+    dq = aq.value();
+  }
+  dy = warp_sum(dy);
+  dq = warp_sum(dq);
+  const int warp = threadIdx.x >> 5;
+  if ((threadIdx.x & 31) == 0) {
+    sh[0][warp] = dy;
+    sh[1][warp] = dq;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double t0 = 0.0, t1 = 0.0;
+    for (int i = 0; i < kWarps; ++i) {
+      t0 += sh[0][i];
+      t1 += sh[1][i];
+    }
+    part[blockIdx.x * 3 + slot] = t0;
+    if (kQ) part[blockIdx.x * 3 + 2] = t1;
+  }
+}
+
+// out[i] = f_i sum_b part[b][i], f = (1, 1, scale); one warp a result
+__global__ void panel_dot_sum_kernel(const double *__restrict__ part, int nb, double scale,
+                                     double *__restrict__ out) {
+  const int i = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double t = 0.0;
+  for (int b = lane; b < nb; b += 32) t += part[b * 3 + i];
+  t = warp_sum(t);
+  if (lane == 0) out[i] = i == 2 ? scale * t : t;
+}
+
+size_t panel_dot_bytes() { return (size_t)kDotBlocks * 3 * sizeof(double); }
+
+static int panel_dot_blocks(int64_t rows, int64_t n) {
+  const int64_t items = rows * ceil_div(n, kDotCols);
+  return (int)(items < kDotBlocks ? items : kDotBlocks);
+}
+
+template <typename T>
+int launch_panel_dot(const T *Y, const T *Lam, const T *Q, int64_t rows, int64_t n, int64_t ld,
+                     int slot, double *part, cudaStream_t s) {
+  const int nb = panel_dot_blocks(rows, n);
+  if (Q)
+    panel_dot_kernel<T, true><<<nb, kThreads, 0, s>>>(Y, Lam, Q, rows, n, ld, slot, part);
+  else
+    panel_dot_kernel<T, false><<<nb, kThreads, 0, s>>>(Y, Lam, Q, rows, n, ld, slot, part);
+  return MFG_LAUNCH_STATUS();
+}
+template int launch_panel_dot<float>(const float *, const float *, const float *, int64_t, int64_t,
+                                     int64_t, int, double *, cudaStream_t);
+template int launch_panel_dot<double>(const double *, const double *, const double *, int64_t, int64_t,
+                                      int64_t, int, double *, cudaStream_t);
+
+int launch_panel_dot_sum(const double *part, int64_t rows, int64_t n, double scale, double *out,
+                         cudaStream_t s) {
+  panel_dot_sum_kernel<<<1, 96, 0, s>>>(part, panel_dot_blocks(rows, n), scale, out);
   return MFG_LAUNCH_STATUS();
 }
 

@@ -472,6 +472,60 @@ static int run_hessenberg(const mfg_operator *op, int64_t k, int64_t p, const T 
 // Batched Hessenberg adjoint (reverse Arnoldi), matfree/decomp.py:480-600.
 // ---------------------------------------------------------------------------
 
+struct ThetaLayout {
+  size_t y, part, status, hi, lo, total;
+};
+
+static ThetaLayout theta_layout(const mfg_operator *op, int64_t rows, int64_t ld) {
+  ThetaLayout L{};
+  size_t off = 0;
+  auto take = [&](size_t bytes) {
+    const size_t o = off;
+    off = align_up(off + bytes, 256);
+    return o;
+  };
+  L.status = take(16);
+  L.y = take((size_t)rows * ld * elem_size_for(op));
+  L.part = take(panel_dot_bytes());
+  L.hi = take(uses_bf16(op) ? (size_t)rows * ld * 2 : 0);
+  L.lo = take(uses_bf16(op) && op->precision == MFG_PREC_BF16X3 ? (size_t)rows * ld * 2 : 0);
+  L.total = off + 256;
+  return L;
+}
+
+// out = (<Lam, (A - shift I) Q>, <Lam, dA Q>, shift <Lam, Q>): one bf16 split of Q
+// for both products, one product panel in flight
+template <typename T>
+static int run_theta(const mfg_operator *op, const mfg_operator *dop, int64_t rows, int64_t ld,
+                     const T *Q, const T *Lam, double *out, const ThetaLayout &L, char *ws,
+                     cudaStream_t s) {
+  T *Y = reinterpret_cast<T *>(ws + L.y);
+  double *part = reinterpret_cast<double *>(ws + L.part);
+  int *status = reinterpret_cast<int *>(ws + L.status);
+  MFG_CUDA_TRY(cudaMemsetAsync(status, 0, sizeof(int), s));
+  __nv_bfloat16 *hi = nullptr, *lo = nullptr;
+  const double panel = (double)op->n * (double)rows * sizeof(T);
+  if constexpr (sizeof(T) == 4) {
+    if (uses_bf16(op)) {
+      hi = reinterpret_cast<__nv_bfloat16 *>(ws + L.hi);
+      lo = op->precision == MFG_PREC_BF16X3 ? reinterpret_cast<__nv_bfloat16 *>(ws + L.lo) : nullptr;
+      MFG_LAUNCH(MFG_PROF_OTHER, panel * (lo ? 2.0 : 1.5), 0.0,
+                 launch_split_bf16(Q, rows, op->n, ld, hi, lo, ld, s));
+    }
+  }
+  mfg_operator base = *op;
+  base.shift = 0.0;
+  double ab = 0.0, af = 0.0;
+  apply_cost(op, rows, &ab, &af);
+  for (int i = 0; i < 2; ++i) {
+    MFG_LAUNCH(MFG_PROF_APPLY, ab, af,
+               apply_op<T>(i == 0 ? &base : dop, Q, ld, Y, ld, rows, hi, lo, ld, nullptr, status, s));
+    MFG_LAUNCH(MFG_PROF_OTHER, panel * (3.0 - i), 4.0 * panel / sizeof(T),
+               launch_panel_dot<T>(Y, Lam, i == 0 ? Q : nullptr, rows, op->n, ld, i, part, s));
+  }
+  return launch_panel_dot_sum(part, rows, op->n, op->shift, out, s);
+}
+
 struct AdjLayout {
   size_t lam, lam2, U, panel, h, g, coef, bp, gamma, scal, beta, Gamma, Pi, M, inv, partials,
       counters, status, hi, lo, total;
@@ -1450,6 +1504,31 @@ int mfg_rbf_build(const float *x, int64_t n, int32_t dim, double s2, double ell,
 int mfg_rbf_build_dlogell(const float *x, int64_t n, int32_t dim, double s2, double ell,
                           int32_t precision, void *a, void *a_lo, int64_t lda, void *stream) {
   return rbf_build(x, n, dim, s2, ell, precision, 1, a, a_lo, lda, stream);
+}
+
+size_t mfg_theta_contractions_workspace_bytes(const mfg_operator *op, int64_t rows, int64_t ld) {
+  if (check_op(op) != MFG_OK || check_panel(op, rows, ld) != MFG_OK) return 0;
+  return theta_layout(op, rows, ld).total;
+}
+
+int mfg_theta_contractions(const mfg_operator *op, const mfg_operator *dop, int64_t rows, int64_t ld,
+                           const void *Q, const void *Lam, double *out, void *workspace,
+                           size_t workspace_bytes, void *stream) {
+  MFG_TRY(check_op(op));
+  MFG_TRY(check_op(dop));
+  MFG_TRY(check_panel(op, rows, ld));
+  if (op->kind != MFG_OP_DENSE || dop->kind != MFG_OP_DENSE || dop->n != op->n ||
+      dop->precision != op->precision)
+    return MFG_ERR_UNSUPPORTED;
+  if (!Q || !Lam || !out || !aligned16(Q) || !aligned16(Lam)) return MFG_ERR_BAD_ARG;
+  const ThetaLayout L = theta_layout(op, rows, ld);
+  if (!workspace || workspace_bytes < L.total) return MFG_ERR_WORKSPACE;
+  char *ws = ws_base(workspace);
+  if (op->precision == MFG_PREC_FP64)
+    return run_theta<double>(op, dop, rows, ld, (const double *)Q, (const double *)Lam, out, L, ws,
+                             as_stream(stream));
+  return run_theta<float>(op, dop, rows, ld, (const float *)Q, (const float *)Lam, out, L, ws,
+                          as_stream(stream));
 }
 
 int mfg_split_bf16(const float *a, int64_t rows, int64_t cols, int64_t lda, void *hi, void *lo,

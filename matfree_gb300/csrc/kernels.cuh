@@ -113,6 +113,14 @@ int launch_adj_lincomb(const T *U, const T *lam, const T *R, const T *dq, int64_
 int launch_axpy_f64(double a, const double *x, double *y, int64_t m, cudaStream_t s);
 int gemm_rule_add(int64_t n_lo, int64_t n_hi, int64_t p_lo, int64_t p_hi, int bn, int split);
 int gemm_rules_clear();
+// bytes of the partial sums of launch_panel_dot; launch_panel_dot writes column
+// `slot` (<Lam, Y>) and, with Q, column 2 (<Lam, Q>) of them
+size_t panel_dot_bytes();
+template <typename T>
+int launch_panel_dot(const T *Y, const T *Lam, const T *Q, int64_t rows, int64_t n, int64_t ld,
+                     int slot, double *part, cudaStream_t s);
+int launch_panel_dot_sum(const double *part, int64_t rows, int64_t n, double scale, double *out,
+                         cudaStream_t s);
 template <typename T>
 int launch_basis_combine(const T *Q, int64_t k, int64_t ld, int64_t n, int64_t p, const double *coef,
                          T *out, cudaStream_t s);
