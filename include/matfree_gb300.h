@@ -281,6 +281,15 @@ MFG_API int mfg_rbf_build(const float *x, int64_t n, int32_t dim, double s2, dou
 MFG_API int mfg_rbf_build_dlogell(const float *x, int64_t n, int32_t dim, double s2, double ell,
                                   int32_t precision, void *a, void *a_lo, int64_t lda, void *stream);
 
+/* Values scale_b e1^T f(T_b) e1 (p) and their cotangent dH (p, k, k) in the
+ * Hessenberg matrix whose symmetrised tridiagonal part is T_b, from eigvals
+ * (p, k), eigvecs (p, k, k; columns), fw = f(eigvals) and fprime_mid (p, k, k)
+ * = f'((w_a + w_b) / 2): the Daleckii-Krein formula behind
+ * matfree/funm.py:322-335.  All float64; dH is zero off the three diagonals. */
+MFG_API int mfg_quadform_dh(int64_t k, int64_t p, const double *eigvals, const double *eigvecs,
+                            const double *fw, const double *fprime_mid, const double *scale,
+                            double *values, double *dH, void *stream);
+
 /* The parameter part of the reverse pass over all stacked adjoint states
  * (matfree/decomp.py:587-589): with rows vectors q_r of Q and lam_r of Lam (ld
  * elements apart), out (device, 3 float64) = (sum lam_r^T A q_r, sum lam_r^T dA q_r,

@@ -70,6 +70,8 @@ SIGNATURES = {
     "mfg_tridiag_eigh": (c_int, [c_int64, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p]),
     "mfg_rbf_build": (c_int, [c_void_p, c_int64, c_int32, c_double, c_double, c_int32, c_void_p, c_void_p, c_int64, c_void_p]),
     "mfg_rbf_build_dlogell": (c_int, [c_void_p, c_int64, c_int32, c_double, c_double, c_int32, c_void_p, c_void_p, c_int64, c_void_p]),
+    "mfg_quadform_dh": (c_int, [c_int64, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
+                                c_void_p, c_void_p]),
     "mfg_theta_contractions_workspace_bytes": (c_size_t, [POINTER(MfgOperator), c_int64, c_int64]),
     "mfg_theta_contractions": (c_int, [POINTER(MfgOperator), POINTER(MfgOperator), c_int64, c_int64, c_void_p,
                                        c_void_p, c_void_p, c_void_p, c_size_t, c_void_p]),

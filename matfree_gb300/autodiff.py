@@ -48,6 +48,17 @@ def quadform_dH(H: torch.Tensor, scale: torch.Tensor, f, fprime) -> tuple[torch.
     p, k = H.shape[0], H.shape[1]
     w, S = tridiag_eigh(H)  # the eigh of T = tridiagonal part of (H + H^T)/2
     fw = f(w)
+    live = torch.is_grad_enabled() and (scale.requires_grad or fw.requires_grad)
+    if not live and fw.dtype == scale.dtype == torch.float64 and scale.shape == (p,) and 0 < p and k <= 4096:
+        fmid = fprime(0.5 * (w[:, :, None] + w[:, None, :])).to(torch.float64)
+        fmid, fw, scale = fmid.expand(p, k, k).contiguous(), fw.contiguous(), scale.contiguous()
+        values = torch.empty(p, dtype=torch.float64, device=w.device)
+        dH = torch.empty((p, k, k), dtype=torch.float64, device=w.device)
+        st = _lib.lib().mfg_quadform_dh(k, p, *(ctypes.c_void_p(t.data_ptr())
+                                                for t in (w, S, fw, fmid, scale, values, dH)), stream_ptr())
+        _lib.check(st, "mfg_quadform_dh")
+        return values, dH
+    # differentiable f or scale, other types
     s1 = S[:, 0, :]
     values = scale * (fw * s1 * s1).sum(-1)
     diff = w[:, :, None] - w[:, None, :]

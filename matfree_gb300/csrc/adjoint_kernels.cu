@@ -345,4 +345,120 @@ int launch_panel_dot_sum(const double *part, int64_t rows, int64_t n, double sca
   return MFG_LAUNCH_STATUS();
 }
 
+// Quadrature values scale e1^T f(T) e1 and their cotangent in H from the
+// eigendecomposition T = S diag(w) S^T: only the three diagonals of
+// G = S (F o s1 s1^T) S^T are wanted, with s1 the first row of S and F the divided
+// differences (f(w_a) - f(w_b)) / (w_a - w_b), f' at the midpoint for equal pairs.
+// With u_ia = S_ia s1_a and, F being symmetric, the lower triangle
+// M_i[a] = sum_{b<a} F_ab u_ib + F_aa u_ia / 2, G_ij = u_i . M_j + u_j . M_i.
+//
+// A CTA per probe, bound by the k^3 / 2 float64 multiply-adds (an SM takes one a
+// warp every 19 cycles).  F lies in shared memory while it fits and in dH, which is
+// written last, beyond; a warp takes kDhRows rows of u, so that one read of F serves
+// them all.  The eigensolver and the cotangent of 32 probes of k = 24: 0.25 ms, where
+// some thirty small batched operations took 0.74; 128 of k = 48: 0.50 ms, 0.73 before.
+constexpr int kDhRows = 2;
+constexpr int kDhThreads = 512;
+constexpr size_t kDhSmem = 160 * 1024;
+
+__global__ void __launch_bounds__(kDhThreads) quadform_dh_kernel(
+    int k, const double *__restrict__ W, const double *__restrict__ S, const double *__restrict__ fW,
+    const double *__restrict__ fpM, const double *__restrict__ scale, int shared_f,
+    double *__restrict__ values, double *dH) {
+  extern __shared__ double sh[];
+  const int64_t b = blockIdx.x;
+  const double *w = W + b * k, *s = S + b * k * k, *fw = fW + b * k, *fp = fpM + b * k * k;
+  double *out = dH + b * k * k;
+  double *gd = sh, *gy = sh + k, *gz = sh + 2 * k;  // u_i . M_i, u_{i+1} . M_i, u_{i-1} . M_i
+  double *F = shared_f ? sh + 3 * k : out;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  for (int64_t t = threadIdx.x; t < (int64_t)k * k; t += blockDim.x) {
+    const int i = (int)(t / k), j = (int)(t - (int64_t)i * k);
+    const double d = w[i] - w[j];
+    const bool same = fabs(d) <= 1e-13 * fmax(fabs(w[i]), 1.0);
+    F[t] = same ? fp[t] : (fw[i] - fw[j]) / d;
+  }
+  __syncthreads();
+  for (int i0 = warp * kDhRows; i0 < k; i0 += nw * kDhRows) {
+    double xd[kDhRows] = {}, xy[kDhRows] = {}, xz[kDhRows] = {};
+    for (int a0 = 0; a0 < k; a0 += 32) {
+      const int a = a0 + lane;
+      const bool in = a < k;
+      double M[kDhRows] = {};
+      for (int b0 = 0; b0 <= a0; b0 += 32) {
+        // u_i[b0 + lane], handed round by shuffles
+        double u[kDhRows];
+        const double s1 = b0 + lane < k ? s[b0 + lane] : 0.0;
+#pragma unroll
+        for (int r = 0; r < kDhRows; ++r)
+          u[r] = (b0 + lane < k && i0 + r < k) ? s[(int64_t)(i0 + r) * k + b0 + lane] * s1 : 0.0;
+        const int nb = k - b0 < 32 ? k - b0 : 32;
+#pragma unroll 4
+        for (int t = 0; t < nb; ++t) {
+          const int bb = b0 + t;
+          double f = (in && bb <= a) ? F[(int64_t)bb * k + a] : 0.0;
+          if (bb == a) f *= 0.5;
+#pragma unroll
+          for (int r = 0; r < kDhRows; ++r) M[r] = fma(f, __shfl_sync(0xffffffffu, u[r], t), M[r]);
+        }
+      }
+      if (in) {
+        const double s1 = s[a];
+#pragma unroll
+        for (int r = 0; r < kDhRows; ++r) {
+          const int i = i0 + r;
+          if (i >= k) continue;
+          const double m = M[r] * s1;
+          xd[r] = fma(s[(int64_t)i * k + a], m, xd[r]);
+          if (i + 1 < k) xy[r] = fma(s[(int64_t)(i + 1) * k + a], m, xy[r]);
+          if (i > 0) xz[r] = fma(s[(int64_t)(i - 1) * k + a], m, xz[r]);
+        }
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < kDhRows; ++r) {
+      const double d = warp_sum(xd[r]), y = warp_sum(xy[r]), z = warp_sum(xz[r]);
+      if (lane == 0 && i0 + r < k) {
+        gd[i0 + r] = d;
+        gy[i0 + r] = y;
+        gz[i0 + r] = z;
+      }
+    }
+  }
+  double v = 0.0;
+  if (warp == 0) {
+    for (int a = lane; a < k; a += 32) v = fma(fw[a] * s[a], s[a], v);
+    v = warp_sum(v);
+  }
+  __syncthreads();
+  const double sc = scale[b];
+  if (threadIdx.x == 0) values[b] = sc * v;
+  for (int64_t t = threadIdx.x; t < (int64_t)k * k; t += blockDim.x) {
+    const int i = (int)(t / k), j = (int)(t - (int64_t)i * k);
+    double g = 0.0;
+    if (i == j)
+      g = 2.0 * gd[i];
+    else if (j == i + 1)
+      g = gy[i] + gz[j];
+    else if (i == j + 1)
+      g = gy[j] + gz[i];
+    out[t] = sc * g;
+  }
+}
+
+int launch_quadform_dh(int64_t k, int64_t p, const double *w, const double *S, const double *fw,
+                       const double *fp, const double *scale, double *values, double *dH, cudaStream_t s) {
+  if (p <= 0) return MFG_OK;
+  const size_t vecs = 3 * (size_t)k * 8, full = vecs + (size_t)k * k * 8;
+  const bool shared_f = full <= kDhSmem;
+  const size_t smem = shared_f ? full : vecs;
+  if (smem > kDhSmem) return MFG_ERR_UNSUPPORTED;
+  MFG_CUDA_TRY(cudaFuncSetAttribute(quadform_dh_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)kDhSmem));
+  const int64_t want = 32 * ceil_div(k, kDhRows);
+  quadform_dh_kernel<<<(unsigned)p, (unsigned)(want < kDhThreads ? want : kDhThreads), smem, s>>>(
+      (int)k, w, S, fw, fp, scale, shared_f, values, dH);
+  return MFG_LAUNCH_STATUS();
+}
+
 }  // namespace mfg

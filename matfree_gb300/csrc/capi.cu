@@ -1316,6 +1316,17 @@ int mfg_tridiag_eigh(int64_t k, int64_t p, const double *H, double *eigvals, dou
   return MFG_OK;
 }
 
+int mfg_quadform_dh(int64_t k, int64_t p, const double *eigvals, const double *eigvecs,
+                    const double *fw, const double *fprime_mid, const double *scale, double *values,
+                    double *dH, void *stream) {
+  if (k <= 0 || p <= 0 || !eigvals || !eigvecs || !fw || !fprime_mid || !scale || !values || !dH)
+    return MFG_ERR_BAD_ARG;
+  cudaStream_t s = as_stream(stream);
+  MFG_LAUNCH(MFG_PROF_QUAD, 8.0 * p * k * k * 3.0, 1.0 * p * k * k * k,
+             launch_quadform_dh(k, p, eigvals, eigvecs, fw, fprime_mid, scale, values, dH, s));
+  return MFG_OK;
+}
+
 int mfg_tridiag_quadrature(int64_t k, int64_t p, const double *H, int32_t fun, double param,
                            const double *scale, double *values, double *eigvals, double *first_sq,
                            void *stream) {

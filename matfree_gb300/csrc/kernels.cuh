@@ -113,6 +113,8 @@ int launch_adj_lincomb(const T *U, const T *lam, const T *R, const T *dq, int64_
 int launch_axpy_f64(double a, const double *x, double *y, int64_t m, cudaStream_t s);
 int gemm_rule_add(int64_t n_lo, int64_t n_hi, int64_t p_lo, int64_t p_hi, int bn, int split);
 int gemm_rules_clear();
+int launch_quadform_dh(int64_t k, int64_t p, const double *w, const double *S, const double *fw,
+                       const double *fp, const double *scale, double *values, double *dH, cudaStream_t s);
 // bytes of the partial sums of launch_panel_dot; launch_panel_dot writes column
 // `slot` (<Lam, Y>) and, with Q, column 2 (<Lam, Q>) of them
 size_t panel_dot_bytes();
