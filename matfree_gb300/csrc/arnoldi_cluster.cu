@@ -120,6 +120,8 @@ __global__ void __launch_bounds__(kCThreads + 32, 2) arnoldi_step_kernel(const C
   __syncthreads();
   // waited for before the first access to another CTA; the copies start at once
   c_cluster_arrive();
+  chain_wait();
+  chain_next();
 
   if (warp == kCWarps) {
     // copy warp: per probe the two vectors, slots 0 .. ns - 1, then every group's
@@ -686,7 +688,7 @@ static CPlan c_plan(int64_t n, int64_t p, int j) {
 // and Hh, nu_{j+1}.
 int launch_arnoldi_step(int j, int64_t k, int64_t n, int64_t p, float *Q, int64_t qb, int64_t ld, const float *W,
                         const float *Vin, int64_t vb, float *Vout, __nv_bfloat16 *hi, __nv_bfloat16 *lo, double *H,
-                        double *Hh, double *nu, int *status, cudaStream_t s) {
+                        double *Hh, double *nu, int *status, bool chained, cudaStream_t s) {
   if (p <= 0) return MFG_OK;
   const CPlan plan = c_plan(n, p, j);
   if (plan.S == 0 || j > kCMaxCols) return MFG_ERR_UNSUPPORTED;
@@ -714,7 +716,7 @@ int launch_arnoldi_step(int j, int64_t k, int64_t n, int64_t p, float *Q, int64_
   a.status = status;
   auto kern = j == 0 ? c_kernel<true>(plan.wr) : c_kernel<false>(plan.wr);
   const size_t smem = c_fixed(plan.R, plan.wr) + (size_t)plan.slots * (kCWarps / plan.wr) * c_gc(plan.wr) * plan.R * 4;
-  return c_launch(kern, plan.S, plan.S * (p < plan.clusters ? p : plan.clusters), smem, a, s);
+  return c_launch(kern, plan.S, plan.S * (p < plan.clusters ? p : plan.clusters), smem, a, chained, s);
 }
 
 // H of every probe from what the steps left (`band`: its tridiagonal part only);

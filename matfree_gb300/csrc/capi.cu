@@ -178,12 +178,28 @@ static char *ws_base(void *workspace) {
   return reinterpret_cast<char *>(align_up((size_t)workspace, 256));
 }
 
+// Whether the launches of a solve's loop are chained (chain_wait in common.cuh); not
+// in a caller's stream capture, whose nodes keep full dependencies.  The bf16
+// products and the steps after any product are (n = 512, k = 16, 32 probes: 547 -> 451
+// us per solve; n = 3001, k = 32, 64: 1290 -> 1123; n = 8192, k = 32, 128 probes of the
+// product form 7.31 -> 6.89 ms); the float32 and float64 products are not: their
+// small CTAs crowd onto the SMs that come free first (n = 2000, k = 32, 64 probes: 1600 ->
+// 1819 us with them, 1497 with the steps alone).
+static bool chain_ok(cudaStream_t s) {
+  cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &c) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return false;
+  }
+  return c == cudaStreamCaptureStatusNone;
+}
+
 // W (ld) = A V (ldv); vhi/vlo are the bf16 copies of V (ldvb) for the
 // tensor-core precisions, panel a contiguous scratch panel for callbacks.
 template <typename T>
 static int apply_op(const mfg_operator *op, const T *V, int64_t ldv, T *W, int64_t ldw, int64_t p,
                     const __nv_bfloat16 *vhi, const __nv_bfloat16 *vlo, int64_t ldvb, T *panel,
-                    int *status, cudaStream_t s) {
+                    int *status, cudaStream_t s, bool chained = false) {
   const int64_t n = op->n;
   switch (op->kind) {
     case MFG_OP_DENSE:
@@ -195,7 +211,7 @@ static int apply_op(const mfg_operator *op, const T *V, int64_t ldv, T *W, int64
             op->precision == MFG_PREC_BF16X3 ? reinterpret_cast<const __nv_bfloat16 *>(op->a_lo) : nullptr;
         return launch_dense_tcgen05(reinterpret_cast<const __nv_bfloat16 *>(op->a), alo, op->lda,
                                     vhi, op->precision == MFG_PREC_BF16X3 ? vlo : nullptr, ldvb,
-                                    V, ldv, W, ldw, n, p, op->shift, status, s);
+                                    V, ldv, W, ldw, n, p, op->shift, status, chained, s);
       }
       return MFG_ERR_UNSUPPORTED;
     case MFG_OP_CSR:
@@ -283,14 +299,15 @@ static int run_two_sweep(const mfg_operator *op, int64_t k, int64_t p, int64_t l
     if (fused) {
       // a step is the product and one launch: while a probe's vector fits the
       // registers of a cluster (n <= 32768)
+      const bool chained = chain_ok(s);
       for (int64_t j = 0; j < k; ++j) {
         MFG_LAUNCH(MFG_PROF_APPLY, ab, af,
-                   apply_op<T>(op, j == 0 ? Q : Vt, j == 0 ? qb : ld, Wb, ld, p, hi, lo, ld, panel, status, s));
+                   apply_op<T>(op, j == 0 ? Q : Vt, j == 0 ? qb : ld, Wb, ld, p, hi, lo, ld, panel, status, s, chained));
         const bool more = j + 1 < k;
         MFG_LAUNCH(MFG_PROF_SUBPROJ, (j + (more || R ? 4.0 : 3.0)) * vecb + (more ? bfb : 0.0),
                    (8.0 * j + 10.0) * vecb / sizeof(T),
                    launch_arnoldi_step((int)j, k, n, p, Q, qb, ld, Wb, j == 0 ? Q : Vt, j == 0 ? qb : ld,
-                                       (more || R) ? Vt : nullptr, more ? hi : nullptr, lo, H, Hh, nu, status, s));
+                                       (more || R) ? Vt : nullptr, more ? hi : nullptr, lo, H, Hh, nu, status, chained, s));
       }
       MFG_LAUNCH(MFG_PROF_OTHER, 24.0 * p * k * k, full_h ? 2.0 / 3.0 * p * k * k * k : 0.0,
                  launch_arnoldi_h(k, p, H, Hh, nu, !full_h, R ? cf : nullptr, s));
@@ -396,10 +413,11 @@ static int run_hessenberg(const mfg_operator *op, int64_t k, int64_t p, const T 
              launch_scale<T>(V, ld, n, p, len0, Q, qb, hi, lo, ld, s));
   if (reortho == 3) return run_two_sweep<T>(op, k, p, ld, Q, H, full_h, R, L, ws, s);
 
+  const bool chained = chain_ok(s);
   for (int64_t j = 0; j < k; ++j) {
     const T *qj = Q + j * ld;
     MFG_LAUNCH(MFG_PROF_APPLY, ab, af,
-               apply_op<T>(op, qj, qb, Wb, ld, p, hi, lo, ld, panel, status, s));
+               apply_op<T>(op, qj, qb, Wb, ld, p, hi, lo, ld, panel, status, s, chained));
     const int ncols = (int)(j + 1);
     const double pb = (ncols + 1.0) * vecb, pf = 2.0 * ncols * vecb / sizeof(T);
     const double ub = (ncols + 2.0) * vecb;
@@ -430,7 +448,7 @@ static int run_hessenberg(const mfg_operator *op, int64_t k, int64_t p, const T 
       MFG_LAUNCH(MFG_PROF_SUBPROJ, (ncols + 2.0) * vecb + (last ? 0.0 : bfb), (reortho ? 4.0 : 2.0) * pf,
                  launch_gs_cluster<T>(Q, qb, ld, ncols, Wb, n, p, reortho ? 4 : 2, nullptr, 0, nullptr, 0, H + j,
                                       k * k, k, norm, hsub, k * k, last ? Wb : nullptr,
-                                      last ? nullptr : Q + (j + 1) * ld, qb, last ? nullptr : hi, lo, status, s));
+                                      last ? nullptr : Q + (j + 1) * ld, qb, last ? nullptr : hi, lo, status, chained, s));
       continue;
     }
     // first pass: h = Q^T w into column j of H
@@ -640,12 +658,13 @@ static int run_adjoint(const mfg_operator *op, int64_t k, int64_t p, int64_t ld,
     MFG_CUDA_TRY(cudaMemcpy2DAsync(Lam + (k - 1) * ld, qb * sizeof(T), lam, ld * sizeof(T), ld * sizeof(T), p,
                                    cudaMemcpyDeviceToDevice, s));
     if (hi) MFG_TRY(launch_split_bf16((const float *)lam, p, n, ld, hi, lo, ld, s));
+    const bool chained = chain_ok(s);
     for (int64_t idx = k - 1; idx >= 0; --idx) {
       MFG_LAUNCH(MFG_PROF_APPLY, ab, af,
-                 apply_op<T>(op, Lam + idx * ld, qb, U, ld, p, hi, lo, ld, panel, status, s));
+                 apply_op<T>(op, Lam + idx * ld, qb, U, ld, p, hi, lo, ld, panel, status, s, chained));
       MFG_LAUNCH(MFG_PROF_SUBPROJ, (2.0 * k - idx + 4.0) * vecb, (4.0 * k + 4.0 * idx + 8.0) * vecb / sizeof(T),
                  launch_adj_cluster<T>(Q, qb, ld, (int)k, (int)idx, U, Lam, R, dQ ? dQ + idx * ld : nullptr, H, Pi, dH,
-                                       gamma, Gamma, c, dv, n, p, hi, lo, status, s));
+                                       gamma, Gamma, c, dv, n, p, hi, lo, status, chained, s));
     }
     return MFG_OK;
   }
@@ -838,22 +857,23 @@ static int run_bidiag(const mfg_operator *A, const mfg_operator *At, int64_t k, 
     return MFG_OK;
   };
 
+  const bool chained = chain_ok(s);
   for (int64_t i = 0; i < k; ++i) {
     const bool last = i + 1 == k;
     // left vector: u_i = (A v_i - beta_i u_{i-1}) reorthogonalised, / alpha_i
     MFG_LAUNCH(MFG_PROF_APPLY, ab, af,
-               apply_op<T>(A, Vb + i * ld, qb, Wb, ld, p, hiA, loA, ld, panel, status, s));
+               apply_op<T>(A, Vb + i * ld, qb, Wb, ld, p, hiA, loA, ld, panel, status, s, chained));
     if (gs_cluster_applies(n, i + 1, 0)) {
       // everything of a side after its product as one launch
       MFG_LAUNCH(MFG_PROF_SUBPROJ, (i + 3.0) * vecb, (8.0 * i + 6.0) * vecb / sizeof(T),
                  launch_gs_cluster<T>(U, qb, ld, (int)i, Wb, n, p, 4, i > 0 ? U + (i - 1) * ld : nullptr, qb, betas + i,
-                                      k, h1, k, 1, norm, alphas + i, k, nullptr, U + i * ld, qb, hi, lo, status, s));
+                                      k, h1, k, 1, norm, alphas + i, k, nullptr, U + i * ld, qb, hi, lo, status, chained, s));
       MFG_LAUNCH(MFG_PROF_APPLY, tb, tf,
-                 apply_op<T>(At, U + i * ld, qb, Wb, ld, p, hiT, loT, ld, panel, status, s));
+                 apply_op<T>(At, U + i * ld, qb, Wb, ld, p, hiT, loT, ld, panel, status, s, chained));
       MFG_LAUNCH(MFG_PROF_SUBPROJ, (i + 4.0) * vecb, (8.0 * i + 14.0) * vecb / sizeof(T),
                  launch_gs_cluster<T>(Vb, qb, ld, (int)(i + 1), Wb, n, p, 4, Vb + i * ld, qb, alphas + i, k, h1, k, 1,
                                       norm, last ? nullptr : betas + i + 1, k, last ? Wb : nullptr,
-                                      last ? nullptr : Vb + (i + 1) * ld, qb, last ? nullptr : hi, lo, status, s));
+                                      last ? nullptr : Vb + (i + 1) * ld, qb, last ? nullptr : hi, lo, status, chained, s));
       continue;
     }
     if (i > 0)
@@ -953,14 +973,15 @@ static int run_cg(const mfg_operator *op, int64_t p, const T *B, T *X, int64_t l
   // Iteration it counts the rows that keep running into nactive[it & 1] and
   // zeroes nactive[(it + 1) & 1] for the next one.
   const bool small = n <= kCgSmallMaxN;
-  auto iteration = [&](int64_t it) -> int {
+  const bool chained = chain_ok(s);
+  auto iteration = [&](int64_t it, bool apply_chained) -> int {
     double *rc = rs[it & 1], *rn = rs[(it + 1) & 1];
     int *na = nactive + (it & 1), *na_next = nactive + ((it + 1) & 1);
-    MFG_LAUNCH(MFG_PROF_APPLY, ab, af, apply_op<T>(op, P, ld, W, ld, p, hi, lo, ld, nullptr, status, s));
+    MFG_LAUNCH(MFG_PROF_APPLY, ab, af, apply_op<T>(op, P, ld, W, ld, p, hi, lo, ld, nullptr, status, s, apply_chained));
     if (small) {
       MFG_LAUNCH(MFG_PROF_SUB, 7.0 * vecb, 10.0 * vecb / sizeof(T),
                  launch_cg_step_small<T>(X, R, P, W, ld, n, p, rc, thr, rn, na, na_next, iters,
-                                         hi, lo, s));
+                                         hi, lo, chained, s));
       return MFG_OK;
     }
     MFG_LAUNCH(MFG_PROF_PROJ, 2.0 * vecb, 2.0 * vecb / sizeof(T),
@@ -990,7 +1011,7 @@ static int run_cg(const mfg_operator *op, int64_t p, const T *B, T *X, int64_t l
         capture_failed = true;
         if (cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
           int st = MFG_OK;
-          for (int64_t t = 0; t < blk && st == MFG_OK; ++t) st = iteration(it + t);
+          for (int64_t t = 0; t < blk && st == MFG_OK; ++t) st = iteration(it + t, chained && t > 0);
           cudaGraph_t g = nullptr;
           const cudaError_t ec = cudaStreamEndCapture(s, &g);
           if (st == MFG_OK && ec == cudaSuccess && g &&
@@ -1002,7 +1023,7 @@ static int run_cg(const mfg_operator *op, int64_t p, const T *B, T *X, int64_t l
       }
       if (exec && cudaGraphLaunch(exec, s) == cudaSuccess) done = true;
     }
-    for (int64_t t = 0; !done && t < blk && rc_loop == MFG_OK; ++t) rc_loop = iteration(it + t);
+    for (int64_t t = 0; !done && t < blk && rc_loop == MFG_OK; ++t) rc_loop = iteration(it + t, chained);
     if (rc_loop != MFG_OK) break;
     const int *last_count = nactive + ((it + blk - 1) & 1);
     it += blk;

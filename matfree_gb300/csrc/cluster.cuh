@@ -200,20 +200,15 @@ inline void c_count_clusters(K kern, int (&clusters)[5]) {
   (void)cudaGetLastError();
 }
 
+// Larger clusters are not chained: placed on SMs as these come free they no longer all
+// fit at once (n = 16384, k = 64, 256 probes, S = 8: 29.0 -> 35.2 ms per solve; S = 4 at n =
+// 8192, 128 probes, k = 48: 17.4 -> 17.0).
+constexpr int kCChainS = 4;
+
 template <typename K, typename A>
-inline int c_launch(K kern, int S, int64_t ctas, size_t smem, const A &args, cudaStream_t s) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)ctas);
-  cfg.blockDim = dim3(kCThreads + 32);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)S;
-  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  MFG_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, args));
+inline int c_launch(K kern, int S, int64_t ctas, size_t smem, const A &args, bool chained, cudaStream_t s) {
+  MFG_CUDA_TRY(launch_kernel(kern, dim3((unsigned)ctas), kCThreads + 32, smem, (unsigned)S, chained && S <= kCChainS, s,
+                             args));
   return MFG_LAUNCH_STATUS();
 }
 

@@ -101,6 +101,53 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar_saddr, uint32_t p
     }
   }
 }
+
+// ---------------------------------------------------------------------------
+// Chained launches: inside a solve's loop a kernel may be launched while the one
+// before it on the stream still runs (programmatic stream serialization), so that
+// its launch, barrier set-up, TMEM allocation and first operator reads overlap that
+// kernel's end.  Every thread calls chain_wait() before it touches memory that an
+// earlier kernel of the loop reads or writes: it returns once the kernel before
+// has completed and its writes are visible.  chain_next() afterwards lets the kernel
+// after it start, so at most two kernels of a chain are resident, and all that came
+// before the first of them has completed.  Only the operator, which no kernel of the
+// loop writes, may be read before chain_wait(): the loop's first kernels are ordinary
+// launches, behind whatever wrote the operator.
+//
+// Two to three microseconds a launch: figures at chain_ok (capi.cu).
+// ---------------------------------------------------------------------------
+
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// A launch on `s`, as clusters of `cluster` CTAs along x (0: the kernel's own) and
+// chained to the kernel before it if asked.
+template <typename... P, typename... A>
+inline cudaError_t launch_kernel(void (*kern)(P...), dim3 grid, unsigned threads, size_t smem, unsigned cluster,
+                                 bool chained, cudaStream_t s, A &&...args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[2];
+  unsigned na = 0;
+  if (cluster) {
+    attr[na].id = cudaLaunchAttributeClusterDimension;
+    attr[na].val.clusterDim.x = cluster;
+    attr[na].val.clusterDim.y = attr[na].val.clusterDim.z = 1;
+    ++na;
+  }
+  if (chained) {
+    attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[na].val.programmaticStreamSerializationAllowed = 1;
+    ++na;
+  }
+  cfg.attrs = attr;
+  cfg.numAttrs = na;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
 // 16-byte vector type per element type: 4 floats or 2 doubles.

@@ -269,6 +269,8 @@ dense_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_ahi,
   // barriers of both CTAs are initialised before any copy or commit reaches them
   cluster_sync_all();
   tc_fence_after();
+  chain_wait();
+  chain_next();
   const uint32_t tmem = sh->tmem_base;
   const uint32_t full0_lead = map_to_rank(smem_u32(&sh->full[0]), 0);
 
@@ -467,17 +469,32 @@ dense_tcgen05_splitk_kernel(const __grid_constant__ CUtensorMap map_ahi,
   tc_fence_after();
   const uint32_t tmem = sh->tmem_base;
 
+  auto load_operator = [&](int kt, int s) {
+    uint8_t *st = tiles + (size_t)s * stage_bytes;
+    mbar_arrive_expect_tx(&sh->full[s], stage_bytes);
+    const int kx = (kb0 + kt) * kSplitKBK;
+    tma_load_2d(st, &map_ahi, &sh->full[s], kx, m0);
+    if (kSplit) tma_load_2d(st + a_bytes + b_bytes, &map_alo, &sh->full[s], kx, m0);
+  };
+  // a ring's worth of the operator before the panel is known to be there
+  const int ahead = num_k < stages ? num_k : stages;
+  if (threadIdx.x == 0)
+    for (int kt = 0; kt < ahead; ++kt) load_operator(kt, kt);
+  __syncwarp();
+  chain_wait();
+  chain_next();
+
   if (warp == 0) {
     if (lane == 0) {
       int issued = 0, s = 0;
       uint32_t ph = 0;
       for (int kt = 0; kt < num_k; ++kt) {
-        if (!mbar_wait(&sh->empty[s], ph ^ 1u, abort_flag, status)) break;
+        if (kt >= ahead) {
+          if (!mbar_wait(&sh->empty[s], ph ^ 1u, abort_flag, status)) break;
+          load_operator(kt, s);
+        }
         uint8_t *st = tiles + (size_t)s * stage_bytes;
-        mbar_arrive_expect_tx(&sh->full[s], stage_bytes);
         const int kx = (kb0 + kt) * kSplitKBK;
-        tma_load_2d(st, &map_ahi, &sh->full[s], kx, m0);
-        if (kSplit) tma_load_2d(st + a_bytes + b_bytes, &map_alo, &sh->full[s], kx, m0);
         tma_load_2d(st + a_bytes, &map_bhi, &sh->full[s], kx, b0);
         if (kSplit) tma_load_2d(st + 2 * a_bytes + b_bytes, &map_blo, &sh->full[s], kx, b0);
         ++issued;
@@ -715,6 +732,8 @@ dense_tcgen05_pair_persistent_kernel(const __grid_constant__ CUtensorMap map_ahi
   tc_fence_before();
   cluster_sync_all();
   tc_fence_after();
+  chain_wait();
+  chain_next();
   const uint32_t tmem = sh->tmem_base;
   const uint32_t full0_lead = map_to_rank(smem_u32(&sh->full[0]), 0);
 
@@ -951,6 +970,10 @@ __device__ __forceinline__ uint4 ld_stream16(const __nv_bfloat16 *p) {
   return v;
 }
 
+__device__ __forceinline__ void l2_prefetch(const void *p) {
+  asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+}
+
 __device__ __forceinline__ void bf16x8_to_float(const uint4 &u, float (&f)[8]) {
   const uint32_t w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
@@ -977,7 +1000,7 @@ __device__ __forceinline__ void gemv_rows(const __nv_bfloat16 *__restrict__ Ahi,
                                           const __nv_bfloat16 *__restrict__ Vlo, int64_t ldvb,
                                           const float *__restrict__ Vf, int64_t ldvf,
                                           float *__restrict__ W, int64_t ldw, int n, int p,
-                                          float shift) {
+                                          float shift, int ahead) {
   constexpr int kAhead = kDeep ? 512 : 256;
   __shared__ float part[kGemvWarps][P];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -986,13 +1009,23 @@ __device__ __forceinline__ void gemv_rows(const __nv_bfloat16 *__restrict__ Ahi,
   float acc[P];
 #pragma unroll
   for (int b = 0; b < P; ++b) acc[b] = 0.f;
+  const int64_t row = m < n ? m : 0;
+  const __nv_bfloat16 *ah = Ahi + row * lda;
+  const __nv_bfloat16 *al = kSplit ? Alo + row * lda : nullptr;
+  const int n8 = n & ~7;
+  const int seg_len = ((n8 / 8 + kGemvSeg - 1) / kGemvSeg) * 8;  // a multiple of 8 columns
+  const int c0 = seg * seg_len;
+  const int c1 = min(c0 + seg_len, n8);
+  if ((int)blockIdx.x < ahead && m < n) {
+    // chained: this segment on its way to L2 while the kernel before ends
+    for (int c = c0 + lane * 64; c < c1; c += 32 * 64) {
+      l2_prefetch(ah + c);
+      if (kSplit) l2_prefetch(al + c);
+    }
+  }
+  chain_wait();
+  chain_next();
   if (m < n) {  // warp-uniform; every warp reaches the barrier below
-    const __nv_bfloat16 *ah = Ahi + m * lda;
-    const __nv_bfloat16 *al = kSplit ? Alo + m * lda : nullptr;
-    const int n8 = n & ~7;
-    const int seg_len = ((n8 / 8 + kGemvSeg - 1) / kGemvSeg) * 8;  // a multiple of 8 columns
-    const int c0 = seg * seg_len;
-    const int c1 = min(c0 + seg_len, n8);
     const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
     uint4 h0 = zero, l0 = zero, h1 = zero, l1 = zero;
     const int cl = c0 + lane * 8;
@@ -1085,8 +1118,8 @@ dense_gemv1_kernel(const __nv_bfloat16 *__restrict__ Ahi, const __nv_bfloat16 *_
                    int64_t lda, const __nv_bfloat16 *__restrict__ Vhi,
                    const __nv_bfloat16 *__restrict__ Vlo, int64_t ldvb,
                    const float *__restrict__ Vf, int64_t ldvf, float *__restrict__ W, int64_t ldw,
-                   int n, int p, float shift) {
-  gemv_rows<1, kSplit, true>(Ahi, Alo, lda, Vhi, Vlo, ldvb, Vf, ldvf, W, ldw, n, p, shift);
+                   int n, int p, float shift, int ahead) {
+  gemv_rows<1, kSplit, true>(Ahi, Alo, lda, Vhi, Vlo, ldvb, Vf, ldvf, W, ldw, n, p, shift, ahead);
 }
 
 template <int P, bool kSplit>
@@ -1095,31 +1128,26 @@ dense_gemv_kernel(const __nv_bfloat16 *__restrict__ Ahi, const __nv_bfloat16 *__
                   int64_t lda, const __nv_bfloat16 *__restrict__ Vhi,
                   const __nv_bfloat16 *__restrict__ Vlo, int64_t ldvb,
                   const float *__restrict__ Vf, int64_t ldvf, float *__restrict__ W, int64_t ldw,
-                  int n, int p, float shift) {
-  gemv_rows<P, kSplit, false>(Ahi, Alo, lda, Vhi, Vlo, ldvb, Vf, ldvf, W, ldw, n, p, shift);
+                  int n, int p, float shift, int ahead) {
+  gemv_rows<P, kSplit, false>(Ahi, Alo, lda, Vhi, Vlo, ldvb, Vf, ldvf, W, ldw, n, p, shift, ahead);
 }
 
+// CTAs that fetch their rows ahead when chained: those resident at first, up to 32 MB
+constexpr int64_t kGemvAheadBytes = 32 << 20;
+
 template <int P>
-static void launch_gemv_p(bool split, const __nv_bfloat16 *A_hi, const __nv_bfloat16 *A_lo,
-                          int64_t lda, const __nv_bfloat16 *V_hi, const __nv_bfloat16 *V_lo,
-                          int64_t ldvb, const float *Vf, int64_t ldvf, float *W, int64_t ldw,
-                          int n, int p, float shift, cudaStream_t s) {
+static int launch_gemv_p(bool split, const __nv_bfloat16 *A_hi, const __nv_bfloat16 *A_lo,
+                         int64_t lda, const __nv_bfloat16 *V_hi, const __nv_bfloat16 *V_lo,
+                         int64_t ldvb, const float *Vf, int64_t ldvf, float *W, int64_t ldw,
+                         int n, int p, float shift, bool chained, cudaStream_t s) {
   const unsigned grid = (unsigned)((n + kGemvRows - 1) / kGemvRows);
-  if constexpr (P == 1) {
-    if (split)
-      dense_gemv1_kernel<true><<<grid, 32 * kGemvWarps, 0, s>>>(A_hi, A_lo, lda, V_hi, V_lo, ldvb,
-                                                                Vf, ldvf, W, ldw, n, p, shift);
-    else
-      dense_gemv1_kernel<false><<<grid, 32 * kGemvWarps, 0, s>>>(A_hi, A_lo, lda, V_hi, V_lo,
-                                                                 ldvb, Vf, ldvf, W, ldw, n, p, shift);
-  } else {
-    if (split)
-      dense_gemv_kernel<P, true><<<grid, 32 * kGemvWarps, 0, s>>>(A_hi, A_lo, lda, V_hi, V_lo,
-                                                                  ldvb, Vf, ldvf, W, ldw, n, p, shift);
-    else
-      dense_gemv_kernel<P, false><<<grid, 32 * kGemvWarps, 0, s>>>(A_hi, A_lo, lda, V_hi, V_lo,
-                                                                   ldvb, Vf, ldvf, W, ldw, n, p, shift);
-  }
+  const int64_t fit = kGemvAheadBytes / ((int64_t)kGemvRows * n * (split ? 4 : 2));
+  const int ahead = !chained ? 0 : (int)(fit < 5 * 152 ? fit : 5 * 152);
+  auto kern = split ? dense_gemv_kernel<P, true> : dense_gemv_kernel<P, false>;
+  if constexpr (P == 1) kern = split ? dense_gemv1_kernel<true> : dense_gemv1_kernel<false>;
+  MFG_CUDA_TRY(launch_kernel(kern, dim3(grid), 32 * kGemvWarps, 0, 0, chained, s, A_hi, A_lo, lda, V_hi, V_lo, ldvb,
+                             Vf, ldvf, W, ldw, n, p, shift, ahead));
+  return MFG_LAUNCH_STATUS();
 }
 
 constexpr int64_t kGemvMaxP = 8;
@@ -1127,19 +1155,17 @@ constexpr int64_t kGemvMaxP = 8;
 static int launch_dense_gemv(const __nv_bfloat16 *A_hi, const __nv_bfloat16 *A_lo, int64_t lda,
                              const __nv_bfloat16 *V_hi, const __nv_bfloat16 *V_lo, int64_t ldvb,
                              const float *Vf, int64_t ldvf, float *W, int64_t ldw, int64_t n,
-                             int64_t p, double shift, cudaStream_t s) {
+                             int64_t p, double shift, bool chained, cudaStream_t s) {
   const bool split = A_lo != nullptr;
   const int ni = (int)n, pi = (int)p;
   const float sh = (float)shift;
   if (p == 1)
-    launch_gemv_p<1>(split, A_hi, A_lo, lda, V_hi, V_lo, ldvb, Vf, ldvf, W, ldw, ni, pi, sh, s);
-  else if (p == 2)
-    launch_gemv_p<2>(split, A_hi, A_lo, lda, V_hi, V_lo, ldvb, Vf, ldvf, W, ldw, ni, pi, sh, s);
-  else if (p <= 4)
-    launch_gemv_p<4>(split, A_hi, A_lo, lda, V_hi, V_lo, ldvb, Vf, ldvf, W, ldw, ni, pi, sh, s);
-  else
-    launch_gemv_p<8>(split, A_hi, A_lo, lda, V_hi, V_lo, ldvb, Vf, ldvf, W, ldw, ni, pi, sh, s);
-  return MFG_LAUNCH_STATUS();
+    return launch_gemv_p<1>(split, A_hi, A_lo, lda, V_hi, V_lo, ldvb, Vf, ldvf, W, ldw, ni, pi, sh, chained, s);
+  if (p == 2)
+    return launch_gemv_p<2>(split, A_hi, A_lo, lda, V_hi, V_lo, ldvb, Vf, ldvf, W, ldw, ni, pi, sh, chained, s);
+  if (p <= 4)
+    return launch_gemv_p<4>(split, A_hi, A_lo, lda, V_hi, V_lo, ldvb, Vf, ldvf, W, ldw, ni, pi, sh, chained, s);
+  return launch_gemv_p<8>(split, A_hi, A_lo, lda, V_hi, V_lo, ldvb, Vf, ldvf, W, ldw, ni, pi, sh, chained, s);
 }
 
 // ---------------------------------------------------------------------------
@@ -1306,7 +1332,7 @@ static SplitKPlan splitk_plan(int64_t n, int64_t p, bool split) {
 static int launch_splitk(const __nv_bfloat16 *A_hi, const __nv_bfloat16 *A_lo, int64_t lda,
                          const __nv_bfloat16 *V_hi, const __nv_bfloat16 *V_lo, int64_t ldvb,
                          const float *Vf, int64_t ldvf, float *W, int64_t ldw, int64_t n, int64_t p,
-                         const SplitKPlan &plan, double shift, int *status, cudaStream_t s) {
+                         const SplitKPlan &plan, double shift, int *status, bool chained, cudaStream_t s) {
   const int bn = plan.bn, S = plan.S, mt = plan.mt;
   const bool split = A_lo != nullptr;
   const uint32_t rows = (uint32_t)(mt * kBM);
@@ -1331,27 +1357,16 @@ static int launch_splitk(const __nv_bfloat16 *A_hi, const __nv_bfloat16 *A_lo, i
   auto kern = mt == 2 ? (split ? dense_tcgen05_splitk_kernel<true, 2> : dense_tcgen05_splitk_kernel<false, 2>)
                       : (split ? dense_tcgen05_splitk_kernel<true, 1> : dense_tcgen05_splitk_kernel<false, 1>);
   MFG_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)S, (unsigned)ceil_div(n, rows), (unsigned)ceil_div(p, bn));
-  cfg.blockDim = dim3(kGemmThreads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)S;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  MFG_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, mahi, malo, mbhi, mblo, Vf, ldvf, W, ldw, (int)n, (int)p,
-                                  bn, stages, cols, (float)shift, vec_ok, status));
+  MFG_CUDA_TRY(launch_kernel(kern, dim3((unsigned)S, (unsigned)ceil_div(n, rows), (unsigned)ceil_div(p, bn)),
+                             kGemmThreads, smem, (unsigned)S, chained, s, mahi, malo, mbhi, mblo, Vf, ldvf, W, ldw,
+                             (int)n, (int)p, bn, stages, cols, (float)shift, vec_ok, status));
   return MFG_LAUNCH_STATUS();
 }
 
 int launch_dense_tcgen05(const __nv_bfloat16 *A_hi, const __nv_bfloat16 *A_lo, int64_t lda,
                          const __nv_bfloat16 *V_hi, const __nv_bfloat16 *V_lo, int64_t ldvb,
                          const float *Vf, int64_t ldvf, float *W, int64_t ldw, int64_t n, int64_t p,
-                         double shift, int *status, cudaStream_t s) {
+                         double shift, int *status, bool chained, cudaStream_t s) {
   if (n <= 0 || p <= 0) return MFG_OK;
   if (!tcgen05_supported_shape(n, p)) return MFG_ERR_UNSUPPORTED;
   const bool split = (A_lo != nullptr);
@@ -1359,7 +1374,8 @@ int launch_dense_tcgen05(const __nv_bfloat16 *A_hi, const __nv_bfloat16 *A_lo, i
   if (lda % 8 != 0 || ldvb % 8 != 0 || ((uintptr_t)A_hi & 15) || ((uintptr_t)V_hi & 15))
     return MFG_ERR_BAD_ARG;
   if (p <= kGemvMaxP)
-    return launch_dense_gemv(A_hi, A_lo, lda, V_hi, V_lo, ldvb, Vf, ldvf, W, ldw, n, p, shift, s);
+    return launch_dense_gemv(A_hi, A_lo, lda, V_hi, V_lo, ldvb, Vf, ldvf, W, ldw, n, p, shift,
+                             chained, s);
   const GemmRule rule = n >= kPairMinRows ? gemm_rule_for(n, p) : GemmRule{0, 0, 0, 0, 0, 0};
   // Few probes are bound by the operator stream, and few tiles leave SMs
   // idle: the split-K cluster form.  More than 128 probes re-read the operator
@@ -1378,7 +1394,8 @@ int launch_dense_tcgen05(const __nv_bfloat16 *A_hi, const __nv_bfloat16 *A_lo, i
   if (!pair_rule && (n < kPairMinRows || p <= kSplitKMaxBN ||
                      row_tiles * ceil_div(p, kSplitKMaxBN) * 9 <= (int64_t)sms * 5)) {
     const SplitKPlan plan = splitk_plan(n, p, split);
-    return launch_splitk(A_hi, A_lo, lda, V_hi, V_lo, ldvb, Vf, ldvf, W, ldw, n, p, plan, shift, status, s);
+    return launch_splitk(A_hi, A_lo, lda, V_hi, V_lo, ldvb, Vf, ldvf, W, ldw, n, p, plan, shift, status,
+                         chained, s);
   }
   // CTA pairs (2-SM MMAs, M = 256); probes per tile: a multiple of 32 in [64, 256]
   const int64_t pt = p < 256 ? p : 256;
@@ -1410,7 +1427,8 @@ int launch_dense_tcgen05(const __nv_bfloat16 *A_hi, const __nv_bfloat16 *A_lo, i
     // grid.x: two CTAs per 256-row tile (the cluster dimension).  When the
     // tiles cover fewer than 60 % of the SMs (e.g. n = 8192: 64 CTAs), each
     // CTA streams its rows at a fixed rate and the SMs idle, so K is split in
-    // two halves (grid.z) whose partial products add into a zeroed W.
+    // two halves (grid.z) whose partial products add into a zeroed W (a zeroing
+    // on the stream ends a chain of launches).
     dim3 grid((unsigned)(2 * ((n + 2 * kBM - 1) / (2 * kBM))), (unsigned)((p + BN - 1) / BN));
     if (grid.y > 65535) return MFG_ERR_UNSUPPORTED;
     const int num_k_all = (int)((n + kBK - 1) / kBK);
@@ -1445,20 +1463,12 @@ int launch_dense_tcgen05(const __nv_bfloat16 *A_hi, const __nv_bfloat16 *A_lo, i
       uint32_t acc_cols = 32;
       while ((int)acc_cols < BN) acc_cols <<= 1;
       const size_t smem_p = 1024 + (size_t)stages * stage_bytes + sizeof(GemmSharedP);
-      dim3 pgrid((unsigned)(2 * sc.P), 1, 1);
-      if (split) {
-        MFG_CUDA_TRY(cudaFuncSetAttribute(dense_tcgen05_pair_persistent_kernel<true>,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_p));
-        dense_tcgen05_pair_persistent_kernel<true><<<pgrid, kGemmThreads, smem_p, s>>>(
-            mahi, malo, mbhi, mblo, Vf, ldvf, W, ldw, (int)n, (int)p, BN, stages, acc_cols, sc,
-            (float)shift, status);
-      } else {
-        MFG_CUDA_TRY(cudaFuncSetAttribute(dense_tcgen05_pair_persistent_kernel<false>,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_p));
-        dense_tcgen05_pair_persistent_kernel<false><<<pgrid, kGemmThreads, smem_p, s>>>(
-            mahi, malo, mbhi, mblo, Vf, ldvf, W, ldw, (int)n, (int)p, BN, stages, acc_cols, sc,
-            (float)shift, status);
-      }
+      const bool zeroed = sc.R > 0 && sc.Km < num_k_all;
+      auto kern = split ? dense_tcgen05_pair_persistent_kernel<true> : dense_tcgen05_pair_persistent_kernel<false>;
+      MFG_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_p));
+      MFG_CUDA_TRY(launch_kernel(kern, dim3((unsigned)(2 * sc.P)), kGemmThreads, smem_p, 0, chained && !zeroed, s, mahi,
+                                 malo, mbhi, mblo, Vf, ldvf, W, ldw, (int)n, (int)p, BN, stages, acc_cols, sc,
+                                 (float)shift, status));
       return MFG_LAUNCH_STATUS();
     }
     if (split_ok) {
@@ -1466,19 +1476,10 @@ int launch_dense_tcgen05(const __nv_bfloat16 *A_hi, const __nv_bfloat16 *A_lo, i
       MFG_CUDA_TRY(cudaMemset2DAsync(W, (size_t)ldw * sizeof(float), 0, (size_t)n * sizeof(float),
                                      (size_t)p, s));
     }
-    if (split) {
-      MFG_CUDA_TRY(cudaFuncSetAttribute(dense_tcgen05_pair_kernel<true>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      dense_tcgen05_pair_kernel<true><<<grid, kGemmThreads, smem, s>>>(
-          mahi, malo, mbhi, mblo, Vf, ldvf, W, ldw, (int)n, (int)p, BN, stages, cols,
-          (float)shift, status);
-    } else {
-      MFG_CUDA_TRY(cudaFuncSetAttribute(dense_tcgen05_pair_kernel<false>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      dense_tcgen05_pair_kernel<false><<<grid, kGemmThreads, smem, s>>>(
-          mahi, malo, mbhi, mblo, Vf, ldvf, W, ldw, (int)n, (int)p, BN, stages, cols,
-          (float)shift, status);
-    }
+    auto kern = split ? dense_tcgen05_pair_kernel<true> : dense_tcgen05_pair_kernel<false>;
+    MFG_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    MFG_CUDA_TRY(launch_kernel(kern, grid, kGemmThreads, smem, 0, chained && !split_ok, s, mahi, malo, mbhi, mblo, Vf,
+                               ldvf, W, ldw, (int)n, (int)p, BN, stages, cols, (float)shift, status));
     return MFG_LAUNCH_STATUS();
   }
 }

@@ -125,6 +125,8 @@ __global__ void __launch_bounds__(kCThreads + 32, 2) gs_cluster_kernel(const GsA
   }
   __syncthreads();
   c_cluster_arrive();  // waited for before the first access to another CTA
+  chain_wait();
+  chain_next();
 
   if (warp == kCWarps) {
     // copy warp: per probe the vectors after idx, then pass 1's slots, then of each
@@ -540,7 +542,7 @@ bool gs_cluster_applies(int64_t n, int64_t ncols, int64_t nextra) {
 // clusters the GPU holds, a round costing its meetings and the CTA's passes (40 GB/s
 // from L2; float64 also its FMAs, 1.7 a clock and SM for two CTAs).
 template <typename T, bool kAdj>
-static int g_run(GsArgs<T> &a, cudaStream_t s) {
+static int g_run(GsArgs<T> &a, bool chained, cudaStream_t s) {
   static const GSlots<T, kAdj> slots;
   if (a.p <= 0) return MFG_OK;
   a.cpad = (a.ncols + 7) / 8 * 8;
@@ -577,7 +579,7 @@ static int g_run(GsArgs<T> &a, cudaStream_t s) {
   if (wr == 0) return MFG_ERR_UNSUPPORTED;
   const size_t smem = g_fixed<T>(a.cpad, a.xpad, a.R, wr) +
                       (size_t)a.slots * (kCWarps / wr) * g_gc<T>(wr) * a.R * sizeof(T);
-  return c_launch(g_kernel<T, kAdj>(wr), a.S, a.S * (a.p < clusters ? a.p : clusters), smem, a, s);
+  return c_launch(g_kernel<T, kAdj>(wr), a.S, a.S * (a.p < clusters ? a.p : clusters), smem, a, chained, s);
 }
 
 // w (panel W; w -= prev_c prev first, if given) against basis vectors 0 .. ncols - 1,
@@ -586,7 +588,7 @@ template <typename T>
 int launch_gs_cluster(const T *Q, int64_t qb, int64_t ld, int ncols, const T *W, int64_t n, int64_t p, int passes,
                       const T *prev, int64_t prev_b, const double *prev_c, int64_t prev_cs, double *h, int64_t h_bs,
                       int64_t h_is, double *norm, double *norm2, int64_t norm2_bs, T *w_out, T *next, int64_t next_b,
-                      __nv_bfloat16 *hi, __nv_bfloat16 *lo, int *status, cudaStream_t s) {
+                      __nv_bfloat16 *hi, __nv_bfloat16 *lo, int *status, bool chained, cudaStream_t s) {
   GsArgs<T> a{};
   a.Q = Q;
   a.qb = qb;
@@ -612,7 +614,7 @@ int launch_gs_cluster(const T *Q, int64_t qb, int64_t ld, int ncols, const T *W,
   a.hi = hi;
   a.lo = lo;
   a.status = status;
-  return g_run<T, false>(a, s);
+  return g_run<T, false>(a, chained, s);
 }
 
 // Step idx of the adjoint after U = A lambda: row idx of Gamma, and lambda of step
@@ -621,7 +623,7 @@ template <typename T>
 int launch_adj_cluster(const T *Q, int64_t qb, int64_t ld, int k, int idx, const T *U, T *Lam, const T *res,
                        const T *dq, const double *H, const double *Pi, const double *dH, const double *gamma,
                        double *Gamma, const double *c, T *dv, int64_t n, int64_t p, __nv_bfloat16 *hi,
-                       __nv_bfloat16 *lo, int *status, cudaStream_t s) {
+                       __nv_bfloat16 *lo, int *status, bool chained, cudaStream_t s) {
   GsArgs<T> a{};
   a.Q = Q;
   a.qb = qb;
@@ -649,18 +651,18 @@ int launch_adj_cluster(const T *Q, int64_t qb, int64_t ld, int k, int idx, const
   a.hi = idx > 0 ? hi : nullptr;
   a.lo = lo;
   a.status = status;
-  return g_run<T, true>(a, s);
+  return g_run<T, true>(a, chained, s);
 }
 
 #define MFG_INST(T)                                                                                               \
   template int launch_gs_cluster<T>(const T *, int64_t, int64_t, int, const T *, int64_t, int64_t, int, const T *, \
                                     int64_t, const double *, int64_t, double *, int64_t, int64_t, double *,        \
                                     double *, int64_t, T *, T *, int64_t, __nv_bfloat16 *, __nv_bfloat16 *, int *, \
-                                    cudaStream_t);                                                                 \
+                                    bool, cudaStream_t);                                                           \
   template int launch_adj_cluster<T>(const T *, int64_t, int64_t, int, int, const T *, T *, const T *, const T *,  \
                                      const double *, const double *, const double *, const double *, double *,    \
                                      const double *, T *, int64_t, int64_t, __nv_bfloat16 *, __nv_bfloat16 *,      \
-                                     int *, cudaStream_t);
+                                     int *, bool, cudaStream_t);
 MFG_INST(float)
 MFG_INST(double)
 #undef MFG_INST

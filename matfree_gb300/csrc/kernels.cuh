@@ -59,9 +59,10 @@ int launch_twosweep_finish(T *Qj, int64_t q_bstride, const T *Z, int64_t w_bstri
 bool arnoldi_cluster_applies(int64_t n);
 int launch_arnoldi_step(int j, int64_t k, int64_t n, int64_t p, float *Q, int64_t qb, int64_t ld, const float *W,
                         const float *Vin, int64_t vb, float *Vout, __nv_bfloat16 *hi, __nv_bfloat16 *lo, double *H,
-                        double *Hh, double *nu, int *status, cudaStream_t s);
+                        double *Hh, double *nu, int *status, bool chained, cudaStream_t s);
 int launch_arnoldi_h(int64_t k, int64_t p, double *H, const double *Hh, const double *nu, bool band,
                      double *nu_last_inv, cudaStream_t s);
+// (chained: see chain_wait in common.cuh)
 // gs_cluster.cu: Gram-Schmidt twice with the norm and the normalisation, and a step
 // of the adjoint, as one launch each (n up to 32768)
 bool gs_cluster_applies(int64_t n, int64_t ncols, int64_t nextra);
@@ -69,12 +70,12 @@ template <typename T>
 int launch_gs_cluster(const T *Q, int64_t qb, int64_t ld, int ncols, const T *W, int64_t n, int64_t p, int passes,
                       const T *prev, int64_t prev_b, const double *prev_c, int64_t prev_cs, double *h, int64_t h_bs,
                       int64_t h_is, double *norm, double *norm2, int64_t norm2_bs, T *w_out, T *next, int64_t next_b,
-                      __nv_bfloat16 *hi, __nv_bfloat16 *lo, int *status, cudaStream_t s);
+                      __nv_bfloat16 *hi, __nv_bfloat16 *lo, int *status, bool chained, cudaStream_t s);
 template <typename T>
 int launch_adj_cluster(const T *Q, int64_t qb, int64_t ld, int k, int idx, const T *U, T *Lam, const T *res,
                        const T *dq, const double *H, const double *Pi, const double *dH, const double *gamma,
                        double *Gamma, const double *c, T *dv, int64_t n, int64_t p, __nv_bfloat16 *hi,
-                       __nv_bfloat16 *lo, int *status, cudaStream_t s);
+                       __nv_bfloat16 *lo, int *status, bool chained, cudaStream_t s);
 // conjugate gradients on probe-major panels (lanczos_kernels.cu)
 template <typename T>
 int launch_cg_init(const T *B, T *X, T *R, T *P, int64_t ld, int64_t n, int64_t p,
@@ -91,7 +92,7 @@ template <typename T>
 int launch_cg_step_small(T *X, T *R, T *P, const T *W, int64_t ld, int64_t n, int64_t p,
                          const double *rs, const double *thr, double *rs_next, int *nactive,
                          int *nactive_clear, int *iters, __nv_bfloat16 *hi, __nv_bfloat16 *lo,
-                         cudaStream_t s);
+                         bool chained, cudaStream_t s);
 template <typename T>
 int launch_cg_direction(T *P, const T *R, int64_t ld, int64_t n, int64_t p, const double *rs,
                         const double *rs_next, const double *thr, __nv_bfloat16 *hi,
@@ -158,7 +159,8 @@ bool make_plain_tensor_map_2d(void *map128, int elem_bytes, const void *base, in
 int launch_dense_tcgen05(const __nv_bfloat16 *A_hi, const __nv_bfloat16 *A_lo, int64_t lda,
                          const __nv_bfloat16 *V_hi, const __nv_bfloat16 *V_lo, int64_t ldvb,
                          const float *Vf, int64_t ldvf, float *W, int64_t ldw, int64_t n,
-                         int64_t p, double shift, int *status, cudaStream_t s);
+                         int64_t p, double shift, int *status, bool chained,
+                         cudaStream_t s);
 bool tcgen05_supported_shape(int64_t n, int64_t p);
 
 // wait_selftest.cu: a bounded wait on an mbarrier nothing arrives on

@@ -1368,6 +1368,8 @@ cg_step_small_kernel(T *__restrict__ X, T *__restrict__ R, T *__restrict__ P,
   __shared__ double red[33];
   __shared__ T coef;  // alpha, then beta: one float64 division each, in thread 0
   __shared__ int run;
+  chain_wait();
+  chain_next();
   const int64_t b = blockIdx.x;
   T *x = X + b * ld, *r = R + b * ld, *pv = P + b * ld;
   const T *w = W + b * ld;
@@ -1465,23 +1467,17 @@ template <typename T>
 int launch_cg_step_small(T *X, T *R, T *P, const T *W, int64_t ld, int64_t n, int64_t p,
                          const double *rs, const double *thr, double *rs_next, int *nactive,
                          int *nactive_clear, int *iters, __nv_bfloat16 *hi, __nv_bfloat16 *lo,
-                         cudaStream_t s) {
+                         bool chained, cudaStream_t s) {
   if (p <= 0 || n <= 0) return MFG_OK;
   if (n > kCgSmallMaxN || p > 0x7fffffff) return MFG_ERR_UNSUPPORTED;
   static_assert(kCgSmallMaxN == 8 * kCgSmallThreads, "elements per thread");
   const unsigned grid = (unsigned)p;
-  if (n <= kCgSmallThreads)
-    cg_step_small_kernel<T, 1><<<grid, kCgSmallThreads, 0, s>>>(
-        X, R, P, W, ld, n, rs, thr, rs_next, nactive, nactive_clear, iters, hi, lo);
-  else if (n <= 2 * kCgSmallThreads)
-    cg_step_small_kernel<T, 2><<<grid, kCgSmallThreads, 0, s>>>(
-        X, R, P, W, ld, n, rs, thr, rs_next, nactive, nactive_clear, iters, hi, lo);
-  else if (n <= 4 * kCgSmallThreads)
-    cg_step_small_kernel<T, 4><<<grid, kCgSmallThreads, 0, s>>>(
-        X, R, P, W, ld, n, rs, thr, rs_next, nactive, nactive_clear, iters, hi, lo);
-  else
-    cg_step_small_kernel<T, 8><<<grid, kCgSmallThreads, 0, s>>>(
-        X, R, P, W, ld, n, rs, thr, rs_next, nactive, nactive_clear, iters, hi, lo);
+  auto kern = n <= kCgSmallThreads       ? cg_step_small_kernel<T, 1>
+              : n <= 2 * kCgSmallThreads ? cg_step_small_kernel<T, 2>
+              : n <= 4 * kCgSmallThreads ? cg_step_small_kernel<T, 4>
+                                         : cg_step_small_kernel<T, 8>;
+  MFG_CUDA_TRY(launch_kernel(kern, dim3(grid), kCgSmallThreads, 0, 0, chained, s, X, R, P, W, ld, n, rs, thr, rs_next,
+                             nactive, nactive_clear, iters, hi, lo));
   return MFG_LAUNCH_STATUS();
 }
 
@@ -1805,7 +1801,7 @@ template int launch_twosweep_finish<float>(float *, int64_t, const float *, int6
                                    unsigned *, double *, int *, int *, int *, cudaStream_t);  \
   template int launch_cg_step_small<T>(T *, T *, T *, const T *, int64_t, int64_t, int64_t,     \
                                        const double *, const double *, double *, int *, int *, \
-                                       int *, __nv_bfloat16 *, __nv_bfloat16 *, cudaStream_t); \
+                                       int *, __nv_bfloat16 *, __nv_bfloat16 *, bool, cudaStream_t); \
   template int launch_cg_direction<T>(T *, const T *, int64_t, int64_t, int64_t,              \
                                       const double *, const double *, const double *,         \
                                       __nv_bfloat16 *, __nv_bfloat16 *, cudaStream_t);        \
