@@ -10,7 +10,7 @@
 //   1. the copy warp streams the probe's basis rows through a shared-memory
 //      ring (slots of GC vectors x R rows); q~ and w stay in registers; the
 //      per-thread products go through a warp butterfly per slot;
-//   2. the CTAs' float64 partial sums meet over distributed shared memory,
+//   2. the CTAs' two-float partial sums meet over distributed shared memory,
 //      every CTA adding all of them in rank order;
 //   3. q~ - Q h and w - Q g from the slots still in the ring first, then from
 //      the earlier vectors read again (from L2: the probes in flight are chosen
@@ -20,7 +20,8 @@
 //
 // The basis thus crosses HBM once per step, and the two vectors once in and once
 // out.  H is not formed here: the raw projections go to the places of H and Hh
-// that they end up in, and arnoldi_h_kernel turns them into H once per solve.
+// that they end up in, the step's scalars to rec, and arnoldi_h_kernel turns them
+// into H in float64 once per solve.
 // Two CTAs share an SM, so that one streams while the other is between passes.
 //
 // What bounds it: for few probes the chain of a step (about 8 us: loads, two
@@ -32,8 +33,8 @@
 // probes 14.7 -> 13.5 ms.  The separate launches remain for n > 32768, where a
 // cluster's registers no longer hold the two vectors.
 //
-// Sums: products and a warp's sum (256 rows) in float32, warps, CTAs and the
-// squared norms in float64 or its two-float equivalent, all in a fixed order.
+// Sums: products and a warp's sum (256 rows) in float32, warps, CTAs, the squared norms
+// and the scalars formed from them as two-float numbers, all in a fixed order.
 // Waits are bounded; after a failure a CTA's warps run on without waiting or
 // computing, still meeting every barrier, and the copies in flight are drained.
 
@@ -44,6 +45,8 @@ namespace mfg {
 
 constexpr int kCMaxCols = kTwoSweepMaxK - 1;  // basis vectors of a step
 static_assert(kCMaxCols == 128, "shared arrays");
+
+constexpr int kCRec = kTwoSweepRec;
 
 struct CStepArgs {
   const float *Q;  // probe stride qb, vector stride ld
@@ -56,7 +59,9 @@ struct CStepArgs {
   __nv_bfloat16 *hi, *lo;
   int64_t n, p;
   int j, k, R, S, slots;  // slots: of one group's ring
-  double *H, *Hh, *nu;  // nu: (p, k + 1), nu_j at [j]
+  // two-float numbers: the projections where H and Hh have their places, and kCRec
+  // numbers a step in rec: ||b'||^2, ||z||^2, b' . z, q~ . w, (Q^T q~) . (Q^T w)
+  float2 *H, *Hh, *rec;
   int *status;
 };
 
@@ -64,11 +69,11 @@ struct CShared {
   uint64_t full[kCMaxSlots], empty[kCMaxSlots];
   uint64_t wq_full, wq_empty;
   uint64_t meet[2];  // cluster barriers: the projections', the norms'
-  double part[2 * kCMaxCols + 1];  // this CTA's projections [h_i, g_i] and q~ . w (read by the cluster)
-  double tot[2 * kCMaxCols + 1];   // the cluster's
-  double npart[3];                 // this CTA's ||b'||^2, ||z||^2, b' . z
-  double wred[kCWarps][4];
-  double hhg[2];  // ||Q^T q~||^2, (Q^T q~) . (Q^T w)
+  float2 part[2 * kCMaxCols + 1];  // this CTA's projections [h_i, g_i] and q~ . w (read by the cluster)
+  float2 tot[2 * kCMaxCols + 1];   // the cluster's
+  float2 npart[3];                 // this CTA's ||b'||^2, ||z||^2, b' . z
+  float2 wred[kCWarps][4];
+  float2 hhg[2];  // ||Q^T q~||^2, (Q^T q~) . (Q^T w)
   float red[kCWarps][2 * kCMaxCols];
   float2 coef[kCMaxCols];
   float fin[3];
@@ -119,25 +124,29 @@ __global__ void __launch_bounds__(kCThreads + 32, 2) arnoldi_step_kernel(const C
   }
   __syncthreads();
   // waited for before the first access to another CTA; the copies start at once
-  c_cluster_arrive();
+  if (S > 1) c_cluster_arrive();
   chain_wait();
   chain_next();
 
   if (warp == kCWarps) {
-    // copy warp: per probe the two vectors, slots 0 .. ns - 1, then every group's
-    // slots that did not stay in its ring again.  Lane g counts group g's fills.
-    int fills = 0, pos = 0, t = 0;
+    // copy warp: per probe the two vectors (the first probe's are loaded directly),
+    // slots 0 .. ns - 1, then every group's slots that did not stay in its ring
+    // again.  Lane g counts group g's fills.
+    int fills = 0, pos = 0, wq_fills = 0;
     uint32_t par = 0;
     bool run = true;
-    for (int64_t b = cluster; run && b < a.p; b += nclusters, ++t) {
-      if (t > 0) run = c_wait(&sh->wq_empty, (uint32_t)(t - 1) & 1u, fail, a.status);
-      if (!run) break;
-      if (lane == 0) {
-        c_expect(&sh->wq_full, 2u * col_bytes);
-        if (col_bytes) {
-          c_bulk(c_smem(wq), a.W + b * a.ld + r0, col_bytes, &sh->wq_full);
-          c_bulk(c_smem(wq + R), a.Vin + b * a.vb + r0, col_bytes, &sh->wq_full);
+    for (int64_t b = cluster; run && b < a.p; b += nclusters) {
+      if (b != cluster) {
+        if (wq_fills > 0) run = c_wait(&sh->wq_empty, (uint32_t)(wq_fills - 1) & 1u, fail, a.status);
+        if (!run) break;
+        if (lane == 0) {
+          c_expect(&sh->wq_full, 2u * col_bytes);
+          if (col_bytes) {
+            c_bulk(c_smem(wq), a.W + b * a.ld + r0, col_bytes, &sh->wq_full);
+            c_bulk(c_smem(wq + R), a.Vin + b * a.vb + r0, col_bytes, &sh->wq_full);
+          }
         }
+        ++wq_fills;
       }
       const float *Qb = a.Q + b * a.qb + r0;
       for (int pass = 0; pass < 2 && run; ++pass)
@@ -173,9 +182,10 @@ __global__ void __launch_bounds__(kCThreads + 32, 2) arnoldi_step_kernel(const C
         for (int f = fills > nslots ? fills - nslots : 0; f < fills; ++f)
           mbar_wait_bounded(c_smem(&sh->full[lane * nslots + f % nslots]), (uint32_t)(f / nslots) & 1u, nullptr,
                             kMbarWaitNs / 8);
-      if (lane == 0 && t > 0) mbar_wait_bounded(c_smem(&sh->wq_full), (uint32_t)(t - 1) & 1u, nullptr, kMbarWaitNs / 8);
+      if (lane == 0 && wq_fills > 0)
+        mbar_wait_bounded(c_smem(&sh->wq_full), (uint32_t)(wq_fills - 1) & 1u, nullptr, kMbarWaitNs / 8);
     }
-    c_cluster_wait();
+    if (S > 1) c_cluster_wait();
   } else {
     const int wr = warp % kWR, group = warp / kWR;
     const int row = wr * kCRows + lane * 4;  // rows row .. row + 3 and row + 128 .. row + 131
@@ -192,31 +202,42 @@ __global__ void __launch_bounds__(kCThreads + 32, 2) arnoldi_step_kernel(const C
         sp ^= 1u;
       }
     };
-    bool met = false;  // the cluster's start
+    bool met = S == 1;  // the cluster's start
+    uint32_t wq_par = 0;
     for (int64_t b = cluster; b < a.p; b += nclusters, par ^= 1u) {
       float w[8], q[8];
-      bool ready = c_wait(&sh->wq_full, par, fail, a.status);
+      bool ready = true;
       {
-        auto load = [&](const float *src, float (&x)[8]) {
-          const float4 u = ready && ok0 ? *reinterpret_cast<const float4 *>(src + row) : zero4;
-          const float4 v = ready && ok1 ? *reinterpret_cast<const float4 *>(src + row + 128) : zero4;
+        auto take = [&](const float4 &u, const float4 &v, float (&x)[8]) {
           x[0] = u.x; x[1] = u.y; x[2] = u.z; x[3] = u.w;
           x[4] = v.x; x[5] = v.y; x[6] = v.z; x[7] = v.w;
 #pragma unroll
           for (int e = 0; e < 8; ++e)
             if (row + (e < 4 ? e : 124 + e) >= nloc) x[e] = 0.f;  // a panel's padding is not data
         };
-        load(wq, w);
-        load(wq + R, q);
+        if (b == cluster) {  // a read of L2 is shorter than a copy's round trip
+          const float4 *gw = reinterpret_cast<const float4 *>(a.W + b * a.ld + r0 + row);
+          const float4 *gq = reinterpret_cast<const float4 *>(a.Vin + b * a.vb + r0 + row);
+          const float4 w0 = ok0 ? __ldcg(gw) : zero4, q0 = ok0 ? __ldcg(gq) : zero4;
+          const float4 w1 = ok1 ? __ldcg(gw + 32) : zero4, q1 = ok1 ? __ldcg(gq + 32) : zero4;
+          take(w0, w1, w);
+          take(q0, q1, q);
+        } else {
+          ready = c_wait(&sh->wq_full, wq_par, fail, a.status);
+          wq_par ^= 1u;
+          const float4 *sw = reinterpret_cast<const float4 *>(wq + row), *sq = reinterpret_cast<const float4 *>(wq + R + row);
+          take(ready && ok0 ? sw[0] : zero4, ready && ok1 ? sw[32] : zero4, w);
+          take(ready && ok0 ? sq[0] : zero4, ready && ok1 ? sq[32] : zero4, q);
+          __syncwarp();
+          if (lane == 0) c_arrive(&sh->wq_empty);
+        }
       }
-      __syncwarp();
-      if (lane == 0) c_arrive(&sh->wq_empty);
 
       if (group == 0) {
         float s0 = 0.f, e0 = 0.f;
 #pragma unroll
         for (int e = 0; e < 8; ++e) two_add(s0, e0, w[e] * q[e]);
-        const double v = warp_sum2(s0, e0);
+        const float2 v = warp_pair(s0, e0);
         if (lane == 0) sh->wred[wr][3] = v;
       }
 
@@ -255,21 +276,21 @@ __global__ void __launch_bounds__(kCThreads + 32, 2) arnoldi_step_kernel(const C
         next();
       }
       c_sync();
-      double *mine = S > 1 ? sh->part : sh->tot;
+      float2 *mine = S > 1 ? sh->part : sh->tot;
       for (int i = threadIdx.x; i < 2 * j + 1; i += kCThreads) {
+        float2 v;
         if (i < 2 * j) {
           float s0 = sh->red[0][i], e0 = 0.f;
 #pragma unroll
           for (int r = 1; r < kWR; ++r) two_add(s0, e0, sh->red[r][i]);
-          const double v = (double)s0 + (double)e0;
-          mine[i] = v;
-          if (S == 1) reinterpret_cast<float *>(sh->coef)[i] = (float)v;
+          v = pair(s0, e0);
+          if (S == 1) reinterpret_cast<float *>(sh->coef)[i] = v.x;
         } else {
-          double v = sh->wred[0][3];
+          v = sh->wred[0][3];
 #pragma unroll
-          for (int r = 1; r < kWR; ++r) v += sh->wred[r][3];
-          mine[i] = v;
+          for (int r = 1; r < kWR; ++r) v = pair_add(v, sh->wred[r][3]);
         }
+        mine[i] = v;
       }
       c_sync();
       if (!met) {
@@ -281,35 +302,24 @@ __global__ void __launch_bounds__(kCThreads + 32, 2) arnoldi_step_kernel(const C
         c_wait<true>(&sh->meet[0], par, fail, a.status);
         for (int i = threadIdx.x; i < 2 * j + 1; i += kCThreads) {
           const uint32_t at = c_smem(&sh->part[i]);
-          double x[kCMaxS];
+          float2 x[kCMaxS];
 #pragma unroll
-          for (int r = 0; r < kCMaxS; ++r) x[r] = r < S ? c_ld_f64(c_map(at, (uint32_t)r)) : 0.0;
-          double v = x[0];
+          for (int r = 0; r < kCMaxS; ++r)
+            if (r < S) x[r] = c_ld_pair(c_map(at, (uint32_t)r));
+          float2 v = x[0];
 #pragma unroll
           for (int r = 1; r < kCMaxS; ++r)
-            if (r < S) v += x[r];
+            if (r < S) v = pair_add(v, x[r]);
           sh->tot[i] = v;
-          if (i < 2 * j) reinterpret_cast<float *>(sh->coef)[i] = (float)v;
+          if (i < 2 * j) reinterpret_cast<float *>(sh->coef)[i] = v.x;
         }
         c_sync();
-      }
-      if (!kFirst && rank == 0) {
-        // the raw projections, where their final values will be: Q^T q~ in column
-        // j - 1 of Hh (column-major), Q^T w in column j of H
-        double *hh = a.Hh + b * (int64_t)(a.k + 1) * a.k + (int64_t)(j - 1) * (a.k + 1);
-        double *hc = a.H + b * (int64_t)a.k * a.k + j;
-        for (int i = threadIdx.x; i < 2 * j; i += kCThreads) {
-          if (i & 1)
-            hc[(int64_t)(i >> 1) * a.k] = sh->tot[i];
-          else
-            hh[i >> 1] = sh->tot[i];
-        }
       }
 
       // pass 2: q~ - Q h and w - Q g, even and odd vectors summed apart: the
       // slots that stayed, then the others again
       if (kFirst) {
-        const float c = (float)sh->tot[0];
+        const float c = sh->tot[0].x;
 #pragma unroll
         for (int e = 0; e < 8; ++e) w[e] = fmaf(-q[e], c, w[e]);
       } else {
@@ -405,23 +415,28 @@ __global__ void __launch_bounds__(kCThreads + 32, 2) arnoldi_step_kernel(const C
             two_add(s3[2], e3[2], q[e] * w[e]);
           }
         }
-        double v3[3];
-        warp_sum2x3(s3, e3, v3);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+          for (int i = 0; i < 3; ++i) {
+            const float s2 = __shfl_xor_sync(0xffffffffu, s3[i], o), e2 = __shfl_xor_sync(0xffffffffu, e3[i], o);
+            two_add(s3[i], e3[i], s2);
+            e3[i] += e2;
+          }
         if (lane == 0) {
-          sh->wred[wr][0] = v3[0];
-          sh->wred[wr][1] = v3[1];
-          sh->wred[wr][2] = v3[2];
+#pragma unroll
+          for (int i = 0; i < 3; ++i) sh->wred[wr][i] = pair(s3[i], e3[i]);
         }
       }
       if (!kFirst && warp == kCWarps - 1) {
-        double hh = 0.0, hg = 0.0;
+        float2 hh = make_float2(0.f, 0.f), hg = hh;
         for (int i = lane; i < j; i += 32) {
-          const double h = sh->tot[2 * i];
-          hh = fma(h, h, hh);
-          hg = fma(h, sh->tot[2 * i + 1], hg);
+          const float2 h = sh->tot[2 * i];
+          hh = pair_add(hh, pair_mul(h, h));
+          hg = pair_add(hg, pair_mul(h, sh->tot[2 * i + 1]));
         }
-        hh = warp_sum(hh);
-        hg = warp_sum(hg);
+        hh = warp_pair(hh.x, hh.y);
+        hg = warp_pair(hg.x, hg.y);
         if (lane == 0) {
           sh->hhg[0] = hh;
           sh->hhg[1] = hg;
@@ -430,66 +445,59 @@ __global__ void __launch_bounds__(kCThreads + 32, 2) arnoldi_step_kernel(const C
       c_sync();
       if (warp == 0) {
         if (lane < 3) {
-          double v = sh->wred[0][lane];
+          float2 v = sh->wred[0][lane];
 #pragma unroll
-          for (int r = 1; r < kWR; ++r) v += sh->wred[r][lane];
+          for (int r = 1; r < kWR; ++r) v = pair_add(v, sh->wred[r][lane]);
           sh->npart[lane] = v;
         }
         __syncwarp();
         c_meet_arrive(&sh->meet[1], S);
         if (S > 1) c_wait<true>(&sh->meet[1], par, fail, a.status);
         // lane r holds rank r's sums; a butterfly adds them in a fixed order
-        double nb = 0.0, nz = 0.0, bz = 0.0;
+        float2 nb = make_float2(0.f, 0.f), nz = nb, bz = nb;
         if (lane < S) {
           const uint32_t at = S > 1 ? c_map(c_smem(&sh->npart[0]), (uint32_t)lane) : c_smem(&sh->npart[0]);
-          nb = c_ld_f64(at);
-          nz = c_ld_f64(at + 8);
-          bz = c_ld_f64(at + 16);
+          nb = c_ld_pair(at);
+          nz = c_ld_pair(at + 8);
+          bz = c_ld_pair(at + 16);
         }
         for (int o = S / 2; o > 0; o >>= 1) {
-          nz += __shfl_xor_sync(0xffffffffu, nz, o);
+          nz = pair_add(nz, pair_shfl_xor(nz, o));
           if (!kFirst) {
-            nb += __shfl_xor_sync(0xffffffffu, nb, o);
-            bz += __shfl_xor_sync(0xffffffffu, bz, o);
+            nb = pair_add(nb, pair_shfl_xor(nb, o));
+            bz = pair_add(bz, pair_shfl_xor(bz, o));
           }
         }
-        const double c = sh->tot[2 * j];
+        auto first_lane = [](float2 v) {
+          return make_float2(__shfl_sync(0xffffffffu, v.x, 0), __shfl_sync(0xffffffffu, v.y, 0));
+        };
+        nb = first_lane(nb);
+        nz = first_lane(nz);
+        bz = first_lane(bz);
+        const float2 c = sh->tot[2 * j];
+        float2 hg = make_float2(0.f, 0.f);
         if (kFirst) {
-          if (lane == 0) {
-            const double nu1 = sqrt(nz);
-            sh->fin[0] = (float)nu1;
-            if (rank == 0) {
-              a.H[b * (int64_t)a.k * a.k] = c;
-              a.nu[b * (a.k + 1) + 1] = nu1;
-            }
-          }
+          // nu_1 = ||z||, to a float from the root's remainder
+          const float r = sqrtf(nz.x);
+          if (lane == 0) sh->fin[0] = r > 0.f ? r + (fmaf(-r, r, nz.x) + nz.y) / (2.f * r) : r;
         } else {
           // rho = sqrt(nb) = ||w''_{j-1}|| / nu_j, qw = q_j . A q~_j = e / rho, and for
-          // y = z - q_j qw:  nb ||y||^2 = nb ||z||^2 - 2 e (b' . z) + e^2 =: d.  Float64
-          // divisions and roots are long here (2 FMA a clock and SM): everything
-          // comes from 1 / sqrt(nb) and 1 / sqrt(nb d), taken side by side.
-          nb = __shfl_sync(0xffffffffu, nb, 0);
-          nz = __shfl_sync(0xffffffffu, nz, 0);
-          bz = __shfl_sync(0xffffffffu, bz, 0);
-          const double e = c - sh->hhg[1], zz = nb * nz;
-          double d = fma(e, e, fma(-2.0 * e, bz, zz));
-          if (!(d > 1e-12 * zz)) d = zz;
-          const double root = rsqrt(lane == 0 ? nb : nb * d);
-          const double ir = __shfl_sync(0xffffffffu, root, 0), id = __shfl_sync(0xffffffffu, root, 1);
+          // y = z - q_j qw:  nb ||y||^2 = nb ||z||^2 - 2 e (b' . z) + e^2 =: d
+          hg = sh->hhg[1];
+          const float2 e = pair_add(c, pair_neg(hg)), zz = pair_mul(nb, nz), eb = pair_mul(e, bz);
+          float2 d = pair_add(pair_add(zz, make_float2(-2.f * eb.x, -2.f * eb.y)), pair_mul(e, e));
+          if (!(d.x > 1e-12f * zz.x)) d = zz;
+          const float2 ir = pair_rsqrt(nb), id = pair_rsqrt(pair_mul(nb, d));
           if (lane == 0) {
-            sh->fin[0] = (float)ir;          // 1 / rho
-            sh->fin[1] = (float)(nb * id);   // 1 / ||y||
-            sh->fin[2] = (float)(e * id);    // qw / (rho ||y||)
-            if (rank == 0) {
-              const double hh = sh->hhg[0], nuj = a.nu[b * (a.k + 1) + j];
-              if (hh > 0.01 * (hh + nb) && a.status) atomicExch(a.status, (int)MFG_ERR_RETRY);
-              double *Hb = a.H + b * (int64_t)a.k * a.k;
-              Hb[(int64_t)j * a.k + j - 1] = nuj * (nb * ir);  // beta_j
-              Hb[(int64_t)j * a.k + j] = e * ir;               // raw: arnoldi_h_kernel completes it
-              a.nu[b * (a.k + 1) + j + 1] = d * id * ir;       // u_{j+1} = y / rho = nu_{j+1} q~_{j+1}
-            }
+            sh->fin[0] = ir.x;                  // 1 / rho
+            sh->fin[1] = pair_mul(nb, id).x;    // 1 / ||y||
+            sh->fin[2] = pair_mul(e, id).x;     // qw / (rho ||y||)
+            const float hh = sh->hhg[0].x;
+            if (rank == 0 && hh > 0.01f * (hh + nb.x) && a.status) atomicExch(a.status, (int)MFG_ERR_RETRY);
           }
         }
+        if (lane < kCRec && rank == 0)
+          a.rec[(b * a.k + j) * kCRec + lane] = lane == 0 ? nb : (lane == 1 ? nz : (lane == 2 ? bz : (lane == 3 ? c : hg)));
       }
       c_sync();
       if (group == 0) {
@@ -526,43 +534,92 @@ __global__ void __launch_bounds__(kCThreads + 32, 2) arnoldi_step_kernel(const C
           }
         }
       }
+      if (!kFirst && rank == 0) {
+        // the raw projections, where their final values will be: Q^T q~ in column
+        // j - 1 of Hh (column-major), Q^T w in column j of H
+        float2 *hh = a.Hh + b * (int64_t)(a.k + 1) * a.k + (int64_t)(j - 1) * (a.k + 1);
+        float2 *hc = a.H + b * (int64_t)a.k * a.k + j;
+        for (int i = threadIdx.x; i < 2 * j; i += kCThreads) {
+          if (i & 1)
+            hc[(int64_t)(i >> 1) * a.k] = sh->tot[i];
+          else
+            hh[i >> 1] = sh->tot[i];
+        }
+      }
     }
   }
   // no CTA leaves while the others may read its sums or arrive on its barriers
-  c_cluster_arrive();
-  c_cluster_wait();
+  if (S > 1) {
+    c_cluster_arrive_relaxed();
+    c_cluster_wait();
+  }
 }
 
 // ---------------------------------------------------------------------------
-// H from the raw projections that the step kernels left: with hq = Q^T q~_j
-// (column j - 1 of Hh), g = Q^T w (column j of H) and qw (H[j][j]),
-//   Hh[:, j - 1] = H[:, j - 1] + nu_j hq (rows < j), beta_j in row j
+// H from what the step kernels left as two-float numbers: hq = Q^T q~_j (column j - 1
+// of Hh), g = Q^T w (column j of H), and of step j (rec) nb = ||b'||^2, nz = ||z||^2,
+// bz = b' . z, c = q~ . w, hg = hq . g:
+//   rho = sqrt(nb), qw = (c - hg) / rho, nu_{j+1} = ||z - qw b' / rho|| / rho,
+//   Hh[:, j - 1] = H[:, j - 1] + nu_j hq (rows < j), beta_j = nu_j rho in row j
 //   H[:, j] = (nu_j [g; qw] - Hh[0 : j + 1, 0 : j] hq) / beta_j
-// for j = 1 .. k - 1.  One CTA per probe keeps Hh in shared memory; a row's sum
-// over the columns is cut in four.  With `band` only the tridiagonal part is
-// formed (all that the quadrature reads): Hh is upper Hessenberg, so rows j - 1
-// and j of the product have two terms and one, and the steps are independent.
+// for j = 1 .. k - 1, and H[0][0] = c, nu_1 = ||z|| of step 0.  One CTA per probe; the
+// full form keeps Hh in shared memory and cuts a row's sum over the columns in
+// four.  With `band` only the tridiagonal part is formed (all that the quadrature
+// reads): Hh is upper Hessenberg, so rows j - 1 and j of the product have two terms
+// and one, and the steps are independent.
 // ---------------------------------------------------------------------------
 
+__device__ __forceinline__ double h_raw(const double *p) {
+  const float2 v = *reinterpret_cast<const float2 *>(p);
+  return (double)v.x + (double)v.y;
+}
+
+// beta[1 .. k - 1], qw[0 .. k - 1] (qw[0] = H[0][0]) and nu[1 .. k] of one probe, by all threads
+__device__ __forceinline__ void h_scalars(const double *__restrict__ rec, int k, double *beta, double *qw, double *nu) {
+  for (int j = threadIdx.x; j < k; j += blockDim.x) {
+    const double *r = rec + (int64_t)j * kCRec;
+    const double nz = h_raw(r + 1), c = h_raw(r + 3);
+    if (j == 0) {
+      qw[0] = c;
+      nu[1] = sqrt(nz);
+    } else {
+      const double nb = h_raw(r), bz = h_raw(r + 2), e = c - h_raw(r + 4), zz = nb * nz;
+      double d = fma(e, e, fma(-2.0 * e, bz, zz));
+      if (!(d > 1e-12 * zz)) d = zz;
+      const double ir = rsqrt(nb), id = rsqrt(nb * d);
+      beta[j] = nb * ir;
+      qw[j] = e * ir;
+      nu[j + 1] = d * id * ir;
+    }
+  }
+  __syncthreads();
+  for (int j = threadIdx.x; j < k; j += blockDim.x)
+    if (j > 0) beta[j] *= nu[j];
+  __syncthreads();
+}
+
 __global__ void arnoldi_h_kernel(double *__restrict__ H, const double *__restrict__ Hh,
-                                 const double *__restrict__ nu, int k, double *__restrict__ nu_last_inv) {
-  extern __shared__ double hs[];  // Hh, column-major with k + 1 rows; then hq, partial sums
+                                 const double *__restrict__ rec, int k, double *__restrict__ nu_last_inv) {
+  extern __shared__ double hs[];  // Hh, column-major with k + 1 rows; then hq, partial sums, the steps' scalars
   const int64_t b = blockIdx.x;
   double *Hb = H + b * (int64_t)k * k;
   const double *raw = Hh + b * (int64_t)(k + 1) * k;
-  const double *nub = nu + b * (k + 1);
   const int ld = k + 1, rows = blockDim.x / 4;
   double *hq = hs + (size_t)ld * k, *part = hq + k;  // part: [4][rows]
+  double *beta = part + 4 * rows, *qw = beta + k, *nu = qw + k;
+  h_scalars(rec + b * k * kCRec, k, beta, qw, nu);
   const int i = threadIdx.x % rows, quarter = threadIdx.x / rows;
-  double hlast = i == 0 ? Hb[0] : 0.0;  // H[i][j - 1] (quarter 0)
+  double hlast = i == 0 ? qw[0] : 0.0;  // H[i][j - 1] (quarter 0)
+  if (threadIdx.x == 0) Hb[0] = qw[0];
   for (int j = 1; j < k; ++j) {
-    const double nuj = nub[j], beta = Hb[(int64_t)j * k + j - 1];
+    const double nuj = nu[j], bj = beta[j];
+    double top = 0.0;
     if (quarter == 0 && i <= j) {
-      const double h = i < j ? raw[(int64_t)(j - 1) * ld + i] : 0.0;
+      const double h = i < j ? h_raw(raw + (int64_t)(j - 1) * ld + i) : 0.0;
       if (i < j) hq[i] = h;
-      hs[(size_t)(j - 1) * ld + i] = i < j ? hlast + nuj * h : beta;
+      hs[(size_t)(j - 1) * ld + i] = i < j ? hlast + nuj * h : bj;
+      top = i < j ? h_raw(Hb + (int64_t)i * k + j) : qw[j];
     }
-    const double top = (quarter == 0 && i <= j) ? Hb[(int64_t)i * k + j] : 0.0;
     __syncthreads();
     if (i <= j) {
       // columns max(i - 1, 0) .. j - 1 of row i, a quarter of them
@@ -575,36 +632,38 @@ __global__ void arnoldi_h_kernel(double *__restrict__ H, const double *__restric
     __syncthreads();
     if (quarter == 0 && i <= j) {
       const double m = (part[i] + part[rows + i]) + (part[2 * rows + i] + part[3 * rows + i]);
-      hlast = nuj * (top - m) / beta;
+      hlast = nuj * (top - m) / bj;
       Hb[(int64_t)i * k + j] = hlast;
+      if (i == j) Hb[(int64_t)j * k + j - 1] = bj;
     }
   }
-  if (threadIdx.x == 0 && nu_last_inv) nu_last_inv[b] = 1.0 / nub[k];
+  if (threadIdx.x == 0 && nu_last_inv) nu_last_inv[b] = 1.0 / nu[k];
 }
 
 __global__ void arnoldi_h_band_kernel(double *__restrict__ H, const double *__restrict__ Hh,
-                                      const double *__restrict__ nu, int k) {
+                                      const double *__restrict__ rec, int k) {
+  __shared__ double beta[kCMaxCols + 1], qw[kCMaxCols + 1], nu[kCMaxCols + 2];
   const int64_t b = blockIdx.x;
   const int j = threadIdx.x + 1;
   double *Hb = H + b * (int64_t)k * k;
-  const double *raw = Hh + b * (int64_t)(k + 1) * k, *nub = nu + b * (k + 1);
+  const double *raw = Hh + b * (int64_t)(k + 1) * k;
+  h_scalars(rec + b * k * kCRec, k, beta, qw, nu);
   double up = 0.0, diag = 0.0;
   if (j < k) {
-    auto beta = [&](int i) { return Hb[(int64_t)i * k + i - 1]; };             // of step i >= 1
-    auto hq = [&](int i, int r) { return raw[(int64_t)(i - 1) * (k + 1) + r]; };  // row r of Q^T q~_i
-    auto diag_of = [&](int i) {
-      return i == 0 ? Hb[0] : nub[i] * (Hb[(int64_t)i * k + i] - beta(i) * hq(i, i - 1)) / beta(i);
-    };
-    const double nuj = nub[j], bj = beta(j), h1 = hq(j, j - 1);
-    double m = (diag_of(j - 1) + nuj * h1) * h1;
-    if (j > 1) m = fma(beta(j - 1), hq(j, j - 2), m);
-    up = nuj * (Hb[(int64_t)(j - 1) * k + j] - m) / bj;
+    auto hq = [&](int i, int r) { return h_raw(raw + (int64_t)(i - 1) * (k + 1) + r); };  // row r of Q^T q~_i
+    auto diag_of = [&](int i) { return i == 0 ? qw[0] : nu[i] * (qw[i] - beta[i] * hq(i, i - 1)) / beta[i]; };
+    const double h1 = hq(j, j - 1);
+    double m = (diag_of(j - 1) + nu[j] * h1) * h1;
+    if (j > 1) m = fma(beta[j - 1], hq(j, j - 2), m);
+    up = nu[j] * (h_raw(Hb + (int64_t)(j - 1) * k + j) - m) / beta[j];
     diag = diag_of(j);
   }
   __syncthreads();  // every raw value has been read
+  if (j == 1) Hb[0] = qw[0];
   if (j < k) {
     Hb[(int64_t)(j - 1) * k + j] = up;
     Hb[(int64_t)j * k + j] = diag;
+    Hb[(int64_t)j * k + j - 1] = beta[j];
   }
 }
 
@@ -685,10 +744,10 @@ static CPlan c_plan(int64_t n, int64_t p, int j) {
 // Q: the basis (probe stride qb, vector stride ld); W = A q~_j; Vin: q~_j with
 // probe stride vb (j = 0: row 0 of Q).  Writes row j of Q (j > 0), the next q~
 // into Vout with its bf16 copies (null: not formed), the raw projections into H
-// and Hh, nu_{j+1}.
+// and Hh, the scalars of the step into rec.
 int launch_arnoldi_step(int j, int64_t k, int64_t n, int64_t p, float *Q, int64_t qb, int64_t ld, const float *W,
                         const float *Vin, int64_t vb, float *Vout, __nv_bfloat16 *hi, __nv_bfloat16 *lo, double *H,
-                        double *Hh, double *nu, int *status, bool chained, cudaStream_t s) {
+                        double *Hh, double *rec, int *status, bool chained, cudaStream_t s) {
   if (p <= 0) return MFG_OK;
   const CPlan plan = c_plan(n, p, j);
   if (plan.S == 0 || j > kCMaxCols) return MFG_ERR_UNSUPPORTED;
@@ -710,9 +769,9 @@ int launch_arnoldi_step(int j, int64_t k, int64_t n, int64_t p, float *Q, int64_
   a.R = plan.R;
   a.S = plan.S;
   a.slots = plan.slots;
-  a.H = H;
-  a.Hh = Hh;
-  a.nu = nu;
+  a.H = reinterpret_cast<float2 *>(H);
+  a.Hh = reinterpret_cast<float2 *>(Hh);
+  a.rec = reinterpret_cast<float2 *>(rec);
   a.status = status;
   auto kern = j == 0 ? c_kernel<true>(plan.wr) : c_kernel<false>(plan.wr);
   const size_t smem = c_fixed(plan.R, plan.wr) + (size_t)plan.slots * (kCWarps / plan.wr) * c_gc(plan.wr) * plan.R * 4;
@@ -721,17 +780,17 @@ int launch_arnoldi_step(int j, int64_t k, int64_t n, int64_t p, float *Q, int64_
 
 // H of every probe from what the steps left (`band`: its tridiagonal part only);
 // nu_last_inv (optional): 1 / nu_k.
-int launch_arnoldi_h(int64_t k, int64_t p, double *H, const double *Hh, const double *nu, bool band,
+int launch_arnoldi_h(int64_t k, int64_t p, double *H, const double *Hh, const double *rec, bool band,
                      double *nu_last_inv, cudaStream_t s) {
   if (p <= 0 || k < 2) return MFG_OK;
   const int rows = (int)ceil_div(k, 32) * 32;
   if (band) {
-    arnoldi_h_band_kernel<<<(unsigned)p, rows, 0, s>>>(H, Hh, nu, (int)k);
+    arnoldi_h_band_kernel<<<(unsigned)p, rows, 0, s>>>(H, Hh, rec, (int)k);
     return MFG_LAUNCH_STATUS();
   }
-  const size_t smem = ((size_t)(k + 1) * k + k + 4 * (size_t)rows) * sizeof(double);
+  const size_t smem = ((size_t)(k + 1) * k + 4 * k + 1 + 4 * (size_t)rows) * sizeof(double);
   MFG_CUDA_TRY(cudaFuncSetAttribute(arnoldi_h_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  arnoldi_h_kernel<<<(unsigned)p, 4 * rows, smem, s>>>(H, Hh, nu, (int)k, nu_last_inv);
+  arnoldi_h_kernel<<<(unsigned)p, 4 * rows, smem, s>>>(H, Hh, rec, (int)k, nu_last_inv);
   return MFG_LAUNCH_STATUS();
 }
 

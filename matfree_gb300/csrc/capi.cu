@@ -89,8 +89,9 @@ static void prof_end(size_t e0, int cls, double bytes, double flops, cudaStream_
 struct WsLayout {
   size_t w, panel, norm, len0, h2, partials, counters, status, hi, lo, q, h, values, eig, fsq;
   // two-sweep Arnoldi: qt (float panel), X2 (p (2k + 1)), dots (p 3), nu
-  // (p (k + 1)), finish coefficients (p 4), full coefficients Hh (p (k + 1) k)
-  size_t vt, x2, dots, nu, cf, hh;
+  // (p (k + 1)), finish coefficients (p 4), full coefficients Hh (p (k + 1) k),
+  // the steps' scalars (p k kTwoSweepRec)
+  size_t vt, x2, dots, nu, cf, hh, rec;
   size_t total;
 };
 
@@ -146,6 +147,7 @@ static WsLayout layout(const mfg_operator *op, int64_t k, int64_t p, int64_t ld,
     L.nu = take((size_t)p * (kk + 1) * 8);
     L.cf = take((size_t)p * 4 * 8);
     L.hh = take((size_t)p * (kk + 1) * kk * 8);
+    L.rec = take((size_t)p * kk * kTwoSweepRec * 8);
   }
   L.total = off + 256;  // slack for aligning the caller's base pointer
   return L;
@@ -285,6 +287,7 @@ static int run_two_sweep(const mfg_operator *op, int64_t k, int64_t p, int64_t l
     double *nu = reinterpret_cast<double *>(ws + L.nu);
     double *cf = reinterpret_cast<double *>(ws + L.cf);
     double *Hh = reinterpret_cast<double *>(ws + L.hh);
+    double *rec = reinterpret_cast<double *>(ws + L.rec);
     double *partials = reinterpret_cast<double *>(ws + L.partials);
     unsigned *counters = reinterpret_cast<unsigned *>(ws + L.counters);
     int *status = reinterpret_cast<int *>(ws + L.status);
@@ -307,10 +310,10 @@ static int run_two_sweep(const mfg_operator *op, int64_t k, int64_t p, int64_t l
         MFG_LAUNCH(MFG_PROF_SUBPROJ, (j + (more || R ? 4.0 : 3.0)) * vecb + (more ? bfb : 0.0),
                    (8.0 * j + 10.0) * vecb / sizeof(T),
                    launch_arnoldi_step((int)j, k, n, p, Q, qb, ld, Wb, j == 0 ? Q : Vt, j == 0 ? qb : ld,
-                                       (more || R) ? Vt : nullptr, more ? hi : nullptr, lo, H, Hh, nu, status, chained, s));
+                                       (more || R) ? Vt : nullptr, more ? hi : nullptr, lo, H, Hh, rec, status, chained, s));
       }
       MFG_LAUNCH(MFG_PROF_OTHER, 24.0 * p * k * k, full_h ? 2.0 / 3.0 * p * k * k * k : 0.0,
-                 launch_arnoldi_h(k, p, H, Hh, nu, !full_h, R ? cf : nullptr, s));
+                 launch_arnoldi_h(k, p, H, Hh, rec, !full_h, R ? cf : nullptr, s));
     } else {
       // step 0 as the reference: w = A q_0, h_0 = q_0 . w, u_1 = w - q_0 h_0
       MFG_LAUNCH(MFG_PROF_APPLY, ab, af, apply_op<T>(op, Q, qb, Wb, ld, p, hi, lo, ld, panel, status, s));

@@ -56,6 +56,12 @@ __device__ __forceinline__ void c_sync() {
   __syncwarp();
 }
 
+// Arrival without a release: for a barrier that orders no data
+__device__ __forceinline__ void c_cluster_arrive_relaxed() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");
+}
+
 __device__ __forceinline__ void c_cluster_arrive() {
   __syncwarp();
   asm volatile("barrier.cluster.arrive.release;" ::: "memory");
@@ -72,6 +78,56 @@ __device__ __forceinline__ void two_add(float &s, float &e, float x) {
   s = t;
 }
 
+// Two-float numbers x + y, |y| <= half an ulp of x: some 2^-45 of relative error per
+// operation, in a few float instructions of 4 cycles each.  A float64 instruction holds
+// its warp for 64 cycles here, a dependent chain of them (or one division or root)
+// for thousands, on the path of every step.
+__device__ __forceinline__ float2 pair(float s, float e) {
+  const float t = s + e;
+  return make_float2(t, e - (t - s));
+}
+
+__device__ __forceinline__ float2 pair_add(float2 a, float2 b) {
+  two_add(a.x, a.y, b.x);
+  return pair(a.x, a.y + b.y);
+}
+
+__device__ __forceinline__ float2 pair_neg(float2 a) { return make_float2(-a.x, -a.y); }
+
+__device__ __forceinline__ float2 pair_mul(float2 a, float2 b) {
+  const float p = a.x * b.x;
+  return pair(p, fmaf(a.y, b.x, fmaf(a.x, b.y, fmaf(a.x, b.x, -p))));
+}
+
+// 1 / sqrt(a): a Newton step on the float result
+__device__ __forceinline__ float2 pair_rsqrt(float2 a) {
+  const float r = rsqrtf(a.x), r2 = r * r;
+  const float t = fmaf(-a.y, r2, fmaf(-a.x, fmaf(r, r, -r2), fmaf(-a.x, r2, 1.0f)));
+  return pair(r, 0.5f * r * t);
+}
+
+__device__ __forceinline__ float2 pair_shfl_xor(float2 a, int o) {
+  return make_float2(__shfl_xor_sync(0xffffffffu, a.x, o), __shfl_xor_sync(0xffffffffu, a.y, o));
+}
+
+__device__ __forceinline__ float2 c_ld_pair(uint32_t addr) {
+  float2 v;
+  asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr) : "memory");
+  return v;
+}
+
+// Sum of the lanes' two-float values (all lanes).
+__device__ __forceinline__ float2 warp_pair(float s, float e) {
+  float2 v = make_float2(s, e);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const float2 u = pair_shfl_xor(v, o);
+    two_add(v.x, v.y, u.x);
+    v.y += u.y;
+  }
+  return pair(v.x, v.y);
+}
+
 // Sum of the lanes' two-float values in float64 (all lanes).
 __device__ __forceinline__ double warp_sum2(float s, float e) {
 #pragma unroll
@@ -81,26 +137,6 @@ __device__ __forceinline__ double warp_sum2(float s, float e) {
     e += e2;
   }
   return (double)s + (double)e;
-}
-
-// The same for three values.
-__device__ __forceinline__ void warp_sum2x3(float (&s)[3], float (&e)[3], double (&out)[3]) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    float s2[3], e2[3];
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      s2[i] = __shfl_xor_sync(0xffffffffu, s[i], o);
-      e2[i] = __shfl_xor_sync(0xffffffffu, e[i], o);
-    }
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      two_add(s[i], e[i], s2[i]);
-      e[i] += e2[i];
-    }
-  }
-#pragma unroll
-  for (int i = 0; i < 3; ++i) out[i] = (double)s[i] + (double)e[i];
 }
 
 // Halving butterfly: N per-lane values to their warp sums; lane l ends with the

@@ -36,6 +36,7 @@ int launch_inv(const double *x, double *y, int64_t p, cudaStream_t s);
 // two-sweep Arnoldi step (lanczos_kernels.cu; float bases).  One two-vector
 // pass covers at most kTwoSweepPassCols basis vectors (both vectors' sums stay
 // in registers); steps with more run it on column blocks.  k <= kTwoSweepMaxK.
+constexpr int kTwoSweepRec = 5;  // 8-byte scalars a step leaves for H (arnoldi_cluster.cu)
 constexpr int kTwoSweepPassCols = 64;
 constexpr int kTwoSweepMaxK = 129;
 template <typename T>
@@ -59,8 +60,8 @@ int launch_twosweep_finish(T *Qj, int64_t q_bstride, const T *Z, int64_t w_bstri
 bool arnoldi_cluster_applies(int64_t n);
 int launch_arnoldi_step(int j, int64_t k, int64_t n, int64_t p, float *Q, int64_t qb, int64_t ld, const float *W,
                         const float *Vin, int64_t vb, float *Vout, __nv_bfloat16 *hi, __nv_bfloat16 *lo, double *H,
-                        double *Hh, double *nu, int *status, bool chained, cudaStream_t s);
-int launch_arnoldi_h(int64_t k, int64_t p, double *H, const double *Hh, const double *nu, bool band,
+                        double *Hh, double *rec, int *status, bool chained, cudaStream_t s);
+int launch_arnoldi_h(int64_t k, int64_t p, double *H, const double *Hh, const double *rec, bool band,
                      double *nu_last_inv, cudaStream_t s);
 // (chained: see chain_wait in common.cuh)
 // gs_cluster.cu: Gram-Schmidt twice with the norm and the normalisation, and a step
