@@ -128,17 +128,6 @@ __device__ __forceinline__ float2 warp_pair(float s, float e) {
   return pair(v.x, v.y);
 }
 
-// Sum of the lanes' two-float values in float64 (all lanes).
-__device__ __forceinline__ double warp_sum2(float s, float e) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float s2 = __shfl_xor_sync(0xffffffffu, s, o), e2 = __shfl_xor_sync(0xffffffffu, e, o);
-    two_add(s, e, s2);
-    e += e2;
-  }
-  return (double)s + (double)e;
-}
-
 // Halving butterfly: N per-lane values to their warp sums; lane l ends with the
 // sum of value idx(l), kept by the lanes of equal idx (32 / N of them).
 template <int N, typename T>

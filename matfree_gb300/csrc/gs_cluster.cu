@@ -20,6 +20,13 @@
 // that does not comes from HBM once and from L2 three times, as far as the probes in
 // flight fit there.  As separate launches over all probes every pass came from HBM,
 // with the vector written and read between them.
+//
+// What bounds it: for few probes the chain of loads, meetings and reductions (sums of
+// floats across warps and CTAs are two-float numbers for that reason: adjoint steps of
+// n = 1501, 32 probes 18.4 -> 15.8 us, n = 8192, 128 probes 87 -> 83 us), for many the reads.
+// Against separate launches (four to five for Gram-Schmidt twice, twelve for an adjoint
+// step): n = 8192, 128 probes, k = 32 bidiagonalisation half step 76 -> 44 us, adjoint
+// k = 48 150 -> 83 us a step; float64 n = 1000, 100 probes, k = 30 62 -> 44 us a step.
 #include "cluster.cuh"
 #include "kernels.cuh"
 
@@ -51,7 +58,7 @@ struct GsArgs {
   const T *lam, *Lam;   // lambda (row idx of Lambda) and Lambda, probe stride qb
   const T *res, *dq;    // residual (probe stride ld), row idx of dQ (stride qb; null: none)
   const double *H, *Pi, *dH, *gamma, *out_scale;  // out_scale: last step, times out_scale[b]
-  double *Gamma;
+  double *Gamma;  // GSum numbers
   // the result: q_next, lambda' or (idx 0) dv; its bf16 copies (probe stride ld)
   T *next;
   int64_t next_b;
@@ -59,9 +66,41 @@ struct GsArgs {
   int *status;
 };
 
+// Sums across warps and CTAs: two-float numbers of floats, float64 of doubles.
+template <typename T> struct GSum { using type = double; };
+template <> struct GSum<float> { using type = float2; };
+__device__ __forceinline__ double g_add(double a, double b) { return a + b; }
+__device__ __forceinline__ float2 g_add(float2 a, float2 b) { return pair_add(a, b); }
+__device__ __forceinline__ double g_sub(double a, double b) { return a - b; }
+__device__ __forceinline__ float2 g_sub(float2 a, float2 b) { return pair_add(a, pair_neg(b)); }
+__device__ __forceinline__ double g_twice(double a, double f) { return a * f; }
+__device__ __forceinline__ float2 g_twice(float2 a, float f) { return make_float2(a.x * f, a.y * f); }  // f: a power of two
+__device__ __forceinline__ double g_round(double a) { return a; }
+__device__ __forceinline__ float g_round(float2 a) { return a.x; }
+__device__ __forceinline__ double g_double(double a) { return a; }
+__device__ __forceinline__ double g_double(float2 a) { return (double)a.x + (double)a.y; }
+__device__ __forceinline__ double g_sum_of(double v) { return v; }
+__device__ __forceinline__ float2 g_sum_of(float v) { return make_float2(v, 0.f); }
+template <typename S> __device__ __forceinline__ S g_from(double v);
+template <> __device__ __forceinline__ double g_from<double>(double v) { return v; }
+template <> __device__ __forceinline__ float2 g_from<float2>(double v) {
+  const float x = (float)v;
+  return make_float2(x, (float)(v - (double)x));
+}
+__device__ __forceinline__ double g_load_rank(const double *p, int rank) { return c_ld_f64(c_map(c_smem(p), (uint32_t)rank)); }
+__device__ __forceinline__ float2 g_load_rank(const float2 *p, int rank) { return c_ld_pair(c_map(c_smem(p), (uint32_t)rank)); }
+__device__ __forceinline__ double g_xor(double v, int o) { return __shfl_xor_sync(0xffffffffu, v, o); }
+__device__ __forceinline__ float2 g_xor(float2 v, int o) { return pair_shfl_xor(v, o); }
+__device__ __forceinline__ double g_sqrt(double v) { return sqrt(v); }
+__device__ __forceinline__ float2 g_sqrt(float2 v) {
+  const float r = sqrtf(v.x);
+  return r > 0.f ? pair(r, (fmaf(-r, r, v.x) + v.y) / (2.f * r)) : make_float2(r, 0.f);
+}
+
 struct GShared {
   uint64_t full[kCMaxSlots], empty[kCMaxSlots];
   uint64_t meet[3];
+  // GSum numbers
   double npart[2];  // this CTA's ||w||^2, by the probe's parity
   double wred[kCWarps];
   double fin;
@@ -72,7 +111,7 @@ template <typename T>
 __host__ __device__ inline size_t g_fixed(int cpad, int xpad, int R, int wr) {
   const size_t groups = kCWarps / wr;
   size_t b = (sizeof(GShared) + 15) / 16 * 16;
-  b += (size_t)cpad * 8 * 4;                             // part[2][2]
+  b += (size_t)cpad * 8 * 6;                             // part[2][2], h_pi, dh
   b += (size_t)(wr * cpad + cpad + xpad) * sizeof(T);    // red, coef, extra coefficients
   if (groups > 1) b += groups * (size_t)R * sizeof(T);   // partial updates
   return (b + 127) / 128 * 128;
@@ -90,11 +129,16 @@ template <typename T, int kWR, int kGC, bool kAdj>
 __global__ void __launch_bounds__(kCThreads + 32, 2) gs_cluster_kernel(const GsArgs<T> a) {
   constexpr int kWC = kCWarps / kWR, VW = 16 / (int)sizeof(T), NV = 8 / VW;
   using Vt = typename Vec<T>::type;
+  using Sum = typename GSum<T>::type;
+  static_assert(sizeof(Sum) == 8, "shared arrays");
   extern __shared__ __align__(128) uint8_t g_raw[];
   GShared *sh = reinterpret_cast<GShared *>(g_raw);
   const int R = a.R, S = a.S, nslots = a.slots, nc = a.ncols, nx = kAdj ? a.nx : 0;
-  double *part = reinterpret_cast<double *>(g_raw + (sizeof(GShared) + 15) / 16 * 16);  // [2][2][cpad]
-  T *red = reinterpret_cast<T *>(part + 4 * a.cpad);  // [kWR][cpad]
+  Sum *part = reinterpret_cast<Sum *>(g_raw + (sizeof(GShared) + 15) / 16 * 16);  // [2][2][cpad]
+  Sum *wred = reinterpret_cast<Sum *>(sh->wred), *npart = reinterpret_cast<Sum *>(sh->npart);
+  Sum *fin = reinterpret_cast<Sum *>(&sh->fin);
+  Sum *h_pi = part + 4 * a.cpad, *dh = h_pi + a.cpad;  // row idx of Pi, then the first projections; column of dH
+  T *red = reinterpret_cast<T *>(dh + a.cpad);  // [kWR][cpad]
   T *coef = red + kWR * a.cpad, *xcoef = coef + a.cpad;
   T *comb = xcoef + a.xpad;  // [kWC][R]
   T *ring = reinterpret_cast<T *>(g_raw + g_fixed<T>(a.cpad, a.xpad, R, kWR));  // [kWC][nslots][kGC][R]
@@ -124,7 +168,7 @@ __global__ void __launch_bounds__(kCThreads + 32, 2) gs_cluster_kernel(const GsA
     if (i <= kCMaxSlots) asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
-  c_cluster_arrive();  // waited for before the first access to another CTA
+  if (S > 1) c_cluster_arrive();  // waited for before the first access to another CTA
   chain_wait();
   chain_next();
 
@@ -178,7 +222,7 @@ __global__ void __launch_bounds__(kCThreads + 32, 2) gs_cluster_kernel(const GsA
         mbar_wait_bounded(c_smem(&sh->full[lane * nslots + f % nslots]), (uint32_t)(f / nslots) & 1u, nullptr,
                           kMbarWaitNs / 8);
     }
-    c_cluster_wait();
+    if (S > 1) c_cluster_wait();
   } else {
     const int wr = warp % kWR, group = warp / kWR;
     int rv[NV];  // first rows of this lane's 16-byte vectors
@@ -277,18 +321,19 @@ __global__ void __launch_bounds__(kCThreads + 32, 2) gs_cluster_kernel(const GsA
         }
       }
     };
-    bool met = false;
+    bool met = S == 1;
     // the cluster's sums of red[.][0 .. nc) into tot; use(i, tot) sets coef and outputs
     auto meet_sums = [&](int which, auto use) {
-      double *mine = part + ((size_t)which * 2 + par) * a.cpad;
+      Sum *mine = part + ((size_t)which * 2 + par) * a.cpad;
       c_sync();
-      for (int i = threadIdx.x; i < nc; i += kCThreads) {
-        double v;
+      const int i = threadIdx.x;  // nc <= kCThreads
+      if (i < nc) {
+        Sum v;
         if constexpr (sizeof(T) == 4) {
           float s0 = red[i], e0 = 0.f;
 #pragma unroll
           for (int r = 1; r < kWR; ++r) two_add(s0, e0, red[r * a.cpad + i]);
-          v = (double)s0 + (double)e0;
+          v = pair(s0, e0);
         } else {
           v = red[i];
 #pragma unroll
@@ -305,15 +350,15 @@ __global__ void __launch_bounds__(kCThreads + 32, 2) gs_cluster_kernel(const GsA
       if (S > 1) {
         c_meet_arrive(&sh->meet[which], S);
         c_wait<true>(&sh->meet[which], par, fail, a.status);
-        for (int i = threadIdx.x; i < nc; i += kCThreads) {
-          const uint32_t at = c_smem(mine + i);
-          double x[kCMaxS];
+        if (i < nc) {
+          Sum v = g_sum_of((T)0);
+          for (int r0 = 0; r0 < S; r0 += 4) {
+            Sum x[4];
 #pragma unroll
-          for (int r = 0; r < kCMaxS; ++r) x[r] = r < S ? c_ld_f64(c_map(at, (uint32_t)r)) : 0.0;
-          double v = x[0];
+            for (int r = 0; r < 4; ++r) x[r] = r0 + r < S ? g_load_rank(mine + i, r0 + r) : g_sum_of((T)0);
 #pragma unroll
-          for (int r = 1; r < kCMaxS; ++r)
-            if (r < S) v += x[r];
+            for (int r = 0; r < 4; ++r) v = g_add(v, x[r]);
+          }
           use(i, v);
         }
         c_sync();
@@ -349,20 +394,19 @@ __global__ void __launch_bounds__(kCThreads + 32, 2) gs_cluster_kernel(const GsA
       load_rows(a.W + b * a.ld, v);
 #pragma unroll
       for (int e = 0; e < 8; ++e) acc[e] = (T)0;
-      double my_pi = 0.0, my_dh = 0.0;  // of basis vector threadIdx.x (ncols <= 256)
       const double *Hb = nullptr;
-      double *Gb = nullptr;
+      Sum *Gb = nullptr;
       T beta = (T)1;
       if constexpr (kAdj) {
         const int64_t kk = (int64_t)a.k * a.k;
         Hb = a.H + b * kk;
-        Gb = a.Gamma + b * kk;
+        Gb = reinterpret_cast<Sum *>(a.Gamma) + b * kk;
         if ((int)threadIdx.x < nc) {
-          my_pi = a.Pi[b * kk + (int64_t)a.idx * a.k + threadIdx.x];
-          if (a.idx > 0) my_dh = a.dH[b * kk + (int64_t)threadIdx.x * a.k + a.idx - 1];
+          h_pi[threadIdx.x] = g_from<Sum>(a.Pi[b * kk + (int64_t)a.idx * a.k + threadIdx.x]);
+          if (a.idx > 0) dh[threadIdx.x] = g_from<Sum>(a.dH[b * kk + (int64_t)threadIdx.x * a.k + a.idx - 1]);
         }
         for (int i = threadIdx.x; i < nx; i += kCThreads) {
-          xcoef[i] = (T)Gb[(int64_t)(a.idx + 1 + i) * a.k + a.idx];
+          xcoef[i] = g_round(Gb[(int64_t)(a.idx + 1 + i) * a.k + a.idx]);
           xcoef[nx + i] = (T)(-Hb[(int64_t)a.idx * a.k + a.idx + 1 + i]);
         }
         if (a.idx > 0) beta = (T)Hb[(int64_t)a.idx * a.k + a.idx - 1];
@@ -399,14 +443,14 @@ __global__ void __launch_bounds__(kCThreads + 32, 2) gs_cluster_kernel(const GsA
 
       if (nc > 0) {
         dots(1, v);
-        meet_sums(0, [&](int i, double t) {
+        meet_sums(0, [&](int i, Sum t) {  // i == threadIdx.x
           if constexpr (kAdj) {
-            const double row = (i < a.idx ? 1.0 : 0.5) * (my_pi - t);  // i == threadIdx.x: nc <= kCThreads
-            if (rank == 0) Gb[(int64_t)a.idx * a.k + i] = row;
-            coef[i] = (T)(i < a.idx ? row : 2.0 * row);
+            const Sum row = g_sub(h_pi[i], t);
+            h_pi[i] = g_twice(row, i < a.idx ? (T)1 : (T)0.5);
+            coef[i] = g_round(row);
           } else {
-            if (rank == 0) a.h[b * a.h_bs + i * a.h_is] = t;
-            coef[i] = (T)(-t);
+            h_pi[i] = t;
+            coef[i] = -g_round(t);
           }
         });
         pass(2, [&](int c0, const T *slot, bool ready) { axpy_slot(coef, c0, nc, slot, ready, acc); });
@@ -418,7 +462,7 @@ __global__ void __launch_bounds__(kCThreads + 32, 2) gs_cluster_kernel(const GsA
         }
         if (a.passes == 4) {
           dots(3, v);
-          meet_sums(1, [&](int i, double t) { coef[i] = (T)(kAdj ? my_dh - t : -t); });
+          meet_sums(1, [&](int i, Sum t) { coef[i] = kAdj ? g_round(g_sub(dh[i], t)) : -g_round(t); });
 #pragma unroll
           for (int e = 0; e < 8; ++e) acc[e] = (T)0;
           pass(4, [&](int c0, const T *slot, bool ready) { axpy_slot(coef, c0, nc, slot, ready, acc); });
@@ -429,19 +473,19 @@ __global__ void __launch_bounds__(kCThreads + 32, 2) gs_cluster_kernel(const GsA
       bool divide = false;
       if constexpr (!kAdj) {
         if (group == 0) {
-          double s;
+          Sum s;
           if constexpr (sizeof(T) == 4) {
             float s0 = 0.f, e0 = 0.f;
 #pragma unroll
             for (int e = 0; e < 8; ++e) two_add(s0, e0, v[e] * v[e]);
-            s = warp_sum2(s0, e0);
+            s = warp_pair(s0, e0);
           } else {
             s = v[0] * v[0];
 #pragma unroll
             for (int e = 1; e < 8; ++e) s = fma(v[e], v[e], s);
             s = warp_sum(s);
           }
-          if (lane == 0) sh->wred[wr] = s;
+          if (lane == 0) wred[wr] = s;
         }
         c_sync();
         if (!met) {
@@ -450,27 +494,21 @@ __global__ void __launch_bounds__(kCThreads + 32, 2) gs_cluster_kernel(const GsA
         }
         if (warp == 0) {
           if (lane == 0) {
-            double s = sh->wred[0];
+            Sum s = wred[0];
 #pragma unroll
-            for (int r = 1; r < kWR; ++r) s += sh->wred[r];
-            sh->npart[par] = s;
+            for (int r = 1; r < kWR; ++r) s = g_add(s, wred[r]);
+            npart[par] = s;
           }
           __syncwarp();
           c_meet_arrive(&sh->meet[2], S);
           if (S > 1) c_wait<true>(&sh->meet[2], par, fail, a.status);
-          double s = lane < S ? c_ld_f64(S > 1 ? c_map(c_smem(&sh->npart[par]), (uint32_t)lane) : c_smem(&sh->npart[par])) : 0.0;
-          for (int o = S / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-          if (lane == 0) {
-            const double nv = sqrt(s);
-            sh->fin = nv;
-            if (rank == 0) {
-              if (a.norm) a.norm[b] = nv;
-              if (a.norm2) a.norm2[b * a.norm2_bs] = nv;
-            }
-          }
+          Sum s = g_sum_of((T)0);
+          if (lane < S) s = S > 1 ? g_load_rank(npart + par, lane) : npart[par];
+          for (int o = S / 2; o > 0; o >>= 1) s = g_add(s, g_xor(s, o));
+          if (lane == 0) *fin = g_sqrt(s);
         }
         c_sync();
-        scale = (T)sh->fin;
+        scale = g_round(*fin);
         rscale = (T)1 / scale;
         divide = true;
       } else if (a.out_scale) {
@@ -503,11 +541,26 @@ __global__ void __launch_bounds__(kCThreads + 32, 2) gs_cluster_kernel(const GsA
           }
         }
       }
+      if (rank == 0) {  // what the next step does not wait for
+        if ((int)threadIdx.x < nc) {
+          if constexpr (kAdj)
+            Gb[(int64_t)a.idx * a.k + threadIdx.x] = h_pi[threadIdx.x];
+          else
+            a.h[b * a.h_bs + threadIdx.x * a.h_is] = g_double(h_pi[threadIdx.x]);
+        }
+        if (!kAdj && threadIdx.x == 0) {
+          const double nv = g_double(*fin);
+          if (a.norm) a.norm[b] = nv;
+          if (a.norm2) a.norm2[b * a.norm2_bs] = nv;
+        }
+      }
     }
   }
   // no CTA leaves while the others may read its sums or arrive on its barriers
-  c_cluster_arrive();
-  c_cluster_wait();
+  if (S > 1) {
+    c_cluster_arrive_relaxed();
+    c_cluster_wait();
+  }
 }
 
 // ---------------------------------------------------------------------------
