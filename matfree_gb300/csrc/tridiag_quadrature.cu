@@ -330,11 +330,11 @@ static int launch_tridiag_eigh_ql(int64_t k, int64_t p, const double *H, double 
 //    orthogonal to working precision; the new first/last rows are
 //    [f; 0]^T u_j and [0; l]^T u_j.
 //
-// One CTA owns one problem.  The serial parts of a merge (the sorted merge
-// of the two halves with deflated poles, the deflation scan) run on one thread per
-// merge; the merge where nothing deflates runs on a thread per element, and the roots,
-// the Loewner products and the vector rows on a group of lanes per root, over all
-// merges of a level at once.
+// One CTA owns one problem.  The sorted merge and the deflation run on a thread per
+// element, the roots, the Loewner products and the vector rows on a group of lanes per
+// root, over all merges of a level at once.  (One thread took 64000 clocks for the
+// deflation of a merge of 64, and the slowest problem of a launch decides: k = 40, 48
+// problems 240 -> 150 us with it.)
 
 constexpr int kDcMinK = 16;          // below this the QL chase is as fast
 constexpr int kDcMaxK = 2048;        // shared-memory bound (about 200 KB)
@@ -408,11 +408,30 @@ __device__ __forceinline__ double dc_quadratic(double c, double h, double a0, bo
   return div_step(small ? a0 : t, small ? t : c);
 }
 
+// The same in float32, for the first steps of a root.
+__device__ __forceinline__ float dc_quadratic(float c, float h, float a0, bool right) {
+  const float sq = sqrtf(fmaxf(fmaf(h, h, -c * a0), 0.f));
+  const bool up = h > 0.f;
+  const float t = up ? h + sq : h - sq;
+  const bool small = up != right;
+  return __fdividef(small ? a0 : t, small ? t : c);
+}
+
+// 2^e just above the largest of a merge's end poles and 2 rho, as the biased exponent
+// (0: out of the range in which a float32 copy of the merge is used)
+__device__ __forceinline__ int dc_exponent(double p0, double p1, double rho) {
+  auto e = [](double v) { return (__double2hiint(v) >> 20) & 0x7ff; };
+  int m = e(p0) > e(p1) ? e(p0) : e(p1);
+  m = m > e(rho) + 1 ? m : e(rho) + 1;
+  return m > 100 && m < 1900 ? m : 0;
+}
+__device__ __forceinline__ double dc_pow2(int biased) { return __hiloint2double(biased << 20, 0); }
+
 // Sum (product) over the G lanes of a group (lanes G m .. G m + G - 1 of a warp).
 // Every lane gets the same bits (each level adds the same two values in either
 // order), so the lanes of a group take the same branches afterwards.
-template <int G>
-__device__ __forceinline__ double group_sum(double v, unsigned mask) {
+template <int G, typename T>
+__device__ __forceinline__ T group_sum(T v, unsigned mask) {
 #pragma unroll
   for (int o = 1; o < G; o <<= 1) v += __shfl_xor_sync(mask, v, o);
   return v;
@@ -431,10 +450,18 @@ __device__ __forceinline__ double group_prod(double v, unsigned mask) {
 // time, 64 clocks each whatever its active lanes, and an SM about four warps'
 // (measured), so what counts is the number of a warp's float64 instructions:
 // comparisons run on integers, and a step is one chain for all its cases.
+// The first steps run in float32 on copies of the poles (PF: two-float numbers, so
+// that close poles keep their distance) and weights (ZF), scaled to 1: a pass over
+// the poles is some 500 clocks instead of 4000 there.  They give the nearer pole and x to
+// some 1e-6, from where two float64 passes reach rounding level; where they cannot
+// tell (a sign within their rounding, a root closer to a pole than float32 reaches) the
+// float64 midpoint decides as it would alone.  The float64 iteration is
+// safeguarded by the interval of the poles either way.  Quadrature of k = 16, 32 problems
+// 84 -> 56 us, k = 32, 64 152 -> 100 us.
 // Returns false when the iteration limit is reached.
 template <int G>
-__device__ bool dc_secular_root(const double *P, const double *ZZ, int mk, int j, double rho,
-                                double upper, int sub, unsigned gm, double &x_out, int &o_out) {
+__device__ bool dc_secular_root(const double *P, const double *ZZ, const float2 *PF, const float *ZF, int mk, int j,
+                                double rho, double upper, int sub, unsigned gm, double &x_out, int &o_out) {
   o_out = j;
   if (mk == 1) {
     x_out = rho * ZZ[0];
@@ -476,26 +503,110 @@ __device__ bool dc_secular_root(const double *P, const double *ZZ, int mk, int j
       t1 = __shfl_sync(gm, t1, lane0 + (m1 & (G - 1)));
     }
   };
-  // the sign at the midpoint names the nearer pole, the origin of the offsets
-  const double xma = 0.5 * (lo_pole + hi_pole);
-  pass(0.0, xma);
-  const double cmid = ir + (below + above), fmid = cmid + (t0 + t1);
-  const int o = (!last && !positive(fmid)) ? j + 1 : j;
-  const double base = P[o];
-  double lo = lo_pole - base, hi = hi_pole - base;
-  const double U = PU - base, V = PV - base, M = 0.5 * (U + V);
-  const double xm = 0.5 * (lo + hi);
-  // first guess: the two poles of the model exact, the other terms frozen at
-  // the midpoint of the interval
-  double x;
-  if (last) {
-    const double u = U - xm, v = V - xm;
-    x = xm + dc_quadratic(cmid, fma(cmid, M - xm, wh), u * v * fmid, true);
-    if (!positive(cmid)) x = xm;
-  } else {
-    x = dc_quadratic(cmid, fma(cmid, M, wh), fma(cmid, U * V, fma(w0, V, w1 * U)), false);
+  int o = j;
+  double x = 0.0;
+  bool found = false;
+  const int ex = dc_exponent(P[0], P[mk - 1], rho);
+  if (ex) {
+    const double sc = dc_pow2(2046 - ex);  // 2^-e
+    const float irf = 1.0f / (float)(rho * sc), f0w = ZF[m0], f1w = ZF[m1];
+    float2 bf = PF[j];
+    const float gap = last ? (float)((upper - P[j]) * sc) : (PF[m1].x - bf.x) + (PF[m1].y - bf.y);
+    float s_below, s_above, s_slope, s0, s1;
+    auto passf = [&](float y) {
+      s_below = s_above = s_slope = s0 = s1 = 0.f;
+      for (int i = sub; i < mk; i += G) {
+        const float inv = __frcp_rn(((PF[i].x - bf.x) + (PF[i].y - bf.y)) - y);
+        const float v = ZF[i] * inv;
+        if (i == m0) {
+          s0 = v;
+        } else if (i == m1) {
+          s1 = v;
+        } else {
+          s_slope = fmaf(v, inv, s_slope);
+          if (i < m0)
+            s_below += v;
+          else
+            s_above += v;
+        }
+      }
+      s_below = group_sum<G>(s_below, gm);
+      s_above = group_sum<G>(s_above, gm);
+      s_slope = group_sum<G>(s_slope, gm);
+      if (G > 1) {
+        s0 = __shfl_sync(gm, s0, lane0 + (m0 & (G - 1)));
+        s1 = __shfl_sync(gm, s1, lane0 + (m1 & (G - 1)));
+      }
+    };
+    float y = 0.5f * gap;
+    passf(y);
+    const float cm = irf + (s_below + s_above), fm = cm + (s0 + s1);
+    const float mag = (irf + (s_above - s_below)) + (fabsf(s0) + fabsf(s1));
+    if (fabsf(fm) > 2e-5f * mag) {
+      // the guess and the steps of the float64 iteration below
+      o = (!last && fm < 0.f) ? j + 1 : j;
+      bf = PF[o];
+      const float U = (PF[m0].x - bf.x) + (PF[m0].y - bf.y), V = (PF[m1].x - bf.x) + (PF[m1].y - bf.y);
+      const float M = 0.5f * (U + V), whf = 0.5f * (f0w + f1w);
+      float lo = o == j ? 0.f : -gap, hi = o == j ? gap : 0.f;
+      const float ym = 0.5f * (lo + hi);
+      if (last) {
+        const float u = U - ym, v = V - ym;
+        y = cm > 0.f ? ym + dc_quadratic(cm, fmaf(cm, M - ym, whf), u * v * fm, true) : ym;
+      } else {
+        y = dc_quadratic(cm, fmaf(cm, M, whf), fmaf(cm, U * V, fmaf(f0w, V, f1w * U)), false);
+      }
+      if (!(lo < y && y < hi)) y = ym;
+      for (int it = 0; it < 6; ++it) {
+        passf(y);
+        const float c0 = irf + (s_below + s_above), f = c0 + (s0 + s1);
+        if (f > 0.f)
+          hi = y;
+        else
+          lo = y;
+        const float u = U - y, v = V - y;
+        const float E = (last || o != j) ? u : v, se = s_slope * E;
+        const float c = c0 - se;
+        const float eta = dc_quadratic(c, fmaf(c, M - y, fmaf(se, 0.5f * E, whf)), u * v * f, last);
+        float yn = y + eta;
+        const bool done = fabsf(eta) < 1e-6f * fabsf(y);
+        if (!(lo < yn && yn < hi) || (last && !(c > 0.f))) {
+          if (done) break;
+          yn = 0.5f * (lo + hi);
+        }
+        y = yn;
+        if (done) break;
+      }
+      x = (double)y * dc_pow2(ex);
+      found = fabsf(y) > 1e-30f;
+    }
   }
-  if (!(less_than(lo, x) && less_than(x, hi))) x = xm;
+  double base = P[o], lo = lo_pole - base, hi = hi_pole - base;
+  double U = PU - base, V = PV - base;
+  if (!(found && less_than(lo, x) && less_than(x, hi))) {
+    // the sign at the midpoint names the nearer pole, the origin of the offsets
+    const double xma = 0.5 * (lo_pole + hi_pole);
+    pass(0.0, xma);
+    const double cmid = ir + (below + above), fmid = cmid + (t0 + t1);
+    o = (!last && !positive(fmid)) ? j + 1 : j;
+    base = P[o];
+    lo = lo_pole - base;
+    hi = hi_pole - base;
+    U = PU - base;
+    V = PV - base;
+    const double mid = 0.5 * (U + V), xm = 0.5 * (lo + hi);
+    // first guess: the two poles of the model exact, the other terms frozen at
+    // the midpoint of the interval
+    if (last) {
+      const double u = U - xm, v = V - xm;
+      x = xm + dc_quadratic(cmid, fma(cmid, mid - xm, wh), u * v * fmid, true);
+      if (!positive(cmid)) x = xm;
+    } else {
+      x = dc_quadratic(cmid, fma(cmid, mid, wh), fma(cmid, U * V, fma(w0, V, w1 * U)), false);
+    }
+    if (!(less_than(lo, x) && less_than(x, hi))) x = xm;
+  }
+  const double M = 0.5 * (U + V);
   bool conv = false;
   const double eps_mk = DBL_EPSILON * mk;
   for (int it = 0; it < kSecularMaxIt; ++it) {
@@ -528,6 +639,12 @@ __device__ bool dc_secular_root(const double *P, const double *ZZ, int mk, int j
         conv = true;
         break;
       }
+    } else if (less_than(fabs(eta), 1e-10 * fabs(x))) {
+      // convergence is quadratic, the other poles being no nearer than the origin:
+      // what is left is below the rounding of x
+      x = xn;
+      conv = true;
+      break;
     }
     x = xn;
   }
@@ -539,20 +656,31 @@ __device__ bool dc_secular_root(const double *P, const double *ZZ, int mk, int j
 struct DcArrays {
   double *D, *Z, *F, *L, *X, *NF, *NL, *RH, *UB;
   int *O, *MS;
+  float *ZF;  // in LAM, whose values D holds between phases A and E
 };
 constexpr int kFlipBit = 1 << 30;   // in MS: the merge was negated
 
-// Phase A of one level where nothing deflates, on all threads: the merged
-// position of each element of the two halves by binary search in the other half,
-// its value, weight and rows written there.  A merge with a negligible weight or
-// two close poles gets MS[q] = -1 and is left to the serial scan.  kVec: the
-// weights come from the eigenvector columns S, and CI keeps each pole's column.
+// The next pole of positive weight behind pole r of a merge (hi: none); flags as below.
+__device__ __forceinline__ int dc_next(const int *O, int r, int hi) {
+  do ++r;
+  while (r < hi && O[r] == 0);
+  return r;
+}
+
+// Phase A of one level, on all threads: the merged position of each element of the two
+// halves by binary search in the other half, its value, weight and rows written there.
+// Then the deflation: poles of negligible weight, and of each run of close ones all but
+// the last, whose weight is rotated onto the next one (by the thread of the run's
+// first), move behind the kept poles.  MS[q]: the kept count and kFlipBit.  kVec: the
+// weights come from the eigenvector columns S, CI keeps each pole's column, and a
+// rotation (kept in F and L) turns two columns.  LAM, FR and LR are free once their
+// values are in D, F and L.
 template <bool kVec>
-__device__ void dc_sorted_merge(const DcArrays &Ar, const double *LAM, const double *FR, const double *LR,
-                                const double *EO, const double *S, int *CI, int k, int s, int nm, double *RH,
-                                double *UB) {
+__device__ void dc_sorted_merge(const DcArrays &Ar, double *LAM, double *FR, double *LR, const double *EO, double *S,
+                                int *CI, int k, int s, int nm, double *RH, double *UB) {
+  constexpr int kLive = 1, kClose = 2, kGone = 4;  // of positive weight, close to the one before it, rotated away
   const int w = 1 << s;
-  int *MS = Ar.MS;
+  int *MS = Ar.MS, *O = Ar.O;
   for (int q = threadIdx.x; q < nm; q += blockDim.x) MS[q] = 0;
   for (int r = threadIdx.x; r < k; r += blockDim.x) {
     const int q = r >> (s + 1);
@@ -587,22 +715,138 @@ __device__ void dc_sorted_merge(const DcArrays &Ar, const double *LAM, const dou
     }
   }
   __syncthreads();
+  auto tol_of = [&](int a, int hi, double rho) {
+    const double maxabs = fmax(fabs(Ar.D[a]), fabs(Ar.D[hi - 1]));  // of the sorted values
+    return 8.0 * DBL_EPSILON * fmax(maxabs, 2.0 * rho);
+  };
+  // the weights are two unit rows: the largest root lies below d + 2 rho
+  auto bound = [](double d, double rho) { return d + 2.0 * rho * (1.0 + 1e-12) + 16.0 * DBL_EPSILON * fabs(d); };
+  int deflates = 0;
   for (int r = threadIdx.x; r < k; r += blockDim.x) {
     const int q = r >> (s + 1);
     if (q >= nm) continue;
     const int a = q * 2 * w, mid = a + w, hi = min(a + 2 * w, k);
     const double rho = fabs(EO[mid - 1]);
-    const double maxabs = fmax(fabs(Ar.D[a]), fabs(Ar.D[hi - 1]));  // of the sorted values
-    const double tol = 8.0 * DBL_EPSILON * fmax(maxabs, 2.0 * rho);
-    const double d = Ar.D[r];
-    if (!(rho * fabs(Ar.Z[r]) > tol) || (r > a && !(d - Ar.D[r - 1] > tol))) MS[q] = -1;
+    const bool drop = rho * fabs(Ar.Z[r]) <= tol_of(a, hi, rho);
+    O[r] = drop ? 0 : kLive;
+    if (drop) MS[q] = deflates = 1;
     if (r == hi - 1) {
       RH[q] = rho;
-      // the weights are two unit rows: the largest root lies below d + 2 rho
-      UB[q] = d + 2.0 * rho * (1.0 + 1e-12) + 16.0 * DBL_EPSILON * fabs(d);
+      UB[q] = bound(Ar.D[r], rho);
     }
   }
   __syncthreads();
+  int turns = 0;
+  for (int r = threadIdx.x; r < k; r += blockDim.x) {
+    const int q = r >> (s + 1);
+    if (q >= nm || O[r] == 0) continue;
+    const int a = q * 2 * w, hi = min(a + 2 * w, k);
+    int prev = r - 1;
+    while (prev >= a && O[prev] == 0) --prev;
+    if (prev >= a && Ar.D[r] - Ar.D[prev] <= tol_of(a, hi, RH[q])) {
+      O[r] = kLive | kClose;
+      MS[q] = deflates = turns = 1;
+    }
+  }
+  if (__syncthreads_or(deflates)) {
+    if (__syncthreads_or(turns)) {
+      for (int r = threadIdx.x; r < k; r += blockDim.x) {
+        const int q = r >> (s + 1);
+        if (q >= nm || (O[r] & (kLive | kClose)) != kLive) continue;
+        const int hi = min(q * 2 * w + 2 * w, k);
+        for (int p = r, n = dc_next(O, r, hi); n < hi && (O[n] & kClose); p = n, n = dc_next(O, n, hi)) {
+          const double zp = Ar.Z[p], z = Ar.Z[n], h = hypot(zp, z), c = z / h, sn = zp / h;
+          O[p] |= kGone;
+          Ar.Z[n] = h;
+          if (kVec) {
+            Ar.F[p] = c;
+            Ar.L[p] = sn;
+          } else {
+            const double fp = Ar.F[p], f = Ar.F[n], lp = Ar.L[p], l = Ar.L[n];
+            Ar.F[p] = c * fp - sn * f;
+            Ar.L[p] = c * lp - sn * l;
+            Ar.F[n] = sn * fp + c * f;
+            Ar.L[n] = sn * lp + c * l;
+          }
+        }
+      }
+      __syncthreads();
+      if (kVec)
+        for (int p = 0; p < nm * 2 * w && p < k; ++p) {
+          if (!(O[p] & kGone)) continue;  // the same for all threads
+          const int a = p >> (s + 1) << (s + 1), hi = min(a + 2 * w, k);
+          double *vp = S + (size_t)CI[p] * k, *vc = S + (size_t)CI[dc_next(O, p, hi)] * k;
+          const double c = Ar.F[p], sn = Ar.L[p];
+          for (int i = a + threadIdx.x; i < hi; i += blockDim.x) {
+            const double x = vp[i], y = vc[i];
+            vp[i] = c * x - sn * y;
+            vc[i] = sn * x + c * y;
+          }
+          __syncthreads();
+        }
+    }
+    // the kept poles in front, by way of the free arrays
+    int *kept_count = reinterpret_cast<int *>(Ar.NL), *ci = reinterpret_cast<int *>(FR);
+    for (int r = threadIdx.x; r < k; r += blockDim.x) {
+      const int q = r >> (s + 1);
+      if (q >= nm || MS[q] == 0) continue;
+      const int a = q * 2 * w, hi = min(a + 2 * w, k);
+      int before = 0, mk = 0;
+      for (int i = a; i < hi; ++i) {
+        if (i == r) before = mk;
+        mk += O[i] != 0 && !(O[i] & kGone);
+      }
+      const bool kept = O[r] != 0 && !(O[r] & kGone);
+      const int pos = kept ? a + before : a + mk + (r - a - before);
+      LAM[pos] = Ar.D[r];
+      Ar.X[pos] = Ar.Z[r];
+      if (kVec) {
+        ci[pos] = CI[r];
+      } else {
+        FR[pos] = Ar.F[r];
+        LR[pos] = Ar.L[r];
+      }
+      if (kept && before == mk - 1) UB[q] = bound(Ar.D[r], RH[q]);
+      if (r == a) kept_count[q] = mk;
+    }
+    __syncthreads();
+    for (int r = threadIdx.x; r < k; r += blockDim.x) {
+      const int q = r >> (s + 1);
+      if (q >= nm || MS[q] == 0) continue;
+      Ar.D[r] = LAM[r];
+      Ar.Z[r] = Ar.X[r];
+      Ar.NF[r] = Ar.X[r] * Ar.X[r];
+      if (kVec) {
+        CI[r] = ci[r];
+      } else {
+        Ar.F[r] = FR[r];
+        Ar.L[r] = LR[r];
+      }
+    }
+    __syncthreads();
+  }
+  for (int q = threadIdx.x; q < nm; q += blockDim.x) {
+    const int a = q * 2 * w, hi = min(a + 2 * w, k);
+    MS[q] = (MS[q] == 0 ? hi - a : reinterpret_cast<const int *>(Ar.NL)[q]) | (EO[a + w - 1] < 0.0 ? kFlipBit : 0);
+  }
+  __syncthreads();
+}
+
+// Phase E: where element r (root r - a < mk or dropped pole) of a merge with dropped
+// poles comes, both kinds being ascending: a dropped pole behind the roots that do not
+// exceed it (counted, into C[r], by dc_drop_rank), the roots in order around them.
+__device__ __forceinline__ void dc_drop_rank(const double *X, const double *D, double *C, int a, int mk, int r) {
+  const long long key = order_key(D[r]);
+  int c = 0;
+  for (int i = a; i < a + mk; ++i) c += order_key(X[i]) <= key;
+  *reinterpret_cast<int *>(C + r) = c;
+}
+__device__ __forceinline__ int dc_merged_place(const double *C, int a, int mk, int hi, int r) {
+  const int j = r - a;
+  if (j >= mk) return j - mk + *reinterpret_cast<const int *>(C + r);
+  int c = 0;
+  for (int i = a + mk; i < hi; ++i) c += *reinterpret_cast<const int *>(C + i) <= j;
+  return j + c;
 }
 
 // Phases B-D of one level (merges of width 2^(s+1)): the secular roots, the
@@ -616,10 +860,25 @@ __device__ bool dc_merge_roots(const DcArrays &Ar, int k, int s, int nm, double 
   const double *RH = Ar.RH, *UB = Ar.UB;
   int *O = Ar.O;
   const int *MS = Ar.MS;
+  float *ZF = Ar.ZF;
   const int sub = threadIdx.x & (G - 1);
   const int grp = threadIdx.x / G, ngrp = (int)blockDim.x / G;
   const unsigned gm = (G == 1 ? 1u : (1u << G) - 1u) << (threadIdx.x & 31 & ~(G - 1));
   bool ok = true;
+  // float32 copies of the kept poles (in NL) and weights (in ZF), scaled per merge
+  for (int r = threadIdx.x; r < k; r += blockDim.x) {
+    const int q = r >> (s + 1);
+    if (q >= nm) continue;
+    const int a = q << (s + 1);
+    const int mk = MS[q] & (kFlipBit - 1);
+    if (r - a >= mk) continue;
+    const int ex = dc_exponent(D[a], D[a + mk - 1], RH[q]);
+    const double d = D[r] * (ex ? dc_pow2(2046 - ex) : 0.0);
+    const float h = (float)d;
+    reinterpret_cast<float2 *>(NL)[r] = make_float2(h, (float)(d - (double)h));
+    ZF[r] = (float)NF[r];
+  }
+  __syncthreads();
   // B: secular roots over all merges of the level
   for (int r = grp; r < k; r += ngrp) {
     const int q = r >> (s + 1);
@@ -630,7 +889,8 @@ __device__ bool dc_merge_roots(const DcArrays &Ar, int k, int s, int nm, double 
     if (j >= mk) continue;
     double x;
     int o;
-    ok &= dc_secular_root<G>(D + a, NF + a, mk, j, RH[q], UB[q], sub, gm, x, o);
+    ok &= dc_secular_root<G>(D + a, NF + a, reinterpret_cast<const float2 *>(NL) + a, ZF + a, mk, j, RH[q], UB[q], sub,
+                             gm, x, o);
     if (sub == 0) {
       X[r] = x;
       O[r] = o;
@@ -764,7 +1024,7 @@ __global__ void __launch_bounds__(kDcMaxThreads, 1)
   double *UB = RH + Ly.kh;  // per merge: bound of the largest root
   int *O = reinterpret_cast<int *>(UB + Ly.kh);  // per root: origin pole
   int *MS = O + k;        // per merge: kept count and kFlipBit
-  const DcArrays Ar{D, Z, F, L, X, NF, NL, RH, UB, O, MS};
+  const DcArrays Ar{D, Z, F, L, X, NF, NL, RH, UB, O, MS, reinterpret_cast<float *>(LAM)};
 
   const double *Hb = H + (size_t)b * k * k;
   for (int i = tid; i < k; i += nt)
@@ -780,151 +1040,28 @@ __global__ void __launch_bounds__(kDcMaxThreads, 1)
   for (int s = 0; (1 << s) < k; ++s) {
     const int w = 1 << s;
     const int nm = (k - w - 1) / (2 * w) + 1;
-    // A: sorted merge of the two halves, and deflation by one thread per merge that
-    // has any (a merge of 32 took that thread 31000 clocks, all threads 2000)
+    // A: sorted merge of the two halves, deflation
     dc_sorted_merge<false>(Ar, LAM, FR, LR, EO, nullptr, nullptr, k, s, nm, RH, UB);
-    for (int q = tid; q < nm; q += nt) {
-      const int a = q * 2 * w, mid = a + w, hi = min(a + 2 * w, k);
-      double rho = EO[mid - 1];
-      const bool flip = rho < 0.0;
-      if (MS[q] == 0) {
-        MS[q] = (hi - a) | (flip ? kFlipBit : 0);
-        continue;
-      }
-      const double sg = flip ? -1.0 : 1.0;
-      rho = fabs(rho);
-      const double maxabs = fmax(fmax(fabs(LAM[a]), fabs(LAM[mid - 1])),
-                                 fmax(fabs(LAM[mid]), fabs(LAM[hi - 1])));
-      const double tol = 8.0 * DBL_EPSILON * fmax(maxabs, 2.0 * rho);
-      const int n1 = mid - a, n2 = hi - mid;
-      int c1 = 0, c2 = 0, kp = a, dp = hi;
-      double zs = 0.0;
-      for (int t = a; t < hi; ++t) {
-        bool take1;
-        if (c1 == n1)
-          take1 = false;
-        else if (c2 == n2)
-          take1 = true;
-        else
-          take1 = sg * LAM[flip ? mid - 1 - c1 : a + c1] <= sg * LAM[flip ? hi - 1 - c2 : mid + c2];
-        double d, z, f, l;
-        if (take1) {
-          const int i1 = flip ? mid - 1 - c1 : a + c1;
-          d = sg * LAM[i1];
-          z = LR[i1];
-          f = FR[i1];
-          l = 0.0;
-          ++c1;
-        } else {
-          const int i2 = flip ? hi - 1 - c2 : mid + c2;
-          d = sg * LAM[i2];
-          z = FR[i2];
-          f = 0.0;
-          l = LR[i2];
-          ++c2;
-        }
-        if (rho * fabs(z) <= tol) {  // negligible coupling: d is an eigenvalue
-          --dp;
-          D[dp] = d;
-          F[dp] = f;
-          L[dp] = l;
-          continue;
-        }
-        zs = fma(z, z, zs);
-        if (kp > a && d - D[kp - 1] <= tol) {
-          // two poles closer than tol: rotate the weight of the earlier one
-          // onto this one and drop the earlier one
-          const double zp = Z[kp - 1];
-          const double r = hypot(zp, z);
-          const double c = z / r, sn = zp / r;
-          const double fp = F[kp - 1], lp = L[kp - 1];
-          --dp;
-          D[dp] = D[kp - 1];
-          F[dp] = c * fp - sn * f;
-          L[dp] = c * lp - sn * l;
-          D[kp - 1] = d;
-          Z[kp - 1] = r;
-          NF[kp - 1] = r * r;
-          F[kp - 1] = sn * fp + c * f;
-          L[kp - 1] = sn * lp + c * l;
-        } else {
-          D[kp] = d;
-          Z[kp] = z;
-          NF[kp] = z * z;
-          F[kp] = f;
-          L[kp] = l;
-          ++kp;
-        }
-      }
-      // the dropped poles sit in [dp, hi) in reverse push order, ascending
-      // except for rotated ones: reverse, then insertion-sort the short run
-      for (int u = dp, v = hi - 1; u < v; ++u, --v) {
-        double tmp = D[u]; D[u] = D[v]; D[v] = tmp;
-        tmp = F[u]; F[u] = F[v]; F[v] = tmp;
-        tmp = L[u]; L[u] = L[v]; L[v] = tmp;
-      }
-      for (int u = dp + 1; u < hi; ++u) {
-        const double dv = D[u], fv = F[u], lv = L[u];
-        int v = u - 1;
-        while (v >= dp && D[v] > dv) {
-          D[v + 1] = D[v];
-          F[v + 1] = F[v];
-          L[v + 1] = L[v];
-          --v;
-        }
-        D[v + 1] = dv;
-        F[v + 1] = fv;
-        L[v + 1] = lv;
-      }
-      const int mk = kp - a;
-      MS[q] = mk | (flip ? kFlipBit : 0);
-      RH[q] = rho;
-      // the largest root lies below d_max + rho |z|^2; the margin keeps it
-      // strictly inside when a single pole is kept
-      UB[q] = mk > 0 ? D[kp - 1] + rho * zs * (1.0 + 16.0 * DBL_EPSILON) +
-                           16.0 * DBL_EPSILON * fabs(D[kp - 1])
-                     : 0.0;
+    ok &= dc_merge_level<false>(G, Ar, k, s, nm);
+    // E: merge the roots [a, a+mk) with the dropped poles [a+mk, hi); a negated merge
+    // is negated back and reversed
+    for (int r = tid; r < k; r += nt) {
+      const int q = r >> (s + 1);
+      const int a = q * 2 * w, mk = q < nm ? MS[q] & (kFlipBit - 1) : 0;
+      if (q < nm && r - a >= mk) dc_drop_rank(X, D, NL, a, mk, r);
     }
     __syncthreads();
-    ok &= dc_merge_level<false>(G, Ar, k, s, nm);
-    // E: merge the roots [a, a+mk) with the dropped poles [a+mk, hi), both
-    // ascending; a negated merge is negated back and reversed
-    for (int r = tid; r < k; r += nt) {  // merges without dropped poles
+    for (int r = tid; r < k; r += nt) {
       const int q = r >> (s + 1);
       if (q >= nm) continue;
-      const int a = q * 2 * w, hi = min(a + 2 * w, k);
-      if ((MS[q] & (kFlipBit - 1)) != hi - a) continue;
-      const bool flip = (MS[q] & kFlipBit) != 0;
-      const int pos = flip ? hi - 1 - (r - a) : r;
-      LAM[pos] = flip ? -X[r] : X[r];
-      FR[pos] = NF[r];
-      LR[pos] = NL[r];
-    }
-    for (int q = tid; q < nm; q += nt) {
-      const int a = q * 2 * w, hi = min(a + 2 * w, k);
-      const int mk = MS[q] & (kFlipBit - 1);
-      if (mk == hi - a) continue;
-      const bool flip = (MS[q] & kFlipBit) != 0;
-      const double sg = flip ? -1.0 : 1.0;
-      int c1 = a, c2 = a + mk;
-      for (int t = 0; t < hi - a; ++t) {
-        double v, fv, lv;
-        if (c1 < a + mk && (c2 >= hi || X[c1] <= D[c2])) {
-          v = X[c1];
-          fv = NF[c1];
-          lv = NL[c1];
-          ++c1;
-        } else {
-          v = D[c2];
-          fv = F[c2];
-          lv = L[c2];
-          ++c2;
-        }
-        const int pos = flip ? hi - 1 - t : a + t;
-        LAM[pos] = sg * v;
-        FR[pos] = fv;
-        LR[pos] = lv;
-      }
+      const int a = q * 2 * w, hi = min(a + 2 * w, k), mk = MS[q] & (kFlipBit - 1);
+      const bool flip = (MS[q] & kFlipBit) != 0, root = r - a < mk;
+      const int at = mk == hi - a ? r - a : dc_merged_place(NL, a, mk, hi, r);
+      const int pos = flip ? hi - 1 - at : a + at;
+      const double v = root ? X[r] : D[r];
+      LAM[pos] = flip ? -v : v;
+      FR[pos] = root ? NF[r] : F[r];
+      LR[pos] = root ? NL[r] : L[r];
     }
     __syncthreads();
   }
@@ -968,10 +1105,9 @@ __global__ void __launch_bounds__(kDcMaxThreads, 1)
 // tridiag_dc_kernel, carrying every eigenvector column (rows a..hi-1 of its
 // merge; zero elsewhere) in shared memory instead of first and last rows.
 // S, S2 and U are k x k, column c of S at S[c * k].
-//   A (one thread per merge): sorted merge of the halves with deflation; each
-//     pole keeps the index CI of its column in S (z is that column's entry in
-//     row mid-1 or mid), and a close-pole rotation combines two columns in
-//     place;
+//   A: sorted merge of the halves with deflation; each pole keeps the index CI of
+//     its column in S (z is that column's entry in row mid-1 or mid), and a
+//     close-pole rotation combines two columns in place;
 //   B, C, D: dc_merge_roots<G, true>, which leaves each root's normalised
 //     coefficients in U;
 //   D' (all threads over (column, row) pairs): S2[:, a+j] = S[:, CI[a..a+mk)]
@@ -995,7 +1131,7 @@ __global__ void __launch_bounds__(kDcMaxThreads, 1)
   const int64_t b = blockIdx.x;
   const DcLayout Ly = dc_layout(k);
   double *LAM = sm;
-  double *FR = LAM + k;  // unused here (same layout as tridiag_dc_kernel)
+  double *FR = LAM + k;  // scratch here (same layout as tridiag_dc_kernel)
   double *LR = FR + k;
   double *D = LR + k;
   double *Z = D + k;
@@ -1013,7 +1149,7 @@ __global__ void __launch_bounds__(kDcMaxThreads, 1)
   double *S2 = S + (size_t)k * k;
   double *U = S2 + (size_t)k * k;
   int *CI = reinterpret_cast<int *>(U + (size_t)k * k);
-  const DcArrays Ar{D, Z, F, L, X, NF, NL, RH, UB, O, MS};
+  const DcArrays Ar{D, Z, F, L, X, NF, NL, RH, UB, O, MS, reinterpret_cast<float *>(LAM)};
 
   const double *Hb = H + (size_t)b * k * k;
   for (int i = tid; i < k; i += nt)
@@ -1028,105 +1164,7 @@ __global__ void __launch_bounds__(kDcMaxThreads, 1)
     const int span = 2 * w;
     const int nm = (k - w - 1) / span + 1;
     // A
-    dc_sorted_merge<true>(Ar, LAM, nullptr, nullptr, EO, S, CI, k, s, nm, RH, UB);
-    for (int q = tid; q < nm; q += nt) {
-      const int a = q * span, mid = a + w, hi = min(a + span, k);
-      double rho = EO[mid - 1];
-      const bool flip = rho < 0.0;
-      if (MS[q] == 0) {
-        MS[q] = (hi - a) | (flip ? kFlipBit : 0);
-        continue;
-      }
-      const double sg = flip ? -1.0 : 1.0;
-      rho = fabs(rho);
-      const double maxabs = fmax(fmax(fabs(LAM[a]), fabs(LAM[mid - 1])),
-                                 fmax(fabs(LAM[mid]), fabs(LAM[hi - 1])));
-      const double tol = 8.0 * DBL_EPSILON * fmax(maxabs, 2.0 * rho);
-      const int n1 = mid - a, n2 = hi - mid;
-      int c1 = 0, c2 = 0, kp = a, dp = hi;
-      double zs = 0.0;
-      for (int t = a; t < hi; ++t) {
-        bool take1;
-        if (c1 == n1)
-          take1 = false;
-        else if (c2 == n2)
-          take1 = true;
-        else
-          take1 = sg * LAM[flip ? mid - 1 - c1 : a + c1] <= sg * LAM[flip ? hi - 1 - c2 : mid + c2];
-        double d, z;
-        int col;
-        if (take1) {
-          col = flip ? mid - 1 - c1 : a + c1;
-          z = S[(size_t)col * k + (mid - 1)];  // last row of the upper block
-          ++c1;
-        } else {
-          col = flip ? hi - 1 - c2 : mid + c2;
-          z = S[(size_t)col * k + mid];  // first row of the lower block
-          ++c2;
-        }
-        d = sg * LAM[col];
-        if (rho * fabs(z) <= tol) {
-          --dp;
-          D[dp] = d;
-          CI[dp] = col;
-          continue;
-        }
-        zs = fma(z, z, zs);
-        if (kp > a && d - D[kp - 1] <= tol) {
-          // close poles: the dropped column is c Vprev - sn Vcur (in column
-          // cp), the kept one sn Vprev + c Vcur (in column col)
-          const double zp = Z[kp - 1];
-          const double r = hypot(zp, z);
-          const double c = z / r, sn = zp / r;
-          const int cp = CI[kp - 1];
-          for (int t2 = a; t2 < hi; ++t2) {
-            const double vp = S[(size_t)cp * k + t2], vc = S[(size_t)col * k + t2];
-            S[(size_t)cp * k + t2] = c * vp - sn * vc;
-            S[(size_t)col * k + t2] = sn * vp + c * vc;
-          }
-          --dp;
-          D[dp] = D[kp - 1];
-          CI[dp] = cp;
-          D[kp - 1] = d;
-          Z[kp - 1] = r;
-          NF[kp - 1] = r * r;
-          CI[kp - 1] = col;
-        } else {
-          D[kp] = d;
-          Z[kp] = z;
-          NF[kp] = z * z;
-          CI[kp] = col;
-          ++kp;
-        }
-      }
-      for (int u = dp, v = hi - 1; u < v; ++u, --v) {
-        const double tmp = D[u];
-        D[u] = D[v];
-        D[v] = tmp;
-        const int ti = CI[u];
-        CI[u] = CI[v];
-        CI[v] = ti;
-      }
-      for (int u = dp + 1; u < hi; ++u) {
-        const double dv = D[u];
-        const int cv = CI[u];
-        int v = u - 1;
-        while (v >= dp && D[v] > dv) {
-          D[v + 1] = D[v];
-          CI[v + 1] = CI[v];
-          --v;
-        }
-        D[v + 1] = dv;
-        CI[v + 1] = cv;
-      }
-      const int mk = kp - a;
-      MS[q] = mk | (flip ? kFlipBit : 0);
-      RH[q] = rho;
-      UB[q] = mk > 0 ? D[kp - 1] + rho * zs * (1.0 + 16.0 * DBL_EPSILON) +
-                           16.0 * DBL_EPSILON * fabs(D[kp - 1])
-                     : 0.0;
-    }
-    __syncthreads();
+    dc_sorted_merge<true>(Ar, LAM, FR, LR, EO, S, CI, k, s, nm, RH, UB);
     ok &= dc_merge_level<true>(G, Ar, k, s, nm, U);
     // D': the merged columns into S2 (rows a..hi-1)
     for (int idx = tid; idx < nm * span * span; idx += nt) {
@@ -1148,37 +1186,22 @@ __global__ void __launch_bounds__(kDcMaxThreads, 1)
     }
     // E: ascending merge of the roots [a, a+mk) and the dropped poles
     // [a+mk, hi); a negated merge is negated back and reversed
-    for (int r = tid; r < k; r += nt) {  // merges without dropped poles
+    for (int r = tid; r < k; r += nt) {
+      const int q = r >> (s + 1);
+      const int a = q * span, mk = q < nm ? MS[q] & (kFlipBit - 1) : 0;
+      if (q < nm && r - a >= mk) dc_drop_rank(X, D, NL, a, mk, r);
+    }
+    __syncthreads();
+    for (int r = tid; r < k; r += nt) {
       const int q = r >> (s + 1);
       if (q >= nm) continue;
-      const int a = q * span, hi = min(a + span, k);
-      if ((MS[q] & (kFlipBit - 1)) != hi - a) continue;
-      const bool flip = (MS[q] & kFlipBit) != 0;
-      const int pos = flip ? hi - 1 - (r - a) : r;
-      LAM[pos] = flip ? -X[r] : X[r];
+      const int a = q * span, hi = min(a + span, k), mk = MS[q] & (kFlipBit - 1);
+      const bool flip = (MS[q] & kFlipBit) != 0, root = r - a < mk;
+      const int at = mk == hi - a ? r - a : dc_merged_place(NL, a, mk, hi, r);
+      const int pos = flip ? hi - 1 - at : a + at;
+      const double v = root ? X[r] : D[r];
+      LAM[pos] = flip ? -v : v;
       O[pos] = r;
-    }
-    for (int q = tid; q < nm; q += nt) {
-      const int a = q * span, hi = min(a + span, k);
-      const int mk = MS[q] & (kFlipBit - 1);
-      if (mk == hi - a) continue;
-      const bool flip = (MS[q] & kFlipBit) != 0;
-      const double sg = flip ? -1.0 : 1.0;
-      int c1 = a, c2 = a + mk;
-      for (int t = 0; t < hi - a; ++t) {
-        double v;
-        int src;
-        if (c1 < a + mk && (c2 >= hi || X[c1] <= D[c2])) {
-          v = X[c1];
-          src = c1++;
-        } else {
-          v = D[c2];
-          src = c2++;
-        }
-        const int pos = flip ? hi - 1 - t : a + t;
-        LAM[pos] = sg * v;
-        O[pos] = src;
-      }
     }
     __syncthreads();
     for (int idx = tid; idx < nm * span * span; idx += nt) {

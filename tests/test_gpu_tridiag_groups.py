@@ -35,3 +35,23 @@ def test_groups_of_lanes_match_eigh(k, p):
         v, Q = (t.cpu().numpy() for t in mf.funm.tridiag_eigh(torch.tensor(T, device="cuda")))
         assert np.abs(Q.transpose(0, 2, 1) @ Q - np.eye(k)).max() <= 1e-12 * k
         assert np.abs((Q * v[:, None, :]) @ Q.transpose(0, 2, 1) - T).max() <= 1e-12 * k * scale
+
+
+@pytest.mark.parametrize("k", [16, 33, 64, 100])
+@pytest.mark.parametrize("exponent", [-400, 0, 400])
+def test_scaled_problems_have_scaled_eigenvalues(k, exponent):
+    """The float32 first steps run on poles scaled to 1: powers of two do not change a result beyond the
+    tolerances of the equal-scale test.  (Squares of distances leave the float64 range past 2^-500 and 2^500.)"""
+    rng = np.random.default_rng(k)
+    d = rng.uniform(0.5, 4.0, (6, k))
+    e = rng.uniform(-1.0, 1.0, (6, k - 1)) * 10.0 ** rng.integers(-13, 1, (6, k - 1))
+    i = np.arange(k)
+    T = np.zeros((6, k, k))
+    T[:, i, i] = d
+    T[:, i[:-1], i[1:]] = T[:, i[1:], i[:-1]] = e
+    w, S = np.linalg.eigh(T)
+    lam, fsq = (t.cpu().numpy() for t in mf.funm.tridiag_eigh_first(torch.tensor(np.ldexp(T, exponent), device="cuda")))
+    lam = np.ldexp(lam, -exponent)
+    assert np.abs(lam - w).max() <= 1e-12 * np.abs(w).max()
+    got, want = (np.exp(lam) * fsq).sum(-1), (np.exp(w) * S[:, 0] ** 2).sum(-1)
+    assert np.abs(got - want).max() <= 1e-12 * np.exp(w).max()
