@@ -333,8 +333,7 @@ static int launch_tridiag_eigh_ql(int64_t k, int64_t p, const double *H, double 
 // One CTA owns one problem.  The sorted merge and the deflation run on a thread per
 // element, the roots, the Loewner products and the vector rows on a group of lanes per
 // root, over all merges of a level at once.  (One thread took 64000 clocks for the
-// deflation of a merge of 64, and the slowest problem of a launch decides: k = 40, 48
-// problems 240 -> 150 us with it.)
+// deflation of a merge of 64, and the slowest problem of a launch decides.)
 
 constexpr int kDcMinK = 16;          // below this the QL chase is as fast
 constexpr int kDcMaxK = 2048;        // shared-memory bound (about 200 KB)
@@ -457,7 +456,7 @@ __device__ __forceinline__ double group_prod(double v, unsigned mask) {
 // tell (a sign within their rounding, a root closer to a pole than float32 reaches) the
 // float64 midpoint decides as it would alone.  The float64 iteration is
 // safeguarded by the interval of the poles either way.  Quadrature of k = 16, 32 problems
-// 84 -> 56 us, k = 32, 64 152 -> 100 us.
+// 98 -> 61 us, k = 32, 64 146 -> 92, k = 64, 1000 1593 -> 660.
 // Returns false when the iteration limit is reached.
 template <int G>
 __device__ bool dc_secular_root(const double *P, const double *ZZ, const float2 *PF, const float *ZF, int mk, int j,
@@ -550,13 +549,8 @@ __device__ bool dc_secular_root(const double *P, const double *ZZ, const float2 
       const float M = 0.5f * (U + V), whf = 0.5f * (f0w + f1w);
       float lo = o == j ? 0.f : -gap, hi = o == j ? gap : 0.f;
       const float ym = 0.5f * (lo + hi);
-      if (last) {
-        const float u = U - ym, v = V - ym;
-        y = cm > 0.f ? ym + dc_quadratic(cm, fmaf(cm, M - ym, whf), u * v * fm, true) : ym;
-      } else {
-        y = dc_quadratic(cm, fmaf(cm, M, whf), fmaf(cm, U * V, fmaf(f0w, V, f1w * U)), false);
-      }
-      if (!(lo < y && y < hi)) y = ym;
+      y = dc_quadratic(cm, fmaf(cm, M, whf), fmaf(cm, U * V, fmaf(f0w, V, f1w * U)), last);
+      if (!(lo < y && y < hi) || (last && !(cm > 0.f))) y = ym;
       for (int it = 0; it < 6; ++it) {
         passf(y);
         const float c0 = irf + (s_below + s_above), f = c0 + (s0 + s1);
@@ -596,15 +590,10 @@ __device__ bool dc_secular_root(const double *P, const double *ZZ, const float2 
     V = PV - base;
     const double mid = 0.5 * (U + V), xm = 0.5 * (lo + hi);
     // first guess: the two poles of the model exact, the other terms frozen at
-    // the midpoint of the interval
-    if (last) {
-      const double u = U - xm, v = V - xm;
-      x = xm + dc_quadratic(cmid, fma(cmid, mid - xm, wh), u * v * fmid, true);
-      if (!positive(cmid)) x = xm;
-    } else {
-      x = dc_quadratic(cmid, fma(cmid, mid, wh), fma(cmid, U * V, fma(w0, V, w1 * U)), false);
-    }
-    if (!(less_than(lo, x) && less_than(x, hi))) x = xm;
+    // the midpoint of the interval, as an offset from the origin (a shift from the
+    // midpoint loses a root that is close to its pole)
+    x = dc_quadratic(cmid, fma(cmid, mid, wh), fma(cmid, U * V, fma(w0, V, w1 * U)), last);
+    if (!(less_than(lo, x) && less_than(x, hi)) || (last && !positive(cmid))) x = xm;
   }
   const double M = 0.5 * (U + V);
   bool conv = false;
@@ -961,10 +950,9 @@ __device__ bool dc_merge_roots(const DcArrays &Ar, int k, int s, int nm, double 
 // about 8 k / G + 3 log2 G + 29 float64 instructions of 64 clocks, and the SM's
 // warps share one such instruction per 19 clocks; a warp of more roots waits for
 // the slowest of more of them, which other warps hide where an SM has several
-// problems.  Measured: k = 16, 32 problems 252 us with one lane per root -> 98 us
-// (8); k = 32, 64: 320 -> 146 (4); k = 40, 48: 281 with 2, 219 with 4; k = 64, 256:
-// 866 -> 552 (2; with 1 654); k = 96, 32: 919 with 1, 639 with 4; k = 64, 1000: 2806 ->
-// 1593 (1).
+// problems.  Measured: k = 16, 32 problems 100 us with one lane per root -> 61 us
+// (8); k = 32, 64: 199 -> 92 (4); k = 48, 128: 344 -> 143 (4); k = 64, 256: 671 -> 301
+// (2).
 static int dc_group(int64_t k, int64_t p) {
   static int sms = 0;
   if (sms == 0) {
