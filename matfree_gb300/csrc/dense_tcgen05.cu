@@ -179,6 +179,13 @@ __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
+// The same where no data is handed over (a CTA must only not leave before the others
+// have read its shared memory): does not wait for this CTA's stores.
+__device__ __forceinline__ void cluster_sync_relaxed() {
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+}
+
 // 2-D tile copy into this CTA's shared memory completing on a barrier that
 // may live in the peer CTA (shared::cluster address).
 __device__ __forceinline__ void tma_load_2d_pair(void *dst, const CUtensorMap *map, uint32_t bar_cluster,
@@ -419,6 +426,72 @@ constexpr int kSplitKMaxBN = 128;
 constexpr int kSplitKMaxS = 8;  // portable cluster size
 constexpr size_t kSplitKRing = 220 * 1024;
 
+template <int S> struct Ranks { static constexpr int value = S; };
+
+// This CTA's share of a cluster's tile: columns (probe, row tile) i = i0, i0 + 6, ... <
+// items of four rows a lane, the S partial tiles summed in rank order.  U columns at a
+// time, so that U S reads of other CTAs' shared memory (some 1500 cycles each) and
+// the shift's reads are under way together: one by one they took 11 of the 62 us of
+// n = 8192, 128 probes.
+template <int S, int MT>
+__device__ __forceinline__ void splitk_reduce(uint32_t base, int c0, int items, int b0, int m0, int n, int p,
+                                              const float *__restrict__ Vf, int64_t ldvf, float *__restrict__ W,
+                                              int64_t ldw, float shift, int vec_ok) {
+  constexpr int U = S <= 2 ? 8 : (S <= 4 ? 4 : 2), kStep = kGemmThreads / 32;
+  const int lane = threadIdx.x & 31;
+  for (int i0 = threadIdx.x >> 5; i0 < items; i0 += U * kStep) {
+    float4 x[U][S], sv[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int i = i0 + u * kStep, c = c0 + i / MT, t = i % MT;
+      const int b = b0 + c, m = m0 + t * kBM + lane * 4;
+      const bool live = i < items && b < p && m < n;
+#pragma unroll
+      for (int r = 0; r < S; ++r)
+        x[u][r] = live ? ld_dsmem_f4(map_to_rank(base + (uint32_t)(c * MT + t) * (kBM * 4u), (uint32_t)r))
+                       : make_float4(0.f, 0.f, 0.f, 0.f);
+      sv[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (live && shift != 0.f) {
+        const float *vf = Vf + (int64_t)b * ldvf + m;
+        if (vec_ok && m + 4 <= n) {
+          sv[u] = __ldg(reinterpret_cast<const float4 *>(vf));
+        } else {
+          sv[u].x = __ldg(vf);
+          if (m + 1 < n) sv[u].y = __ldg(vf + 1);
+          if (m + 2 < n) sv[u].z = __ldg(vf + 2);
+          if (m + 3 < n) sv[u].w = __ldg(vf + 3);
+        }
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int i = i0 + u * kStep, c = c0 + i / MT, t = i % MT;
+      const int b = b0 + c, m = m0 + t * kBM + lane * 4;
+      if (!(i < items && b < p && m < n)) continue;
+      float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int r = 0; r < S; ++r) {
+        sum.x += x[u][r].x;
+        sum.y += x[u][r].y;
+        sum.z += x[u][r].z;
+        sum.w += x[u][r].w;
+      }
+      if (shift != 0.f)
+        sum = make_float4(fmaf(shift, sv[u].x, sum.x), fmaf(shift, sv[u].y, sum.y), fmaf(shift, sv[u].z, sum.z),
+                          fmaf(shift, sv[u].w, sum.w));
+      float *w = W + (int64_t)b * ldw + m;
+      if (vec_ok && m + 4 <= n) {
+        *reinterpret_cast<float4 *>(w) = sum;
+      } else {
+        w[0] = sum.x;
+        if (m + 1 < n) w[1] = sum.y;
+        if (m + 2 < n) w[2] = sum.z;
+        if (m + 3 < n) w[3] = sum.w;
+      }
+    }
+  }
+}
+
 template <bool kSplit, int MT>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 dense_tcgen05_splitk_kernel(const __grid_constant__ CUtensorMap map_ahi,
@@ -573,43 +646,24 @@ dense_tcgen05_splitk_kernel(const __grid_constant__ CUtensorMap map_ahi,
   }
   // this CTA's columns [c0, c1) of the tile; a warp takes whole columns, a
   // lane four consecutive rows
-  const int c0 = BN * part / S, c1 = BN * (part + 1) / S;
+  const int c0 = BN * part / S, items = MT * (BN * (part + 1) / S - c0);
   const uint32_t base = smem_u32(tiles) + (uint32_t)lane * 16u;
-  for (int i = warp; i < MT * (c1 - c0); i += kGemmThreads / 32) {
-    const int c = c0 + i / MT, t = i % MT;
-    const int b = b0 + c, m = m0 + t * kBM + lane * 4;
-    if (b >= p || m >= n) continue;
-    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
-    float4 x[kSplitKMaxS];
-#pragma unroll
-    for (int r = 0; r < kSplitKMaxS; ++r)
-      if (r < S) x[r] = ld_dsmem_f4(map_to_rank(base + (uint32_t)(c * MT + t) * (kBM * 4u), (uint32_t)r));
-#pragma unroll
-    for (int r = 0; r < kSplitKMaxS; ++r)
-      if (r < S) {
-        sum.x += x[r].x;
-        sum.y += x[r].y;
-        sum.z += x[r].z;
-        sum.w += x[r].w;
-      }
-    float *w = W + (int64_t)b * ldw + m;
-    const float *vf = Vf + (int64_t)b * ldvf + m;
-    if (vec_ok && m + 4 <= n) {
-      if (shift != 0.f) {
-        const float4 sv = __ldg(reinterpret_cast<const float4 *>(vf));
-        sum = make_float4(fmaf(shift, sv.x, sum.x), fmaf(shift, sv.y, sum.y), fmaf(shift, sv.z, sum.z),
-                          fmaf(shift, sv.w, sum.w));
-      }
-      *reinterpret_cast<float4 *>(w) = sum;
-    } else {
-      const float o[4] = {sum.x, sum.y, sum.z, sum.w};
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        if (m + j < n) w[j] = shift != 0.f ? fmaf(shift, __ldg(vf + j), o[j]) : o[j];
-    }
+  auto reduce = [&](auto s) {
+    splitk_reduce<decltype(s)::value, MT>(base, c0, items, b0, m0, n, p, Vf, ldvf, W, ldw, shift, vec_ok);
+  };
+  static_assert(kSplitKMaxS == 8, "cases below");
+  switch (S) {
+    case 1: reduce(Ranks<1>{}); break;
+    case 2: reduce(Ranks<2>{}); break;
+    case 3: reduce(Ranks<3>{}); break;
+    case 4: reduce(Ranks<4>{}); break;
+    case 5: reduce(Ranks<5>{}); break;
+    case 6: reduce(Ranks<6>{}); break;
+    case 7: reduce(Ranks<7>{}); break;
+    default: reduce(Ranks<8>{});
   }
   __syncwarp();
-  cluster_sync_all();  // no CTA leaves while the others may read its partial tile
+  cluster_sync_relaxed();  // no CTA leaves while the others may read its partial tile
 }
 
 // ---------------------------------------------------------------------------
@@ -1289,14 +1343,15 @@ struct SplitKPlan {
 };
 
 // The cheapest (S, mt) by the time of the rounds of CTAs: a 64-wide K slice
-// takes as long as the slowest of the SM's own intake (measured 75 GB/s with
-// three or more stages in the ring, 62 with two), the operator's share of HBM
+// takes as long as the slowest of the SM's own intake (measured 80 GB/s with
+// three or more stages in the ring, 60 with two), the operator's share of HBM
 // (6.4 TB/s over the CTAs running) and the L2 share of everything read
-// (11 TB/s); a round adds 6 us of pipeline fill and cluster reduction, and
-// 20 ns per accumulator column.  The model ranks the measured (n, p) grid
+// (11 TB/s); a round adds 5 us of pipeline fill and cluster reduction, and
+// 10 ns per accumulator column.  The model ranks the measured (n, p) grid
 // right to within a few percent: e.g. n = 23170, 32 probes S = 3 of two row
-// tiles (334 us; S = 1: 452 with one, 352 with two), n = 5000, 48 probes S = 3
-// (27 us; S = 1: 56, S = 4: 39, a second round), n = 512 S = 8 (11 us; S = 1: 17).
+// tiles (333 us; S = 1: 447 with one, 345 with two), n = 8192, 128 probes S = 2 of one
+// (55 us; S = 4 of two: 60), n = 5000, 48 probes S = 3 (20 us; S = 1: 46, S = 4: 30, a
+// second round), n = 512 S = 8 (4 us; S = 1: 7).
 static SplitKPlan splitk_plan(int64_t n, int64_t p, bool split) {
   static const SplitKSlots slots;
   const int64_t tiles_p = ceil_div(p, kSplitKMaxBN);
@@ -1307,9 +1362,9 @@ static SplitKPlan splitk_plan(int64_t n, int64_t p, bool split) {
   for (int mt = 1; mt <= 2; ++mt) {
     const double a = copies * mt * kBM * kSplitKBK * 2.0;
     const int64_t tiles = ceil_div(n, mt * kBM) * tiles_p;
-    const double intake = kSplitKRing >= 3.0 * (a + v) ? 75e3 : 62e3;  // bytes per us
+    const double intake = kSplitKRing >= 3.0 * (a + v) ? 80e3 : 60e3;  // bytes per us
     for (int S = 1; S <= kSplitKMaxS && S <= slices; ++S) {
-      const double ks = (double)ceil_div(slices, S), fixed = 6.0 + 0.02 * best.bn * mt;
+      const double ks = (double)ceil_div(slices, S), fixed = 5.0 + 0.01 * best.bn * mt;
       auto round_us = [&](double ctas) {
         double t = (a + v) / intake;
         if (ctas * a / 6.4e6 > t) t = ctas * a / 6.4e6;

@@ -103,7 +103,10 @@ __device__ __forceinline__ void d_reduce_store(const T *part, const T *__restric
       if (q < S) sum += x[q];
     W[b * ldw + m] = fma(shift, __ldg(V + b * ldv + m), sum);
   }
-  d_cluster_sync();
+  // no CTA leaves while the others may read its tile; nothing waits for the stores
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
 }
 
 // float32: 256 threads, TM x TP outputs each, rows tx + i BM / TM and probes ty + j
