@@ -47,44 +47,62 @@ __device__ __forceinline__ T d_load_rank(const T *local, int rank) {
 
 // Slices [kb, ke) of BK columns of A's rows m0.. and V's probes b0.. through the
 // stages; body(As, Vs) consumes one.  Columns past n, rows past n and probes past
-// p read as zero.
+// p read as zero.  A thread copies the same 16-byte column of kPer rows in every slice, by
+// pointers that only advance (index arithmetic per copy cost as much as a slice's FMAs).
 template <typename T, int BM, int BP, int BK, int THREADS, typename F>
 __device__ __forceinline__ void d_pipeline(T *stages, const T *__restrict__ A, int64_t lda, const T *__restrict__ V,
                                            int64_t ldv, int64_t n, int64_t p, int64_t m0, int64_t b0, int64_t kb,
                                            int64_t ke, F body) {
-  constexpr int VW = Vec<T>::width, LD = BK + VW, PER = BK / VW;
-  constexpr int64_t kStage = (int64_t)(BM + BP) * LD;
-  auto load = [&](int64_t slice) {
-    if (slice < ke) {
-      T *st = stages + (slice - kb) % kDStages * kStage;
-      for (int i = threadIdx.x; i < (BM + BP) * PER; i += THREADS) {
-        const int r = i / PER, c = i % PER * VW;
-        const int64_t k = slice * BK + c;
-        const bool isA = r < BM;
-        const int64_t row = isA ? m0 + r : b0 + (r - BM);
-        const int64_t left = row < (isA ? n : p) ? n - k : 0;
-        const int bytes = left >= VW ? 16 : (left > 0 ? (int)(left * sizeof(T)) : 0);
-        const T *src = bytes ? (isA ? A + row * lda : V + row * ldv) + k : A;
-        cp_async16(st + (int64_t)r * LD + c, src, bytes);
+  constexpr int VW = Vec<T>::width, LD = BK + VW, PER = BK / VW, kStage = (BM + BP) * LD;
+  constexpr int kRowStep = THREADS / PER, kPer = (BM + BP + kRowStep - 1) / kRowStep;
+  static_assert(THREADS % PER == 0, "a thread's column");
+  const int row = threadIdx.x / PER, c = threadIdx.x % PER * VW;
+  const T *src[kPer];
+  bool live[kPer];
+#pragma unroll
+  for (int q = 0; q < kPer; ++q) {
+    const int r = row + q * kRowStep;
+    const bool isA = r < BM;
+    const int64_t at = isA ? m0 + r : b0 + (r - BM);
+    live[q] = r < BM + BP && at < (isA ? n : p);
+    src[q] = live[q] ? (isA ? A + at * lda : V + at * ldv) + kb * BK + c : A;
+  }
+  int left = (int)(ke - kb), fill = 0;                  // slices to load; the stage they go to
+  int64_t cols = n - kb * BK - c;                       // columns left at this thread's
+  auto load = [&]() {
+    if (left > 0) {
+      T *st = stages + fill * kStage + row * LD + c;
+      const int bytes = cols >= VW ? 16 : (cols > 0 ? (int)cols * (int)sizeof(T) : 0);
+#pragma unroll
+      for (int q = 0; q < kPer; ++q) {
+        if (row + q * kRowStep < BM + BP)
+          cp_async16(st + q * kRowStep * LD, live[q] && bytes ? src[q] : A, live[q] ? bytes : 0);
+        src[q] += live[q] ? BK : 0;
       }
+      cols -= BK;
+      --left;
+      if (++fill == kDStages) fill = 0;
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
 #pragma unroll
-  for (int s = 0; s < kDStages - 1; ++s) load(kb + s);
-  for (int64_t slice = kb; slice < ke; ++slice) {
+  for (int s = 0; s < kDStages - 1; ++s) load();
+  int use = 0;
+  for (int slices = (int)(ke - kb); slices > 0; --slices) {
     asm volatile("cp.async.wait_group %0;" ::"n"(kDStages - 2) : "memory");
     __syncthreads();  // this slice has landed, and the stage loaded next is no longer read
-    load(slice + kDStages - 1);
-    const T *st = stages + (slice - kb) % kDStages * kStage;
-    body(st, st + (int64_t)BM * LD);
+    load();
+    const T *st = stages + use * kStage;
+    body(st, st + BM * LD);
+    if (++use == kDStages) use = 0;
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
   __syncthreads();
 }
 
-// The cluster's partial tiles part[BP][BM] into W, this CTA's share of the probes.
-template <typename T, int BM, int BP, int THREADS>
+// The cluster's partial tiles part[BP][BM] (probes PITCH apart) into W, this CTA's
+// share of the probes.
+template <typename T, int BM, int BP, int PITCH, int THREADS>
 __device__ __forceinline__ void d_reduce_store(const T *part, const T *__restrict__ V, int64_t ldv, T *__restrict__ W,
                                                int64_t ldw, int64_t n, int64_t p, int64_t m0, int64_t b0, int rank,
                                                int S, T shift) {
@@ -96,7 +114,7 @@ __device__ __forceinline__ void d_reduce_store(const T *part, const T *__restric
     if (m >= n || b >= p) continue;
     T x[kDMaxS];
 #pragma unroll
-    for (int q = 0; q < kDMaxS; ++q) x[q] = q < S ? d_load_rank(part + c * BM + r, q) : (T)0;
+    for (int q = 0; q < kDMaxS; ++q) x[q] = q < S ? d_load_rank(part + c * PITCH + r, q) : (T)0;
     T sum = x[0];
 #pragma unroll
     for (int q = 1; q < kDMaxS; ++q)
@@ -109,51 +127,72 @@ __device__ __forceinline__ void d_reduce_store(const T *part, const T *__restric
   asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
 }
 
-// float32: 256 threads, TM x TP outputs each, rows tx + i BM / TM and probes ty + j
-// BP / TP; four columns at a time from 16-byte reads, 8 of them for 64 FMAs.  Bound by
-// the FMA pipes and, for small operators, by too few tiles.  Against 32 x 32 and
-// 128 x 64 tiles staged through registers: n = 2000, 64 probes 54 -> 27 us; n = 512, 32
-// 17 -> 7; n = 4096, 256 598 -> 279 (31 TFLOP/s); n = 16384, 256 5.84 -> 4.18 ms.
-template <int BM, int BP, int TM, int TP>
-__global__ void __launch_bounds__(256)
+// float32: tiles of 64 rows x BP probes by G groups of threads, each group the whole
+// tile over a G-th of every slice's columns; a thread has 8 rows tx + 8 i and four probes
+// ty + TY j, read 16 bytes (four columns) at a time and summed as pairs of columns by
+// two-float FMAs: 12 reads for 64 of these, two CTAs an SM so that one's reads overlap
+// the other's FMAs.  Bound by those reads (four cycles of shared memory each) and the FMA
+// pipes.  Against 4 x 4 outputs a thread and copies indexed anew in every slice: n =
+// 2000, 64 probes 27 -> 22.8 us; n = 4096, 256 279 -> 228; n = 16384, 256 4.18 -> 3.38 ms (41
+// TFLOP/s).  8 x 8 outputs, one CTA an SM: 22.8, 261, 3.43; 64-column slices 24.6, 240, 3.53.
+// two float FMAs in one instruction, and the sum of the two
+__device__ __forceinline__ void fma2(unsigned long long &acc, unsigned long long a, unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ float sum2(unsigned long long v) {
+  return __uint_as_float((uint32_t)v) + __uint_as_float((uint32_t)(v >> 32));
+}
+
+template <int BP, int BK, int G>
+__global__ void __launch_bounds__(256, 2)
 dense_f32_kernel(const float *__restrict__ A, int64_t lda, const float *__restrict__ V, int64_t ldv,
                  float *__restrict__ W, int64_t ldw, int64_t n, int64_t p, float shift) {
-  constexpr int BK = 32, LD = BK + 4, RX = BM / TM, RY = BP / TP;
-  static_assert(RX * RY == 256, "thread layout");
+  constexpr int BM = 64, LD = BK + 4, TY = 32 / G, TP = BP / TY, PITCH = BM + 8, KG = BK / G;
   extern __shared__ __align__(16) uint8_t d_raw[];
   float *stages = reinterpret_cast<float *>(d_raw);
   const int S = (int)gridDim.x, rank = (int)blockIdx.x;
   const int64_t m0 = (int64_t)blockIdx.y * BM, b0 = (int64_t)blockIdx.z * BP;
   const int64_t slices = (n + BK - 1) / BK;
-  const int tx = threadIdx.x % RX, ty = threadIdx.x / RX;
-  float acc[TM][TP];
+  const int tx = threadIdx.x & 7, ty = (threadIdx.x >> 3) % TY, group = threadIdx.x / (8 * TY);
+  unsigned long long acc[8][TP];
 #pragma unroll
-  for (int i = 0; i < TM; ++i)
+  for (int i = 0; i < 8; ++i)
 #pragma unroll
-    for (int j = 0; j < TP; ++j) acc[i][j] = 0.f;
+    for (int j = 0; j < TP; ++j) acc[i][j] = 0;
   d_pipeline<float, BM, BP, BK, 256>(
       stages, A, lda, V, ldv, n, p, m0, b0, slices * rank / S, slices * (rank + 1) / S,
       [&](const float *As, const float *Vs) {
 #pragma unroll
-        for (int k = 0; k < BK; k += 4) {
-          float a[TM][4], v[TP][4];
+        for (int kk = 0; kk < KG; kk += 4) {
+          const int k = group * KG + kk;
+          ulonglong2 v[TP];
 #pragma unroll
-          for (int i = 0; i < TM; ++i) vec_to_array<float>(*reinterpret_cast<const float4 *>(As + (tx + i * RX) * LD + k), a[i]);
+          for (int j = 0; j < TP; ++j) v[j] = *reinterpret_cast<const ulonglong2 *>(Vs + (ty + j * TY) * LD + k);
 #pragma unroll
-          for (int j = 0; j < TP; ++j) vec_to_array<float>(*reinterpret_cast<const float4 *>(Vs + (ty + j * RY) * LD + k), v[j]);
+          for (int i = 0; i < 8; ++i) {
+            const ulonglong2 a = *reinterpret_cast<const ulonglong2 *>(As + (tx + i * 8) * LD + k);
 #pragma unroll
-          for (int u = 0; u < 4; ++u)
-#pragma unroll
-            for (int i = 0; i < TM; ++i)
-#pragma unroll
-              for (int j = 0; j < TP; ++j) acc[i][j] = fmaf(a[i][u], v[j][u], acc[i][j]);
+            for (int j = 0; j < TP; ++j) {
+              fma2(acc[i][j], a.x, v[j].x);
+              fma2(acc[i][j], a.y, v[j].y);
+            }
+          }
         }
       });
+  // the groups' partial tiles, probes PITCH apart (no bank twice), summed in order
 #pragma unroll
   for (int j = 0; j < TP; ++j)
 #pragma unroll
-    for (int i = 0; i < TM; ++i) stages[(ty + j * RY) * BM + tx + i * RX] = acc[i][j];
-  d_reduce_store<float, BM, BP, 256>(stages, V, ldv, W, ldw, n, p, m0, b0, rank, S, shift);
+    for (int i = 0; i < 8; ++i) stages[(group * BP + ty + j * TY) * PITCH + tx + i * 8] = sum2(acc[i][j]);
+  __syncthreads();
+  for (int i = threadIdx.x; i < BP * BM; i += 256) {
+    const int at = i / BM * PITCH + i % BM;
+    float sum = stages[at];
+#pragma unroll
+    for (int g = 1; g < G; ++g) sum += stages[g * BP * PITCH + at];
+    stages[at] = sum;
+  }
+  d_reduce_store<float, BM, BP, PITCH, 256>(stages, V, ldv, W, ldw, n, p, m0, b0, rank, S, shift);
 }
 
 // float64: four warps, warp w the probes 8 w .. 8 w + 7 of the tile, its rows as M / 8
@@ -161,8 +200,8 @@ dense_f32_kernel(const float *__restrict__ A, int64_t lda, const float *__restri
 // instructions (measured), whatever a warp's independent chains, so tiles are small
 // and many: up to five CTAs share an SM's pipe, MMAs past the last row or probe are
 // left out, and no operand is reused in registers.  Against 32 x 32 tiles of FMA
-// instructions on one CTA each: n = 1000, 100 probes 272 -> 242 us (0.83 TFLOP/s, 0.80 of
-// that rate); n = 1500, 100 785 -> 480; n = 700, 37 193 -> 57; n = 200, 16 60 -> 11.
+// instructions on one CTA each: n = 1000, 100 probes 272 -> 234 us (0.86 TFLOP/s, 0.83 of
+// that rate); n = 1500, 100 785 -> 470; n = 700, 37 193 -> 54; n = 200, 16 60 -> 11.
 constexpr int kF64M = 16, kF64P = 32, kF64K = 32;
 
 __global__ void __launch_bounds__(128)
@@ -201,7 +240,7 @@ dense_f64_kernel(const double *__restrict__ A, int64_t lda, const double *__rest
   for (int i = 0; i < kRows; ++i)
 #pragma unroll
     for (int e = 0; e < 2; ++e) stages[(warp * 8 + 2 * fk + e) * M + i * 8 + fr] = c[i][e];
-  d_reduce_store<double, M, kF64P, 128>(stages, V, ldv, W, ldw, n, p, m0, b0, rank, S, shift);
+  d_reduce_store<double, M, kF64P, M, 128>(stages, V, ldv, W, ldw, n, p, m0, b0, rank, S, shift);
 }
 
 template <typename K, typename T>
@@ -224,6 +263,16 @@ static int launch_dense_cluster(K kern, int bm, int bp, int threads, size_t smem
   cfg.numAttrs = 1;
   MFG_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, A, lda, V, ldv, W, ldw, n, p, shift));
   return MFG_LAUNCH_STATUS();
+}
+
+// the launch of one float32 form, with the shared memory that the form needs
+template <int BP, int BK, int G>
+static int launch_f32(int S, const float *A, int64_t lda, const float *V, int64_t ldv, float *W, int64_t ldw, int64_t n,
+                      int64_t p, float shift, cudaStream_t s) {
+  constexpr size_t kRing = (size_t)kDStages * (64 + BP) * (BK + 4) * sizeof(float);
+  constexpr size_t kPart = (size_t)G * BP * 72 * sizeof(float);
+  return launch_dense_cluster(dense_f32_kernel<BP, BK, G>, 64, BP, 256, kRing > kPart ? kRing : kPart, S, A, lda, V,
+                              ldv, W, ldw, n, p, shift, s);
 }
 
 template <typename T>
@@ -257,17 +306,25 @@ int launch_dense_simt(const T *A, int64_t lda, const T *V, int64_t ldv, T *W, in
     const size_t smem = (size_t)kDStages * (kF64M + kF64P) * (kF64K + 2) * sizeof(double);
     return launch_dense_cluster(dense_f64_kernel, kF64M, kF64P, 128, smem, S, A, lda, V, ldv, W, ldw, n, p, shift, s);
   } else {
-    // four to eight K ranges of at least two slices (n = 2000, 64 probes: one range 104
-    // us, two 56, four 31, eight 27; n = 4096, 256: 330, 322, 279, 299)
+    // the K ranges of least time: an SM's CTAs share its pipes, so what counts is the
+    // CTAs of the busiest SM (clusters of three to eight leave SMs of a GPC over) times the
+    // slices of one; a range more is a tile more to add.  n = 2000, 64 probes S = 8 22.8 us (4:
+    // 24.8, 5: 33.0); n = 3001, 64 S = 5 45 (4: 55, 6: 56, 8: 48); n = 4096, 256 S = 4 228 (2: 258).
+    static const int kFit[kDMaxS + 1] = {0, 152, 152, 138, 148, 140, 138, 105, 144};  // SMs of clusters of S
     const int bp = p <= 32 ? 32 : 64;
-    const int64_t tiles = ceil_div(n, 64) * ceil_div(p, bp), slices = ceil_div(n, 32);
-    int64_t S = ceil_div(4 * (int64_t)sms, tiles);
-    S = S < 4 ? 4 : (S > kDMaxS ? kDMaxS : S);
-    if (S > slices / 2) S = slices / 2;
-    if (S < 1) S = 1;
-    const size_t smem = (size_t)kDStages * (64 + bp) * 36 * sizeof(float);
-    return launch_dense_cluster(bp == 32 ? dense_f32_kernel<64, 32, 4, 2> : dense_f32_kernel<64, 64, 4, 4>, 64, bp, 256,
-                                smem, (int)S, A, lda, V, ldv, W, ldw, n, p, (float)shift, s);
+    const int64_t tiles = ceil_div(n, 64) * ceil_div(p, bp), slices = ceil_div(n, 64);
+    int S = 1;
+    double best = 1e300;
+    for (int c = 1; c <= kDMaxS && c <= slices; ++c) {
+      const double busiest = (double)ceil_div(tiles * c * 152, (int64_t)kFit[c] * sms);
+      const double cost = busiest * (double)ceil_div(slices, c) * (1.0 + 0.15 * sms / (double)(tiles * c)) + 0.15 * c;
+      if (cost < best) {
+        best = cost;
+        S = c;
+      }
+    }
+    if (bp == 32) return launch_f32<32, 64, 4>(S, A, lda, V, ldv, W, ldw, n, p, (float)shift, s);
+    return launch_f32<64, 32, 2>(S, A, lda, V, ldv, W, ldw, n, p, (float)shift, s);
   }
 }
 template int launch_dense_simt<float>(const float *, int64_t, const float *, int64_t, float *,
