@@ -49,7 +49,8 @@ def quadform_dH(H: torch.Tensor, scale: torch.Tensor, f, fprime) -> tuple[torch.
     w, S = tridiag_eigh(H)  # the eigh of T = tridiagonal part of (H + H^T)/2
     fw = f(w)
     live = torch.is_grad_enabled() and (scale.requires_grad or fw.requires_grad)
-    if not live and fw.dtype == scale.dtype == torch.float64 and scale.shape == (p,) and 0 < p and k <= 4096:
+    if (w.is_cuda and not live and fw.dtype == scale.dtype == torch.float64 and scale.shape == (p,) and 0 < p
+            and k <= 4096):
         fmid = fprime(0.5 * (w[:, :, None] + w[:, None, :])).to(torch.float64)
         fmid, fw, scale = fmid.expand(p, k, k).contiguous(), fw.contiguous(), scale.contiguous()
         values = torch.empty(p, dtype=torch.float64, device=w.device)
@@ -58,7 +59,7 @@ def quadform_dH(H: torch.Tensor, scale: torch.Tensor, f, fprime) -> tuple[torch.
                                                 for t in (w, S, fw, fmid, scale, values, dH)), stream_ptr())
         _lib.check(st, "mfg_quadform_dh")
         return values, dH
-    # differentiable f or scale, other types
+    # differentiable f or scale, other types and devices
     s1 = S[:, 0, :]
     values = scale * (fw * s1 * s1).sum(-1)
     diff = w[:, :, None] - w[:, None, :]
