@@ -48,7 +48,9 @@ def require_cuda(t, what: str) -> torch.Tensor:
 
 
 def stream_ptr() -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    """The current stream of the current device (``torch.cuda.current_stream()`` without its
+    Python objects: a solve asks four to eight times)."""
+    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
 
 def empty_panel(p: int, n: int, dtype, device="cuda") -> torch.Tensor:

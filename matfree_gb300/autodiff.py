@@ -31,7 +31,7 @@ import torch
 
 from . import _lib
 from ._panel import Workspace, as_panel, padded_ld, require_cuda, stream_ptr
-from .decomp import run_hessenberg, two_sweep_applies
+from .decomp import retry_needed, run_hessenberg, two_sweep_applies
 from .operators import CallbackOperator, DenseOperator, RBFKernelOperator
 from .tree import _rebuild, tree_leaves
 
@@ -152,8 +152,13 @@ class _RBFLogdet(torch.autograd.Function):
         chunks = probe_chunks(p, n, k, op.basis_dtype, budget_bytes)
         vals, saved = [], []
         for b0, b1 in chunks:
-            Q, H, R, c = _forward_panels(op, k, panel[b0:b1], ld)
+            # the solve is checked once the quadrature is enqueued behind it
+            deferred = []
+            Q, H, R, c = _forward_panels(op, k, panel[b0:b1], ld, deferred)
             values, dH = quadform_dH(H, 1.0 / (c * c), _log, _dlog)
+            if retry_needed(deferred):
+                Q, H, R, c = _forward_panels(op, k, panel[b0:b1], ld)
+                values, dH = quadform_dH(H, 1.0 / (c * c), _log, _dlog)
             vals.append(values)
             if len(chunks) == 1:
                 saved.append((Q, H, R, c, dH))
@@ -180,8 +185,9 @@ class _RBFLogdet(torch.autograd.Function):
         return grad.to(device=theta.device, dtype=theta.dtype), None, None, None, None, None
 
 
-def _forward_panels(op, k, panel, ld):
-    """mfg_hessenberg keeping the padded (p, k, ld) / (p, ld) panels."""
+def _forward_panels(op, k, panel, ld, deferred=None):
+    """mfg_hessenberg keeping the padded (p, k, ld) / (p, ld) panels (deferred: as in
+    ``run_hessenberg``)."""
     p = panel.shape[0]
     dt = op.basis_dtype
     Q = torch.zeros((p, k, ld), dtype=dt, device=panel.device)
@@ -206,6 +212,9 @@ def _forward_panels(op, k, panel, ld):
             raise err
         _lib.check(st, "mfg_hessenberg")
         if mode == 1:
+            break
+        if deferred is not None:
+            deferred.append(ws)
             break
         dst = lib.mfg_workspace_status(ws, stream_ptr())
         if dst != _lib.MFG_ERR_RETRY:

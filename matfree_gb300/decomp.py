@@ -54,7 +54,7 @@ def full_reortho(op, k: int) -> str:
     return "full-two-sweep" if two_sweep_applies(op, k) else "full"
 
 
-def run_hessenberg(op, k: int, V: torch.Tensor, *, reortho: str = "full", workspace=None):
+def run_hessenberg(op, k: int, V: torch.Tensor, *, reortho: str = "full", workspace=None, deferred=None):
     """Batched Arnoldi over the rows of V (p, n) on the GPU.
 
     ``reortho``: "full" (Gram-Schmidt twice, three reads of the basis per
@@ -62,6 +62,10 @@ def run_hessenberg(op, k: int, V: torch.Tensor, *, reortho: str = "full", worksp
     the device reports a step near an invariant subspace), "none", or
     "lanczos" (the three-term recurrence).
     Returns (Q (p, k, n), H (p, k, k) float64, residual (p, n), 1/||v|| (p,)).
+
+    Reading the device's report waits for the solve.  With a list ``deferred`` the
+    wait is left to the caller, who enqueues what follows first and then asks
+    :func:`retry_needed`; on True everything is to be done again without it.
     """
     V = require_cuda(V, "vectors")
     n = op.n
@@ -90,13 +94,28 @@ def run_hessenberg(op, k: int, V: torch.Tensor, *, reortho: str = "full", worksp
         op.error = None
         raise err
     _lib.check(st, "mfg_hessenberg")
-    if mode == 3:
+    if mode == 3 and deferred is not None:
+        deferred.append(ws)
+    elif mode == 3:
         # the two-sweep step asks for the three-sweep form near an invariant subspace
         dst = lib.mfg_workspace_status(ws, stream_ptr())
         if dst == _lib.MFG_ERR_RETRY:
             return run_hessenberg(op, k, V, reortho="full", workspace=workspace)
         _lib.check(dst, "mfg_hessenberg (device status)")
     return Q[:, :, :n], H, R[:, :n], c
+
+
+def retry_needed(deferred: list) -> bool:
+    """Wait for the solves whose check was ``deferred`` (workspaces, none used since by
+    another solve); True if one asks for the three-sweep form."""
+    retry = False
+    for ws in deferred:
+        dst = _lib.lib().mfg_workspace_status(ws, stream_ptr())
+        if dst == _lib.MFG_ERR_RETRY:
+            retry = True
+        else:
+            _lib.check(dst, "mfg_hessenberg (device status)")
+    return retry
 
 
 def _tridiag_from_hessenberg(H):
@@ -136,7 +155,7 @@ class _Decomposition:
                              init_length_inv=c[0])
 
 
-def _differentiable_forward(dec, op, k, V):
+def _differentiable_forward(dec, op, k, V, deferred=None):
     """run_hessenberg with full reorthogonalisation, behind the Hessenberg
     adjoint when V or the matvec's parameters require gradients (the custom
     VJP of matfree/decomp.py:393-422); plain otherwise."""
@@ -148,7 +167,7 @@ def _differentiable_forward(dec, op, k, V):
                 "gradients of the decomposition need custom_vjp=True: the Krylov loop runs as CUDA "
                 "kernels, so it is differentiated by the Hessenberg adjoint, not traced")
         return arnoldi_full(op, k, V)
-    return run_hessenberg(op, k, V, reortho=full_reortho(op, k))
+    return run_hessenberg(op, k, V, reortho=full_reortho(op, k), deferred=deferred)
 
 
 class _TridiagSymFull(_Decomposition):
@@ -157,10 +176,13 @@ class _TridiagSymFull(_Decomposition):
 
         Differentiable in V and in the tensor leaves of a callable matvec's
         parameters (custom_vjp=True, the default)."""
+        return self._batched(matvec, V, params)
+
+    def _batched(self, matvec, V: torch.Tensor, params, deferred=None) -> _DecompResult:
         V = require_cuda(V, "vectors")
         op = as_operator(matvec, V.shape[1], V.dtype, params)
         k = self.num_matvecs
-        Q, H, r, c = _differentiable_forward(self, op, k, V)
+        Q, H, r, c = _differentiable_forward(self, op, k, V, deferred)
         d, e = _tridiag_from_hessenberg(H)
         out_dt = V.dtype if V.dtype in (torch.float32, torch.float64) else torch.float32
         d, e = d.to(out_dt), e.to(out_dt)

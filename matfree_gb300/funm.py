@@ -241,12 +241,29 @@ class FunmLanczosSym:
         return unravel(self.batched(op, flat[None, :])[0])
 
     def batched(self, matvec, V: torch.Tensor, *parameters) -> torch.Tensor:
+        from .decomp import _TridiagSymFull, retry_needed
+
+        V = require_cuda(V, "vectors")
+        # with a closed-form f and an operator descriptor nothing below runs the
+        # caller's code: the solve is checked once all of it is enqueued
+        deferred = []
+        if self.dense_funm.kind is not None and isinstance(matvec, Operator) \
+                and type(self.tridiag_sym) is _TridiagSymFull:
+            out = self._apply(matvec, V, parameters, deferred)
+            if not retry_needed(deferred):
+                return out
+        return self._apply(matvec, V, parameters, None)
+
+    def _apply(self, matvec, V, parameters, deferred):
         from .autodiff import basis_combine, funm_e1
         from .decomp import _todense_tridiag_sym
 
-        V = require_cuda(V, "vectors")
         length = torch.linalg.vector_norm(V, dim=1)
-        Q, T, *_ = self.tridiag_sym.batched(matvec, V / length[:, None], *parameters)
+        X = V / length[:, None]
+        if deferred is None:
+            Q, T, *_ = self.tridiag_sym.batched(matvec, X, *parameters)
+        else:
+            Q, T, *_ = self.tridiag_sym._batched(matvec, X, parameters, deferred)
         if isinstance(T, tuple):
             T = _todense_tridiag_sym(*T)
         if T.shape[-1] == 0:
