@@ -1047,7 +1047,13 @@ constexpr int kGemvRows = kGemvWarps / kGemvSeg;  // rows per CTA
 // kDeep: loads of two iterations ahead in flight instead of one (for one
 // probe, whose products are too few to cover the latency; with more probes
 // the deeper ring costs occupancy).
-template <int P, bool kSplit, bool kDeep>
+// NR rows of a warp share the panel's values, loaded and widened once: two, but one for
+// one probe (the deeper ring serves it better).  A CG iteration of n = 8192, 2 probes 60.0
+// -> 55.4 us, 4 probes 81.5 -> 76.9, 8 probes 162 -> 165 (bound by the FMAs; n = 5000, 6
+// probes 56.7 -> 52.8); four rows: 58.4, 98.0, 190.  The sums are those of one row a warp.
+constexpr int gemv_warp_rows(int P) { return P > 1 ? 2 : 1; }
+
+template <int P, bool kSplit, bool kDeep, int NR>
 __device__ __forceinline__ void gemv_rows(const __nv_bfloat16 *__restrict__ Ahi,
                                           const __nv_bfloat16 *__restrict__ Alo, int64_t lda,
                                           const __nv_bfloat16 *__restrict__ Vhi,
@@ -1056,58 +1062,64 @@ __device__ __forceinline__ void gemv_rows(const __nv_bfloat16 *__restrict__ Ahi,
                                           float *__restrict__ W, int64_t ldw, int n, int p,
                                           float shift, int ahead) {
   constexpr int kAhead = kDeep ? 512 : 256;
-  __shared__ float part[kGemvWarps][P];
+  __shared__ float part[kGemvWarps][NR][P];
+  static_assert(kGemvRows * NR * P <= 32 * kGemvWarps, "a thread per result");
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int seg = warp % kGemvSeg;
-  const int64_t m = (int64_t)blockIdx.x * kGemvRows + warp / kGemvSeg;
-  float acc[P];
+  const int64_t m = ((int64_t)blockIdx.x * kGemvRows + warp / kGemvSeg) * NR;
+  float acc[NR][P];
+  const __nv_bfloat16 *ah[NR], *al[NR];
 #pragma unroll
-  for (int b = 0; b < P; ++b) acc[b] = 0.f;
-  const int64_t row = m < n ? m : 0;
-  const __nv_bfloat16 *ah = Ahi + row * lda;
-  const __nv_bfloat16 *al = kSplit ? Alo + row * lda : nullptr;
+  for (int r = 0; r < NR; ++r) {
+    const int64_t row = m + r < n ? m + r : n - 1;  // rows past the last repeat it and are not stored
+    ah[r] = Ahi + row * lda;
+    al[r] = kSplit ? Alo + row * lda : nullptr;
+#pragma unroll
+    for (int b = 0; b < P; ++b) acc[r][b] = 0.f;
+  }
   const int n8 = n & ~7;
   const int seg_len = ((n8 / 8 + kGemvSeg - 1) / kGemvSeg) * 8;  // a multiple of 8 columns
   const int c0 = seg * seg_len;
   const int c1 = min(c0 + seg_len, n8);
-  if ((int)blockIdx.x < ahead && m < n) {
+  if ((int)blockIdx.x < ahead) {
     // chained: this segment on its way to L2 while the kernel before ends
     for (int c = c0 + lane * 64; c < c1; c += 32 * 64) {
-      l2_prefetch(ah + c);
-      if (kSplit) l2_prefetch(al + c);
+#pragma unroll
+      for (int r = 0; r < NR; ++r) {
+        l2_prefetch(ah[r] + c);
+        if (kSplit) l2_prefetch(al[r] + c);
+      }
     }
   }
   chain_wait();
   chain_next();
-  if (m < n) {  // warp-uniform; every warp reaches the barrier below
+  {
     const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-    uint4 h0 = zero, l0 = zero, h1 = zero, l1 = zero;
+    uint4 h0[NR], l0[NR], h1[NR], l1[NR];
     const int cl = c0 + lane * 8;
-    if (cl < c1) {
-      h0 = ld_stream16(ah + cl);
-      if (kSplit) l0 = ld_stream16(al + cl);
-    }
-    if (kDeep && cl + 256 < c1) {
-      h1 = ld_stream16(ah + cl + 256);
-      if (kSplit) l1 = ld_stream16(al + cl + 256);
-    }
-    for (int c = cl; c < c1; c += 256) {
-      uint4 h2 = zero, l2 = zero;
-      if (c + kAhead < c1) {
-        h2 = ld_stream16(ah + c + kAhead);
-        if (kSplit) l2 = ld_stream16(al + c + kAhead);
+    auto fetch = [&](int c, uint4(&h)[NR], uint4(&l)[NR]) {
+#pragma unroll
+      for (int r = 0; r < NR; ++r) {
+        h[r] = c < c1 ? ld_stream16(ah[r] + c) : zero;
+        if (kSplit) l[r] = c < c1 ? ld_stream16(al[r] + c) : zero;
       }
-      float a1[8], a2[8];
-      bf16x8_to_float(h0, a1);
-      if (kSplit) bf16x8_to_float(l0, a2);
-      if (kDeep) {
-        h0 = h1;
-        l0 = l1;
-        h1 = h2;
-        l1 = l2;
-      } else {
-        h0 = h2;
-        l0 = l2;
+    };
+    fetch(cl, h0, l0);
+    if (kDeep) fetch(cl + 256, h1, l1);
+    for (int c = cl; c < c1; c += 256) {
+      uint4 h2[NR], l2[NR];
+      fetch(c + kAhead, h2, l2);
+      float a1[NR][8], a2[NR][8];
+#pragma unroll
+      for (int r = 0; r < NR; ++r) {
+        bf16x8_to_float(h0[r], a1[r]);
+        if (kSplit) bf16x8_to_float(l0[r], a2[r]);
+        h0[r] = kDeep ? h1[r] : h2[r];
+        if (kSplit) l0[r] = kDeep ? l1[r] : l2[r];
+        if (kDeep) {
+          h1[r] = h2[r];
+          if (kSplit) l1[r] = l2[r];
+        }
       }
 #pragma unroll
       for (int b = 0; b < P; ++b) {
@@ -1117,49 +1129,53 @@ __device__ __forceinline__ void gemv_rows(const __nv_bfloat16 *__restrict__ Ahi,
         if (kSplit)
           bf16x8_to_float(__ldg(reinterpret_cast<const uint4 *>(Vlo + b * ldvb + c)), v2);
 #pragma unroll
-        for (int t = 0; t < 8; ++t) {
-          acc[b] = fmaf(a1[t], v1[t], acc[b]);
-          if (kSplit) {
-            acc[b] = fmaf(a1[t], v2[t], acc[b]);
-            acc[b] = fmaf(a2[t], v1[t], acc[b]);
+        for (int t = 0; t < 8; ++t)
+#pragma unroll
+          for (int r = 0; r < NR; ++r) {
+            acc[r][b] = fmaf(a1[r][t], v1[t], acc[r][b]);
+            if (kSplit) {
+              acc[r][b] = fmaf(a1[r][t], v2[t], acc[r][b]);
+              acc[r][b] = fmaf(a2[r][t], v1[t], acc[r][b]);
+            }
           }
-        }
       }
     }
     if (seg == kGemvSeg - 1) {
       for (int c = n8 + lane; c < n; c += 32) {  // columns past the last multiple of 8
-        const float x1 = __bfloat162float(ah[c]);
-        const float x2 = kSplit ? __bfloat162float(al[c]) : 0.f;
 #pragma unroll
-        for (int b = 0; b < P; ++b) {
-          if (b >= p) break;
-          const float y1 = __bfloat162float(Vhi[b * ldvb + c]);
-          acc[b] = fmaf(x1, y1, acc[b]);
-          if (kSplit) {
-            acc[b] = fmaf(x1, __bfloat162float(Vlo[b * ldvb + c]), acc[b]);
-            acc[b] = fmaf(x2, y1, acc[b]);
+        for (int r = 0; r < NR; ++r) {
+          const float x1 = __bfloat162float(ah[r][c]);
+          const float x2 = kSplit ? __bfloat162float(al[r][c]) : 0.f;
+#pragma unroll
+          for (int b = 0; b < P; ++b) {
+            if (b >= p) break;
+            const float y1 = __bfloat162float(Vhi[b * ldvb + c]);
+            acc[r][b] = fmaf(x1, y1, acc[r][b]);
+            if (kSplit) {
+              acc[r][b] = fmaf(x1, __bfloat162float(Vlo[b * ldvb + c]), acc[r][b]);
+              acc[r][b] = fmaf(x2, y1, acc[r][b]);
+            }
           }
         }
       }
     }
 #pragma unroll
-    for (int b = 0; b < P; ++b) {
+    for (int r = 0; r < NR; ++r)
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) acc[b] += __shfl_xor_sync(0xffffffffu, acc[b], o);
-    }
-  }
-  if (lane == 0) {
+      for (int b = 0; b < P; ++b) {
 #pragma unroll
-    for (int b = 0; b < P; ++b) part[warp][b] = acc[b];
+        for (int o = 16; o > 0; o >>= 1) acc[r][b] += __shfl_xor_sync(0xffffffffu, acc[r][b], o);
+        if (lane == 0) part[warp][r][b] = acc[r][b];
+      }
   }
   __syncthreads();
-  if (threadIdx.x < kGemvRows * P) {
-    const int r = threadIdx.x / P, b = threadIdx.x % P;
-    const int64_t row = (int64_t)blockIdx.x * kGemvRows + r;
+  if (threadIdx.x < kGemvRows * NR * P) {
+    const int g = threadIdx.x / (NR * P), r = threadIdx.x / P % NR, b = threadIdx.x % P;
+    const int64_t row = ((int64_t)blockIdx.x * kGemvRows + g) * NR + r;
     if (row < n && b < p) {
       float t = 0.f;
 #pragma unroll
-      for (int q = 0; q < kGemvSeg; ++q) t += part[r * kGemvSeg + q][b];
+      for (int q = 0; q < kGemvSeg; ++q) t += part[g * kGemvSeg + q][r][b];
       W[b * ldw + row] = fmaf(shift, __ldg(Vf + b * ldvf + row), t);
     }
   }
@@ -1173,32 +1189,33 @@ dense_gemv1_kernel(const __nv_bfloat16 *__restrict__ Ahi, const __nv_bfloat16 *_
                    const __nv_bfloat16 *__restrict__ Vlo, int64_t ldvb,
                    const float *__restrict__ Vf, int64_t ldvf, float *__restrict__ W, int64_t ldw,
                    int n, int p, float shift, int ahead) {
-  gemv_rows<1, kSplit, true>(Ahi, Alo, lda, Vhi, Vlo, ldvb, Vf, ldvf, W, ldw, n, p, shift, ahead);
+  gemv_rows<1, kSplit, true, 1>(Ahi, Alo, lda, Vhi, Vlo, ldvb, Vf, ldvf, W, ldw, n, p, shift, ahead);
 }
 
 template <int P, bool kSplit>
-__global__ void __launch_bounds__(32 * kGemvWarps)
+__global__ void __launch_bounds__(32 * kGemvWarps, P == 8 ? 2 : 3)
 dense_gemv_kernel(const __nv_bfloat16 *__restrict__ Ahi, const __nv_bfloat16 *__restrict__ Alo,
                   int64_t lda, const __nv_bfloat16 *__restrict__ Vhi,
                   const __nv_bfloat16 *__restrict__ Vlo, int64_t ldvb,
                   const float *__restrict__ Vf, int64_t ldvf, float *__restrict__ W, int64_t ldw,
                   int n, int p, float shift, int ahead) {
-  gemv_rows<P, kSplit, false>(Ahi, Alo, lda, Vhi, Vlo, ldvb, Vf, ldvf, W, ldw, n, p, shift, ahead);
+  gemv_rows<P, kSplit, false, gemv_warp_rows(P)>(Ahi, Alo, lda, Vhi, Vlo, ldvb, Vf, ldvf, W, ldw, n, p, shift, ahead);
 }
 
-// CTAs that fetch their rows ahead when chained: those resident at first, up to 32 MB
-constexpr int64_t kGemvAheadBytes = 32 << 20;
+// CTAs that fetch their rows ahead when chained: those resident at first, up to 48 MB
+constexpr int64_t kGemvAheadBytes = 48 << 20;
 
 template <int P>
 static int launch_gemv_p(bool split, const __nv_bfloat16 *A_hi, const __nv_bfloat16 *A_lo,
                          int64_t lda, const __nv_bfloat16 *V_hi, const __nv_bfloat16 *V_lo,
                          int64_t ldvb, const float *Vf, int64_t ldvf, float *W, int64_t ldw,
                          int n, int p, float shift, bool chained, cudaStream_t s) {
-  const unsigned grid = (unsigned)((n + kGemvRows - 1) / kGemvRows);
-  const int64_t fit = kGemvAheadBytes / ((int64_t)kGemvRows * n * (split ? 4 : 2));
-  const int ahead = !chained ? 0 : (int)(fit < 5 * 152 ? fit : 5 * 152);
+  constexpr int kRowsPerCta = kGemvRows * gemv_warp_rows(P);
   auto kern = split ? dense_gemv_kernel<P, true> : dense_gemv_kernel<P, false>;
   if constexpr (P == 1) kern = split ? dense_gemv1_kernel<true> : dense_gemv1_kernel<false>;
+  const unsigned grid = (unsigned)((n + kRowsPerCta - 1) / kRowsPerCta);
+  const int64_t fit = kGemvAheadBytes / ((int64_t)kRowsPerCta * n * (split ? 4 : 2)), resident = (P == 1 ? 5 : 3) * 152;
+  const int ahead = !chained ? 0 : (int)(fit < resident ? fit : resident);
   MFG_CUDA_TRY(launch_kernel(kern, dim3(grid), 32 * kGemvWarps, 0, 0, chained, s, A_hi, A_lo, lda, V_hi, V_lo, ldvb,
                              Vf, ldvf, W, ldw, n, p, shift, ahead));
   return MFG_LAUNCH_STATUS();
