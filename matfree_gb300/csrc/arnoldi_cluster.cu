@@ -600,6 +600,8 @@ __device__ __forceinline__ void h_scalars(const double *__restrict__ rec, int k,
 
 __global__ void arnoldi_h_kernel(double *__restrict__ H, const double *__restrict__ Hh,
                                  const double *__restrict__ rec, int k, double *__restrict__ nu_last_inv) {
+  chain_wait();
+  chain_next();
   extern __shared__ double hs[];  // Hh, column-major with k + 1 rows; then hq, partial sums, the steps' scalars
   const int64_t b = blockIdx.x;
   double *Hb = H + b * (int64_t)k * k;
@@ -642,6 +644,8 @@ __global__ void arnoldi_h_kernel(double *__restrict__ H, const double *__restric
 
 __global__ void arnoldi_h_band_kernel(double *__restrict__ H, const double *__restrict__ Hh,
                                       const double *__restrict__ rec, int k) {
+  chain_wait();
+  chain_next();
   __shared__ double beta[kCMaxCols + 1], qw[kCMaxCols + 1], nu[kCMaxCols + 2];
   const int64_t b = blockIdx.x;
   const int j = threadIdx.x + 1;
@@ -781,16 +785,16 @@ int launch_arnoldi_step(int j, int64_t k, int64_t n, int64_t p, float *Q, int64_
 // H of every probe from what the steps left (`band`: its tridiagonal part only);
 // nu_last_inv (optional): 1 / nu_k.
 int launch_arnoldi_h(int64_t k, int64_t p, double *H, const double *Hh, const double *rec, bool band,
-                     double *nu_last_inv, cudaStream_t s) {
+                     double *nu_last_inv, bool chained, cudaStream_t s) {
   if (p <= 0 || k < 2) return MFG_OK;
   const int rows = (int)ceil_div(k, 32) * 32;
   if (band) {
-    arnoldi_h_band_kernel<<<(unsigned)p, rows, 0, s>>>(H, Hh, rec, (int)k);
+    MFG_CUDA_TRY(launch_kernel(arnoldi_h_band_kernel, dim3((unsigned)p), (unsigned)rows, 0, 0, chained, s, H, Hh, rec, (int)k));
     return MFG_LAUNCH_STATUS();
   }
   const size_t smem = ((size_t)(k + 1) * k + 4 * k + 1 + 4 * (size_t)rows) * sizeof(double);
   MFG_CUDA_TRY(cudaFuncSetAttribute(arnoldi_h_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  arnoldi_h_kernel<<<(unsigned)p, 4 * rows, smem, s>>>(H, Hh, rec, (int)k, nu_last_inv);
+  MFG_CUDA_TRY(launch_kernel(arnoldi_h_kernel, dim3((unsigned)p), 4u * rows, smem, 0, chained, s, H, Hh, rec, (int)k, nu_last_inv));
   return MFG_LAUNCH_STATUS();
 }
 

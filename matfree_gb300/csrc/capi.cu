@@ -313,7 +313,7 @@ static int run_two_sweep(const mfg_operator *op, int64_t k, int64_t p, int64_t l
                                        (more || R) ? Vt : nullptr, more ? hi : nullptr, lo, H, Hh, rec, status, chained, s));
       }
       MFG_LAUNCH(MFG_PROF_OTHER, 24.0 * p * k * k, full_h ? 2.0 / 3.0 * p * k * k * k : 0.0,
-                 launch_arnoldi_h(k, p, H, Hh, rec, !full_h, R ? cf : nullptr, s));
+                 launch_arnoldi_h(k, p, H, Hh, rec, !full_h, R ? cf : nullptr, chained, s));
     } else {
       // step 0 as the reference: w = A q_0, h_0 = q_0 . w, u_1 = w - q_0 h_0
       MFG_LAUNCH(MFG_PROF_APPLY, ab, af, apply_op<T>(op, Q, qb, Wb, ld, p, hi, lo, ld, panel, status, s));
@@ -401,10 +401,18 @@ static int run_hessenberg(const mfg_operator *op, int64_t k, int64_t p, const T 
 
   const double bfb = hi ? (double)n * (double)p * 2.0 * (lo ? 2.0 : 1.0) : 0.0;
 
-  // initial length (decomp.py:436) -> 1 / length
-  MFG_LAUNCH(MFG_PROF_OTHER, vecb, 2.0 * vecb / sizeof(T),
-             launch_sub<T>(nullptr, 0, 0, 0, nullptr, 0, 0, V, nullptr, ld, n, p, true, false,
-                           partials, counters, len0, nullptr, 0, s));
+  // initial length (decomp.py:436) -> 1 / length, and q_0; as one launch where a
+  // cluster's registers hold a vector.  Not chained: what wrote the operator and the
+  // vectors is complete before the loop's first product.
+  const bool one = k > 0 && gs_cluster_applies(n, 0, 0);
+  if (one)
+    MFG_LAUNCH(MFG_PROF_OTHER, 2.0 * vecb + bfb, 3.0 * vecb / sizeof(T),
+               launch_gs_cluster<T>(Q, qb, ld, 0, V, n, p, 4, nullptr, 0, nullptr, 0, nullptr, 0, 0, len0, nullptr, 0,
+                                    nullptr, Q, qb, hi, lo, status, false, s));
+  else
+    MFG_LAUNCH(MFG_PROF_OTHER, vecb, 2.0 * vecb / sizeof(T),
+               launch_sub<T>(nullptr, 0, 0, 0, nullptr, 0, 0, V, nullptr, ld, n, p, true, false,
+                             partials, counters, len0, nullptr, 0, s));
   if (init_len_inv) MFG_LAUNCH(MFG_PROF_OTHER, 16.0 * p, (double)p, launch_inv(len0, init_len_inv, p, s));
   if (k == 0) {
     if (R)
@@ -412,8 +420,9 @@ static int run_hessenberg(const mfg_operator *op, int64_t k, int64_t p, const T 
                                      cudaMemcpyDeviceToDevice, s));
     return MFG_OK;
   }
-  MFG_LAUNCH(MFG_PROF_SCALE, 2.0 * vecb + bfb, vecb / sizeof(T),
-             launch_scale<T>(V, ld, n, p, len0, Q, qb, hi, lo, ld, s));
+  if (!one)
+    MFG_LAUNCH(MFG_PROF_SCALE, 2.0 * vecb + bfb, vecb / sizeof(T),
+               launch_scale<T>(V, ld, n, p, len0, Q, qb, hi, lo, ld, s));
   if (reortho == 3) return run_two_sweep<T>(op, k, p, ld, Q, H, full_h, R, L, ws, s);
 
   const bool chained = chain_ok(s);
@@ -717,12 +726,14 @@ static int run_adjoint(const mfg_operator *op, int64_t k, int64_t p, int64_t ld,
 }
 
 __global__ void square_kernel(const double *x, double *y, int64_t p) {
+  chain_wait();
+  chain_next();
   const int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (b < p) y[b] = x[b] * x[b];
 }
 
-static int launch_square(const double *x, double *y, int64_t p, cudaStream_t s) {
-  square_kernel<<<(unsigned)ceil_div(p, 128), 128, 0, s>>>(x, y, p);
+static int launch_square(const double *x, double *y, int64_t p, bool chained, cudaStream_t s) {
+  MFG_CUDA_TRY(launch_kernel(square_kernel, dim3((unsigned)ceil_div(p, 128)), 128, 0, 0, chained, s, x, y, p));
   return MFG_LAUNCH_STATUS();
 }
 
@@ -1389,11 +1400,12 @@ static int slq_impl(const mfg_operator *op, int64_t k, int64_t p, const void *pr
     MFG_TRY(run_hessenberg<float>(op, k, p, (const float *)probes, ld, two ? 3 : 1, (float *)Qb, Hb,
                                   H != nullptr, nullptr, nullptr, L, ws, s));
   // funm.py:240-241: length^2 * e1^T f(T) e1 with length = ||v||
-  MFG_LAUNCH(MFG_PROF_OTHER, 16.0 * p, (double)p, launch_square(len0, scale, p, s));
+  const bool chained = chain_ok(s);
+  MFG_LAUNCH(MFG_PROF_OTHER, 16.0 * p, (double)p, launch_square(len0, scale, p, chained, s));
   MFG_LAUNCH(MFG_PROF_QUAD, 8.0 * p * k * k + 16.0 * p * k, 0.0,
              launch_tridiag_quadrature(k, p, Hb, fun, param, scale, values,
                                        reinterpret_cast<double *>(ws + L.eig),
-                                       reinterpret_cast<double *>(ws + L.fsq), status, s));
+                                       reinterpret_cast<double *>(ws + L.fsq), status, s, chained));
   if (mean_sem) MFG_LAUNCH(MFG_PROF_QUAD, 8.0 * p, 3.0 * p, launch_mean_sem(values, p, mean_sem, s));
   return MFG_OK;
 }
@@ -1488,7 +1500,8 @@ int mfg_slq_product(const mfg_operator *A, const mfg_operator *At, int64_t k, in
   MFG_CUDA_TRY(cudaMemsetAsync(gram, 0, (size_t)p * k * k * 8, s));
   bidiag_gram_kernel<<<(unsigned)ceil_div(p * k, 128), 128, 0, s>>>(alphas, betas, k, p, gram);
   MFG_TRY(MFG_LAUNCH_STATUS());
-  MFG_LAUNCH(MFG_PROF_OTHER, 16.0 * p, (double)p, launch_square(len0, scale, p, s));
+  const bool chained = chain_ok(s);
+  MFG_LAUNCH(MFG_PROF_OTHER, 16.0 * p, (double)p, launch_square(len0, scale, p, chained, s));
   MFG_LAUNCH(MFG_PROF_QUAD, 8.0 * p * k * k + 16.0 * p * k, 0.0,
              launch_tridiag_quadrature(k, p, gram, fun, param, scale, values,
                                        reinterpret_cast<double *>(ws + L.base.eig),

@@ -62,7 +62,7 @@ int launch_arnoldi_step(int j, int64_t k, int64_t n, int64_t p, float *Q, int64_
                         const float *Vin, int64_t vb, float *Vout, __nv_bfloat16 *hi, __nv_bfloat16 *lo, double *H,
                         double *Hh, double *rec, int *status, bool chained, cudaStream_t s);
 int launch_arnoldi_h(int64_t k, int64_t p, double *H, const double *Hh, const double *rec, bool band,
-                     double *nu_last_inv, cudaStream_t s);
+                     double *nu_last_inv, bool chained, cudaStream_t s);
 // (chained: see chain_wait in common.cuh)
 // gs_cluster.cu: Gram-Schmidt twice with the norm and the normalisation, and a step
 // of the adjoint, as one launch each (n up to 32768)
@@ -134,7 +134,8 @@ int launch_tridiag_eigh_full(int64_t k, int64_t p, const double *H, double *w, d
                              double *Z, int *status, cudaStream_t s);
 int launch_tridiag_quadrature(int64_t k, int64_t p, const double *H, int32_t fun, double param,
                               const double *scale, double *values, double *eigvals,
-                              double *first_sq, int *status, cudaStream_t s);
+                              double *first_sq, int *status, cudaStream_t s,
+                              bool chained = false);
 int launch_mean_sem(const double *values, int64_t p, double *mean_sem, cudaStream_t s);
 
 // operators.cu

@@ -992,6 +992,8 @@ __global__ void __launch_bounds__(kDcMaxThreads, 1)
                       const double *__restrict__ scale, double *__restrict__ values,
                       double *__restrict__ eigvals, double *__restrict__ first_sq,
                       int *__restrict__ status) {
+  chain_wait();
+  chain_next();
   extern __shared__ double sm[];
   const int tid = threadIdx.x;
   const int nt = blockDim.x;
@@ -1215,7 +1217,7 @@ __global__ void __launch_bounds__(kDcMaxThreads, 1)
 
 int launch_tridiag_quadrature(int64_t k, int64_t p, const double *H, int32_t fun, double param,
                               const double *scale, double *values, double *eigvals,
-                              double *first_sq, int *status, cudaStream_t s) {
+                              double *first_sq, int *status, cudaStream_t s, bool chained) {
   if (p <= 0 || k <= 0) return MFG_OK;
   if (k >= kDcMinK && k <= kDcMaxK) {
     // one problem per CTA, G lanes per root, up to 512 threads
@@ -1226,8 +1228,8 @@ int launch_tridiag_quadrature(int64_t k, int64_t p, const double *H, int32_t fun
     const int G = dc_group(k, p);
     const int64_t want = (k * G + 31) / 32 * 32;
     const int threads = (int)(want < kDcMaxThreads ? want : kDcMaxThreads);
-    tridiag_dc_kernel<<<(unsigned)p, threads, smem, s>>>((int)k, p, G, H, fun, param, scale, values,
-                                                        eigvals, first_sq, status);
+    MFG_CUDA_TRY(launch_kernel(tridiag_dc_kernel, dim3((unsigned)p), (unsigned)threads, smem, 0, chained, s, (int)k, p, G,
+                               H, fun, param, scale, values, eigvals, first_sq, status));
     return MFG_LAUNCH_STATUS();
   }
   const size_t per_thread = (size_t)3 * k * sizeof(double);
