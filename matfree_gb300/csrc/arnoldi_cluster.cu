@@ -461,7 +461,7 @@ __global__ void __launch_bounds__(kCThreads + 32, 2) arnoldi_step_kernel(const C
           nz = c_ld_pair(at + 8);
           bz = c_ld_pair(at + 16);
         }
-        for (int o = S / 2; o > 0; o >>= 1) {
+        for (int o = c_half(S); o > 0; o >>= 1) {
           nz = pair_add(nz, pair_shfl_xor(nz, o));
           if (!kFirst) {
             nb = pair_add(nb, pair_shfl_xor(nb, o));
@@ -697,7 +697,7 @@ static size_t c_fixed(int R, int wr) {
 
 // clusters held at a time, per log2 of the row warps
 struct CSlots {
-  int clusters[4][5];
+  int clusters[4][kCSizes];
   CSlots() {
     for (int w = 0; w < 4; ++w) {
       c_prepare(c_kernel<true>(1 << w));
@@ -716,13 +716,15 @@ struct CPlan {
 // 40 GB/s.  Measured, whole solves' steps: n = 512, 256 probes S = 1 193 us
 // (2: 353, 4: 572); n = 3001, 64 probes S = 4 550 us (2: 596, 8: 788); n = 8192,
 // 128 probes S = 4 2.15 ms (8: 2.87); n = 16384, 256 probes S = 8 12.1 ms (16: 18.9,
-// whose clusters leave a quarter of the SMs over).
+// whose clusters leave a quarter of the SMs over).  Sizes between the powers of two where
+// those leave rows or SMs unused: n = 23170, 96 steps, 32 probes S = 12 5.8 ms (16: 6.7), n = 18000, 64,
+// 64 3.9 (16: 5.8), n = 10000, 32, 128 S = 6 1.34 (8: 1.64).
 static CPlan c_plan(int64_t n, int64_t p, int j) {
   static const CSlots slots;
   CPlan best{0, 0, 0, 0, 0};
   double best_us = 1e300;
-  for (int i = 0; i < 5; ++i) {
-    const int S = 1 << i;
+  for (int i = 0; i < kCSizes; ++i) {
+    const int S = kCSize[i];
     const int64_t R = ceil_div(ceil_div(n, S), 4) * 4;
     if (R > kCMaxR) continue;
     const int wr = c_row_warps(R);

@@ -194,8 +194,14 @@ __device__ __forceinline__ void c_meet_arrive(uint64_t *bar, int S) {
   __syncwarp();
 }
 
-// Row warps for R rows of a CTA, and the clusters of S = 1, 2, 4, 8, 16 CTAs that
-// the GPU holds at a time for a kernel of kCThreads + 32 threads and kCSmem bytes.
+// CTAs per probe to choose from
+constexpr int kCSizes = 9;
+constexpr int kCSize[kCSizes] = {1, 2, 4, 6, 8, 10, 12, 14, 16};
+
+// first distance of a butterfly over the ranks (lanes past the last hold zero)
+__device__ __forceinline__ int c_half(int S) { return S > 8 ? 8 : (S > 4 ? 4 : S / 2); }
+
+// Row warps for R rows of a CTA, and the clusters of each size that the GPU holds at a time for a kernel of kCThreads + 32 threads and kCSmem bytes.
 inline int c_row_warps(int64_t R) { return R <= kCRows ? 1 : (R <= 2 * kCRows ? 2 : (R <= 4 * kCRows ? 4 : 8)); }
 
 template <typename K>
@@ -205,16 +211,16 @@ inline bool c_prepare(K kern) {
 }
 
 template <typename K>
-inline void c_count_clusters(K kern, int (&clusters)[5]) {
+inline void c_count_clusters(K kern, int (&clusters)[kCSizes]) {
   const bool set = c_prepare(kern);
-  for (int i = 0; i < 5; ++i) {
+  for (int i = 0; i < kCSizes; ++i) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(1024);
+    cfg.gridDim = dim3(64u * kCSize[i]);
     cfg.blockDim = dim3(kCThreads + 32);
     cfg.dynamicSmemBytes = kCSmem;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 1u << i;
+    attr[0].val.clusterDim.x = (unsigned)kCSize[i];
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;

@@ -504,7 +504,7 @@ __global__ void __launch_bounds__(kCThreads + 32, 2) gs_cluster_kernel(const GsA
           if (S > 1) c_wait<true>(&sh->meet[2], par, fail, a.status);
           Sum s = g_sum_of((T)0);
           if (lane < S) s = S > 1 ? g_load_rank(npart + par, lane) : npart[par];
-          for (int o = S / 2; o > 0; o >>= 1) s = g_add(s, g_xor(s, o));
+          for (int o = c_half(S); o > 0; o >>= 1) s = g_add(s, g_xor(s, o));
           if (lane == 0) *fin = g_sqrt(s);
         }
         c_sync();
@@ -581,7 +581,7 @@ static auto g_kernel(int wr) -> void (*)(const GsArgs<T>) {
 
 template <typename T, bool kAdj>
 struct GSlots {
-  int clusters[4][5];
+  int clusters[4][kCSizes];
   GSlots() {
     for (int w = 0; w < 4; ++w) c_count_clusters(g_kernel<T, kAdj>(1 << w), clusters[w]);
   }
@@ -604,8 +604,8 @@ static int g_run(GsArgs<T> &a, bool chained, cudaStream_t s) {
   double best_us = 1e300;
   int64_t clusters = 0;
   int wr = 0;
-  for (int i = 0; i < 5; ++i) {
-    const int S = 1 << i;
+  for (int i = 0; i < kCSizes; ++i) {
+    const int S = kCSize[i];
     const int64_t R = ceil_div(ceil_div(a.n, S), 4) * 4;
     if (R > kCMaxR) continue;
     const int w = c_row_warps(R);

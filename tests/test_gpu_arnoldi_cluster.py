@@ -17,8 +17,8 @@ pytestmark = pytest.mark.gpu
 # the largest cluster, the last size of this form and the first past it; p: fewer and more probes than clusters
 # fit at a time, of every size; k: no full slot, slots that stay in the ring, slots read again, the deepest
 @pytest.mark.parametrize("n,k,p", [(33, 20, 2), (255, 30, 5), (257, 64, 3), (600, 40, 310), (1021, 129, 4), (1023, 33, 160),
-                                   (2049, 66, 80), (4098, 100, 40), (5003, 70, 9), (8191, 48, 45), (16385, 24, 17),
-                                   (32768, 11, 3), (32770, 6, 2)])
+                                   (2049, 66, 80), (4098, 100, 40), (5003, 70, 9), (8191, 48, 45), (10001, 16, 9), (16385, 24, 17),
+                                   (24577, 9, 3), (32768, 11, 3), (32770, 6, 2)])
 def test_cluster_step_matches_oracle(n, k, p):
     rng = np.random.default_rng(n)
     off = -rng.uniform(0.2, 1.0, n - 1)
