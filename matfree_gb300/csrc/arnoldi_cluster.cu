@@ -718,7 +718,8 @@ struct CPlan {
 // 128 probes S = 4 2.15 ms (8: 2.87); n = 16384, 256 probes S = 8 12.1 ms (16: 18.9,
 // whose clusters leave a quarter of the SMs over).  Sizes between the powers of two where
 // those leave rows or SMs unused: n = 23170, 96 steps, 32 probes S = 12 5.8 ms (16: 6.7), n = 18000, 64,
-// 64 3.9 (16: 5.8), n = 10000, 32, 128 S = 6 1.34 (8: 1.64).
+// 64 3.9 (16: 5.8), n = 10000, 32, 128 S = 6 1.34 (8: 1.64).  Of equal sizes the one whose launches
+// are chained: n = 3001, k = 16, 40 probes 464 us per solve with S = 4, 507 with 6.
 static CPlan c_plan(int64_t n, int64_t p, int j) {
   static const CSlots slots;
   CPlan best{0, 0, 0, 0, 0};
@@ -734,7 +735,7 @@ static CPlan c_plan(int64_t n, int64_t p, int j) {
     if (c < 1) continue;
     const double rounds = (double)ceil_div(p, c);
     if (c_fixed((int)R, wr) + (size_t)(kCWarps / wr) * c_gc(wr) * R * 4 > kCSmem) continue;  // no slot per group
-    const double us = rounds * ((S == 1 ? 5.0 : 6.5) + 0.1 * S + (2.0 * j + 8.0) * R * 4.0 / 40e3);
+    const double us = rounds * ((S == 1 ? 5.0 : 6.5) + 0.1 * S + (2.0 * j + 8.0) * R * 4.0 / 40e3) + (S > kCChainS ? kCUnchainedUs : 0.0);
     if (us < best_us) {
       best_us = us;
       int sl = (int)((kCSmem - c_fixed((int)R, wr)) / ((size_t)c_gc(wr) * R * 4));

@@ -235,6 +235,7 @@ inline void c_count_clusters(K kern, int (&clusters)[kCSizes]) {
 // fit at once (n = 16384, k = 64, 256 probes, S = 8: 29.0 -> 35.2 ms per solve; S = 4 at n =
 // 8192, 128 probes, k = 48: 17.4 -> 17.0).
 constexpr int kCChainS = 4;
+constexpr double kCUnchainedUs = 2.7;  // a step whose launch is not chained, in the plans' costs
 
 template <typename K, typename A>
 inline int c_launch(K kern, int S, int64_t ctas, size_t smem, const A &args, bool chained, cudaStream_t s) {

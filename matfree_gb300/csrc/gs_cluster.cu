@@ -617,7 +617,7 @@ static int g_run(GsArgs<T> &a, bool chained, cudaStream_t s) {
     if (c < 1 || fixed + slot * groups > kCSmem) continue;
     double us = (S == 1 ? 6.0 : 9.0) + 0.15 * S + cols * R * sizeof(T) / 40e3;
     if (sizeof(T) == 8) us += cols * R / 1630.0;
-    us *= (double)ceil_div(a.p, c);
+    us = us * (double)ceil_div(a.p, c) + (S > kCChainS ? kCUnchainedUs : 0.0);
     if (us < best_us) {
       best_us = us;
       a.S = S;
