@@ -38,6 +38,18 @@ from .tree import _rebuild, tree_leaves
 _WS = Workspace()
 
 
+def _plain(*tensors) -> bool:
+    """Whether a kernel may stand in for torch operations on these: plain tensors that no
+    gradient, forward-mode tangent or function transform (vmap, jvp) follows."""
+    return all(type(t) is torch.Tensor and not torch._C._functorch.is_functorch_wrapped_tensor(t)
+               and not (torch.is_grad_enabled() and t.requires_grad)
+               and torch.autograd.forward_ad.unpack_dual(t).tangent is None for t in tensors)
+
+
+def _plain_float64(device, *tensors) -> bool:
+    return _plain(*tensors) and all(t.dtype == torch.float64 and t.device == device for t in tensors)
+
+
 def quadform_dH(H: torch.Tensor, scale: torch.Tensor, f, fprime) -> tuple[torch.Tensor, torch.Tensor]:
     """Values scale_b e1^T f(T_b) e1 and their cotangent with respect to H.
 
@@ -48,10 +60,10 @@ def quadform_dH(H: torch.Tensor, scale: torch.Tensor, f, fprime) -> tuple[torch.
     p, k = H.shape[0], H.shape[1]
     w, S = tridiag_eigh(H)  # the eigh of T = tridiagonal part of (H + H^T)/2
     fw = f(w)
-    live = torch.is_grad_enabled() and (scale.requires_grad or fw.requires_grad)
-    if (w.is_cuda and not live and fw.dtype == scale.dtype == torch.float64 and scale.shape == (p,) and 0 < p
-            and k <= 4096):
-        fmid = fprime(0.5 * (w[:, :, None] + w[:, None, :])).to(torch.float64)
+    fmid = fprime(0.5 * (w[:, :, None] + w[:, None, :]))
+    # one kernel, which reads fw (p, k), fmid (p, k, k) and scale (p,) as they lie in memory
+    if (w.is_cuda and 0 < p and k <= 4096 and _plain_float64(w.device, fw, fmid, scale) and fw.shape == (p, k)
+            and scale.shape == (p,) and fmid.dim() <= 3):
         fmid, fw, scale = fmid.expand(p, k, k).contiguous(), fw.contiguous(), scale.contiguous()
         values = torch.empty(p, dtype=torch.float64, device=w.device)
         dH = torch.empty((p, k, k), dtype=torch.float64, device=w.device)
@@ -59,13 +71,13 @@ def quadform_dH(H: torch.Tensor, scale: torch.Tensor, f, fprime) -> tuple[torch.
                                                 for t in (w, S, fw, fmid, scale, values, dH)), stream_ptr())
         _lib.check(st, "mfg_quadform_dh")
         return values, dH
-    # differentiable f or scale, other types and devices
+    # differentiable or transformed f, f' or scale; other shapes, types and devices
     s1 = S[:, 0, :]
     values = scale * (fw * s1 * s1).sum(-1)
     diff = w[:, :, None] - w[:, None, :]
     same = diff.abs() <= 1e-13 * torch.clamp(w.abs()[:, :, None], min=1.0)
     F = (fw[:, :, None] - fw[:, None, :]) / torch.where(same, torch.ones_like(diff), diff)
-    F = torch.where(same, fprime(0.5 * (w[:, :, None] + w[:, None, :])), F)
+    F = torch.where(same, fmid, F)
     G = S @ (F * s1[:, :, None] * s1[:, None, :]) @ S.transpose(-1, -2)
     G = G * scale[:, None, None]
     # T_dense = diag(d) + diag(e, 1) + diag(e, -1), d = diag(H), e = (H[i,i+1] + H[i+1,i])/2
@@ -232,13 +244,13 @@ def rbf_theta_contractions(op: RBFKernelOperator, x, Q, Lam, dl=None) -> torch.T
     n = op.n
     if dl is None:
         dl = _rbf_dlogell_operator(op, x)
-    live = torch.is_grad_enabled() and (Q.requires_grad or Lam.requires_grad)
-    if (not live and Q.dtype == Lam.dtype == op.basis_dtype and Q.shape == Lam.shape and p * k > 0
-            and dl.precision == op.precision and dl.n == n and ld >= n and ld % 8 == 0):
+    if (_plain(Q, Lam) and Q.device == Lam.device and Q.dtype == Lam.dtype == op.basis_dtype and Q.shape == Lam.shape
+            and p * k > 0 and isinstance(dl, DenseOperator) and dl.precision == op.precision and dl.n == n
+            and ld >= n and ld % 8 == 0):
         Q, Lam = Q.contiguous(), Lam.contiguous()
         if Q.data_ptr() % 16 == 0 and Lam.data_ptr() % 16 == 0:
             return _device_contractions(op, dl, Q, Lam)
-    # panels the kernel does not read in place, mixed types
+    # panels the kernel does not read in place, mixed types, other operators
     rows = Q.reshape(p * k, ld)[:, :n]
     lam = Lam.reshape(p * k, ld)[:, :n].double()
     # the stored exponential part (without the nugget) is dK/dlog s2
