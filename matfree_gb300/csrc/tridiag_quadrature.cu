@@ -392,6 +392,13 @@ __device__ __forceinline__ long long order_key(double x) {
 }
 __device__ __forceinline__ bool less_than(double x, double y) { return order_key(x) < order_key(y); }
 __device__ __forceinline__ bool positive(double x) { return order_key(x) > 0; }
+__device__ __forceinline__ bool is_nan(double x) { return order_key(fabs(x)) > 0x7ff0000000000000ll; }
+
+// The first failure on the stream is what the caller is told (a solve that asked to be
+// repeated leaves NaN behind it).
+__device__ __forceinline__ void dc_failed(int *status) {
+  if (status) atomicCAS(status, 0, (int)MFG_ERR_NO_CONVERGENCE);
+}
 
 // Root of c x^2 - 2 h x + a0 with c + s0/(U - x) + s1/(V - x) = 0, U < V its poles:
 // the one between them, or (right) the one above both, for c > 0.  The
@@ -457,14 +464,14 @@ __device__ __forceinline__ double group_prod(double v, unsigned mask) {
 // float64 midpoint decides as it would alone.  The float64 iteration is
 // safeguarded by the interval of the poles either way.  Quadrature of k = 16, 32 problems
 // 98 -> 61 us, k = 32, 64 146 -> 92, k = 64, 1000 1593 -> 660.
-// Returns false when the iteration limit is reached.
+// Returns false when the iteration limit is reached, or on NaN.
 template <int G>
 __device__ bool dc_secular_root(const double *P, const double *ZZ, const float2 *PF, const float *ZF, int mk, int j,
                                 double rho, double upper, int sub, unsigned gm, double &x_out, int &o_out) {
   o_out = j;
   if (mk == 1) {
     x_out = rho * ZZ[0];
-    return true;
+    return !is_nan(x_out);
   }
   const double ir = rcp_any(rho);
   const bool last = j + 1 >= mk;
@@ -602,6 +609,7 @@ __device__ bool dc_secular_root(const double *P, const double *ZZ, const float2 
     pass(base, x);
     const double c0 = ir + (below + above);
     const double f = c0 + (t0 + t1);
+    if (is_nan(f)) break;
     if (positive(f))
       hi = x;
     else
@@ -1020,12 +1028,22 @@ __global__ void __launch_bounds__(kDcMaxThreads, 1)
   for (int i = tid; i < k; i += nt)
     EO[i] = (i + 1 < k) ? 0.5 * (Hb[(size_t)i * k + i + 1] + Hb[(size_t)(i + 1) * k + i]) : 0.0;
   __syncthreads();
+  int bad = 0;
   for (int i = tid; i < k; i += nt) {
     LAM[i] = Hb[(size_t)i * k + i] - (i > 0 ? EO[i - 1] : 0.0) - EO[i];
     FR[i] = 1.0;
     LR[i] = 1.0;
+    bad |= is_nan(LAM[i]);
   }
-  __syncthreads();
+  if (__syncthreads_or(bad)) {
+    for (int i = tid; i < k; i += nt) {
+      if (eigvals) eigvals[(size_t)b * k + i] = nan("");
+      if (first_sq) first_sq[(size_t)b * k + i] = nan("");
+    }
+    if (tid == 0 && values) values[b] = nan("");
+    if (tid == 0) dc_failed(status);
+    return;
+  }
   bool ok = true;
   for (int s = 0; (1 << s) < k; ++s) {
     const int w = 1 << s;
@@ -1049,7 +1067,7 @@ __global__ void __launch_bounds__(kDcMaxThreads, 1)
       const int at = mk == hi - a ? r - a : dc_merged_place(NL, a, mk, hi, r);
       const int pos = flip ? hi - 1 - at : a + at;
       const double v = root ? X[r] : D[r];
-      LAM[pos] = flip ? -v : v;
+      LAM[pos] = (flip ? -v : v) + 0.0;  // one zero: the order of the keys is that of the values
       FR[pos] = root ? NF[r] : F[r];
       LR[pos] = root ? NL[r] : L[r];
     }
@@ -1083,7 +1101,7 @@ __global__ void __launch_bounds__(kDcMaxThreads, 1)
     for (int w = 0; w < (nt >> 5); ++w) acc += red[w];
     if (!ok) {
       acc = nan("");
-      if (status) atomicExch(status, (int)MFG_ERR_NO_CONVERGENCE);
+      dc_failed(status);
     }
     if (values) values[b] = (scale ? scale[b] : 1.0) * acc;
   }
@@ -1105,7 +1123,9 @@ __global__ void __launch_bounds__(kDcMaxThreads, 1)
 //     poles c >= a+mk;
 //   E: the order of the merged eigenvalues as a column map (in O), then S
 //     from S2 through that map.
-// A direct restatement runs on the CPU as dc_full in the tests.
+// On the CPU, tests/test_dc_model.py runs the merges with a serial deflation and the float64
+// iteration from the midpoint (dc_full), tests/test_dc_merge_model.py the index work of phases
+// A and E element by element.
 constexpr int kDcvMaxK = 64;  // S, S2, U: 3 k^2 doubles (96 KB at k = 64)
 
 __host__ inline size_t dcv_smem_bytes(int k) {
@@ -1145,9 +1165,19 @@ __global__ void __launch_bounds__(kDcMaxThreads, 1)
   for (int i = tid; i < k; i += nt)
     EO[i] = (i + 1 < k) ? 0.5 * (Hb[(size_t)i * k + i + 1] + Hb[(size_t)(i + 1) * k + i]) : 0.0;
   __syncthreads();
-  for (int i = tid; i < k; i += nt) LAM[i] = Hb[(size_t)i * k + i] - (i > 0 ? EO[i - 1] : 0.0) - EO[i];
+  int bad = 0;
+  for (int i = tid; i < k; i += nt) {
+    LAM[i] = Hb[(size_t)i * k + i] - (i > 0 ? EO[i - 1] : 0.0) - EO[i];
+    CI[i] = i;  // a column at all times, also where a failure leaves the poles unordered
+    bad |= is_nan(LAM[i]);
+  }
   for (int idx = tid; idx < k * k; idx += nt) S[idx] = (idx / k == idx % k) ? 1.0 : 0.0;
-  __syncthreads();
+  if (__syncthreads_or(bad)) {
+    for (int i = tid; i < k; i += nt) w_out[(size_t)b * k + i] = nan("");
+    for (int idx = tid; idx < k * k; idx += nt) S_out[(size_t)b * k * k + idx] = nan("");
+    if (tid == 0) dc_failed(status);
+    return;
+  }
   bool ok = true;
   for (int s = 0; (1 << s) < k; ++s) {
     const int w = 1 << s;
@@ -1190,7 +1220,7 @@ __global__ void __launch_bounds__(kDcMaxThreads, 1)
       const int at = mk == hi - a ? r - a : dc_merged_place(NL, a, mk, hi, r);
       const int pos = flip ? hi - 1 - at : a + at;
       const double v = root ? X[r] : D[r];
-      LAM[pos] = flip ? -v : v;
+      LAM[pos] = (flip ? -v : v) + 0.0;  // one zero: the order of the keys is that of the values
       O[pos] = r;
     }
     __syncthreads();
@@ -1212,7 +1242,7 @@ __global__ void __launch_bounds__(kDcMaxThreads, 1)
     const int row = idx / k, j = idx - row * k;
     Sb[idx] = S[(size_t)j * k + row];
   }
-  if (!ok && tid == 0 && status) atomicExch(status, (int)MFG_ERR_NO_CONVERGENCE);
+  if (!ok && tid == 0) dc_failed(status);
 }
 
 int launch_tridiag_quadrature(int64_t k, int64_t p, const double *H, int32_t fun, double param,
