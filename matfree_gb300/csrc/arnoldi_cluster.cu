@@ -218,8 +218,8 @@ __global__ void __launch_bounds__(kCThreads + 32, 2) arnoldi_step_kernel(const C
         if (b == cluster) {  // a read of L2 is shorter than a copy's round trip
           const float4 *gw = reinterpret_cast<const float4 *>(a.W + b * a.ld + r0 + row);
           const float4 *gq = reinterpret_cast<const float4 *>(a.Vin + b * a.vb + r0 + row);
-          const float4 w0 = ok0 ? __ldcg(gw) : zero4, q0 = ok0 ? __ldcg(gq) : zero4;
-          const float4 w1 = ok1 ? __ldcg(gw + 32) : zero4, q1 = ok1 ? __ldcg(gq + 32) : zero4;
+          const float4 w0 = ok0 ? c_ld_l2(gw) : zero4, q0 = ok0 ? c_ld_l2(gq) : zero4;
+          const float4 w1 = ok1 ? c_ld_l2(gw + 32) : zero4, q1 = ok1 ? c_ld_l2(gq + 32) : zero4;
           take(w0, w1, w);
           take(q0, q1, q);
         } else {
@@ -575,7 +575,7 @@ __device__ __forceinline__ double h_raw(const double *p) {
 }
 
 // beta[1 .. k - 1], qw[0 .. k - 1] (qw[0] = H[0][0]) and nu[1 .. k] of one probe, by all threads
-__device__ __forceinline__ void h_scalars(const double *__restrict__ rec, int k, double *beta, double *qw, double *nu) {
+__device__ __forceinline__ void h_scalars(const double *rec, int k, double *beta, double *qw, double *nu) {
   for (int j = threadIdx.x; j < k; j += blockDim.x) {
     const double *r = rec + (int64_t)j * kCRec;
     const double nz = h_raw(r + 1), c = h_raw(r + 3);
@@ -598,8 +598,7 @@ __device__ __forceinline__ void h_scalars(const double *__restrict__ rec, int k,
   __syncthreads();
 }
 
-__global__ void arnoldi_h_kernel(double *__restrict__ H, const double *__restrict__ Hh,
-                                 const double *__restrict__ rec, int k, double *__restrict__ nu_last_inv) {
+__global__ void arnoldi_h_kernel(double *H, const double *Hh, const double *rec, int k, double *__restrict__ nu_last_inv) {
   chain_wait();
   chain_next();
   extern __shared__ double hs[];  // Hh, column-major with k + 1 rows; then hq, partial sums, the steps' scalars
@@ -642,8 +641,7 @@ __global__ void arnoldi_h_kernel(double *__restrict__ H, const double *__restric
   if (threadIdx.x == 0 && nu_last_inv) nu_last_inv[b] = 1.0 / nu[k];
 }
 
-__global__ void arnoldi_h_band_kernel(double *__restrict__ H, const double *__restrict__ Hh,
-                                      const double *__restrict__ rec, int k) {
+__global__ void arnoldi_h_band_kernel(double *H, const double *Hh, const double *rec, int k) {
   chain_wait();
   chain_next();
   __shared__ double beta[kCMaxCols + 1], qw[kCMaxCols + 1], nu[kCMaxCols + 2];

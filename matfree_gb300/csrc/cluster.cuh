@@ -35,6 +35,13 @@ __device__ __forceinline__ double c_ld_f64(uint32_t addr) {
   return v;
 }
 
+// from L2, in program order with the waits
+__device__ __forceinline__ float4 c_ld_l2(const float4 *p) {
+  float4 v;
+  asm volatile("ld.global.cg.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
+  return v;
+}
+
 __device__ __forceinline__ void c_bulk(uint32_t dst, const void *src, uint32_t bytes, uint64_t *bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
                "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes), "r"(c_smem(bar))

@@ -114,6 +114,10 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar_saddr, uint32_t p
 // loop writes, may be read before chain_wait(): the loop's first kernels are ordinary
 // launches, behind whatever wrote the operator.
 //
+// What an earlier kernel of the loop wrote is not read-only while this one runs: it is read
+// by plain or volatile loads through pointers without __restrict__ (which would let the
+// compiler use the non-coherent path or move a load above the wait), never by __ldg.
+//
 // Two to three microseconds a launch: figures at chain_ok (capi.cu).
 // ---------------------------------------------------------------------------
 

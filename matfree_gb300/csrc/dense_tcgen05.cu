@@ -229,7 +229,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
 dense_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_ahi,
                           const __grid_constant__ CUtensorMap map_alo,
                           const __grid_constant__ CUtensorMap map_bhi,
-                          const __grid_constant__ CUtensorMap map_blo, const float *__restrict__ Vf,
+                          const __grid_constant__ CUtensorMap map_blo, const float *Vf,
                           int64_t ldvf, float *__restrict__ W, int64_t ldw, int n, int p, int BN,
                           int stages, uint32_t tmem_cols, float shift, int *status) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -353,8 +353,7 @@ dense_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_ahi,
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
         const int b = b0 + c + j;
-        dst[j] = (shift != 0.f && blockIdx.z == 0 && m < n && b < p) ? __ldg(Vf + (int64_t)b * ldvf + m)
-                                                                      : 0.f;
+        dst[j] = (shift != 0.f && blockIdx.z == 0 && m < n && b < p) ? Vf[(int64_t)b * ldvf + m] : 0.f;
       }
     };
     load_shift(0, sv);
@@ -435,7 +434,7 @@ template <int S> struct Ranks { static constexpr int value = S; };
 // n = 8192, 128 probes.
 template <int S, int MT>
 __device__ __forceinline__ void splitk_reduce(uint32_t base, int c0, int items, int b0, int m0, int n, int p,
-                                              const float *__restrict__ Vf, int64_t ldvf, float *__restrict__ W,
+                                              const float *Vf, int64_t ldvf, float *__restrict__ W,
                                               int64_t ldw, float shift, int vec_ok) {
   constexpr int U = S <= 2 ? 8 : (S <= 4 ? 4 : 2), kStep = kGemmThreads / 32;
   const int lane = threadIdx.x & 31;
@@ -454,12 +453,12 @@ __device__ __forceinline__ void splitk_reduce(uint32_t base, int c0, int items, 
       if (live && shift != 0.f) {
         const float *vf = Vf + (int64_t)b * ldvf + m;
         if (vec_ok && m + 4 <= n) {
-          sv[u] = __ldg(reinterpret_cast<const float4 *>(vf));
+          sv[u] = *reinterpret_cast<const float4 *>(vf);
         } else {
-          sv[u].x = __ldg(vf);
-          if (m + 1 < n) sv[u].y = __ldg(vf + 1);
-          if (m + 2 < n) sv[u].z = __ldg(vf + 2);
-          if (m + 3 < n) sv[u].w = __ldg(vf + 3);
+          sv[u].x = vf[0];
+          if (m + 1 < n) sv[u].y = vf[1];
+          if (m + 2 < n) sv[u].z = vf[2];
+          if (m + 3 < n) sv[u].w = vf[3];
         }
       }
     }
@@ -498,7 +497,7 @@ dense_tcgen05_splitk_kernel(const __grid_constant__ CUtensorMap map_ahi,
                             const __grid_constant__ CUtensorMap map_alo,
                             const __grid_constant__ CUtensorMap map_bhi,
                             const __grid_constant__ CUtensorMap map_blo,
-                            const float *__restrict__ Vf, int64_t ldvf, float *__restrict__ W,
+                            const float *Vf, int64_t ldvf, float *__restrict__ W,
                             int64_t ldw, int n, int p, int BN, int stages, uint32_t tmem_cols,
                             float shift, int vec_ok, int *status) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -744,7 +743,7 @@ dense_tcgen05_pair_persistent_kernel(const __grid_constant__ CUtensorMap map_ahi
                                      const __grid_constant__ CUtensorMap map_alo,
                                      const __grid_constant__ CUtensorMap map_bhi,
                                      const __grid_constant__ CUtensorMap map_blo,
-                                     const float *__restrict__ Vf, int64_t ldvf,
+                                     const float *Vf, int64_t ldvf,
                                      float *__restrict__ W, int64_t ldw, int n, int p, int BN,
                                      int stages, uint32_t acc_cols, PairSchedule sc, float shift,
                                      int *status) {
@@ -893,7 +892,7 @@ dense_tcgen05_pair_persistent_kernel(const __grid_constant__ CUtensorMap map_ahi
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
           const int b = b0 + c + j;
-          dst[j] = (with_shift && m < n && b < p) ? __ldg(Vf + (int64_t)b * ldvf + m) : 0.f;
+          dst[j] = (with_shift && m < n && b < p) ? Vf[(int64_t)b * ldvf + m] : 0.f;
         }
       };
       load_shift(0, sv);
@@ -1056,9 +1055,8 @@ constexpr int gemv_warp_rows(int P) { return P > 1 ? 2 : 1; }
 template <int P, bool kSplit, bool kDeep, int NR>
 __device__ __forceinline__ void gemv_rows(const __nv_bfloat16 *__restrict__ Ahi,
                                           const __nv_bfloat16 *__restrict__ Alo, int64_t lda,
-                                          const __nv_bfloat16 *__restrict__ Vhi,
-                                          const __nv_bfloat16 *__restrict__ Vlo, int64_t ldvb,
-                                          const float *__restrict__ Vf, int64_t ldvf,
+                                          const __nv_bfloat16 *Vhi, const __nv_bfloat16 *Vlo,
+                                          int64_t ldvb, const float *Vf, int64_t ldvf,
                                           float *__restrict__ W, int64_t ldw, int n, int p,
                                           float shift, int ahead) {
   constexpr int kAhead = kDeep ? 512 : 256;
@@ -1125,9 +1123,9 @@ __device__ __forceinline__ void gemv_rows(const __nv_bfloat16 *__restrict__ Ahi,
       for (int b = 0; b < P; ++b) {
         if (b >= p) break;
         float v1[8], v2[8];
-        bf16x8_to_float(__ldg(reinterpret_cast<const uint4 *>(Vhi + b * ldvb + c)), v1);
+        bf16x8_to_float(*reinterpret_cast<const uint4 *>(Vhi + b * ldvb + c), v1);
         if (kSplit)
-          bf16x8_to_float(__ldg(reinterpret_cast<const uint4 *>(Vlo + b * ldvb + c)), v2);
+          bf16x8_to_float(*reinterpret_cast<const uint4 *>(Vlo + b * ldvb + c), v2);
 #pragma unroll
         for (int t = 0; t < 8; ++t)
 #pragma unroll
@@ -1176,7 +1174,7 @@ __device__ __forceinline__ void gemv_rows(const __nv_bfloat16 *__restrict__ Ahi,
       float t = 0.f;
 #pragma unroll
       for (int q = 0; q < kGemvSeg; ++q) t += part[g * kGemvSeg + q][r][b];
-      W[b * ldw + row] = fmaf(shift, __ldg(Vf + b * ldvf + row), t);
+      W[b * ldw + row] = fmaf(shift, Vf[b * ldvf + row], t);
     }
   }
 }
@@ -1185,9 +1183,9 @@ __device__ __forceinline__ void gemv_rows(const __nv_bfloat16 *__restrict__ Ahi,
 template <bool kSplit>
 __global__ void __launch_bounds__(32 * kGemvWarps, 5)
 dense_gemv1_kernel(const __nv_bfloat16 *__restrict__ Ahi, const __nv_bfloat16 *__restrict__ Alo,
-                   int64_t lda, const __nv_bfloat16 *__restrict__ Vhi,
-                   const __nv_bfloat16 *__restrict__ Vlo, int64_t ldvb,
-                   const float *__restrict__ Vf, int64_t ldvf, float *__restrict__ W, int64_t ldw,
+                   int64_t lda, const __nv_bfloat16 *Vhi,
+                   const __nv_bfloat16 *Vlo, int64_t ldvb,
+                   const float *Vf, int64_t ldvf, float *__restrict__ W, int64_t ldw,
                    int n, int p, float shift, int ahead) {
   gemv_rows<1, kSplit, true, 1>(Ahi, Alo, lda, Vhi, Vlo, ldvb, Vf, ldvf, W, ldw, n, p, shift, ahead);
 }
@@ -1195,9 +1193,9 @@ dense_gemv1_kernel(const __nv_bfloat16 *__restrict__ Ahi, const __nv_bfloat16 *_
 template <int P, bool kSplit>
 __global__ void __launch_bounds__(32 * kGemvWarps, P == 8 ? 2 : 3)
 dense_gemv_kernel(const __nv_bfloat16 *__restrict__ Ahi, const __nv_bfloat16 *__restrict__ Alo,
-                  int64_t lda, const __nv_bfloat16 *__restrict__ Vhi,
-                  const __nv_bfloat16 *__restrict__ Vlo, int64_t ldvb,
-                  const float *__restrict__ Vf, int64_t ldvf, float *__restrict__ W, int64_t ldw,
+                  int64_t lda, const __nv_bfloat16 *Vhi,
+                  const __nv_bfloat16 *Vlo, int64_t ldvb,
+                  const float *Vf, int64_t ldvf, float *__restrict__ W, int64_t ldw,
                   int n, int p, float shift, int ahead) {
   gemv_rows<P, kSplit, false, gemv_warp_rows(P)>(Ahi, Alo, lda, Vhi, Vlo, ldvb, Vf, ldvf, W, ldw, n, p, shift, ahead);
 }

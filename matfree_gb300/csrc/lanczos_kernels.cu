@@ -1359,11 +1359,8 @@ __device__ __forceinline__ double cta_sum_small(T v, double *red) {
 
 template <typename T, int E>
 __global__ void __launch_bounds__(kCgSmallThreads)
-cg_step_small_kernel(T *__restrict__ X, T *__restrict__ R, T *__restrict__ P,
-                     const T *__restrict__ W, int64_t ld, int64_t n,
-                     const double *__restrict__ rs, const double *__restrict__ thr,
-                     double *__restrict__ rs_next, int *__restrict__ nactive,
-                     int *__restrict__ nactive_clear, int *__restrict__ iters,
+cg_step_small_kernel(T *X, T *R, T *P, const T *W, int64_t ld, int64_t n, const double *rs,
+                     const double *thr, double *rs_next, int *nactive, int *nactive_clear, int *iters,
                      __nv_bfloat16 *hi, __nv_bfloat16 *lo) {
   __shared__ double red[33];
   __shared__ T coef;  // alpha, then beta: one float64 division each, in thread 0
@@ -1382,9 +1379,12 @@ cg_step_small_kernel(T *__restrict__ X, T *__restrict__ R, T *__restrict__ P,
     pe[e] = in ? pv[i] : (T)0;
     we[e] = in ? w[i] : (T)0;
   }
+  double rsb = 0.0, thrb = 0.0;  // thread 0's
   if (threadIdx.x == 0) {
+    rsb = rs[b];
+    thrb = thr[b];
     if (b == 0) *nactive_clear = 0;  // the next iteration's count
-    run = rs[b] > thr[b];
+    run = rsb > thrb;
   }
   __syncthreads();
   const bool active = run != 0;  // uniform over the CTA
@@ -1394,15 +1394,21 @@ cg_step_small_kernel(T *__restrict__ X, T *__restrict__ R, T *__restrict__ P,
 #pragma unroll
     for (int e = 0; e < E; ++e) acc = fma(pe[e], we[e], acc);
     const double pap = cta_sum_small<T>(acc, red);
-    if (threadIdx.x == 0) coef = (T)(rs[b] / pap);
+    if (threadIdx.x == 0) coef = (T)(rsb / pap);
     __syncthreads();
     const T alpha = coef;
+    T xe[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) {  // X is read only here, before the stores
+      const int i = (int)threadIdx.x + e * kCgSmallThreads;
+      xe[e] = i < n ? x[i] : (T)0;
+    }
 #pragma unroll
     for (int e = 0; e < E; ++e) {
       const int i = (int)threadIdx.x + e * kCgSmallThreads;  // n <= kCgSmallMaxN
       rv[e] = fma(-alpha, we[e], rv[e]);
       if (i < n) {
-        x[i] = fma(alpha, pe[e], x[i]);  // X is read only here
+        x[i] = fma(alpha, pe[e], xe[e]);
         r[i] = rv[e];
       }
     }
@@ -1414,8 +1420,8 @@ cg_step_small_kernel(T *__restrict__ X, T *__restrict__ R, T *__restrict__ P,
     rs_next[b] = t;
     if (active) {
       if (iters) iters[b] += 1;
-      if (t > thr[b]) atomicAdd(nactive, 1);
-      coef = (T)(t / rs[b]);
+      if (t > thrb) atomicAdd(nactive, 1);
+      coef = (T)(t / rsb);
     }
   }
   if (!active) return;

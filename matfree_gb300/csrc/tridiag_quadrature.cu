@@ -996,8 +996,8 @@ __device__ bool dc_merge_level(int G, const DcArrays &Ar, int k, int s, int nm, 
 }
 
 __global__ void __launch_bounds__(kDcMaxThreads, 1)
-    tridiag_dc_kernel(int k, int64_t p, int G, const double *__restrict__ H, int fun, double param,
-                      const double *__restrict__ scale, double *__restrict__ values,
+    tridiag_dc_kernel(int k, int64_t p, int G, const double *H, int fun, double param,
+                      const double *scale, double *__restrict__ values,
                       double *__restrict__ eigvals, double *__restrict__ first_sq,
                       int *__restrict__ status) {
   chain_wait();
