@@ -176,15 +176,14 @@ __global__ void __launch_bounds__(kCThreads + 32, 2) arnoldi_step_kernel(const C
           }
         }
     }
-    if (*fail) {
-      // copies in flight land (bounded) before the shared memory goes away
-      if (lane < kWC)
-        for (int f = fills > nslots ? fills - nslots : 0; f < fills; ++f)
-          mbar_wait_bounded(c_smem(&sh->full[lane * nslots + f % nslots]), (uint32_t)(f / nslots) & 1u, nullptr,
-                            kMbarWaitNs / 8);
-      if (lane == 0 && wq_fills > 0)
-        mbar_wait_bounded(c_smem(&sh->wq_full), (uint32_t)(wq_fills - 1) & 1u, nullptr, kMbarWaitNs / 8);
-    }
+    // the last copies land (bounded) before this warp is done: a compute warp that gives up
+    // later leaves none in flight into shared memory that goes to another CTA
+    if (lane < kWC)
+      for (int f = fills > nslots ? fills - nslots : 0; f < fills; ++f)
+        mbar_wait_bounded(c_smem(&sh->full[lane * nslots + f % nslots]), (uint32_t)(f / nslots) & 1u, nullptr,
+                          kMbarWaitNs / 8);
+    if (lane == 0 && wq_fills > 0)
+      mbar_wait_bounded(c_smem(&sh->wq_full), (uint32_t)(wq_fills - 1) & 1u, nullptr, kMbarWaitNs / 8);
     if (S > 1) c_cluster_wait();
   } else {
     const int wr = warp % kWR, group = warp / kWR;

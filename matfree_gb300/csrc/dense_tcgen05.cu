@@ -575,11 +575,10 @@ dense_tcgen05_splitk_kernel(const __grid_constant__ CUtensorMap map_ahi,
           ph ^= 1u;
         }
       }
-      if (*abort_flag) {
-        for (int kt = (issued > stages ? issued - stages : 0); kt < issued; ++kt)
-          mbar_wait_bounded(smem_u32(&sh->full[kt % stages]), (uint32_t)(kt / stages) & 1u, nullptr,
-                            kMbarWaitNs / 8);
-      }
+      // the last copies land (bounded) before this role is done, whichever role gives up and
+      // when; the slices fetched ahead are among them: no wait comes before their panel parts
+      for (int kt = (issued > stages ? issued - stages : 0); kt < issued; ++kt)
+        mbar_wait_bounded(smem_u32(&sh->full[kt % stages]), (uint32_t)(kt / stages) & 1u, nullptr, kMbarWaitNs / 8);
     }
   } else if (warp == 1) {
     if (lane == 0) {
