@@ -40,10 +40,11 @@ _WS = Workspace()
 
 def _plain(*tensors) -> bool:
     """Whether a kernel may stand in for torch operations on these: plain tensors that no
-    gradient, forward-mode tangent or function transform (vmap, jvp) follows."""
-    return all(type(t) is torch.Tensor and not torch._C._functorch.is_functorch_wrapped_tensor(t)
-               and not (torch.is_grad_enabled() and t.requires_grad)
-               and torch.autograd.forward_ad.unpack_dual(t).tangent is None for t in tensors)
+    gradient follows, outside of function transforms (vmap, jvp) and forward-mode levels."""
+    if torch._C._functorch.peek_interpreter_stack() is not None or torch.autograd.forward_ad._current_level >= 0:
+        return False
+    live = torch.is_grad_enabled()
+    return all(type(t) is torch.Tensor and not (live and t.requires_grad) for t in tensors)
 
 
 def _plain_float64(device, *tensors) -> bool:

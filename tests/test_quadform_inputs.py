@@ -25,7 +25,7 @@ def test_plain_tensors():
         assert _plain(live)
     with fwad.dual_level():
         assert not _plain(fwad.make_dual(t, t))
-        assert _plain(t)
+    assert _plain(t)
     seen = []
     torch.vmap(lambda x: (seen.append(_plain(x)), x)[1])(t)
     torch.func.jvp(lambda x: (seen.append(_plain(x)), x)[1], (t,), (t,))
