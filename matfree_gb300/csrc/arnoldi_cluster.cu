@@ -692,16 +692,15 @@ static size_t c_fixed(int R, int wr) {
   return (sizeof(CShared) + 127) / 128 * 128 + (size_t)(2 * R + (kCWarps / wr - 1) * 2 * R) * 4;
 }
 
-// clusters held at a time, per log2 of the row warps
-struct CSlots {
-  int clusters[4][kCSizes];
-  CSlots() {
-    for (int w = 0; w < 4; ++w) {
-      c_prepare(c_kernel<true>(1 << w));
-      c_count_clusters(c_kernel<false>(1 << w), clusters[w]);
-    }
-  }
-};
+// the current device's counts (its kernels prepared with them); null: not to be had
+static const CSlots *c_slots() {
+  static PerDevice<CSlots> table;
+  return table.get(current_device(), [](CSlots &t) {
+    for (int w = 0; w < 4; ++w)
+      if (!c_prepare(c_kernel<true>(1 << w)) || !c_count_clusters(c_kernel<false>(1 << w), t.clusters[w])) return false;
+    return true;
+  });
+}
 
 struct CPlan {
   int S, R, wr, slots, clusters;
@@ -717,8 +716,7 @@ struct CPlan {
 // those leave rows or SMs unused: n = 23170, 96 steps, 32 probes S = 12 5.8 ms (16: 6.7), n = 18000, 64,
 // 64 3.9 (16: 5.8), n = 10000, 32, 128 S = 6 1.34 (8: 1.64).  Of equal sizes the one whose launches
 // are chained: n = 3001, k = 16, 40 probes 464 us per solve with S = 4, 507 with 6.
-static CPlan c_plan(int64_t n, int64_t p, int j) {
-  static const CSlots slots;
+static CPlan c_plan(const CSlots &slots, int64_t n, int64_t p, int j) {
   CPlan best{0, 0, 0, 0, 0};
   double best_us = 1e300;
   for (int i = 0; i < kCSizes; ++i) {
@@ -753,7 +751,8 @@ int launch_arnoldi_step(int j, int64_t k, int64_t n, int64_t p, float *Q, int64_
                         const float *Vin, int64_t vb, float *Vout, __nv_bfloat16 *hi, __nv_bfloat16 *lo, double *H,
                         double *Hh, double *rec, int *status, bool chained, cudaStream_t s) {
   if (p <= 0) return MFG_OK;
-  const CPlan plan = c_plan(n, p, j);
+  const CSlots *slots = c_slots();
+  const CPlan plan = slots ? c_plan(*slots, n, p, j) : CPlan{0, 0, 0, 0, 0};
   if (plan.S == 0 || j > kCMaxCols) return MFG_ERR_UNSUPPORTED;
   CStepArgs a;
   a.Q = Q;
@@ -792,8 +791,13 @@ int launch_arnoldi_h(int64_t k, int64_t p, double *H, const double *Hh, const do
     MFG_CUDA_TRY(launch_kernel(arnoldi_h_band_kernel, dim3((unsigned)p), (unsigned)rows, 0, 0, chained, s, H, Hh, rec, (int)k));
     return MFG_LAUNCH_STATUS();
   }
-  const size_t smem = ((size_t)(k + 1) * k + 4 * k + 1 + 4 * (size_t)rows) * sizeof(double);
-  MFG_CUDA_TRY(cudaFuncSetAttribute(arnoldi_h_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  auto bytes = [](int64_t kk) {
+    return ((size_t)(kk + 1) * kk + 4 * kk + 1 + 4 * (size_t)(ceil_div(kk, 32) * 32)) * sizeof(double);
+  };
+  const size_t smem = bytes(k);
+  // the same limit in every launch: another thread's shorter solve must not lower it under this one
+  MFG_CUDA_TRY(cudaFuncSetAttribute(arnoldi_h_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)bytes(kTwoSweepMaxK)));
   MFG_CUDA_TRY(launch_kernel(arnoldi_h_kernel, dim3((unsigned)p), 4u * rows, smem, 0, chained, s, H, Hh, rec, (int)k, nu_last_inv));
   return MFG_LAUNCH_STATUS();
 }

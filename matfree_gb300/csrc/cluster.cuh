@@ -217,10 +217,17 @@ inline bool c_prepare(K kern) {
          cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
 }
 
+// Clusters that the current device holds at a time, per log2 of the row warps and size
+// (0: that size does not run there).
+struct CSlots {
+  int clusters[4][kCSizes];
+};
+
+// False if the kernel could not be prepared or asked about for another reason than a cluster size.
 template <typename K>
-inline void c_count_clusters(K kern, int (&clusters)[kCSizes]) {
-  const bool set = c_prepare(kern);
-  for (int i = 0; i < kCSizes; ++i) {
+inline bool c_count_clusters(K kern, int (&clusters)[kCSizes]) {
+  bool ok = c_prepare(kern);
+  for (int i = 0; i < kCSizes && ok; ++i) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(64u * kCSize[i]);
     cfg.blockDim = dim3(kCThreads + 32);
@@ -232,10 +239,13 @@ inline void c_count_clusters(K kern, int (&clusters)[kCSizes]) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int c = 0;
-    if (!set || cudaOccupancyMaxActiveClusters(&c, kern, &cfg) != cudaSuccess) c = 0;
+    const cudaError_t e = cudaOccupancyMaxActiveClusters(&c, kern, &cfg);
+    if (e != cudaSuccess) c = 0;
+    ok = e == cudaSuccess || e == cudaErrorInvalidClusterSize || e == cudaErrorInvalidConfiguration;
     clusters[i] = c;
   }
   (void)cudaGetLastError();
+  return ok;
 }
 
 // Larger clusters are not chained: placed on SMs as these come free they no longer all

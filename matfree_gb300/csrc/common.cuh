@@ -7,6 +7,7 @@
 #include <stddef.h>
 
 #include "../../include/matfree_gb300.h"
+#include "per_device.cuh"
 
 namespace mfg {
 // Records the call site and CUDA error text of the most recent failure on
@@ -43,6 +44,21 @@ constexpr int kWarps = kThreads / 32;
 inline cudaStream_t as_stream(void *s) { return reinterpret_cast<cudaStream_t>(s); }
 
 inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
+
+inline int current_device() {
+  int dev = 0;
+  return cudaGetDevice(&dev) == cudaSuccess ? dev : -1;
+}
+
+// Multiprocessors of the current device (152 where it cannot be asked).
+inline int sm_count() {
+  static PerDevice<int> counts;
+  const int dev = current_device();
+  const int *sms = counts.get(dev, [&](int &n) {
+    return cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && n > 0;
+  });
+  return sms ? *sms : 152;
+}
 
 // ---------------------------------------------------------------------------
 // mbarrier waits, bounded in wall-clock time (%globaltimer) and given up

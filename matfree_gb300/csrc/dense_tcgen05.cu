@@ -1323,19 +1323,23 @@ int64_t schedule_cost(const PairSchedule &sc, int K) {
 // 138, 144, 140, 138, 105, 120 on a GB300).
 struct SplitKSlots {
   int cta[kSplitKMaxS + 1];
-  SplitKSlots() {
-    int dev = 0, sms = 152;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-      sms = 152;
+};
+
+// Dynamic shared memory that the split-K kernels are allowed, whatever a launch takes of it.
+constexpr int kSplitKSmem = 1024 + (int)kSplitKRing + (int)sizeof(GemmShared);
+
+static SplitKSlots splitk_slots() {
+  static PerDevice<SplitKSlots> table;
+  const int sms = sm_count();
+  auto fill = [&](SplitKSlots &t) {
     auto kern = dense_tcgen05_splitk_kernel<true, 1>;
-    const int smem = 1024 + (int)kSplitKRing + (int)sizeof(GemmShared);
-    const bool set = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess;
+    bool ok = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSplitKSmem) == cudaSuccess;
+    t.cta[0] = sms;
     for (int S = 1; S <= kSplitKMaxS; ++S) {
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3((unsigned)S, 1024, 1);
       cfg.blockDim = dim3(kGemmThreads);
-      cfg.dynamicSmemBytes = (size_t)smem;
+      cfg.dynamicSmemBytes = (size_t)kSplitKSmem;
       cudaLaunchAttribute attr[1];
       attr[0].id = cudaLaunchAttributeClusterDimension;
       attr[0].val.clusterDim.x = (unsigned)S;
@@ -1343,14 +1347,20 @@ struct SplitKSlots {
       cfg.attrs = attr;
       cfg.numAttrs = 1;
       int clusters = 0;
-      if (!set || cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) != cudaSuccess || clusters < 1)
+      if (!ok || cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) != cudaSuccess || clusters < 1) {
+        ok = false;
         clusters = sms / S > 0 ? sms / S : 1;
-      cta[S] = clusters * S;
+      }
+      t.cta[S] = clusters * S;
     }
-    cta[0] = sms;
     (void)cudaGetLastError();
-  }
-};
+    return ok;
+  };
+  if (const SplitKSlots *t = table.get(current_device(), fill)) return *t;
+  SplitKSlots t;  // counts that could not be asked, for this call only
+  fill(t);
+  return t;
+}
 
 struct SplitKPlan {
   int bn, S, mt;  // probe tile, K ranges, 128-row tiles per CTA
@@ -1367,7 +1377,7 @@ struct SplitKPlan {
 // (55 us; S = 4 of two: 60), n = 5000, 48 probes S = 3 (20 us; S = 1: 46, S = 4: 30, a
 // second round), n = 512 S = 8 (4 us; S = 1: 7).
 static SplitKPlan splitk_plan(int64_t n, int64_t p, bool split) {
-  static const SplitKSlots slots;
+  const SplitKSlots slots = splitk_slots();
   const int64_t tiles_p = ceil_div(p, kSplitKMaxBN);
   SplitKPlan best{(int)(ceil_div(ceil_div(p, tiles_p), 16) * 16), 1, 1};
   const int64_t slices = ceil_div(n, kSplitKBK);
@@ -1409,6 +1419,7 @@ static int launch_splitk(const __nv_bfloat16 *A_hi, const __nv_bfloat16 *A_lo, i
   int stages = (int)(kSplitKRing / stage_bytes);
   if (stages > kGemmMaxStages) stages = kGemmMaxStages;
   const size_t ring = (size_t)stages * stage_bytes, part = (size_t)bn * rows * 4;
+  static_assert((size_t)kSplitKMaxBN * 2 * kBM * 4 <= kSplitKRing, "the partial tile fits the ring");
   const size_t smem = 1024 + (ring > part ? ring : part) + sizeof(GemmShared);
   CUtensorMap mahi, malo, mbhi, mblo;
   if (!make_map(&mahi, A_hi, n, n, lda, rows, kSplitKBK)) return MFG_ERR_CUDA;
@@ -1425,7 +1436,8 @@ static int launch_splitk(const __nv_bfloat16 *A_hi, const __nv_bfloat16 *A_lo, i
   const int vec_ok = ldw % 4 == 0 && ldvf % 4 == 0 && ((uintptr_t)W & 15) == 0 && ((uintptr_t)Vf & 15) == 0;
   auto kern = mt == 2 ? (split ? dense_tcgen05_splitk_kernel<true, 2> : dense_tcgen05_splitk_kernel<false, 2>)
                       : (split ? dense_tcgen05_splitk_kernel<true, 1> : dense_tcgen05_splitk_kernel<false, 1>);
-  MFG_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // the same limit in every launch: another thread's smaller product must not lower it under this one
+  MFG_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSplitKSmem));
   MFG_CUDA_TRY(launch_kernel(kern, dim3((unsigned)S, (unsigned)ceil_div(n, rows), (unsigned)ceil_div(p, bn)),
                              kGemmThreads, smem, (unsigned)S, chained, s, mahi, malo, mbhi, mblo, Vf, ldvf, W, ldw,
                              (int)n, (int)p, bn, stages, cols, (float)shift, vec_ok, status));
@@ -1451,13 +1463,7 @@ int launch_dense_tcgen05(const __nv_bfloat16 *A_hi, const __nv_bfloat16 *A_lo, i
   // per probe tile there, which pays while the tiles (of one K range) cover
   // up to 5/9 of the SMs (256 probes: n = 5000 52 against 71 us for CTA pairs;
   // n = 6144 73 against 66).  Rules of the autotuner name CTA-pair forms.
-  static int sms = 0;
-  if (sms == 0) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-      sms = 152;
-  }
+  const int sms = sm_count();
   const bool pair_rule = (rule.split != 0 || rule.bn != 0) && p >= 64;
   const int64_t row_tiles = ceil_div(n, kBM);
   if (!pair_rule && (n < kPairMinRows || p <= kSplitKMaxBN ||

@@ -579,13 +579,16 @@ static auto g_kernel(int wr) -> void (*)(const GsArgs<T>) {
   }
 }
 
+// the current device's counts (its kernels prepared with them); null: not to be had
 template <typename T, bool kAdj>
-struct GSlots {
-  int clusters[4][kCSizes];
-  GSlots() {
-    for (int w = 0; w < 4; ++w) c_count_clusters(g_kernel<T, kAdj>(1 << w), clusters[w]);
-  }
-};
+static const CSlots *g_slots() {
+  static PerDevice<CSlots> table;
+  return table.get(current_device(), [](CSlots &t) {
+    for (int w = 0; w < 4; ++w)
+      if (!c_count_clusters(g_kernel<T, kAdj>(1 << w), t.clusters[w])) return false;
+    return true;
+  });
+}
 
 bool gs_cluster_applies(int64_t n, int64_t ncols, int64_t nextra) {
   return n <= (int64_t)kCMaxS * kCMaxR && ncols <= kGMaxCols && nextra <= kGMaxCols;
@@ -596,8 +599,9 @@ bool gs_cluster_applies(int64_t n, int64_t ncols, int64_t nextra) {
 // from L2; float64 also its FMAs, 1.7 a clock and SM for two CTAs).
 template <typename T, bool kAdj>
 static int g_run(GsArgs<T> &a, bool chained, cudaStream_t s) {
-  static const GSlots<T, kAdj> slots;
   if (a.p <= 0) return MFG_OK;
+  const CSlots *slots = g_slots<T, kAdj>();
+  if (!slots) return MFG_ERR_UNSUPPORTED;
   a.cpad = (a.ncols + 7) / 8 * 8;
   a.xpad = (2 * (kAdj ? a.nx : 0) + 7) / 8 * 8;
   const double cols = (double)a.passes * a.ncols + 2.0 * (kAdj ? a.nx : 0) + 4.0;
@@ -611,7 +615,7 @@ static int g_run(GsArgs<T> &a, bool chained, cudaStream_t s) {
     const int w = c_row_warps(R);
     int lw = 0;
     while ((1 << lw) < w) ++lw;
-    const int64_t c = slots.clusters[lw][i];
+    const int64_t c = slots->clusters[lw][i];
     const size_t slot = (size_t)g_gc<T>(w) * R * sizeof(T), fixed = g_fixed<T>(a.cpad, a.xpad, (int)R, w);
     const int groups = kCWarps / w;
     if (c < 1 || fixed + slot * groups > kCSmem) continue;

@@ -279,13 +279,7 @@ template <typename T>
 int launch_dense_simt(const T *A, int64_t lda, const T *V, int64_t ldv, T *W, int64_t ldw,
                       int64_t n, int64_t p, double shift, cudaStream_t s) {
   if (n <= 0 || p <= 0) return MFG_OK;
-  static int sms = 0;
-  if (sms == 0) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-      sms = 152;
-  }
+  const int sms = sm_count();
   if constexpr (sizeof(T) == 8) {
     // the K ranges of least time: an SM's CTAs one after the other on its pipe (five
     // at a time; past that a tail of two), slower with few of them to hide each
@@ -588,20 +582,18 @@ static int launch_csr_spmm_t(const int32_t *row_ptr, const int32_t *col_idx, con
                              const float *V, int64_t ldv, float *W, int64_t ldw, int64_t p, double shift,
                              int *status, cudaStream_t s) {
   const size_t smem = sizeof(WinShared);
-  static int per_sm = 0, sms = 0;
-  if (per_sm == 0) {
-    int dev = 0;
-    MFG_CUDA_TRY(cudaGetDevice(&dev));
-    MFG_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    MFG_CUDA_TRY(cudaFuncSetAttribute(csr_spmm_window_kernel<RMAX>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    int q = 0;
-    MFG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&q, csr_spmm_window_kernel<RMAX>,
-                                                               kWThreads + 32, smem));
-    if (q < 1) return MFG_ERR_UNSUPPORTED;
-    per_sm = q;
-  }
-  const int64_t G = (int64_t)sms * per_sm;
+  static PerDevice<int> table;
+  const int *per_sm = table.get(current_device(), [&](int &q) {
+    return cuda_status(cudaFuncSetAttribute(csr_spmm_window_kernel<RMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            (int)smem),
+                       __FILE__, __LINE__) == MFG_OK &&
+           cuda_status(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&q, csr_spmm_window_kernel<RMAX>, kWThreads + 32,
+                                                                     smem),
+                       __FILE__, __LINE__) == MFG_OK;
+  });
+  if (!per_sm) return MFG_ERR_CUDA;
+  if (*per_sm < 1) return MFG_ERR_UNSUPPORTED;
+  const int64_t G = (int64_t)sm_count() * *per_sm;
   const int64_t tile_rows = kWRows;
   const int64_t ntiles = ceil_div(n, tile_rows);
   const int64_t grid = G < ntiles ? G : ntiles;

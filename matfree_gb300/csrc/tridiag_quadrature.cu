@@ -962,13 +962,7 @@ __device__ bool dc_merge_roots(const DcArrays &Ar, int k, int s, int nm, double 
 // (8); k = 32, 64: 199 -> 92 (4); k = 48, 128: 344 -> 143 (4); k = 64, 256: 671 -> 301
 // (2).
 static int dc_group(int64_t k, int64_t p) {
-  static int sms = 0;
-  if (sms == 0) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-      sms = 152;
-  }
+  const int sms = sm_count();
   int best = 1;
   double best_clk = 1e300;
   for (int G = 1, lg = 0; G <= 8; G *= 2, ++lg) {
