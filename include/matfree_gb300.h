@@ -281,6 +281,15 @@ MFG_API int mfg_rbf_build(const float *x, int64_t n, int32_t dim, double s2, dou
 MFG_API int mfg_rbf_build_dlogell(const float *x, int64_t n, int32_t dim, double s2, double ell,
                                   int32_t precision, void *a, void *a_lo, int64_t lda, void *stream);
 
+/* The cluster size that a step of a solve is launched with, and 0 where the separate launches
+ * run, for a GPU that holds clusters[4][9] clusters at a time (1, 2, 4, 8 warps of rows a CTA x
+ * 1, 2, 4, 6, 8, 10, 12, 14, 16 CTAs a cluster; 0: not that size).  Host arithmetic only.
+ * kind 0: the two-sweep Arnoldi step against ncols vectors, 1: Gram-Schmidt against ncols
+ * vectors, 2: the adjoint of a basis of ncols (its plan of the last step; 0 if any step has
+ * none).  plan[4]: CTAs per probe, rows and row warps of a CTA, slots of a ring. */
+MFG_API int mfg_step_plan(int32_t kind, int32_t precision, int64_t n, int64_t p, int64_t ncols,
+                          const int32_t *clusters, int32_t *plan);
+
 /* Values scale_b e1^T f(T_b) e1 (p) and their cotangent dH (p, k, k) in the
  * Hessenberg matrix whose symmetrised tridiagonal part is T_b, from eigvals
  * (p, k), eigvecs (p, k, k; columns), fw = f(eigvals) and fprime_mid (p, k, k)

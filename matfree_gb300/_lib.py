@@ -70,6 +70,7 @@ SIGNATURES = {
     "mfg_tridiag_eigh": (c_int, [c_int64, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p]),
     "mfg_rbf_build": (c_int, [c_void_p, c_int64, c_int32, c_double, c_double, c_int32, c_void_p, c_void_p, c_int64, c_void_p]),
     "mfg_rbf_build_dlogell": (c_int, [c_void_p, c_int64, c_int32, c_double, c_double, c_int32, c_void_p, c_void_p, c_int64, c_void_p]),
+    "mfg_step_plan": (c_int, [c_int32, c_int32, c_int64, c_int64, c_int64, c_void_p, c_void_p]),
     "mfg_quadform_dh": (c_int, [c_int64, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                 c_void_p, c_void_p]),
     "mfg_theta_contractions_workspace_bytes": (c_size_t, [POINTER(MfgOperator), c_int64, c_int64]),

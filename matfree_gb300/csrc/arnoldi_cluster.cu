@@ -672,8 +672,6 @@ __global__ void arnoldi_h_band_kernel(double *H, const double *Hh, const double 
 // Host side
 // ---------------------------------------------------------------------------
 
-bool arnoldi_cluster_applies(int64_t n) { return n <= (int64_t)kCMaxS * kCMaxR; }
-
 static int c_gc(int wr) { return wr >= 4 ? 2 : 4; }
 
 using CKernel = void (*)(const CStepArgs);
@@ -740,6 +738,25 @@ static CPlan c_plan(const CSlots &slots, int64_t n, int64_t p, int j) {
     }
   }
   return best;
+}
+
+// Whether a step of n rows has a plan on the current device (which does not depend on j);
+// the separate launches run otherwise.
+bool arnoldi_cluster_applies(int64_t n, int64_t p) {
+  if (n > (int64_t)kCMaxS * kCMaxR) return false;
+  const CSlots *slots = c_slots();
+  return slots && c_plan(*slots, n, p, 1).S > 0;
+}
+
+// The plan for a table of clusters (host only): see mfg_step_plan.
+int arnoldi_plan_query(const CSlots &slots, int64_t n, int64_t p, int64_t j, int *out) {
+  if (n > (int64_t)kCMaxS * kCMaxR || j > kCMaxCols) return 0;
+  const CPlan c = c_plan(slots, n, p, (int)j);
+  out[0] = c.S;
+  out[1] = c.R;
+  out[2] = c.wr;
+  out[3] = c.slots;
+  return c.S;
 }
 
 // Step j of the two-sweep iteration for every probe (j = 0: the first step).

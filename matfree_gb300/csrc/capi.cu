@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "cluster.cuh"
 #include "kernels.cuh"
 
 namespace mfg {
@@ -298,7 +299,7 @@ static int run_two_sweep(const mfg_operator *op, int64_t k, int64_t p, int64_t l
     const double bfb = hi ? (double)n * (double)p * 2.0 * (lo ? 2.0 : 1.0) : 0.0;
     const int64_t qb = k * ld;
     const int64_t koff = k, xs = 2 * k + 1;
-    const bool fused = arnoldi_cluster_applies(n);
+    const bool fused = arnoldi_cluster_applies(n, p);
     if (fused) {
       // a step is the product and one launch: while a probe's vector fits the
       // registers of a cluster (n <= 32768)
@@ -404,7 +405,7 @@ static int run_hessenberg(const mfg_operator *op, int64_t k, int64_t p, const T 
   // initial length (decomp.py:436) -> 1 / length, and q_0; as one launch where a
   // cluster's registers hold a vector.  Not chained: what wrote the operator and the
   // vectors is complete before the loop's first product.
-  const bool one = k > 0 && gs_cluster_applies(n, 0, 0);
+  const bool one = k > 0 && gs_cluster_applies<T>(n, p, 0);
   if (one)
     MFG_LAUNCH(MFG_PROF_OTHER, 2.0 * vecb + bfb, 3.0 * vecb / sizeof(T),
                launch_gs_cluster<T>(Q, qb, ld, 0, V, n, p, 4, nullptr, 0, nullptr, 0, nullptr, 0, 0, len0, nullptr, 0,
@@ -455,7 +456,7 @@ static int run_hessenberg(const mfg_operator *op, int64_t k, int64_t p, const T 
     }
     const bool last = (j + 1 == k);
     double *hsub = last ? nullptr : H + (j + 1) * k + j;
-    if (gs_cluster_applies(n, ncols, 0)) {
+    if (gs_cluster_applies<T>(n, p, ncols)) {
       // the step after the product as one launch
       MFG_LAUNCH(MFG_PROF_SUBPROJ, (ncols + 2.0) * vecb + (last ? 0.0 : bfb), (reortho ? 4.0 : 2.0) * pf,
                  launch_gs_cluster<T>(Q, qb, ld, ncols, Wb, n, p, reortho ? 4 : 2, nullptr, 0, nullptr, 0, H + j,
@@ -657,7 +658,7 @@ static int run_adjoint(const mfg_operator *op, int64_t k, int64_t p, int64_t ld,
              launch_sub<T>(Q, qb, ld, (int)k, coef, k, 1, lam, lam, ld, n, p, false, true, partials,
                            counters, nullptr, nullptr, 0, s, status));
 
-  if (gs_cluster_applies(n, k, 2 * k)) {
+  if (adj_cluster_applies<T>(n, p, k)) {
     // lambda of step k - 1 reprojected (decomp.py:576-584), then a step is the product
     // and one launch
     MFG_LAUNCH(MFG_PROF_PROJ, (k + 1.0) * vecb, 2.0 * k * vecb / sizeof(T),
@@ -877,7 +878,7 @@ static int run_bidiag(const mfg_operator *A, const mfg_operator *At, int64_t k, 
     // left vector: u_i = (A v_i - beta_i u_{i-1}) reorthogonalised, / alpha_i
     MFG_LAUNCH(MFG_PROF_APPLY, ab, af,
                apply_op<T>(A, Vb + i * ld, qb, Wb, ld, p, hiA, loA, ld, panel, status, s, chained));
-    if (gs_cluster_applies(n, i + 1, 0)) {
+    if (gs_cluster_applies<T>(n, p, i) && gs_cluster_applies<T>(n, p, i + 1)) {
       // everything of a side after its product as one launch
       MFG_LAUNCH(MFG_PROF_SUBPROJ, (i + 3.0) * vecb, (8.0 * i + 6.0) * vecb / sizeof(T),
                  launch_gs_cluster<T>(U, qb, ld, (int)i, Wb, n, p, 4, i > 0 ? U + (i - 1) * ld : nullptr, qb, betas + i,
@@ -1552,6 +1553,18 @@ int mfg_rbf_build(const float *x, int64_t n, int32_t dim, double s2, double ell,
 int mfg_rbf_build_dlogell(const float *x, int64_t n, int32_t dim, double s2, double ell,
                           int32_t precision, void *a, void *a_lo, int64_t lda, void *stream) {
   return rbf_build(x, n, dim, s2, ell, precision, 1, a, a_lo, lda, stream);
+}
+
+int mfg_step_plan(int32_t kind, int32_t precision, int64_t n, int64_t p, int64_t ncols, const int32_t *clusters,
+                  int32_t *plan) {
+  if (n <= 0 || p <= 0 || ncols < 0 || !clusters || !plan) return 0;
+  CSlots t;
+  for (int w = 0; w < 4; ++w)
+    for (int i = 0; i < kCSizes; ++i) t.clusters[w][i] = clusters[w * kCSizes + i];
+  if (kind == 0) return precision == MFG_PREC_FP64 ? 0 : arnoldi_plan_query(t, n, p, ncols, plan);
+  if (kind != 1 && (kind != 2 || ncols < 1)) return 0;
+  return precision == MFG_PREC_FP64 ? gs_plan_query<double>(t, n, p, ncols, kind == 2, plan)
+                                    : gs_plan_query<float>(t, n, p, ncols, kind == 2, plan);
 }
 
 size_t mfg_theta_contractions_workspace_bytes(const mfg_operator *op, int64_t rows, int64_t ld) {

@@ -590,53 +590,102 @@ static const CSlots *g_slots() {
   });
 }
 
-bool gs_cluster_applies(int64_t n, int64_t ncols, int64_t nextra) {
-  return n <= (int64_t)kCMaxS * kCMaxR && ncols <= kGMaxCols && nextra <= kGMaxCols;
-}
+struct GPlan {
+  int S, R, wr, slots, clusters, cpad, xpad;
+};
 
 // CTAs per probe, as for the Arnoldi step: the fewest rounds of probes over the
 // clusters the GPU holds, a round costing its meetings and the CTA's passes (40 GB/s
-// from L2; float64 also its FMAs, 1.7 a clock and SM for two CTAs).
-template <typename T, bool kAdj>
-static int g_run(GsArgs<T> &a, bool chained, cudaStream_t s) {
-  if (a.p <= 0) return MFG_OK;
-  const CSlots *slots = g_slots<T, kAdj>();
-  if (!slots) return MFG_ERR_UNSUPPORTED;
-  a.cpad = (a.ncols + 7) / 8 * 8;
-  a.xpad = (2 * (kAdj ? a.nx : 0) + 7) / 8 * 8;
-  const double cols = (double)a.passes * a.ncols + 2.0 * (kAdj ? a.nx : 0) + 4.0;
+// from L2; float64 also its FMAs, 1.7 a clock and SM for two CTAs).  S = 0: no size
+// that the GPU holds has room.
+template <typename T>
+static GPlan g_plan(const CSlots &slots, int64_t n, int64_t p, int passes, int ncols, int nx) {
+  GPlan best{};
+  best.cpad = (ncols + 7) / 8 * 8;
+  best.xpad = (2 * nx + 7) / 8 * 8;
+  const double cols = (double)passes * ncols + 2.0 * nx + 4.0;
   double best_us = 1e300;
-  int64_t clusters = 0;
-  int wr = 0;
   for (int i = 0; i < kCSizes; ++i) {
     const int S = kCSize[i];
-    const int64_t R = ceil_div(ceil_div(a.n, S), 4) * 4;
+    const int64_t R = ceil_div(ceil_div(n, S), 4) * 4;
     if (R > kCMaxR) continue;
     const int w = c_row_warps(R);
     int lw = 0;
     while ((1 << lw) < w) ++lw;
-    const int64_t c = slots->clusters[lw][i];
-    const size_t slot = (size_t)g_gc<T>(w) * R * sizeof(T), fixed = g_fixed<T>(a.cpad, a.xpad, (int)R, w);
+    const int c = slots.clusters[lw][i];
+    const size_t slot = (size_t)g_gc<T>(w) * R * sizeof(T), fixed = g_fixed<T>(best.cpad, best.xpad, (int)R, w);
     const int groups = kCWarps / w;
     if (c < 1 || fixed + slot * groups > kCSmem) continue;
     double us = (S == 1 ? 6.0 : 9.0) + 0.15 * S + cols * R * sizeof(T) / 40e3;
     if (sizeof(T) == 8) us += cols * R / 1630.0;
-    us = us * (double)ceil_div(a.p, c) + (S > kCChainS ? kCUnchainedUs : 0.0);
+    us = us * (double)ceil_div(p, c) + (S > kCChainS ? kCUnchainedUs : 0.0);
     if (us < best_us) {
       best_us = us;
-      a.S = S;
-      a.R = (int)R;
+      best.S = S;
+      best.R = (int)R;
+      best.wr = w;
+      best.clusters = c;
       int sl = (int)((kCSmem - fixed) / slot);
       if (sl > kCMaxSlots) sl = kCMaxSlots;
-      a.slots = sl / groups;
-      clusters = c;
-      wr = w;
+      best.slots = sl / groups;
     }
   }
-  if (wr == 0) return MFG_ERR_UNSUPPORTED;
-  const size_t smem = g_fixed<T>(a.cpad, a.xpad, a.R, wr) +
-                      (size_t)a.slots * (kCWarps / wr) * g_gc<T>(wr) * a.R * sizeof(T);
-  return c_launch(g_kernel<T, kAdj>(wr), a.S, a.S * (a.p < clusters ? a.p : clusters), smem, a, chained, s);
+  return best;
+}
+
+static bool g_limits(int64_t n, int64_t ncols, int64_t nextra) {
+  return n <= (int64_t)kCMaxS * kCMaxR && ncols <= kGMaxCols && nextra <= kGMaxCols;
+}
+
+// Whether Gram-Schmidt against ncols vectors, or every step of an adjoint of k, has a plan
+// on the current device; the separate launches run otherwise.
+template <typename T>
+bool gs_cluster_applies(int64_t n, int64_t p, int64_t ncols) {
+  if (!g_limits(n, ncols, 0)) return false;
+  const CSlots *slots = g_slots<T, false>();
+  return slots && g_plan<T>(*slots, n, p, 4, (int)ncols, 0).S > 0;
+}
+
+template <typename T>
+static bool adj_has_plans(const CSlots &slots, int64_t n, int64_t p, int64_t k) {
+  if (!g_limits(n, k, 2 * k)) return false;
+  for (int idx = 0; idx < (int)k; ++idx)
+    if (g_plan<T>(slots, n, p, idx > 0 ? 4 : 2, idx + 1, (int)k - 1 - idx).S == 0) return false;
+  return true;
+}
+
+template <typename T>
+bool adj_cluster_applies(int64_t n, int64_t p, int64_t k) {
+  const CSlots *slots = g_slots<T, true>();
+  return slots && adj_has_plans<T>(*slots, n, p, k);
+}
+
+// The plan for a table of clusters (host only): see mfg_step_plan.
+template <typename T>
+int gs_plan_query(const CSlots &slots, int64_t n, int64_t p, int64_t ncols, bool adj, int *out) {
+  if (adj ? !adj_has_plans<T>(slots, n, p, ncols) : !g_limits(n, ncols, 0)) return 0;
+  const GPlan g = adj ? g_plan<T>(slots, n, p, ncols > 1 ? 4 : 2, (int)ncols, 0) : g_plan<T>(slots, n, p, 4, (int)ncols, 0);
+  out[0] = g.S;
+  out[1] = g.R;
+  out[2] = g.wr;
+  out[3] = g.slots;
+  return g.S;
+}
+
+template <typename T, bool kAdj>
+static int g_run(GsArgs<T> &a, bool chained, cudaStream_t s) {
+  if (a.p <= 0) return MFG_OK;
+  const CSlots *slots = g_slots<T, kAdj>();
+  const GPlan g = slots ? g_plan<T>(*slots, a.n, a.p, a.passes, a.ncols, kAdj ? a.nx : 0) : GPlan{};
+  if (g.S == 0) return MFG_ERR_UNSUPPORTED;
+  a.S = g.S;
+  a.R = g.R;
+  a.slots = g.slots;
+  a.cpad = g.cpad;
+  a.xpad = g.xpad;
+  const size_t smem = g_fixed<T>(a.cpad, a.xpad, a.R, g.wr) +
+                      (size_t)a.slots * (kCWarps / g.wr) * g_gc<T>(g.wr) * a.R * sizeof(T);
+  return c_launch(g_kernel<T, kAdj>(g.wr), a.S, a.S * (a.p < g.clusters ? a.p : g.clusters), smem, a, chained, s);
 }
 
 // w (panel W; w -= prev_c prev first, if given) against basis vectors 0 .. ncols - 1,
@@ -712,6 +761,9 @@ int launch_adj_cluster(const T *Q, int64_t qb, int64_t ld, int k, int idx, const
 }
 
 #define MFG_INST(T)                                                                                               \
+  template bool gs_cluster_applies<T>(int64_t, int64_t, int64_t);                                                  \
+  template bool adj_cluster_applies<T>(int64_t, int64_t, int64_t);                                                 \
+  template int gs_plan_query<T>(const CSlots &, int64_t, int64_t, int64_t, bool, int *);                           \
   template int launch_gs_cluster<T>(const T *, int64_t, int64_t, int, const T *, int64_t, int64_t, int, const T *, \
                                     int64_t, const double *, int64_t, double *, int64_t, int64_t, double *,        \
                                     double *, int64_t, T *, T *, int64_t, __nv_bfloat16 *, __nv_bfloat16 *, int *, \

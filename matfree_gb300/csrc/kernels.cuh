@@ -57,7 +57,9 @@ int launch_twosweep_finish(T *Qj, int64_t q_bstride, const T *Z, int64_t w_bstri
                            int64_t p, const double *cf, T *qt, __nv_bfloat16 *hi,
                            __nv_bfloat16 *lo, int64_t bf_bstride, cudaStream_t s);
 // arnoldi_cluster.cu: the same step as one launch (float bases of n up to 32768)
-bool arnoldi_cluster_applies(int64_t n);
+bool arnoldi_cluster_applies(int64_t n, int64_t p);
+struct CSlots;
+int arnoldi_plan_query(const CSlots &slots, int64_t n, int64_t p, int64_t j, int *out);
 int launch_arnoldi_step(int j, int64_t k, int64_t n, int64_t p, float *Q, int64_t qb, int64_t ld, const float *W,
                         const float *Vin, int64_t vb, float *Vout, __nv_bfloat16 *hi, __nv_bfloat16 *lo, double *H,
                         double *Hh, double *rec, int *status, bool chained, cudaStream_t s);
@@ -66,7 +68,12 @@ int launch_arnoldi_h(int64_t k, int64_t p, double *H, const double *Hh, const do
 // (chained: see chain_wait in common.cuh)
 // gs_cluster.cu: Gram-Schmidt twice with the norm and the normalisation, and a step
 // of the adjoint, as one launch each (n up to 32768)
-bool gs_cluster_applies(int64_t n, int64_t ncols, int64_t nextra);
+template <typename T>
+bool gs_cluster_applies(int64_t n, int64_t p, int64_t ncols);
+template <typename T>
+bool adj_cluster_applies(int64_t n, int64_t p, int64_t k);
+template <typename T>
+int gs_plan_query(const CSlots &slots, int64_t n, int64_t p, int64_t ncols, bool adj, int *out);
 template <typename T>
 int launch_gs_cluster(const T *Q, int64_t qb, int64_t ld, int ncols, const T *W, int64_t n, int64_t p, int passes,
                       const T *prev, int64_t prev_b, const double *prev_c, int64_t prev_cs, double *h, int64_t h_bs,
