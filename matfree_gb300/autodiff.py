@@ -170,7 +170,8 @@ class _RBFLogdet(torch.autograd.Function):
             Q, H, R, c = _forward_panels(op, k, panel[b0:b1], ld, deferred)
             values, dH = quadform_dH(H, 1.0 / (c * c), _log, _dlog)
             if retry_needed(deferred):
-                Q, H, R, c = _forward_panels(op, k, panel[b0:b1], ld)
+                del Q, H, R, c, values, dH  # one chunk's panels at a time
+                Q, H, R, c = _forward_panels(op, k, panel[b0:b1], ld, two_sweep=False)
                 values, dH = quadform_dH(H, 1.0 / (c * c), _log, _dlog)
             vals.append(values)
             if len(chunks) == 1:
@@ -198,9 +199,9 @@ class _RBFLogdet(torch.autograd.Function):
         return grad.to(device=theta.device, dtype=theta.dtype), None, None, None, None, None
 
 
-def _forward_panels(op, k, panel, ld, deferred=None):
+def _forward_panels(op, k, panel, ld, deferred=None, two_sweep=True):
     """mfg_hessenberg keeping the padded (p, k, ld) / (p, ld) panels (deferred: as in
-    ``run_hessenberg``)."""
+    ``run_hessenberg``; two_sweep=False: the three-read form at once)."""
     p = panel.shape[0]
     dt = op.basis_dtype
     Q = torch.zeros((p, k, ld), dtype=dt, device=panel.device)
@@ -211,7 +212,7 @@ def _forward_panels(op, k, panel, ld, deferred=None):
     lib = _lib.lib()
     # full reorthogonalisation in two reads of the basis per step where it
     # applies, repeated in the three-read form if the device asks for it
-    for mode in ((3, 1) if two_sweep_applies(op, k) else (1,)):
+    for mode in ((3, 1) if two_sweep and two_sweep_applies(op, k) else (1,)):
         flags = _lib.MFG_SLQ_TWO_SWEEP if mode == 3 else 0
         nbytes = lib.mfg_slq_ex_workspace_bytes(ctypes.byref(s), k, p, ld, flags)
         ws, wsb = _WS.get(nbytes, panel.device)

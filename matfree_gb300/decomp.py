@@ -65,7 +65,8 @@ def run_hessenberg(op, k: int, V: torch.Tensor, *, reortho: str = "full", worksp
 
     Reading the device's report waits for the solve.  With a list ``deferred`` the
     wait is left to the caller, who enqueues what follows first and then asks
-    :func:`retry_needed`; on True everything is to be done again without it.
+    :func:`retry_needed`; on True everything is to be done again with "full" (the
+    two-sweep form would ask for that again).
     """
     V = require_cuda(V, "vectors")
     n = op.n
@@ -155,10 +156,11 @@ class _Decomposition:
                              init_length_inv=c[0])
 
 
-def _differentiable_forward(dec, op, k, V, deferred=None):
+def _differentiable_forward(dec, op, k, V, deferred=None, reortho=None):
     """run_hessenberg with full reorthogonalisation, behind the Hessenberg
     adjoint when V or the matvec's parameters require gradients (the custom
-    VJP of matfree/decomp.py:393-422); plain otherwise."""
+    VJP of matfree/decomp.py:393-422); plain otherwise (reortho: the form,
+    :func:`full_reortho`'s by default)."""
     from .autodiff import arnoldi_full, wants_grad
 
     if k > 0 and wants_grad(V, op):
@@ -167,7 +169,7 @@ def _differentiable_forward(dec, op, k, V, deferred=None):
                 "gradients of the decomposition need custom_vjp=True: the Krylov loop runs as CUDA "
                 "kernels, so it is differentiated by the Hessenberg adjoint, not traced")
         return arnoldi_full(op, k, V)
-    return run_hessenberg(op, k, V, reortho=full_reortho(op, k), deferred=deferred)
+    return run_hessenberg(op, k, V, reortho=reortho or full_reortho(op, k), deferred=deferred)
 
 
 class _TridiagSymFull(_Decomposition):
@@ -178,11 +180,11 @@ class _TridiagSymFull(_Decomposition):
         parameters (custom_vjp=True, the default)."""
         return self._batched(matvec, V, params)
 
-    def _batched(self, matvec, V: torch.Tensor, params, deferred=None) -> _DecompResult:
+    def _batched(self, matvec, V: torch.Tensor, params, deferred=None, reortho=None) -> _DecompResult:
         V = require_cuda(V, "vectors")
         op = as_operator(matvec, V.shape[1], V.dtype, params)
         k = self.num_matvecs
-        Q, H, r, c = _differentiable_forward(self, op, k, V, deferred)
+        Q, H, r, c = _differentiable_forward(self, op, k, V, deferred, reortho)
         d, e = _tridiag_from_hessenberg(H)
         out_dt = V.dtype if V.dtype in (torch.float32, torch.float64) else torch.float32
         d, e = d.to(out_dt), e.to(out_dt)

@@ -21,7 +21,7 @@ import torch
 from . import _lib
 from ._panel import Workspace, as_panel, require_cuda, stream_ptr
 from .decomp import _flat_operator, _TridiagSymFull, full_reortho, run_hessenberg, two_sweep_applies
-from .operators import CallbackOperator, Operator, as_operator
+from .operators import CallbackOperator, CSROperator, DenseOperator, Operator, as_operator
 from .tree import ravel_pytree
 
 _LOGS = {np.log, math.log, torch.log}
@@ -244,26 +244,24 @@ class FunmLanczosSym:
         from .decomp import _TridiagSymFull, retry_needed
 
         V = require_cuda(V, "vectors")
-        # with a closed-form f and an operator descriptor nothing below runs the
-        # caller's code: the solve is checked once all of it is enqueued
+        # with a closed-form f and a descriptor of the operator's data nothing below runs
+        # the caller's code: the solve is checked once all of it is enqueued
+        if not (self.dense_funm.kind is not None and isinstance(matvec, (DenseOperator, CSROperator))
+                and type(self.tridiag_sym) is _TridiagSymFull):
+            return self._apply(V, lambda X: self.tridiag_sym.batched(matvec, X, *parameters))
         deferred = []
-        if self.dense_funm.kind is not None and isinstance(matvec, Operator) \
-                and type(self.tridiag_sym) is _TridiagSymFull:
-            out = self._apply(matvec, V, parameters, deferred)
-            if not retry_needed(deferred):
-                return out
-        return self._apply(matvec, V, parameters, None)
+        out = self._apply(V, lambda X: self.tridiag_sym._batched(matvec, X, parameters, deferred))
+        if retry_needed(deferred):
+            del out
+            out = self._apply(V, lambda X: self.tridiag_sym._batched(matvec, X, parameters, reortho="full"))
+        return out
 
-    def _apply(self, matvec, V, parameters, deferred):
+    def _apply(self, V, decompose):
         from .autodiff import basis_combine, funm_e1
         from .decomp import _todense_tridiag_sym
 
         length = torch.linalg.vector_norm(V, dim=1)
-        X = V / length[:, None]
-        if deferred is None:
-            Q, T, *_ = self.tridiag_sym.batched(matvec, X, *parameters)
-        else:
-            Q, T, *_ = self.tridiag_sym._batched(matvec, X, parameters, deferred)
+        Q, T, *_ = decompose(V / length[:, None])
         if isinstance(T, tuple):
             T = _todense_tridiag_sym(*T)
         if T.shape[-1] == 0:
