@@ -128,11 +128,12 @@ __global__ void __launch_bounds__(kCThreads + 32, 2) arnoldi_step_kernel(const C
   chain_wait();
   chain_next();
 
+  int fills = 0, wq_fills = 0;  // the copy warp's
   if (warp == kCWarps) {
     // copy warp: per probe the two vectors (the first probe's are loaded directly),
     // slots 0 .. ns - 1, then every group's slots that did not stay in its ring
     // again.  Lane g counts group g's fills.
-    int fills = 0, pos = 0, wq_fills = 0;
+    int pos = 0;
     uint32_t par = 0;
     bool run = true;
     for (int64_t b = cluster; run && b < a.p; b += nclusters) {
@@ -176,14 +177,6 @@ __global__ void __launch_bounds__(kCThreads + 32, 2) arnoldi_step_kernel(const C
           }
         }
     }
-    // the last copies land (bounded) before this warp is done: a compute warp that gives up
-    // later leaves none in flight into shared memory that goes to another CTA
-    if (lane < kWC)
-      for (int f = fills > nslots ? fills - nslots : 0; f < fills; ++f)
-        mbar_wait_bounded(c_smem(&sh->full[lane * nslots + f % nslots]), (uint32_t)(f / nslots) & 1u, nullptr,
-                          kMbarWaitNs / 8);
-    if (lane == 0 && wq_fills > 0)
-      mbar_wait_bounded(c_smem(&sh->wq_full), (uint32_t)(wq_fills - 1) & 1u, nullptr, kMbarWaitNs / 8);
     if (S > 1) c_cluster_wait();
   } else {
     const int wr = warp % kWR, group = warp / kWR;
@@ -551,6 +544,17 @@ __global__ void __launch_bounds__(kCThreads + 32, 2) arnoldi_step_kernel(const C
   if (S > 1) {
     c_cluster_arrive_relaxed();
     c_cluster_wait();
+  } else {
+    __syncthreads();
+  }
+  if (warp == kCWarps && *fail) {
+    // every role is done; copies in flight land (bounded) before the shared memory goes away
+    if (lane < kWC)
+      for (int f = fills > nslots ? fills - nslots : 0; f < fills; ++f)
+        mbar_wait_bounded(c_smem(&sh->full[lane * nslots + f % nslots]), (uint32_t)(f / nslots) & 1u, nullptr,
+                          kMbarWaitNs / 8);
+    if (lane == 0 && wq_fills > 0)
+      mbar_wait_bounded(c_smem(&sh->wq_full), (uint32_t)(wq_fills - 1) & 1u, nullptr, kMbarWaitNs / 8);
   }
 }
 

@@ -556,9 +556,10 @@ dense_tcgen05_splitk_kernel(const __grid_constant__ CUtensorMap map_ahi,
   chain_wait();
   chain_next();
 
+  int issued = 0;  // slices asked for (thread 0's)
   if (warp == 0) {
     if (lane == 0) {
-      int issued = 0, s = 0;
+      int s = 0;
       uint32_t ph = 0;
       for (int kt = 0; kt < num_k; ++kt) {
         if (kt >= ahead) {
@@ -575,10 +576,6 @@ dense_tcgen05_splitk_kernel(const __grid_constant__ CUtensorMap map_ahi,
           ph ^= 1u;
         }
       }
-      // the last copies land (bounded) before this role is done, whichever role gives up and
-      // when; the slices fetched ahead are among them: no wait comes before their panel parts
-      for (int kt = (issued > stages ? issued - stages : 0); kt < issued; ++kt)
-        mbar_wait_bounded(smem_u32(&sh->full[kt % stages]), (uint32_t)(kt / stages) & 1u, nullptr, kMbarWaitNs / 8);
     }
   } else if (warp == 1) {
     if (lane == 0) {
@@ -637,6 +634,13 @@ dense_tcgen05_splitk_kernel(const __grid_constant__ CUtensorMap map_ahi,
   __syncwarp();
   tc_fence_before();
   cluster_sync_all();  // the S partial tiles are complete
+  if (threadIdx.x == 0 && *abort_flag) {
+    // every role is done; copies in flight land (bounded) before the shared memory goes away.
+    // The slices fetched ahead are among them: no wait comes before their panel parts
+    for (int kt = (issued > stages ? issued - stages : 0); kt < issued; ++kt)
+      mbar_wait_bounded(smem_u32(&sh->full[kt % stages]), (uint32_t)(kt / stages) & 1u, nullptr, kMbarWaitNs / 8);
+  }
+  __syncwarp();
   if (warp == 1) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tmem_cols)
