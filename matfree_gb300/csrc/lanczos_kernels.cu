@@ -1390,19 +1390,24 @@ cg_step_small_kernel(T *X, T *R, T *P, const T *W, int64_t ld, int64_t n, const 
   const bool active = run != 0;  // uniform over the CTA
   T rr = (T)0;
   if (active) {
-    T acc = (T)0;
+    // X is read only here: while the sum below meets, or, of eight elements a thread (no
+    // registers for them until then), after it
+    T acc = (T)0, xe[E];
+    auto load_x = [&] {
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        const int i = (int)threadIdx.x + e * kCgSmallThreads;
+        xe[e] = i < n ? x[i] : (T)0;
+      }
+    };
+    if constexpr (E <= 4) load_x();
 #pragma unroll
     for (int e = 0; e < E; ++e) acc = fma(pe[e], we[e], acc);
     const double pap = cta_sum_small<T>(acc, red);
     if (threadIdx.x == 0) coef = (T)(rsb / pap);
     __syncthreads();
     const T alpha = coef;
-    T xe[E];
-#pragma unroll
-    for (int e = 0; e < E; ++e) {  // X is read only here, before the stores
-      const int i = (int)threadIdx.x + e * kCgSmallThreads;
-      xe[e] = i < n ? x[i] : (T)0;
-    }
+    if constexpr (E > 4) load_x();
 #pragma unroll
     for (int e = 0; e < E; ++e) {
       const int i = (int)threadIdx.x + e * kCgSmallThreads;  // n <= kCgSmallMaxN
