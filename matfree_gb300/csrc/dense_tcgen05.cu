@@ -1049,11 +1049,8 @@ constexpr int kGemvRows = kGemvWarps / kGemvSeg;  // rows per CTA
 // kDeep: loads of two iterations ahead in flight instead of one (for one
 // probe, whose products are too few to cover the latency; with more probes
 // the deeper ring costs occupancy).
-// NR rows of a warp share the panel's values, loaded and widened once: two, but one for
-// one probe (the deeper ring serves it better).  A CG iteration of n = 8192, 2 probes 60.0
-// -> 55.4 us, 4 probes 81.5 -> 76.9, 8 probes 162 -> 165 (bound by the FMAs; n = 5000, 6
-// probes 56.7 -> 52.8); four rows: 58.4, 98.0, 190.  The sums are those of one row a warp.
-constexpr int gemv_warp_rows(int P) { return P > 1 ? 2 : 1; }
+// NR rows of a warp share the panel's values, loaded and widened once.  The sums are those
+// of one row a warp.
 
 template <int P, bool kSplit, bool kDeep, int NR>
 __device__ __forceinline__ void gemv_rows(const __nv_bfloat16 *__restrict__ Ahi,
@@ -1193,33 +1190,66 @@ dense_gemv1_kernel(const __nv_bfloat16 *__restrict__ Ahi, const __nv_bfloat16 *_
   gemv_rows<1, kSplit, true, 1>(Ahi, Alo, lda, Vhi, Vlo, ldvb, Vf, ldvf, W, ldw, n, p, shift, ahead);
 }
 
-template <int P, bool kSplit>
-__global__ void __launch_bounds__(32 * kGemvWarps, P == 8 ? 2 : 3)
+template <int P, bool kSplit, int NR>
+__global__ void __launch_bounds__(32 * kGemvWarps, NR == 1 ? (P == 8 ? 4 : 8) : (P == 8 ? 2 : 3))
 dense_gemv_kernel(const __nv_bfloat16 *__restrict__ Ahi, const __nv_bfloat16 *__restrict__ Alo,
-                  int64_t lda, const __nv_bfloat16 *Vhi,
-                  const __nv_bfloat16 *Vlo, int64_t ldvb,
-                  const float *Vf, int64_t ldvf, float *__restrict__ W, int64_t ldw,
-                  int n, int p, float shift, int ahead) {
-  gemv_rows<P, kSplit, false, gemv_warp_rows(P)>(Ahi, Alo, lda, Vhi, Vlo, ldvb, Vf, ldvf, W, ldw, n, p, shift, ahead);
+                  int64_t lda, const __nv_bfloat16 *Vhi, const __nv_bfloat16 *Vlo, int64_t ldvb,
+                  const float *Vf, int64_t ldvf, float *__restrict__ W, int64_t ldw, int n, int p,
+                  float shift, int ahead) {
+  gemv_rows<P, kSplit, false, NR>(Ahi, Alo, lda, Vhi, Vlo, ldvb, Vf, ldvf, W, ldw, n, p, shift, ahead);
 }
 
 // CTAs that fetch their rows ahead when chained: those resident at first, up to 48 MB
 constexpr int64_t kGemvAheadBytes = 48 << 20;
 
-template <int P>
-static int launch_gemv_p(bool split, const __nv_bfloat16 *A_hi, const __nv_bfloat16 *A_lo,
-                         int64_t lda, const __nv_bfloat16 *V_hi, const __nv_bfloat16 *V_lo,
-                         int64_t ldvb, const float *Vf, int64_t ldvf, float *W, int64_t ldw,
-                         int n, int p, float shift, bool chained, cudaStream_t s) {
-  constexpr int kRowsPerCta = kGemvRows * gemv_warp_rows(P);
-  auto kern = split ? dense_gemv_kernel<P, true> : dense_gemv_kernel<P, false>;
-  if constexpr (P == 1) kern = split ? dense_gemv1_kernel<true> : dense_gemv1_kernel<false>;
+// Two rows of a warp, but one for one probe (the deeper ring serves it better) and, for
+// operators well beyond L2, for the two forms that lose by it there: 2 probes of a plain
+// operator, where a row a warp keeps more of the operator under way (eight CTAs an SM), and 5
+// to 8 of a split one, bound by the FMAs.  Product, one row -> two, us: 2 probes, plain, n =
+// 8192 42.0 -> 38.7, 10000 51.1 -> 54.9, 16384 101 -> 107, 23170 193 -> 213; split, 5 probes 10000 166
+// -> 154, 12000 258 -> 262, 23170 846 -> 884, 6 probes 8192 121 -> 109, 12000 282 -> 288, 23170 978
+// -> 1010, 8 probes 8192 178 -> 176, 23170 1237 -> 1254.  The others gain at every size: 4 probes,
+// split, 8192 86.0 -> 82.3, 23170 696 -> 554; 8, plain, 23170 671 -> 661.  Four rows, a CG iteration of n
+// = 8192, split, 2, 4 and 8 probes 58.4, 98.0, 190 (two: 55.4, 76.9, 165).
+constexpr int gemv_two_rows_n(bool split) { return split ? 11000 : 9000; }
+
+template <int P, bool kSplit, int NR>
+static int launch_gemv_rows(const __nv_bfloat16 *A_hi, const __nv_bfloat16 *A_lo, int64_t lda,
+                            const __nv_bfloat16 *V_hi, const __nv_bfloat16 *V_lo, int64_t ldvb,
+                            const float *Vf, int64_t ldvf, float *W, int64_t ldw, int n, int p,
+                            float shift, bool chained, cudaStream_t s) {
+  constexpr int kRowsPerCta = kGemvRows * NR;
+  auto kern = [] {
+    if constexpr (P == 1) return &dense_gemv1_kernel<kSplit>;
+    else return &dense_gemv_kernel<P, kSplit, NR>;
+  }();
   const unsigned grid = (unsigned)((n + kRowsPerCta - 1) / kRowsPerCta);
-  const int64_t fit = kGemvAheadBytes / ((int64_t)kRowsPerCta * n * (split ? 4 : 2)), resident = (P == 1 ? 5 : 3) * 152;
-  const int ahead = !chained ? 0 : (int)(fit < resident ? fit : resident);
+  int ahead = 0;
+  if (chained) {
+    static PerDevice<int> table;
+    const int *resident = table.get(current_device(), [&](int &q) {
+      const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&q, kern, 32 * kGemvWarps, 0);
+      q *= sm_count();
+      return e == cudaSuccess;
+    });
+    const int64_t fit = kGemvAheadBytes / ((int64_t)kRowsPerCta * n * (kSplit ? 4 : 2));
+    if (resident) ahead = (int)(fit < *resident ? fit : *resident);
+  }
   MFG_CUDA_TRY(launch_kernel(kern, dim3(grid), 32 * kGemvWarps, 0, 0, chained, s, A_hi, A_lo, lda, V_hi, V_lo, ldvb,
                              Vf, ldvf, W, ldw, n, p, shift, ahead));
   return MFG_LAUNCH_STATUS();
+}
+
+template <int P, typename... A>
+static int launch_gemv_p(bool split, int n, A... args) {
+  if constexpr (P == 1)
+    return split ? launch_gemv_rows<1, true, 1>(args...) : launch_gemv_rows<1, false, 1>(args...);
+  if constexpr (P == 2)
+    if (!split && n > gemv_two_rows_n(false)) return launch_gemv_rows<2, false, 1>(args...);
+  if constexpr (P == 8)
+    if (split && n > gemv_two_rows_n(true)) return launch_gemv_rows<8, true, 1>(args...);
+  if constexpr (P > 1)
+    return split ? launch_gemv_rows<P, true, 2>(args...) : launch_gemv_rows<P, false, 2>(args...);
 }
 
 constexpr int64_t kGemvMaxP = 8;
@@ -1232,12 +1262,12 @@ static int launch_dense_gemv(const __nv_bfloat16 *A_hi, const __nv_bfloat16 *A_l
   const int ni = (int)n, pi = (int)p;
   const float sh = (float)shift;
   if (p == 1)
-    return launch_gemv_p<1>(split, A_hi, A_lo, lda, V_hi, V_lo, ldvb, Vf, ldvf, W, ldw, ni, pi, sh, chained, s);
+    return launch_gemv_p<1>(split, ni, A_hi, A_lo, lda, V_hi, V_lo, ldvb, Vf, ldvf, W, ldw, ni, pi, sh, chained, s);
   if (p == 2)
-    return launch_gemv_p<2>(split, A_hi, A_lo, lda, V_hi, V_lo, ldvb, Vf, ldvf, W, ldw, ni, pi, sh, chained, s);
+    return launch_gemv_p<2>(split, ni, A_hi, A_lo, lda, V_hi, V_lo, ldvb, Vf, ldvf, W, ldw, ni, pi, sh, chained, s);
   if (p <= 4)
-    return launch_gemv_p<4>(split, A_hi, A_lo, lda, V_hi, V_lo, ldvb, Vf, ldvf, W, ldw, ni, pi, sh, chained, s);
-  return launch_gemv_p<8>(split, A_hi, A_lo, lda, V_hi, V_lo, ldvb, Vf, ldvf, W, ldw, ni, pi, sh, chained, s);
+    return launch_gemv_p<4>(split, ni, A_hi, A_lo, lda, V_hi, V_lo, ldvb, Vf, ldvf, W, ldw, ni, pi, sh, chained, s);
+  return launch_gemv_p<8>(split, ni, A_hi, A_lo, lda, V_hi, V_lo, ldvb, Vf, ldvf, W, ldw, ni, pi, sh, chained, s);
 }
 
 // ---------------------------------------------------------------------------
