@@ -1362,12 +1362,17 @@ struct SplitKSlots {
 // Dynamic shared memory that the split-K kernels are allowed, whatever a launch takes of it.
 constexpr int kSplitKSmem = 1024 + (int)kSplitKRing + (int)sizeof(GemmShared);
 
-static SplitKSlots splitk_slots() {
+// The current device's, the kernels prepared for it.
+static const SplitKSlots &splitk_slots() {
   static PerDevice<SplitKSlots> table;
-  const int sms = sm_count();
-  auto fill = [&](SplitKSlots &t) {
+  auto fill = [](SplitKSlots &t) {
+    const int sms = sm_count();
     auto kern = dense_tcgen05_splitk_kernel<true, 1>;
-    bool ok = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSplitKSmem) == cudaSuccess;
+    // the kernels' limit, the same for all launches: no thread lowers it under another's
+    bool ok = true;
+    for (auto f : {kern, dense_tcgen05_splitk_kernel<true, 2>, dense_tcgen05_splitk_kernel<false, 1>,
+                   dense_tcgen05_splitk_kernel<false, 2>})
+      ok &= cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kSplitKSmem) == cudaSuccess;
     t.cta[0] = sms;
     for (int S = 1; S <= kSplitKMaxS; ++S) {
       cudaLaunchConfig_t cfg = {};
@@ -1382,7 +1387,7 @@ static SplitKSlots splitk_slots() {
       cfg.numAttrs = 1;
       int clusters = 0;
       if (!ok || cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) != cudaSuccess || clusters < 1) {
-        ok = false;
+        ok = false;  // asked again by the next launch
         clusters = sms / S > 0 ? sms / S : 1;
       }
       t.cta[S] = clusters * S;
@@ -1391,7 +1396,7 @@ static SplitKSlots splitk_slots() {
     return ok;
   };
   if (const SplitKSlots *t = table.get(current_device(), fill)) return *t;
-  SplitKSlots t;  // counts that could not be asked, for this call only
+  static thread_local SplitKSlots t;  // counts that could not be asked, for this call only
   fill(t);
   return t;
 }
@@ -1411,7 +1416,7 @@ struct SplitKPlan {
 // (55 us; S = 4 of two: 60), n = 5000, 48 probes S = 3 (20 us; S = 1: 46, S = 4: 30, a
 // second round), n = 512 S = 8 (4 us; S = 1: 7).
 static SplitKPlan splitk_plan(int64_t n, int64_t p, bool split) {
-  const SplitKSlots slots = splitk_slots();
+  const SplitKSlots &slots = splitk_slots();
   const int64_t tiles_p = ceil_div(p, kSplitKMaxBN);
   SplitKPlan best{(int)(ceil_div(ceil_div(p, tiles_p), 16) * 16), 1, 1};
   const int64_t slices = ceil_div(n, kSplitKBK);
@@ -1470,8 +1475,6 @@ static int launch_splitk(const __nv_bfloat16 *A_hi, const __nv_bfloat16 *A_lo, i
   const int vec_ok = ldw % 4 == 0 && ldvf % 4 == 0 && ((uintptr_t)W & 15) == 0 && ((uintptr_t)Vf & 15) == 0;
   auto kern = mt == 2 ? (split ? dense_tcgen05_splitk_kernel<true, 2> : dense_tcgen05_splitk_kernel<false, 2>)
                       : (split ? dense_tcgen05_splitk_kernel<true, 1> : dense_tcgen05_splitk_kernel<false, 1>);
-  // the same limit in every launch: another thread's smaller product must not lower it under this one
-  MFG_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSplitKSmem));
   MFG_CUDA_TRY(launch_kernel(kern, dim3((unsigned)S, (unsigned)ceil_div(n, rows), (unsigned)ceil_div(p, bn)),
                              kGemmThreads, smem, (unsigned)S, chained, s, mahi, malo, mbhi, mblo, Vf, ldvf, W, ldw,
                              (int)n, (int)p, bn, stages, cols, (float)shift, vec_ok, status));
@@ -1497,16 +1500,16 @@ int launch_dense_tcgen05(const __nv_bfloat16 *A_hi, const __nv_bfloat16 *A_lo, i
   // per probe tile there, which pays while the tiles (of one K range) cover
   // up to 5/9 of the SMs (256 probes: n = 5000 52 against 71 us for CTA pairs;
   // n = 6144 73 against 66).  Rules of the autotuner name CTA-pair forms.
-  const int sms = sm_count();
   const bool pair_rule = (rule.split != 0 || rule.bn != 0) && p >= 64;
   const int64_t row_tiles = ceil_div(n, kBM);
   if (!pair_rule && (n < kPairMinRows || p <= kSplitKMaxBN ||
-                     row_tiles * ceil_div(p, kSplitKMaxBN) * 9 <= (int64_t)sms * 5)) {
+                     row_tiles * ceil_div(p, kSplitKMaxBN) * 9 <= (int64_t)sm_count() * 5)) {
     const SplitKPlan plan = splitk_plan(n, p, split);
     return launch_splitk(A_hi, A_lo, lda, V_hi, V_lo, ldvb, Vf, ldvf, W, ldw, n, p, plan, shift, status,
                          chained, s);
   }
   // CTA pairs (2-SM MMAs, M = 256); probes per tile: a multiple of 32 in [64, 256]
+  const int sms = sm_count();
   const int64_t pt = p < 256 ? p : 256;
   int BN = (int)((pt + 31) / 32 * 32);
   if (rule.bn > 0 && rule.bn < BN) BN = rule.bn;  // a narrower probe tile: more tiles per operator
