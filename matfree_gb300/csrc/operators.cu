@@ -243,6 +243,68 @@ dense_f64_kernel(const double *__restrict__ A, int64_t lda, const double *__rest
   d_reduce_store<double, M, kF64P, M, 128>(stages, V, ldv, W, ldw, n, p, m0, b0, rank, S, shift);
 }
 
+// The same product by FMA instructions: a CTA of 256 threads forms a tile of 32 rows x 32
+// probes over all of K, a thread 2 x 2 of it, both operands k-major in shared memory and the
+// next 16 columns on their way in registers.  An SM runs 1.94 FMAs a clock so, against 1.76
+// as MMAs, but a tile is a CTA: the last round of them costs as much as a full one (n =
+// 1000: 278 us for up to 152 tiles, 532 for up to 304).  Bound by the float64 pipe.
+constexpr int kF64Tile = 32, kF64Cols = 16;
+
+__global__ void __launch_bounds__(256)
+dense_f64_fma_kernel(const double *__restrict__ A, int64_t lda, const double *__restrict__ V, int64_t ldv,
+                     double *__restrict__ W, int64_t ldw, int64_t n, int64_t p, double shift) {
+  constexpr int B = kF64Tile, BK = kF64Cols;
+  __shared__ __align__(16) double As[BK][B], Vs[BK][B];
+  static_assert(B * BK == 2 * 256, "a 16-byte load of each operand per thread");
+  const int t = threadIdx.x, tx = t % (B / 2), ty = t / (B / 2);
+  const int64_t m0 = (int64_t)blockIdx.x * B, b0 = (int64_t)blockIdx.y * B;
+  const int row = t / (BK / 2), kq = t % (BK / 2) * 2;  // this thread's load: two columns of a row
+  double ra[2], rv[2];
+  auto load = [&](const double *__restrict__ X, int64_t ldx, int64_t r, int64_t rows, int64_t k, double(&x)[2]) {
+    x[0] = x[1] = 0.0;
+    if (r >= rows) return;
+    if (k + 2 <= n) {
+      const double2 u = __ldg(reinterpret_cast<const double2 *>(X + r * ldx + k));
+      x[0] = u.x;
+      x[1] = u.y;
+    } else if (k < n) {
+      x[0] = X[r * ldx + k];
+    }
+  };
+  double acc[2][2] = {};
+  load(A, lda, m0 + row, n, kq, ra);
+  load(V, ldv, b0 + row, p, kq, rv);
+  for (int64_t k0 = 0; k0 < n; k0 += BK) {
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      As[kq + u][row] = ra[u];
+      Vs[kq + u][row] = rv[u];
+    }
+    __syncthreads();
+    if (k0 + BK < n) {
+      load(A, lda, m0 + row, n, k0 + BK + kq, ra);
+      load(V, ldv, b0 + row, p, k0 + BK + kq, rv);
+    }
+#pragma unroll
+    for (int kk = 0; kk < BK; ++kk) {
+      const double2 a = *reinterpret_cast<const double2 *>(&As[kk][tx * 2]);
+      const double2 v = *reinterpret_cast<const double2 *>(&Vs[kk][ty * 2]);
+      acc[0][0] = fma(a.x, v.x, acc[0][0]);
+      acc[0][1] = fma(a.x, v.y, acc[0][1]);
+      acc[1][0] = fma(a.y, v.x, acc[1][0]);
+      acc[1][1] = fma(a.y, v.y, acc[1][1]);
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int64_t m = m0 + tx * 2 + i, b = b0 + ty * 2 + j;
+      if (m < n && b < p) W[b * ldw + m] = fma(shift, __ldg(V + b * ldv + m), acc[i][j]);
+    }
+}
+
 template <typename K, typename T>
 static int launch_dense_cluster(K kern, int bm, int bp, int threads, size_t smem, int S, const T *A, int64_t lda,
                                 const T *V, int64_t ldv, T *W, int64_t ldw, int64_t n, int64_t p, T shift,
@@ -275,6 +337,9 @@ static int launch_f32(int S, const float *A, int64_t lda, const float *V, int64_
                               ldv, W, ldw, n, p, shift, s);
 }
 
+// SMs of 152 that clusters of S CTAs fill
+constexpr int kFit[kDMaxS + 1] = {0, 152, 152, 138, 148, 140, 138, 105, 144};
+
 template <typename T>
 int launch_dense_simt(const T *A, int64_t lda, const T *V, int64_t ldv, T *W, int64_t ldw,
                       int64_t n, int64_t p, double shift, cudaStream_t s) {
@@ -297,6 +362,22 @@ int launch_dense_simt(const T *A, int64_t lda, const T *V, int64_t ldv, T *W, in
         S = c;
       }
     }
+    // FMA tiles where they fill their rounds and the MMAs' CTAs do not, both counted in the FMAs
+    // of an SM at 1.76 a clock, rows and probes in MMAs of eight.  The MMAs' CTAs share an SM
+    // five at a time; with a few more the first SMs to be done take five again (1.28), and many
+    // even out (1.11, 1.05).  MMAs -> FMAs, us: n = 1000, 128 probes 410 -> 279 (100 probes: 239,
+    // 279), 1200, 512 1642 -> 1237, 2000, 64 675 -> 546 (48: 448, 545), 4096, 256 8739 -> 7239.  Over 323
+    // sizes (200 <= n <= 4096, p <= 1000) the choice is within 3 % of the faster one but for two (10 %).
+    const double ctas = (double)(tiles * S * 152) / ((double)kFit[S] * sms);
+    const double q = ctas <= 5.0 ? ceil(ctas) / ctas : (ctas < 10.0 ? 1.28 : (ctas < 30.0 ? 1.11 : 1.05));
+    const double mma = 64.0 * (double)ceil_div(n, 8) * (double)ceil_div(p, 8) * q;
+    const int64_t fx = ceil_div(n, kF64Tile), fy = ceil_div(p, kF64Tile);
+    const double rounds = (double)ceil_div(fx * fy, sms);
+    if (mma > (double)sms * kF64Tile * kF64Tile * (0.82 * rounds + 0.06)) {
+      if (fy > 65535) return MFG_ERR_UNSUPPORTED;
+      dense_f64_fma_kernel<<<dim3((unsigned)fx, (unsigned)fy), 256, 0, s>>>(A, lda, V, ldv, W, ldw, n, p, shift);
+      return MFG_LAUNCH_STATUS();
+    }
     const size_t smem = (size_t)kDStages * (kF64M + kF64P) * (kF64K + 2) * sizeof(double);
     return launch_dense_cluster(dense_f64_kernel, kF64M, kF64P, 128, smem, S, A, lda, V, ldv, W, ldw, n, p, shift, s);
   } else {
@@ -304,7 +385,6 @@ int launch_dense_simt(const T *A, int64_t lda, const T *V, int64_t ldv, T *W, in
     // CTAs of the busiest SM (clusters of three to eight leave SMs of a GPC over) times the
     // slices of one; a range more is a tile more to add.  n = 2000, 64 probes S = 8 22.8 us (4:
     // 24.8, 5: 33.0); n = 3001, 64 S = 5 45 (4: 55, 6: 56, 8: 48); n = 4096, 256 S = 4 228 (2: 258).
-    static const int kFit[kDMaxS + 1] = {0, 152, 152, 138, 148, 140, 138, 105, 144};  // SMs of clusters of S
     const int bp = p <= 32 ? 32 : 64;
     const int64_t tiles = ceil_div(n, 64) * ceil_div(p, bp), slices = ceil_div(n, 64);
     int S = 1;
