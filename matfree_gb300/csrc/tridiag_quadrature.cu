@@ -365,6 +365,13 @@ __device__ __forceinline__ double rcp_nr(double x) {
   return fma(y, fma(e, e, e), y);
 }
 
+// 1/x to some 2^-20
+__device__ __forceinline__ double rcp_rough(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  return y;
+}
+
 // 1 / rho of a coupling, which may be as small as the whole problem's scale
 __device__ __forceinline__ double rcp_any(double x) { return x > 1e-290 ? rcp_nr(x) : 1.0 / x; }
 
@@ -614,9 +621,15 @@ __device__ bool dc_secular_root(const double *P, const double *ZZ, const float2 
       hi = x;
     else
       lo = x;
-    // |f| within the rounding of its terms
+    // |f| within the rounding of its terms: a Newton step is the last.  From a float32 start x
+    // may still be mk times that rounding off: without the step the eigenvalues' errors were up to
+    // three times those of a float64 start (k = 24: rms 2.8e-16 of the spectral radius, 8.3e-17;
+    // with it 6.3e-17).  Quadrature of k = 16, 32 problems 72.4 -> 72.6 us, 100, 64 396 -> 400.
     const double mag = (ir + (above - below)) + (fabs(t0) + fabs(t1));
     if (!less_than(eps_mk * mag, fabs(f))) {
+      const double fp = fma(t1 * t1, rcp_rough(w1), fma(t0 * t0, rcp_rough(w0), slope));
+      const double xn = fma(-f, rcp_rough(fp), x);
+      if (less_than(lo, xn) && less_than(xn, hi)) x = xn;  // not a NaN step
       conv = true;
       break;
     }
