@@ -615,15 +615,25 @@ __global__ void arnoldi_h_kernel(double *H, const double *Hh, const double *rec,
   const int i = threadIdx.x % rows, quarter = threadIdx.x / rows;
   double hlast = i == 0 ? qw[0] : 0.0;  // H[i][j - 1] (quarter 0)
   if (threadIdx.x == 0) Hb[0] = qw[0];
+  // the raw values of step j, read a step ahead
+  double hraw = 0.0, traw = 0.0;
+  auto fetch = [&](int j) {
+    if (quarter == 0 && i < j && j < k) {
+      hraw = h_raw(raw + (int64_t)(j - 1) * ld + i);
+      traw = h_raw(Hb + (int64_t)i * k + j);
+    }
+  };
+  fetch(1);
   for (int j = 1; j < k; ++j) {
     const double nuj = nu[j], bj = beta[j];
     double top = 0.0;
     if (quarter == 0 && i <= j) {
-      const double h = i < j ? h_raw(raw + (int64_t)(j - 1) * ld + i) : 0.0;
+      const double h = i < j ? hraw : 0.0;
       if (i < j) hq[i] = h;
       hs[(size_t)(j - 1) * ld + i] = i < j ? hlast + nuj * h : bj;
-      top = i < j ? h_raw(Hb + (int64_t)i * k + j) : qw[j];
+      top = i < j ? traw : qw[j];
     }
+    fetch(j + 1);
     __syncthreads();
     if (i <= j) {
       // columns max(i - 1, 0) .. j - 1 of row i, a quarter of them
