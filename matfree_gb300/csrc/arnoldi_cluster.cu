@@ -128,12 +128,11 @@ __global__ void __launch_bounds__(kCThreads + 32, 2) arnoldi_step_kernel(const C
   chain_wait();
   chain_next();
 
-  int fills = 0, wq_fills = 0;  // the copy warp's
   if (warp == kCWarps) {
     // copy warp: per probe the two vectors (the first probe's are loaded directly),
     // slots 0 .. ns - 1, then every group's slots that did not stay in its ring
     // again.  Lane g counts group g's fills.
-    int pos = 0;
+    int fills = 0, pos = 0, wq_fills = 0;
     uint32_t par = 0;
     bool run = true;
     for (int64_t b = cluster; run && b < a.p; b += nclusters) {
@@ -178,6 +177,16 @@ __global__ void __launch_bounds__(kCThreads + 32, 2) arnoldi_step_kernel(const C
         }
     }
     if (S > 1) c_cluster_wait();
+    c_done(S);
+    if (*fail) {
+      // copies in flight land (bounded) before the shared memory goes away
+      if (lane < kWC)
+        for (int f = fills > nslots ? fills - nslots : 0; f < fills; ++f)
+          mbar_wait_bounded(c_smem(&sh->full[lane * nslots + f % nslots]), (uint32_t)(f / nslots) & 1u, nullptr,
+                            kMbarWaitNs / 8);
+      if (lane == 0 && wq_fills > 0)
+        mbar_wait_bounded(c_smem(&sh->wq_full), (uint32_t)(wq_fills - 1) & 1u, nullptr, kMbarWaitNs / 8);
+    }
   } else {
     const int wr = warp % kWR, group = warp / kWR;
     const int row = wr * kCRows + lane * 4;  // rows row .. row + 3 and row + 128 .. row + 131
@@ -208,10 +217,9 @@ __global__ void __launch_bounds__(kCThreads + 32, 2) arnoldi_step_kernel(const C
             if (row + (e < 4 ? e : 124 + e) >= nloc) x[e] = 0.f;  // a panel's padding is not data
         };
         if (b == cluster) {  // a read of L2 is shorter than a copy's round trip
-          const float4 *gw = reinterpret_cast<const float4 *>(a.W + b * a.ld + r0 + row);
-          const float4 *gq = reinterpret_cast<const float4 *>(a.Vin + b * a.vb + r0 + row);
+          const float *gw = a.W + b * a.ld + r0 + row, *gq = a.Vin + b * a.vb + r0 + row;
           const float4 w0 = ok0 ? c_ld_l2(gw) : zero4, q0 = ok0 ? c_ld_l2(gq) : zero4;
-          const float4 w1 = ok1 ? c_ld_l2(gw + 32) : zero4, q1 = ok1 ? c_ld_l2(gq + 32) : zero4;
+          const float4 w1 = ok1 ? c_ld_l2(gw + 128) : zero4, q1 = ok1 ? c_ld_l2(gq + 128) : zero4;
           take(w0, w1, w);
           take(q0, q1, q);
         } else {
@@ -539,22 +547,7 @@ __global__ void __launch_bounds__(kCThreads + 32, 2) arnoldi_step_kernel(const C
         }
       }
     }
-  }
-  // no CTA leaves while the others may read its sums or arrive on its barriers
-  if (S > 1) {
-    c_cluster_arrive_relaxed();
-    c_cluster_wait();
-  } else {
-    __syncthreads();
-  }
-  if (warp == kCWarps && *fail) {
-    // every role is done; copies in flight land (bounded) before the shared memory goes away
-    if (lane < kWC)
-      for (int f = fills > nslots ? fills - nslots : 0; f < fills; ++f)
-        mbar_wait_bounded(c_smem(&sh->full[lane * nslots + f % nslots]), (uint32_t)(f / nslots) & 1u, nullptr,
-                          kMbarWaitNs / 8);
-    if (lane == 0 && wq_fills > 0)
-      mbar_wait_bounded(c_smem(&sh->wq_full), (uint32_t)(wq_fills - 1) & 1u, nullptr, kMbarWaitNs / 8);
+    c_done(S);
   }
 }
 

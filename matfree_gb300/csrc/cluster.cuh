@@ -36,7 +36,7 @@ __device__ __forceinline__ double c_ld_f64(uint32_t addr) {
 }
 
 // from L2, in program order with the waits
-__device__ __forceinline__ float4 c_ld_l2(const float4 *p) {
+__device__ __forceinline__ float4 c_ld_l2(const float *p) {
   float4 v;
   asm volatile("ld.global.cg.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
   return v;
@@ -76,6 +76,18 @@ __device__ __forceinline__ void c_cluster_arrive() {
 __device__ __forceinline__ void c_cluster_wait() {
   asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
   __syncwarp();
+}
+
+// The end of a CTA's work, by every warp: the cluster's CTAs have read each other's sums, and
+// every role of this CTA is done.
+__device__ __forceinline__ void c_done(int S) {
+  if (S > 1) {
+    c_cluster_arrive_relaxed();
+    c_cluster_wait();
+  } else {
+    __syncwarp();
+    asm volatile("barrier.sync 2, %0;" ::"n"(kCThreads + 32) : "memory");
+  }
 }
 
 // s + e += x, exactly up to the rounding of e

@@ -432,10 +432,32 @@ template <int S> struct Ranks { static constexpr int value = S; };
 // time, so that U S reads of other CTAs' shared memory (some 1500 cycles each) and
 // the shift's reads are under way together: one by one they took 11 of the 62 us of
 // n = 8192, 128 probes.
+// The shift's probe values for column i of this CTA's share (zero past its end)
+template <int MT>
+__device__ __forceinline__ float4 splitk_shift(int i, int c0, int items, int b0, int m0, int n, int p, const float *Vf,
+                                               int64_t ldvf, float shift, int vec_ok) {
+  const int b = b0 + c0 + i / MT, m = m0 + i % MT * kBM + (int)(threadIdx.x & 31) * 4;
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (i < items && b < p && m < n && shift != 0.f) {
+    const float *vf = Vf + (int64_t)b * ldvf + m;
+    if (vec_ok && m + 4 <= n) {
+      v = *reinterpret_cast<const float4 *>(vf);
+    } else {
+      v.x = vf[0];
+      if (m + 1 < n) v.y = vf[1];
+      if (m + 2 < n) v.z = vf[2];
+      if (m + 3 < n) v.w = vf[3];
+    }
+  }
+  return v;
+}
+
+constexpr int kSplitKAhead = 2;  // columns a warp whose shift values are read before the cluster meets
+
 template <int S, int MT>
 __device__ __forceinline__ void splitk_reduce(uint32_t base, int c0, int items, int b0, int m0, int n, int p,
                                               const float *Vf, int64_t ldvf, float *__restrict__ W,
-                                              int64_t ldw, float shift, int vec_ok) {
+                                              int64_t ldw, float shift, int vec_ok, const float4 (&ahead)[kSplitKAhead]) {
   constexpr int U = S <= 2 ? 8 : (S <= 4 ? 4 : 2), kStep = kGemmThreads / 32;
   const int lane = threadIdx.x & 31;
   for (int i0 = threadIdx.x >> 5; i0 < items; i0 += U * kStep) {
@@ -449,18 +471,9 @@ __device__ __forceinline__ void splitk_reduce(uint32_t base, int c0, int items, 
       for (int r = 0; r < S; ++r)
         x[u][r] = live ? ld_dsmem_f4(map_to_rank(base + (uint32_t)(c * MT + t) * (kBM * 4u), (uint32_t)r))
                        : make_float4(0.f, 0.f, 0.f, 0.f);
-      sv[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (live && shift != 0.f) {
-        const float *vf = Vf + (int64_t)b * ldvf + m;
-        if (vec_ok && m + 4 <= n) {
-          sv[u] = *reinterpret_cast<const float4 *>(vf);
-        } else {
-          sv[u].x = vf[0];
-          if (m + 1 < n) sv[u].y = vf[1];
-          if (m + 2 < n) sv[u].z = vf[2];
-          if (m + 3 < n) sv[u].w = vf[3];
-        }
-      }
+      sv[u] = u < kSplitKAhead && i0 < kStep
+                  ? ahead[u < kSplitKAhead ? u : 0]
+                  : splitk_shift<MT>(i, c0, items, b0, m0, n, p, Vf, ldvf, shift, vec_ok);
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
@@ -555,6 +568,15 @@ dense_tcgen05_splitk_kernel(const __grid_constant__ CUtensorMap map_ahi,
   __syncwarp();
   chain_wait();
   chain_next();
+  // this CTA's columns [c0, c1) of the tile; a warp takes whole columns, a
+  // lane four consecutive rows
+  const int c0 = BN * part / S, items = MT * (BN * (part + 1) / S - c0);
+  float4 shifts[kSplitKAhead];
+  auto load_shifts = [&] {
+#pragma unroll
+    for (int u = 0; u < kSplitKAhead; ++u)
+      shifts[u] = splitk_shift<MT>(warp + u * (kGemmThreads / 32), c0, items, b0, m0, n, p, Vf, ldvf, shift, vec_ok);
+  };
 
   int issued = 0;  // slices asked for (thread 0's)
   if (warp == 0) {
@@ -616,6 +638,7 @@ dense_tcgen05_splitk_kernel(const __grid_constant__ CUtensorMap map_ahi,
     // CTA's shared memory, probe-major (32 lanes write 32 consecutive rows).
     // Every copy has landed and every MMA has read its stage once tmem_full
     // completes, so the ring may be overwritten.
+    load_shifts();
     const int quarter = warp & 3;
     float *dst = reinterpret_cast<float *>(tiles) + quarter * 32 + lane;
     const bool ok = __all_sync(0xffffffffu, mbar_wait<true>(&sh->tmem_full, 0, abort_flag, status));
@@ -631,27 +654,18 @@ dense_tcgen05_splitk_kernel(const __grid_constant__ CUtensorMap map_ahi,
         }
     }
   }
+  if (warp < 2) load_shifts();
   __syncwarp();
   tc_fence_before();
   cluster_sync_all();  // the S partial tiles are complete
-  if (threadIdx.x == 0 && *abort_flag) {
-    // every role is done; copies in flight land (bounded) before the shared memory goes away.
-    // The slices fetched ahead are among them: no wait comes before their panel parts
-    for (int kt = (issued > stages ? issued - stages : 0); kt < issued; ++kt)
-      mbar_wait_bounded(smem_u32(&sh->full[kt % stages]), (uint32_t)(kt / stages) & 1u, nullptr, kMbarWaitNs / 8);
-  }
-  __syncwarp();
   if (warp == 1) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tmem_cols)
                  : "memory");
   }
-  // this CTA's columns [c0, c1) of the tile; a warp takes whole columns, a
-  // lane four consecutive rows
-  const int c0 = BN * part / S, items = MT * (BN * (part + 1) / S - c0);
   const uint32_t base = smem_u32(tiles) + (uint32_t)lane * 16u;
   auto reduce = [&](auto s) {
-    splitk_reduce<decltype(s)::value, MT>(base, c0, items, b0, m0, n, p, Vf, ldvf, W, ldw, shift, vec_ok);
+    splitk_reduce<decltype(s)::value, MT>(base, c0, items, b0, m0, n, p, Vf, ldvf, W, ldw, shift, vec_ok, shifts);
   };
   static_assert(kSplitKMaxS == 8, "cases below");
   switch (S) {
@@ -666,6 +680,12 @@ dense_tcgen05_splitk_kernel(const __grid_constant__ CUtensorMap map_ahi,
   }
   __syncwarp();
   cluster_sync_relaxed();  // no CTA leaves while the others may read its partial tile
+  if (threadIdx.x == 0 && *abort_flag) {
+    // every role is done; copies in flight land (bounded) before the shared memory goes away.
+    // The slices fetched ahead are among them: no wait comes before their panel parts
+    for (int kt = (issued > stages ? issued - stages : 0); kt < issued; ++kt)
+      mbar_wait_bounded(smem_u32(&sh->full[kt % stages]), (uint32_t)(kt / stages) & 1u, nullptr, kMbarWaitNs / 8);
+  }
 }
 
 // ---------------------------------------------------------------------------

@@ -172,12 +172,11 @@ __global__ void __launch_bounds__(kCThreads + 32, 2) gs_cluster_kernel(const GsA
   chain_wait();
   chain_next();
 
-  int fills = 0;  // the copy warp's, lane g: group g
   if (warp == kCWarps) {
     // copy warp: per probe the vectors after idx, then pass 1's slots, then of each
     // later pass the slots that did not stay.  Pass t takes a group's slots in the
     // order rotated by (t - 1)(slots - kept): those that stayed come first.
-    int pos = 0;  // lane g: group g
+    int fills = 0, pos = 0;  // lane g: group g
     uint32_t par = 0;
     bool run = true;
     auto fill = [&](int g, int s, bool extra, int64_t b) {
@@ -218,6 +217,13 @@ __global__ void __launch_bounds__(kCThreads + 32, 2) gs_cluster_kernel(const GsA
           }
     }
     if (S > 1) c_cluster_wait();
+    c_done(S);
+    if (*fail && lane < kWC) {
+      // copies in flight land (bounded) before the shared memory goes away
+      for (int f = fills > nslots ? fills - nslots : 0; f < fills; ++f)
+        mbar_wait_bounded(c_smem(&sh->full[lane * nslots + f % nslots]), (uint32_t)(f / nslots) & 1u, nullptr,
+                          kMbarWaitNs / 8);
+    }
   } else {
     const int wr = warp % kWR, group = warp / kWR;
     int rv[NV];  // first rows of this lane's 16-byte vectors
@@ -550,19 +556,7 @@ __global__ void __launch_bounds__(kCThreads + 32, 2) gs_cluster_kernel(const GsA
         }
       }
     }
-  }
-  // no CTA leaves while the others may read its sums or arrive on its barriers
-  if (S > 1) {
-    c_cluster_arrive_relaxed();
-    c_cluster_wait();
-  } else {
-    __syncthreads();
-  }
-  if (warp == kCWarps && *fail && lane < kWC) {
-    // every role is done; copies in flight land (bounded) before the shared memory goes away
-    for (int f = fills > nslots ? fills - nslots : 0; f < fills; ++f)
-      mbar_wait_bounded(c_smem(&sh->full[lane * nslots + f % nslots]), (uint32_t)(f / nslots) & 1u, nullptr,
-                        kMbarWaitNs / 8);
+    c_done(S);
   }
 }
 

@@ -14,7 +14,7 @@ CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
 OPERATOR = {"Ahi", "Alo"}
 OUTPUT = {"W", "values", "eigvals", "first_sq", "status", "nu_last_inv"}
 # device functions that are given the pointers of a chained kernel
-SHARED = {"gemv_rows", "splitk_reduce", "h_scalars"}
+SHARED = {"gemv_rows", "splitk_reduce", "splitk_shift", "h_scalars"}
 
 
 def _functions(src):

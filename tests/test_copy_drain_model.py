@@ -87,8 +87,15 @@ def test_asking_in_the_copying_role_is_not_enough():
 def test_the_kernels_ask_after_their_roles_have_met(source, kernel):
     with open(os.path.join(CSRC, source)) as f:
         body = f.read().split(kernel, 1)[1].split("\n}\n", 1)[0]
-    asked = max(body.rfind("*fail)"), body.rfind("*fail &&"), body.rfind("*abort_flag)"))
-    met = max(body.rfind("c_cluster_wait();", 0, asked), body.rfind("cluster_sync_all();", 0, asked))
-    drained = body.rfind("mbar_wait_bounded(")
+    asked = max(body.rfind("(*fail"), body.rfind("&& *abort_flag)"))
+    met = max(body.rfind("c_done(S);", 0, asked), body.rfind("cluster_sync_relaxed();", 0, asked))
+    drained = body.find("full[", asked)
     assert 0 < met < asked < drained
     assert "full[" not in "".join(x.split(")")[0] for x in body[:met].split("mbar_wait_bounded(")[1:])
+
+
+def test_every_role_meets():
+    for source, kernel in (("arnoldi_cluster.cu", "arnoldi_step_kernel(const"), ("gs_cluster.cu", "gs_cluster_kernel(const")):
+        with open(os.path.join(CSRC, source)) as f:
+            copy, compute = f.read().split(kernel, 1)[1].split("\n}\n", 1)[0].split("\n  } else {\n    const int wr", 1)
+        assert copy.count("c_done(S);") == 1 and compute.count("c_done(S);") == 1
