@@ -25,7 +25,7 @@
 // Two CTAs share an SM, so that one streams while the other is between passes.
 //
 // What bounds it: for few probes the chain of a step (about 8 us: loads, two
-// float64 meetings, the scalars), for many the reads (HBM for the first pass, L2
+// meetings, the scalars), for many the reads (HBM for the first pass, L2
 // for the second).  Against the separate launches (projection, update,
 // coefficients, finish) per solve: n = 512, k = 16, 32 probes 0.60 -> 0.22 ms;
 // n = 3001, k = 32, 64 probes 1.14 -> 0.55 ms; n = 8192, k = 64, 512 probes 16.5 ->
@@ -720,7 +720,10 @@ struct CPlan {
 // whose clusters leave a quarter of the SMs over).  Sizes between the powers of two where
 // those leave rows or SMs unused: n = 23170, 96 steps, 32 probes S = 12 5.8 ms (16: 6.7), n = 18000, 64,
 // 64 3.9 (16: 5.8), n = 10000, 32, 128 S = 6 1.34 (8: 1.64).  Of equal sizes the one whose launches
-// are chained: n = 3001, k = 16, 40 probes 464 us per solve with S = 4, 507 with 6.
+// are chained: n = 3001, k = 16, 40 probes 464 us per solve with S = 4, 507 with 6.  The separate
+// launches, which spread any p evenly, stay behind it also where the probes are one more than
+// the clusters: n = 29000, 15 probes on 14 clusters of 16 0.65, 0.65 and 0.70 of their time for
+// k = 8, 32 and 100 (14 probes: 0.55, 0.52, 0.52).
 static CPlan c_plan(const CSlots &slots, int64_t n, int64_t p, int j) {
   CPlan best{0, 0, 0, 0, 0};
   double best_us = 1e300;

@@ -89,9 +89,9 @@ static void prof_end(size_t e0, int cls, double bytes, double flops, cudaStream_
 
 struct WsLayout {
   size_t w, panel, norm, len0, h2, partials, counters, status, hi, lo, q, h, values, eig, fsq;
-  // two-sweep Arnoldi: qt (float panel), X2 (p (2k + 1)), dots (p 3), nu
-  // (p (k + 1)), finish coefficients (p 4), full coefficients Hh (p (k + 1) k),
-  // the steps' scalars (p k kTwoSweepRec)
+  // two-sweep Arnoldi: qt (float panel), X2 (p (2k + 1)), dots (p 3), nu (p),
+  // finish coefficients (p 4), full coefficients Hh (p (k + 1) k), the steps'
+  // scalars (p k kTwoSweepRec)
   size_t vt, x2, dots, nu, cf, hh, rec;
   size_t total;
 };
@@ -145,7 +145,7 @@ static WsLayout layout(const mfg_operator *op, int64_t k, int64_t p, int64_t ld,
     L.vt = take((size_t)p * ld * es);
     L.x2 = take((size_t)p * (2 * kk + 1) * 8);
     L.dots = take((size_t)p * 3 * 8);
-    L.nu = take((size_t)p * (kk + 1) * 8);
+    L.nu = take((size_t)p * 8);
     L.cf = take((size_t)p * 4 * 8);
     L.hh = take((size_t)p * (kk + 1) * kk * 8);
     L.rec = take((size_t)p * kk * kTwoSweepRec * 8);

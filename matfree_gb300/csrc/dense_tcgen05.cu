@@ -406,9 +406,8 @@ dense_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_ahi,
 // chains of n / S terms (the tensor pipe's fp32 accumulation truncates, so
 // shorter chains are also closer to the exact product).
 //
-// What bounds it: the operator stream (4 n^2 bytes in split mode).  The ring
-// takes under half of an SM's shared memory, so two CTAs share an SM and one
-// streams while the other fills its pipeline or reduces.
+// What bounds it: the operator stream (4 n^2 bytes in split mode).  Kernels with
+// TMEM run one CTA per SM, so the ring takes most of the SM's shared memory.
 // ---------------------------------------------------------------------------
 
 __device__ __forceinline__ float4 ld_dsmem_f4(uint32_t addr) {
