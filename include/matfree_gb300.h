@@ -265,6 +265,10 @@ MFG_API int mfg_slq_ex(const mfg_operator *op, int64_t k, int64_t p, const void 
  * code of the call reports launch-time errors only). */
 MFG_API int mfg_workspace_status(const void *workspace, void *stream);
 
+/* Enqueues the copy of that status word to *status, pinned host memory, on `stream` without
+ * waiting: it is there once an event recorded behind the call has completed. */
+MFG_API int mfg_workspace_status_async(const void *workspace, int32_t *status, void *stream);
+
 /* Dense RBF kernel matrix K_ij = s2 exp(-|x_i - x_j|^2 / (2 ell^2)) from
  * points x (n x dim float32, row-major), WITHOUT the nugget (pass tau as the
  * operator shift).  precision selects the storage: FP32 -> a (float),

@@ -1442,6 +1442,13 @@ int mfg_workspace_status(const void *workspace, void *stream) {
   return st;
 }
 
+int mfg_workspace_status_async(const void *workspace, int32_t *status, void *stream) {
+  if (!workspace || !status) return MFG_ERR_BAD_ARG;
+  MFG_CUDA_TRY(cudaMemcpyAsync(status, ws_base(const_cast<void *>(workspace)), sizeof(int), cudaMemcpyDeviceToHost,
+                               as_stream(stream)));
+  return MFG_OK;
+}
+
 static int check_bidiag_ops(const mfg_operator *A, const mfg_operator *At, int64_t p, int64_t ld) {
   MFG_TRY(check_op(A));
   MFG_TRY(check_op(At));

@@ -128,6 +128,17 @@ def _operator_views(slot: _Slot, members_n: int, n: int, ld: int, precision: str
     return out
 
 
+def _status_word(ws, stream) -> torch.Tensor:
+    """The solve's device status in pinned memory, copied behind it on its stream: the loop
+    reads it once the solve's event has completed and never waits for the device itself
+    (a wait there would also keep ``stall_s`` from being looked at)."""
+    word = torch.zeros((1,), dtype=torch.int32, pin_memory=True)
+    st = _lib.lib().mfg_workspace_status_async(ws, ctypes.c_void_p(word.data_ptr()),
+                                               ctypes.c_void_p(stream.cuda_stream))
+    _lib.check(st, "mfg_workspace_status_async")
+    return word
+
+
 class _GroupOperator:
     """Block-diagonal operator over a packed probe panel: rows [start_r,
     start_r + p_r) are multiplied by member r's operator (every member n x n,
@@ -252,11 +263,12 @@ class SLQServer:
             _lib.check(st, "mfg_slq_ex")
             out = torch.empty((2,), dtype=torch.float64, pin_memory=True)
             out.copy_(ms, non_blocking=True)
+            word = _status_word(ws, slot.stream)
             done = torch.cuda.Event()
             done.record(slot.stream)
         # keep every buffer of the solve alive until its completion event fires
         return {"done": done, "out": out, "keep": (xh, xd, op, probes, values, ms), "flags": flags,
-                "ws": ws}
+                "word": word}
 
     def _launch_group(self, slot: _Slot, members, flags=None):
         """One packed solve of several small requests on the slot's stream."""
@@ -312,10 +324,11 @@ class SLQServer:
                               for b0, c in zip(starts.tolist(), counts)])
             out = torch.empty(ms.shape, dtype=torch.float64, pin_memory=True)
             out.copy_(ms, non_blocking=True)
+            word = _status_word(ws, slot.stream)
             done = torch.cuda.Event()
             done.record(slot.stream)
         return {"done": done, "out": out, "keep": (keep, ops, gop, panel, values, ms), "flags": flags,
-                "ws": ws, "group": members}
+                "word": word, "group": members}
 
     def _take_group(self, pending, head, now, realtime):
         """The head request and the waiting requests packed with it."""
@@ -365,14 +378,14 @@ class SLQServer:
                 raise RuntimeError(f"no solve completed for {stall_s} s; in flight: {desc}; "
                                    f"{len(results)} done, {len(pending)} pending")
             for idx, (slot, req, st, fp, t_start) in list(inflight.items()):
-                if st["done"].query() and st["flags"] and _lib.lib().mfg_workspace_status(
-                        st["ws"], ctypes.c_void_p(slot.stream.cuda_stream)) == _lib.MFG_ERR_RETRY:
+                done = st["done"].query()
+                if done and st["flags"] and int(st["word"][0]) == _lib.MFG_ERR_RETRY:
                     # the two-sweep step asked for the three-read form: run it again
                     again = (self._launch_group(slot, st["group"], flags=0) if "group" in st
                              else self._launch(slot, req, flags=0))
                     inflight[idx] = (slot, req, again, fp, t_start)
                     continue
-                if st["done"].query():
+                if done:
                     t_end = time.perf_counter() - t0
                     members = st.get("group", [req])
                     out = st["out"].reshape(len(members), 2)
