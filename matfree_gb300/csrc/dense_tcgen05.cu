@@ -46,6 +46,7 @@ constexpr int kGemmThreads = 192;
 constexpr int64_t kPairMinRows = 1024;  // CTA pairs from this operator size on
 
 constexpr int kGemmMaxStages = 12;
+constexpr uint32_t kPairAlone = 114 * 1024;  // a ring from here on leaves no room for another pair on the SM
 
 struct GemmShared {
   uint64_t full[kGemmMaxStages];
@@ -186,6 +187,51 @@ __device__ __forceinline__ void cluster_sync_relaxed() {
   asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
 }
 
+__device__ __forceinline__ void pair_give_up_right() {
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+
+// TMEM of a CTA pair (cta_group::2).  Allocation, giving up the right to allocate, and release
+// are each the two CTAs' together, and each CTA's part reaches into the other's SM.  So both
+// CTAs run before either allocates, both hold their columns before either gives up the right,
+// and both have released before either leaves (its SM may go to another kernel, which
+// allocates there).  Allocating at once and giving up the right directly behind it left, about
+// once in 30,000 solves on eight streams, one CTA waiting in its allocation for ever while its
+// peer was past it, with no other kernel on the device.  That is so where the pair has its
+// SMs to itself (ring_bytes).  Smaller rings (plain operators, up to 192 probes a tile) let two
+// pairs share them (n = 24576, 160 probes: 1.06 ms for three steps against 1.74 with one), and
+// two that each hold the right on one SM could wait for the other's: there it is given up
+// at once.  All threads of both CTAs call these.
+__device__ __forceinline__ void pair_alloc(uint32_t *base, uint32_t cols, uint32_t ring_bytes, int warp) {
+  const bool alone = ring_bytes >= kPairAlone;
+  __syncwarp();
+  cluster_sync_relaxed();
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(base)), "r"(cols)
+                 : "memory");
+    if (!alone) pair_give_up_right();
+  }
+  tc_fence_before();
+  // the barriers of both CTAs are initialised, too, before any copy or commit reaches them
+  cluster_sync_all();
+  tc_fence_after();
+  if (warp == 1 && alone) pair_give_up_right();
+}
+
+__device__ __forceinline__ void pair_release(uint32_t tmem, uint32_t cols, int warp) {
+  __syncwarp();
+  tc_fence_before();
+  // neither CTA releases its TMEM or shared memory while the pair's MMAs,
+  // copies or commits may still reach it
+  cluster_sync_all();
+  if (warp == 1) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols) : "memory");
+  }
+  __syncwarp();
+  cluster_sync_relaxed();
+}
+
 // 2-D tile copy into this CTA's shared memory completing on a barrier that
 // may live in the peer CTA (shared::cluster address).
 __device__ __forceinline__ void tma_load_2d_pair(void *dst, const CUtensorMap *map, uint32_t bar_cluster,
@@ -264,18 +310,7 @@ dense_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_ahi,
     sh->abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 1) {
-    // one warp of each CTA of the pair allocates, collectively
-    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                     smem_u32(&sh->tmem_base)),
-                 "r"(tmem_cols)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-  }
-  tc_fence_before();
-  // barriers of both CTAs are initialised before any copy or commit reaches them
-  cluster_sync_all();
-  tc_fence_after();
+  pair_alloc(&sh->tmem_base, tmem_cols, (uint32_t)stages * stage_bytes, warp);
   chain_wait();
   chain_next();
   const uint32_t tmem = sh->tmem_base;
@@ -383,16 +418,7 @@ dense_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_ahi,
       }
     }
   }
-  __syncwarp();
-  tc_fence_before();
-  // neither CTA releases its TMEM or shared memory while the pair's MMAs,
-  // copies or commits may still reach it
-  cluster_sync_all();
-  if (warp == 1) {
-    tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tmem_cols)
-                 : "memory");
-  }
+  pair_release(tmem, tmem_cols, warp);
 }
 
 // ---------------------------------------------------------------------------
@@ -797,16 +823,7 @@ dense_tcgen05_pair_persistent_kernel(const __grid_constant__ CUtensorMap map_ahi
     sh->abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                     smem_u32(&sh->tmem_base)),
-                 "r"(2u * acc_cols)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-  }
-  tc_fence_before();
-  cluster_sync_all();
-  tc_fence_after();
+  pair_alloc(&sh->tmem_base, 2u * acc_cols, (uint32_t)stages * stage_bytes, warp);
   chain_wait();
   chain_next();
   const uint32_t tmem = sh->tmem_base;
@@ -951,16 +968,7 @@ dense_tcgen05_pair_persistent_kernel(const __grid_constant__ CUtensorMap map_ahi
                      : "memory");
     }
   }
-  __syncwarp();
-  tc_fence_before();
-  // neither CTA releases its TMEM or shared memory while the pair's MMAs,
-  // copies, commits or remote arrivals may still reach it
-  cluster_sync_all();
-  if (warp == 1) {
-    tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2u * acc_cols)
-                 : "memory");
-  }
+  pair_release(tmem, 2u * acc_cols, warp);
 }
 
 // ---------------------------------------------------------------------------
